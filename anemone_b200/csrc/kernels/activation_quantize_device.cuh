@@ -1,7 +1,8 @@
 /*
  * activation_quantize_device.cuh: one warp's task of the activation quantizer: a load of 64 bfloat16 values of one
  * vector to E4M3 codes, the two E8M0 exponents of its blocks of 32 and the operands (the arithmetic is stated at
- * kernel_activation_quantize.cu). All 32 lanes call.
+ * kernel_activation_quantize.cu), or, with STREAM, the codes once more in stream order (anemone_b200_mx.h) instead of the
+ * operands. All 32 lanes call.
  */
 #ifndef AB_ACTIVATION_QUANTIZE_DEVICE_CUH
 #define AB_ACTIVATION_QUANTIZE_DEVICE_CUH
@@ -11,9 +12,10 @@
 
 #include "anemone_b200_records.h"
 
+template <bool STREAM>
 __device__ __forceinline__ void activation_quantize_load(const struct activation_quantize_arguments &arguments,
 							  unsigned char *arena, uint32_t vector, uint32_t load,
-							  uint32_t lane)
+							  uint32_t lane, uint64_t stream_offset)
 {
 	const uint32_t width = arguments.width;
 	const uint32_t raw = reinterpret_cast<const uint32_t *>(arena + arguments.values_offset)[((uint64_t)vector * width +
@@ -36,6 +38,17 @@ __device__ __forceinline__ void activation_quantize_load(const struct activation
 	unsigned char *const codes = arena + arguments.codes_offset + (uint64_t)vector * width + 64u * load;
 	codes[(t * 4u + s) * 4u + r] = (unsigned char)code_low; /* j = 2 (k % 2) + k / 8: h = 0 */
 	codes[(t * 4u + s) * 4u + 2u + r] = (unsigned char)code_high; /* h = 1 */
+	if (STREAM) {
+		/* block q = s / 2, p = s % 2: byte 32 q + 8 t + 2 j + p, j = 2 h + r */
+		unsigned char *const stream = arena + stream_offset + (uint64_t)vector * width + 64u * load +
+					      (s / 2u) * 32u + t * 8u + s % 2u;
+		stream[2u * r] = (unsigned char)code_low;
+		stream[2u * (2u + r)] = (unsigned char)code_high;
+		if (lane % 16u == 0)
+			(arena + arguments.exponents_offset)[(uint64_t)vector * (width / 32u) + 2u * load + lane / 16u] =
+				(unsigned char)code;
+		return;
+	}
 	const uint32_t placed_low = ((code_low & 0x80u) << 8) | ((code_low & 0x7Fu) << 7);
 	const uint32_t placed_high = ((code_high & 0x80u) << 8) | ((code_high & 0x7Fu) << 7);
 	reinterpret_cast<uint32_t *>(arena + arguments.operands_offset)[((uint64_t)vector * width + 64u * load) / 2u +

@@ -14,5 +14,5 @@
 extern "C" __global__ void __launch_bounds__(32)
 	activation_quantize_entry(struct activation_quantize_arguments arguments, unsigned char *arena)
 {
-	activation_quantize_load(arguments, arena, blockIdx.y, blockIdx.x, threadIdx.x);
+	activation_quantize_load<false>(arguments, arena, blockIdx.y, blockIdx.x, threadIdx.x, 0);
 }

@@ -16,6 +16,8 @@
 #include "activation_quantize_device.cuh"
 #include "router_device.cuh"
 
+#include "anemone_b200_mx.h"
+
 /* router_select_b200's one block */
 __device__ __forceinline__ void router_select_block(const struct router_select_b200_arguments &arguments,
 						    unsigned char *arena)
@@ -76,7 +78,26 @@ extern "C" __global__ void __launch_bounds__(ROUTER_B200_THREADS)
 	const uint32_t warps = blockDim.x / WARP, loads = arguments.quantize.width / 64u;
 	const uint32_t tasks = arguments.vector_count * loads;
 	for (uint32_t task = (blockIdx.x - 1u) * warps + threadIdx.x / WARP; task < tasks; task += (gridDim.x - 1u) * warps)
-		activation_quantize_load(arguments.quantize, arena, task / loads, task % loads, threadIdx.x % WARP);
+		activation_quantize_load<false>(arguments.quantize, arena, task / loads, task % loads, threadIdx.x % WARP, 0);
+}
+
+/* the same with the live rows' codes in stream order, for the tensor-core products (anemone_b200_mx.h), which may take
+ * their places on the card meanwhile */
+extern "C" __global__ void __launch_bounds__(ROUTER_B200_THREADS)
+	mx_route_quantize(struct mx_route_quantize_arguments arguments, unsigned char *arena)
+{
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+	if (blockIdx.x == 0) {
+		router_select_block(arguments.router, arena);
+		return;
+	}
+	const struct mx_quantize_arguments &quantize = arguments.quantize;
+	const struct step_block step = *reinterpret_cast<const struct step_block *>(arena + quantize.step_offset);
+	const uint32_t warps = blockDim.x / WARP, loads = quantize.base.width / 64u;
+	const uint32_t tasks = min(step.row_count, quantize.row_capacity) * loads;
+	for (uint32_t task = (blockIdx.x - 1u) * warps + threadIdx.x / WARP; task < tasks; task += (gridDim.x - 1u) * warps)
+		activation_quantize_load<true>(quantize.base, arena, task / loads, task % loads, threadIdx.x % WARP,
+					       quantize.stream_offset);
 }
 
 /* One block: copy the pool entry the cursor names into the step input area, then advance the cursor. */

@@ -1,5 +1,11 @@
 """One rank's original-weights routed-expert layer (MXFP4 weights by E4M3 block-quantized activations), prepared once
-and run per step through the C-ABI library. Launches of one step, all from libanemone_b200.so:
+and run per step through the C-ABI library. Launches of one step, all from libanemone_b200.so, where the widths are
+multiples of 128 (tensor_products):
+    mx_route_quantize -> mx_gate_up_few -> mx_down_few -> ordered_publish_reduce_flags_bf16
+and for many rows
+    exl3_prefill_picks -> exl3_prefill_group -> exl3_prefill_tiles -> mx_quantize -> mx_gather -> mx_gate_up_many
+    -> mx_down_many -> expert_row_sum_entry -> trunk_rows_add_entry -> ordered_row_sum_publish -> ordered_reduce_bf16
+(the products of the routed and the always-on experts on the fifth-generation tensor cores); otherwise
     router_select_b200 -> activation_quantize_entry -> expert_gate_up_<S> -> activation_quantize_entry (hidden)
     -> expert_down_<S> -> expert_row_sum_entry
     [-> trunk_linear_quantized_<S> (gate, up) -> trunk_hidden_entry -> activation_quantize_entry
@@ -25,6 +31,18 @@ from .moe import LINE, SIGNAL_BYTES, rank_columns
 WEIGHT_FORMAT_E2M1_SCALED = 3
 WEIGHT_FORMAT_E4M3_SCALED = 5
 WEIGHT_FORMAT_E4M3_BLOCK128 = 6
+
+
+# Below this many weights a matrix a call of many rows keeps the mma.sync group products: a unit of the tensor-core
+# launches (128 rows of a matrix, all of its inputs) is then a handful of stages, and a tile of 128 batch rows hardly any.
+TENSOR_WIDE_WEIGHTS = 1 << 18
+
+
+def tensor_products(config, inner_local, wide, many):
+    """Whether the products run on the fifth-generation tensor cores: whole blocks of 128 inputs and units of 128
+    outputs, and for many rows matrices that are worth it."""
+    H = config.hidden
+    return H % 128 == 0 and inner_local % 128 == 0 and (not wide or (many and H * inner_local >= TENSOR_WIDE_WEIGHTS))
 
 
 def matrix_bytes(outputs, inputs):
@@ -82,6 +100,14 @@ class MxLayout:
         self.shared_sizes = {"gate_output": rows * I * 2, "up_output": rows * I * 2, "hidden": rows * I * 2,
                              "hidden_codes": rows * I, "hidden_exponents": rows * I // 32,
                              "hidden_operands": rows * I * 2, "output": rows * H * 2} if c.shared else {}
+        # the tensor-core products' vectors: codes in stream order; for many rows tiles of 128 vectors in operand order
+        self.stream_codes = layout.take(rows * H)
+        tiles = 0
+        if wide and tensor_products(config, I, True, True):
+            tiles = api.prefill_parts(rows, c.picks, 0, c.experts, H, I).tile_capacity + (rows + 31) // 32
+        self.tile_sizes = {"codes": tiles * 128 * H, "exponents": tiles * 4 * H, "hidden_codes": tiles * 128 * I,
+                           "hidden_exponents": tiles * 4 * I}
+        self.tile_at = {name: layout.take(size, 1024) for name, size in self.tile_sizes.items()}
         self.shared_at = {name: layout.take(size) for name, size in self.shared_sizes.items()}
         self.weights_begin = api.align(layout.cursor, 64)
         self.matrices = []
@@ -127,24 +153,153 @@ class MxLayer:
         for peer in range(rank_count):
             peers[peer].region_offset = L.region
         card.upload(L.peer_table, np.frombuffer(bytes(peers), dtype=np.uint8))
+        self.sequence = 0
+        self.step_graph = None  # step(): the copies and the launches as one graph, captured at its first call
+        if tensor_products(config, L.inner_local, wide, many):
+            self._prepare_tensor()
+        else:
+            self._prepare(slices, shared_slices, many, side_run)
+        self._capture()
+
+    def _shared_format(self):
+        if not self.config.shared:
+            return 0
+        return WEIGHT_FORMAT_E4M3_BLOCK128 if self.layout.block128 else WEIGHT_FORMAT_E4M3_SCALED
+
+    def _routing(self):
+        """The record of the prefill's routing launches: every routed expert local, no always-on expert."""
+        c, L = self.config, self.layout
+        routing = R.Exl3Prefill()
+        routing.scores_offset, routing.expert_table_offset = L.scores, L.expert_table
+        routing.picks_offset, routing.weights_offset, routing.workspace_offset = L.picks, L.weights, L.workspace
+        routing.step_offset, routing.input_size, routing.inner_size = L.step, c.hidden, L.inner_local
+        routing.expert_count, routing.local_count, routing.picks = c.experts, c.experts, c.picks
+        routing.row_capacity, routing.scoring, routing.route_scale = c.row_capacity, c.scoring, c.route_scale
+        return routing
+
+    def _router(self):
+        c, L = self.config, self.layout
+        return R.RouterSelectB200(L.scores, L.expert_table, L.picks, L.weights, L.jobs, L.step, c.experts, 0, c.picks,
+                                  c.row_capacity, L.job_capacity, c.scoring, c.route_scale, 0)
+
+    def _prepare_tensor(self):
+        c, L, card, lib = self.config, self.layout, self.card, api.library()
+        H, I, rows = c.hidden, L.inner_local, c.row_capacity
+
+        def prepare(name, record, count):
+            entry = getattr(lib, name)
+            entry.argtypes = [C.c_void_p, C.c_uint64, C.POINTER(api.BackendOperations), C.c_void_p,
+                              C.POINTER(R.KernelLaunch)]
+            launches = (R.KernelLaunch * count)()
+            api.check(entry(C.byref(record), card.arena_bytes, card.ops_pointer, card.handle, launches), name)
+            return list(launches)
+        quantize = R.MxQuantize(R.ActivationQuantize(L.tokens, L.at["codes"], L.at["exponents"], 0, H, 0),
+                                L.stream_codes, L.step, rows, 0)
+        description = R.MxLayerDescription()
+        description.workspace_offset, description.expert_table_offset = L.workspace, L.expert_table
+        description.step_offset = L.step
+        if L.wide:
+            head = prepare("router_tiles_prepare", self._routing(), 3) + prepare("mx_quantize_prepare", quantize, 1)
+            description.row_codes = R.LinearRange(L.stream_codes, rows * H)
+            description.row_exponents = R.LinearRange(L.at["exponents"], L.sizes["exponents"])
+            for name in L.tile_sizes:
+                setattr(description, name, R.LinearRange(L.tile_at[name], L.tile_sizes[name]))
+        else:
+            head = prepare("mx_route_quantize_prepare", R.MxRouteQuantize(self._router(), quantize), 1)
+            description.jobs = R.LinearRange(L.jobs, L.job_capacity * 96)
+            description.codes = R.LinearRange(L.stream_codes, rows * H)
+            for name in ("exponents", "hidden_codes", "hidden_exponents"):
+                setattr(description, name, R.LinearRange(L.at[name], L.sizes[name]))
+        description.pair_output = R.LinearRange(L.at["pair_output"], L.sizes["pair_output"])
+        if c.shared:
+            for name in ("hidden_codes", "hidden_exponents", "output"):
+                setattr(description, "shared_" + name, R.LinearRange(L.shared_at[name], L.shared_sizes[name]))
+            description.shared_weights_offset = (C.c_uint64 * 3)(*L.shared_matrices)
+        description.shared_format, description.hidden_size, description.inner_size = self._shared_format(), H, I
+        description.expert_count, description.picks, description.row_capacity = c.experts, c.picks, rows
+        description.activation_limit = c.activation_limit
+        lib.mx_products_prepare.argtypes = [C.POINTER(R.MxLayerDescription), C.c_uint64,
+                                            C.POINTER(api.BackendOperations), C.c_void_p, C.POINTER(R.KernelLaunch),
+                                            C.POINTER(C.c_uint32)]
+        launches, count = (R.KernelLaunch * 3)(), C.c_uint32()
+        api.check(lib.mx_products_prepare(C.byref(description), card.arena_bytes, card.ops_pointer, card.handle, launches,
+                                          C.byref(count)), "mx_products_prepare")
+        self.expert_launches = list(launches)[count.value - 2:count.value]  # gate/up, down
+        head += list(launches)[:count.value - 2]
+        behind = [] if L.flags else self._row_sums()
+        reduce_launches = self._reduce()
+        if L.flags:
+            reduce_launches[0].branch = R.LAUNCH_CHAIN | R.LAUNCH_OVERLAPS_PREVIOUS
+        self.launches = head + self.expert_launches + behind + reduce_launches
+
+    def _row_sums(self):
+        """FP32 sums of the routed pairs' bfloat16 outputs, and the always-on expert's rows added to them"""
+        c, L, card = self.config, self.layout, self.card
+        record = R.ExpertRowSum(L.at["pair_output"], L.at["row_output"], c.hidden, c.picks)
+        launch = R.KernelLaunch()
+        launch.kernel = card.kernel("kernel_expert_linear", "expert_row_sum_entry", C.sizeof(record))
+        launch.argument_byte_count = C.sizeof(record)
+        launch.grid[:] = ((c.hidden + 255) // 256, c.row_capacity, 1)
+        launch.block[:] = (256, 1, 1)
+        C.memmove(launch.argument, C.byref(record), C.sizeof(record))
+        return [launch] + ([self._rows_add()] if c.shared else [])
+
+    def _rows_add(self):
+        c, L, card, lib = self.config, self.layout, self.card, api.library()
+        lib.linear_rows_add_prepare.argtypes = [C.POINTER(R.LinearRange), C.POINTER(R.LinearRange), C.c_uint32,
+                                                C.c_uint32, C.c_uint64, C.POINTER(api.BackendOperations),
+                                                C.c_void_p, C.POINTER(R.KernelLaunch)]
+        add = R.KernelLaunch()
+        sums = R.LinearRange(L.at["row_output"], L.sizes["row_output"])
+        values = R.LinearRange(L.shared_at["output"], L.shared_sizes["output"])
+        api.check(lib.linear_rows_add_prepare(C.byref(sums), C.byref(values), c.hidden, c.row_capacity, card.arena_bytes,
+                                              card.ops_pointer, card.handle, C.byref(add)), "linear_rows_add_prepare")
+        return add
+
+    def _reduce(self):
+        """The reduction's launches: of the pair outputs and the always-on rows in one, or of the rows' sums in two"""
+        c, L, card, lib, H = self.config, self.layout, self.card, api.library(), self.config.hidden
+        reduce = R.OrderedReduceBf16Description()
+        reduce.reduce.collective = R.OrderedCollective(L.peer_table, L.region, L.slot_input, L.result, 0, L.step,
+                                                       L.parity_stride, c.deadline_cycles, c.row_capacity * H,
+                                                       self.rank_count, self.rank, 0)
+        reduce.reduce.status_offset, reduce.reduce.width = L.status, H
+        reduce.reduce.mode = R.ORDERED_REDUCE_OWNER_RUNS if L.wide else R.ORDERED_REDUCE_EVERY_RANK
+        reduce.pair_output_offset, reduce.arena_byte_count = L.at["row_output"], card.arena_bytes
+        reduce.pairs_per_row, reduce.row_capacity = 1, c.row_capacity
+        lib.ordered_reduce_bf16_prepare.argtypes = [C.POINTER(R.OrderedReduceBf16Description),
+                                                    C.POINTER(api.BackendOperations), C.c_void_p,
+                                                    C.POINTER(R.KernelLaunch)]
+        lib.ordered_publish_reduce_bf16_prepare.argtypes = [C.POINTER(R.OrderedReduceBf16Description), C.c_uint64,
+                                                            C.c_uint64, C.POINTER(api.BackendOperations), C.c_void_p,
+                                                            C.POINTER(R.KernelLaunch)]
+        if L.flags:
+            # row sums of the pair outputs, the always-on expert's rows, READY and the ranks' sum in one launch: it
+            # stands for expert_row_sum_entry, trunk_rows_add_entry and the reduction's two
+            reduce.pair_output_offset, reduce.pairs_per_row = L.at["pair_output"], c.picks
+            reduce_launches = (R.KernelLaunch * 1)()
+            api.check(lib.ordered_publish_reduce_bf16_prepare(
+                C.byref(reduce), L.shared_at["output"] if c.shared else 0, L.at["row_output"], card.ops_pointer,
+                card.handle, reduce_launches), "ordered_publish_reduce_bf16_prepare")
+        else:
+            reduce_launches = (R.KernelLaunch * 2)()
+            api.check(lib.ordered_reduce_bf16_prepare(C.byref(reduce), card.ops_pointer, card.handle, reduce_launches),
+                      "ordered_reduce_bf16_prepare")
+        return list(reduce_launches)
+
+    def _prepare(self, slices, shared_slices, many, side_run):
+        config, L, card, wide = self.config, self.layout, self.card, self.layout.wide
         c, lib, H, I = config, api.library(), config.hidden, L.inner_local
-        router = R.RouterSelectB200(L.scores, L.expert_table, L.picks, L.weights, L.jobs, L.step, c.experts, 0,
-                                    c.picks, c.row_capacity, L.job_capacity, c.scoring, c.route_scale, 0)
+        router = self._router()
         lib.router_select_b200_prepare.argtypes = [C.POINTER(R.RouterSelectB200), C.c_uint64,
                                                    C.POINTER(api.BackendOperations), C.c_void_p,
                                                    C.POINTER(R.KernelLaunch)]
         router_launch = R.KernelLaunch()
         if wide:
-            routing = R.Exl3Prefill()
-            routing.scores_offset, routing.expert_table_offset = L.scores, L.expert_table
-            routing.picks_offset, routing.weights_offset, routing.workspace_offset = L.picks, L.weights, L.workspace
-            routing.step_offset, routing.input_size, routing.inner_size = L.step, H, I
-            routing.expert_count, routing.local_count, routing.picks = c.experts, c.experts, c.picks
-            routing.row_capacity, routing.scoring, routing.route_scale = c.row_capacity, c.scoring, c.route_scale
             lib.router_wide_prepare.argtypes = [C.POINTER(R.RouterWide), C.c_uint64, C.POINTER(api.BackendOperations),
                                                 C.c_void_p, C.POINTER(R.KernelLaunch)]
             router_launches = (R.KernelLaunch * R.ROUTER_WIDE_LAUNCHES)()
-            api.check(lib.router_wide_prepare(C.byref(R.RouterWide(routing, L.jobs, L.job_capacity, 0)),
+            api.check(lib.router_wide_prepare(C.byref(R.RouterWide(self._routing(), L.jobs, L.job_capacity, 0)),
                                               card.arena_bytes, card.ops_pointer, card.handle, router_launches),
                       "router_wide_prepare")
             router_launches = list(router_launches)
@@ -236,43 +391,12 @@ class MxLayer:
             else:
                 api.check(lib.linear_shared_expert_prepare(C.byref(shared), card.arena_bytes, C.byref(kernels), four),
                           "linear_shared_expert_prepare")
-            lib.linear_rows_add_prepare.argtypes = [C.POINTER(R.LinearRange), C.POINTER(R.LinearRange), C.c_uint32,
-                                                    C.c_uint32, C.c_uint64, C.POINTER(api.BackendOperations),
-                                                    C.c_void_p, C.POINTER(R.KernelLaunch)]
-            add = R.KernelLaunch()
-            sums, values = span("row_output"), R.LinearRange(L.shared_at["output"], L.shared_sizes["output"])
-            api.check(lib.linear_rows_add_prepare(C.byref(sums), C.byref(values), H, c.row_capacity, card.arena_bytes,
-                                                  card.ops_pointer, card.handle, C.byref(add)), "linear_rows_add_prepare")
-            shared_launches = list(four) + [add]
-        reduce = R.OrderedReduceBf16Description()
-        reduce.reduce.collective = R.OrderedCollective(L.peer_table, L.region, L.slot_input, L.result, 0, L.step,
-                                                       L.parity_stride, c.deadline_cycles, c.row_capacity * H,
-                                                       rank_count, rank, 0)
-        reduce.reduce.status_offset, reduce.reduce.width = L.status, H
-        reduce.reduce.mode = R.ORDERED_REDUCE_OWNER_RUNS if wide else R.ORDERED_REDUCE_EVERY_RANK
-        reduce.pair_output_offset, reduce.arena_byte_count = L.at["row_output"], card.arena_bytes
-        reduce.pairs_per_row, reduce.row_capacity = 1, c.row_capacity
-        lib.ordered_reduce_bf16_prepare.argtypes = [C.POINTER(R.OrderedReduceBf16Description),
-                                                    C.POINTER(api.BackendOperations), C.c_void_p,
-                                                    C.POINTER(R.KernelLaunch)]
-        lib.ordered_publish_reduce_bf16_prepare.argtypes = [C.POINTER(R.OrderedReduceBf16Description), C.c_uint64,
-                                                            C.c_uint64, C.POINTER(api.BackendOperations), C.c_void_p,
-                                                            C.POINTER(R.KernelLaunch)]
+            shared_launches = list(four) + [self._rows_add()]
+        reduce_launches = self._reduce()
+        self.step_launches = list(self.expert_launches)
         if L.flags:
-            # row sums of the pair outputs, the always-on expert's rows, READY and the ranks' sum in one launch: it
-            # stands for expert_row_sum_entry, trunk_rows_add_entry and the reduction's two
-            reduce.pair_output_offset, reduce.pairs_per_row = L.at["pair_output"], c.picks
-            reduce_launches = (R.KernelLaunch * 1)()
-            api.check(lib.ordered_publish_reduce_bf16_prepare(
-                C.byref(reduce), L.shared_at["output"] if c.shared else 0, L.at["row_output"], card.ops_pointer,
-                card.handle, reduce_launches), "ordered_publish_reduce_bf16_prepare")
-            self.step_launches = list(self.expert_launches)[:3]
+            self.step_launches = self.step_launches[:3]
             shared_launches = shared_launches[:4]
-        else:
-            reduce_launches = (R.KernelLaunch * 2)()
-            api.check(lib.ordered_reduce_bf16_prepare(C.byref(reduce), card.ops_pointer, card.handle, reduce_launches),
-                      "ordered_reduce_bf16_prepare")
-            self.step_launches = list(self.expert_launches)
         # the always-on expert reads the quantized rows alone: its four launches are a side run of the graph beside the
         # routed experts' launches (a decode step's trunk launches are too small to fill the card by themselves);
         # the join is the launch that adds its rows to the routed experts' sums
@@ -285,6 +409,9 @@ class MxLayer:
             self.launches = head + shared_launches[:4] + self.step_launches + behind
         else:
             self.launches = head + self.step_launches + shared_launches[:4] + behind
+
+    def _capture(self):
+        L, card, lib = self.layout, self.card, api.library()
         self.graph = card.graph(self.launches)
         self.resident_graph = None
         if L.pool_entries:
@@ -296,7 +423,6 @@ class MxLayer:
             api.check(lib.step_input_select_prepare(C.byref(select), card.arena_bytes, card.ops_pointer, card.handle,
                                                     C.byref(select_launch)), "step_input_select_prepare")
             self.resident_graph = card.graph([select_launch] + self.launches)
-        self.sequence = 0
 
     def load_pool(self, steps):
         """steps: pool_entries tuples (sequence, tokens, scores), sequences strictly increasing. Their input areas go
@@ -346,8 +472,17 @@ class MxLayer:
         result_at = api.align(L.step_input_bytes, 4096)
         self.stage_step(0, self.sequence, tokens, scores)
         nbytes = rows * self.config.hidden * 2
-        # one library call: inputs in, the graph, status block and result out, wait
-        card.step_run(self.graph, L.step, 0, L.step_input_bytes, L.status, result_at, 16 + nbytes)
+        # one library call: inputs in, the graph, status block and result out, wait. A decode step's copies are nodes of
+        # the step's own graph where its table is a plain chain
+        if self.step_graph is None:
+            captured = None if L.wide else card.step_capture(
+                self.launches, L.step, 0, L.step_input_bytes, L.status, result_at,
+                16 + self.config.row_capacity * self.config.hidden * 2)
+            self.step_graph = -1 if captured is None else captured
+        if self.step_graph >= 0:
+            card.graph_run_wait(self.step_graph)
+        else:
+            card.step_run(self.graph, L.step, 0, L.step_input_bytes, L.status, result_at, 16 + nbytes)
         status = card.staging_view[result_at:result_at + 16].view(np.uint32)
         if status[0] != 0:
             raise RuntimeError("ordered reduction failed: code %d (1 timed out, 2 bad sequence), phase %d, rank %d"

@@ -353,6 +353,27 @@ class LinearSharedExpertDescription(C.Structure):
                [("row_count", C.c_uint32), ("activation_limit", C.c_float)]
 
 
+class MxQuantize(C.Structure):
+    _fields_ = [("base", ActivationQuantize), ("stream_offset", C.c_uint64), ("step_offset", C.c_uint64),
+                ("row_capacity", C.c_uint32), ("reserved_zero", C.c_uint32)]
+
+
+class MxRouteQuantize(C.Structure):
+    _fields_ = [("router", RouterSelectB200), ("quantize", MxQuantize)]
+
+
+class MxLayerDescription(C.Structure):
+    _fields_ = [("jobs", LinearRange), ("workspace_offset", C.c_uint64), ("expert_table_offset", C.c_uint64),
+                ("step_offset", C.c_uint64)] + \
+               [(name, LinearRange) for name in ("row_codes", "row_exponents", "codes", "exponents", "hidden_codes",
+                                                 "hidden_exponents", "pair_output", "shared_hidden_codes",
+                                                 "shared_hidden_exponents", "shared_output")] + \
+               [("shared_weights_offset", C.c_uint64 * 3)] + \
+               [(name, C.c_uint32) for name in ("shared_format", "hidden_size", "inner_size", "expert_count", "picks",
+                                                "row_capacity")] + \
+               [("activation_limit", C.c_float), ("reserved_zero", C.c_uint32)]
+
+
 class KernelLaunch(C.Structure):
     _fields_ = [("kernel", C.c_uint32), ("grid", C.c_uint32 * 3), ("block", C.c_uint32 * 3),
                 ("dynamic_shared_byte_count", C.c_uint32), ("argument_byte_count", C.c_uint32),
@@ -360,6 +381,7 @@ class KernelLaunch(C.Structure):
 
 
 LAUNCH_CHAIN, LAUNCH_SIDE, LAUNCH_RESUME, LAUNCH_JOIN, LAUNCH_SIDE_MORE = range(5)
+LAUNCH_OVERLAPS_PREVIOUS = 0x100
 BACKEND_COPY, EXCHANGE_OWN_ARENA = 0xFFFFFFFE, 0xFFFFFFFFFFFFFFFF
 
 

@@ -24,7 +24,7 @@ Further objects of the same line, each with its own value, e2e and roofline wher
   prefill            cfg4: the same layer for M = 4096 rows, Zipf(1.1) routing, experts sharded over the ranks,
                      tensor-core (tcgen05) grouped products, ordered reduction with owner runs;
   original_weights   cfg5 decode: MXFP4 routed experts and the E4M3 always-on expert, E4M3 block-quantized activations;
-  original_weights_prefill  cfg5 prefill: the same layer for M = 2048 rows (group products: two jobs of eight rows a block);
+  original_weights_prefill  cfg5 prefill: the same layer for M = 2048 rows (tcgen05 block-scaled products);
   reduction          (N > 1) cfg2: the fixed-order reduction alone, FP32 [M][4096] a rank, M in {1, 8, 64}, in this
                      library's four forms, microseconds a call and NVLink bytes a second;
   reference_kernels  (N = 1) the reference's own EXL3 kernels, recompiled for sm_100a from its sources into oracle/_ref,
@@ -53,7 +53,7 @@ SEED = 20261125
 GATE_UP_TRAFFIC_RATIO = 1.03
 # the same for the prefill's gate/up products (one capture at 32 experts and 1024 rows: 401.3 MB read and 45.0 MB
 # written against 444 MB of codes, scales, operand blocks read and down operand blocks written) and for the
-# original-weights gate/up products (one capture at 64 experts: 360.1 MB against 356.8 MB)
+# original-weights gate/up products (one capture of the mma.sync launch at 64 experts: 360.1 MB against 356.8 MB)
 PREFILL_TRAFFIC_RATIO = 1.00
 MX_GATE_UP_TRAFFIC_RATIO = 1.01
 
@@ -556,7 +556,7 @@ def run_original_weights(args, api, base, rank, world, local_rank, dist, barrier
     from anemone_b200 import records as R
     from anemone_b200 import synthetic
     from anemone_b200.moe import MoeConfig
-    from anemone_b200.mx import MxLayer, MxLayout, matrix_bytes
+    from anemone_b200.mx import MxLayer, MxLayout, matrix_bytes, shared_matrix_bytes
     rows, steps, warmup = args.rows, args.steps, args.warmup
     config = MoeConfig(hidden=base.hidden, inner=base.inner, experts=base.experts, shared=1, picks=base.picks,
                        row_capacity=rows, activation_limit=7.0)
@@ -610,12 +610,12 @@ def run_original_weights(args, api, base, rank, world, local_rank, dist, barrier
         layer.step(tokens, scores)
     e2e_ms = maximum(1000.0 * (time.perf_counter() - wall_begin)) / steps
     barrier()
-    # ---- roofline: expert_gate_up alone ----
+    # ---- roofline: the gate/up products alone ----
     roofline = None
     if rank == 0:
         peak, source = measured_peaks()
         gate_up = (R.KernelLaunch * 1)(R.KernelLaunch.from_buffer_copy(bytes(layer.expert_launches[0])))
-        gate_up[0].branch = 0  # alone: in the step's graph it resumes the main run beside the always-on expert's
+        gate_up[0].branch = 0  # alone: in the step's graph it overlaps the launch before it
         card.run(gate_up)
         card.wait()
         card.measure_begin()
@@ -626,9 +626,11 @@ def run_original_weights(args, api, base, rank, world, local_rank, dist, barrier
         picks = card.download(layout.picks, rows * config.picks * 4, np.uint32)
         active = len(set(picks.tolist()))
         pairs = rows * config.picks
-        byte_total = active * 2 * matrix_bytes(I, H) + rows * H * 2 + rows * H // 32 + pairs * I * 2
+        # gate and up of the active experts and of the always-on one; the rows' codes in, the hidden vectors' codes out
+        byte_total = active * 2 * matrix_bytes(I, H) + 2 * shared_matrix_bytes(I, H, True) + \
+            rows * H + rows * H // 32 + (pairs + rows) * (I + I // 32)
         achieved = byte_total / us / 1000.0
-        roofline = {"kernel": "expert_gate_up_2", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+        roofline = {"kernel": "mx_gate_up_few", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                     "frac": achieved / peak, "peak_source": source, "traffic": MX_GATE_UP_TRAFFIC_RATIO * byte_total,
                     "algorithmic_bytes_per_launch": byte_total, "us_per_launch": us, "active_experts": active}
     card.wait()
@@ -650,8 +652,8 @@ def run_original_weights(args, api, base, rank, world, local_rank, dist, barrier
 
 def run_original_weights_prefill(args, api, base, rank, world, local_rank, dist, barrier, maximum):
     """cfg5 prefill: the same original-weights layer for M = 2048 rows, tensor parallel by intermediate columns. The
-    products are linear_routed_experts_wide_prepare's (a group of two jobs of eight rows and several tiles a block, the
-    thin instances' arithmetic bit for bit), not yet a tcgen05 grouped GEMM: the number says where that stands."""
+    products are mx_gate_up_many and mx_down_many (tcgen05 block-scaled products over tiles of up to 128 rows of one
+    expert)."""
     from anemone_b200 import synthetic
     from anemone_b200.moe import MoeConfig
     from anemone_b200.mx import MxLayer, MxLayout
@@ -715,7 +717,7 @@ def run_original_weights_prefill(args, api, base, rank, world, local_rank, dist,
             "dtype": "e2m1 x e4m3 -> f32", "jobs": layout.job_capacity,
             "config": {"workload": "cfg5 original-weights MoE layer prefill: M=%d, %d routed MXFP4 experts, top-%d, 1 "
                                    "always-on expert E4M3 with one FP32 scale per 128x128 weights, hidden %d, "
-                                   "intermediate %d; group products (two jobs of eight rows a block, mma.sync, the thin instances' bits)" %
+                                   "intermediate %d; tcgen05 block-scaled products, tiles of up to 128 rows of one expert" %
                                    (rows, config.experts, config.picks, H, config.inner),
                        "parallelism": "tp%d by intermediate columns, ordered FP32->bf16 reduce (owner runs)" % world}}
 

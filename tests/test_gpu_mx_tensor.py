@@ -1,0 +1,110 @@
+"""The original-weights layer's tensor-core products (mx_gate_up_*, mx_down_*) against the CPU oracle, on the card's own
+picks and quantized rows: tiles that are full, ragged and of one row, widths whose last stage of 256 inputs is half
+empty, both storage forms of the always-on expert and none."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from anemone_b200 import records as R
+from anemone_b200 import synthetic
+from oracle.binding import ptr, u8p
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,capacity,hidden,inner,experts,picks,shared", [
+    (8, 8, 640, 384, 12, 4, "block128"),  # the decode form, half stages
+    (1, 8, 512, 128, 9, 2, "e8m0"),
+    (33, 64, 256, 256, 6, 3, None),  # the decode form with several jobs an expert
+    (257, 512, 2048, 128, 3, 1, None),  # many rows, a single block of 128 inputs in down
+    (130, 160, 1152, 256, 5, 2, "e8m0"),  # 1152 = four stages and a half; an always-on tile of two rows
+    (203, 256, 1024, 384, 12, 3, "block128"),  # ragged tiles, one of two and more; 384 = a stage and a half
+    (9, 16, 1024, 512, 40, 8, "block128"),  # a row or two an expert
+])
+def test_layer_matches_oracle(oracle, rows, capacity, hidden, inner, experts, picks, shared):
+    from anemone_b200 import api
+    from anemone_b200.moe import MoeConfig
+    from anemone_b200.mx import MxLayer, MxLayout
+    from oracle import moe_reference
+    wide = capacity > 64 or (shared is not None and capacity > 8)
+    config = MoeConfig(hidden=hidden, inner=inner, experts=experts, shared=0 if shared is None else 1, picks=picks,
+                       row_capacity=capacity, activation_limit=7.0)
+    H, I, block128 = hidden, inner, shared == "block128"
+    rng = np.random.default_rng(rows)
+    matrices = [(synthetic.mx_matrix(rng, I, H), synthetic.mx_matrix(rng, I, H), synthetic.mx_matrix(rng, H, I))
+                for _ in range(experts)]
+    draw = synthetic.e4m3_block128_matrix if block128 else synthetic.e4m3_matrix
+    always = None if shared is None else (draw(rng, I, H), draw(rng, I, H), draw(rng, H, I))
+    tokens = synthetic.tokens(rng, rows, H)
+    scores = rng.normal(0, 1, size=(rows, experts)).astype(np.float32)
+    scores[:, 1] += 1.5  # one expert with many rows
+    L = MxLayout(config, 1, 0, block128=block128, wide=wide)
+    card = api.Card(0, L.arena_bytes)
+    try:
+        layer = MxLayer(card, config, matrices, slices=(1, 1), shared_matrices=always, block128=block128, wide=wide)
+        layer.connect_local([layer])
+        assert len(layer.expert_launches) == 2  # the tensor-core launches are the ones that run
+        for _ in range(2):  # both parity slots
+            result = layer.step(tokens, scores)
+            assert not card.waits_expired()
+        received = card.download(0, L.arena_bytes)
+    finally:
+        card.close()
+    chosen, weights = moe_reference.route(oracle, config, scores)
+    picked = received[L.picks:L.picks + rows * picks * 4].view(np.uint32).reshape(rows, picks)
+    assert np.array_equal(picked, chosen)
+    # the jobs of the oracle: expert ascending, rows ascending, eight to a job
+    table = received[L.expert_table:L.expert_table + experts * 24].view(np.uint64)
+    jobs = (R.ExpertJob * L.job_capacity)()
+    job = 0
+    for expert in range(experts):
+        held = [(row, slot) for row in range(rows) for slot in range(picks) if chosen[row, slot] == expert]
+        for first in range(0, len(held), 8):
+            record = jobs[job]
+            record.gate_offset, record.up_offset, record.down_offset = (int(x) for x in table[3 * expert:3 * expert + 3])
+            record.expert, record.row_count = expert, min(8, len(held) - first)
+            for column, (row, slot) in enumerate(held[first:first + 8]):
+                record.pair_index[column] = row * picks + slot
+                record.route_weight[column] = float(weights[row, slot])
+            job += 1
+    expected = received.copy()
+    expected[L.jobs:L.jobs + L.job_capacity * 96] = np.frombuffer(bytes(jobs), dtype=np.uint8)
+    at = L.at
+    oracle.orc_mx_experts(C.byref(R.ExpertGateUp(L.jobs, at["codes"], at["exponents"], at["operands"], at["hidden"], I, H,
+                                                 L.pairs, picks, 7.0, 0)),
+                          C.byref(R.ExpertDown(L.jobs, at["hidden_codes"], at["hidden_exponents"], at["hidden_operands"],
+                                               at["pair_output"], H, I, L.pairs, 0)),
+                          L.job_capacity, 1, 1, at["hidden_codes"], at["hidden_exponents"], at["hidden_operands"],
+                          ptr(expected, u8p))
+
+    def outputs(image, where, count):
+        return synthetic.from_bfloat16(image[where:where + count * H * 2].view(np.uint16)).reshape(count, H)
+
+    def close(got, want):
+        assert np.isfinite(got).all() and np.abs(want).max() > 0
+        assert np.abs(got - want).max() <= max(2e-2, 2.0 ** -6 * np.abs(want).max())
+        a, b = got.reshape(-1).astype(np.float64), want.reshape(-1).astype(np.float64)
+        assert a @ b / (np.linalg.norm(a) * np.linalg.norm(b)) >= 0.9999
+    got = outputs(received, at["pair_output"], rows * picks)
+    close(got, outputs(expected, at["pair_output"], rows * picks))
+    summed = np.zeros((rows, H), dtype=np.float32)
+    for slot in range(picks):
+        summed = (summed + got.reshape(rows, picks, H)[:, slot, :]).astype(np.float32)
+    if shared is not None:
+        S = L.shared_at
+        gate_up = R.TrunkLinearQuantized((C.c_uint64 * 2)(L.shared_matrices[0], L.shared_matrices[1]),
+                                         (C.c_uint64 * 2)(S["gate_output"], S["up_output"]), at["codes"], at["exponents"],
+                                         at["operands"], (C.c_uint32 * 2)(I, I), H, rows)
+        down = R.TrunkLinearQuantized((C.c_uint64 * 2)(L.shared_matrices[2], 0), (C.c_uint64 * 2)(S["output"], 0),
+                                      S["hidden_codes"], S["hidden_exponents"], S["hidden_operands"],
+                                      (C.c_uint32 * 2)(H, 0), I, rows)
+        (oracle.orc_shared_expert_block128 if block128 else oracle.orc_shared_expert)(
+            C.byref(gate_up), C.byref(R.TrunkHidden(S["gate_output"], S["up_output"], S["hidden"], I, 7.0)),
+            C.byref(R.ActivationQuantize(S["hidden"], S["hidden_codes"], S["hidden_exponents"], S["hidden_operands"], I, 0)),
+            C.byref(down), 1, 1, ptr(expected, u8p))
+        joined = outputs(received, S["output"], rows)
+        close(joined, outputs(expected, S["output"], rows))
+        summed = (summed + joined).astype(np.float32)
+    # row sums, the join and the reduction: bit for bit given what the card wrote
+    assert np.array_equal(result, synthetic.to_bfloat16(np.float32(0.0) + summed))
