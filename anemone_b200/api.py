@@ -94,6 +94,8 @@ def library():
                                                   C.c_uint64, C.c_uint64, C.c_void_p, C.c_uint64,
                                                   C.POINTER(C.c_uint32)]
         lib.backend_b200_graph_run_wait.argtypes = [_card, C.c_uint32]
+        lib.backend_b200_step_call.argtypes = [_card, C.c_uint32, C.POINTER(R.HostRange), C.c_uint32,
+                                               C.POINTER(R.HostRange), C.c_uint32, C.c_void_p, C.c_uint64]
         lib.backend_b200_ipc_export.argtypes = [_card, C.c_char_p]
         lib.backend_b200_ipc_connect.argtypes = [_card, C.c_char_p, C.c_uint64, C.c_uint64]
         lib.exl3_reconstruct_prepare.argtypes = [C.POINTER(R.Exl3Reconstruct), C.c_uint64, C.c_uint32,
@@ -178,6 +180,37 @@ class Layout:
         return offset
 
 
+class StepStaging:
+    """Views of the places in a card's staging block where a decode step's inputs are written and its outputs appear:
+    step block, tokens and scores as in the layer's step input area, then at result_at the status block and the
+    bfloat16 rows. The views of a row count are made once."""
+
+    def __init__(self, card, layout, config):
+        self.card, self.layout, self.config = card, layout, config
+        self.result_at = align(layout.step_input_bytes, 4096)
+        self.of_rows = {}
+
+    def views(self, rows):
+        held = self.of_rows.get(rows)
+        if held is None:
+            c, L, view = self.config, self.layout, self.card.staging_view
+            tokens, scores, result = L.tokens - L.step, L.scores - L.step, self.result_at + 16
+            held = self.of_rows[rows] = (
+                view[0:16].view(np.uint64), view[tokens:tokens + rows * c.hidden * 2].view(np.uint16).reshape(rows, -1),
+                view[scores:scores + rows * c.experts * 4].view(np.float32).reshape(rows, -1),
+                view[self.result_at:self.result_at + 16].view(np.uint32),
+                view[result:result + rows * c.hidden * 2].view(np.uint16).reshape(rows, -1))
+        return held
+
+    def write(self, sequence, tokens, scores):
+        """Writes a step's inputs; returns the views of its status block and result."""
+        block, tokens_at, scores_at, status, result = self.views(tokens.shape[0])
+        block[0], block[1] = sequence, tokens.shape[0]  # struct step_block: the sequence, then the row count
+        tokens_at[...] = tokens if tokens.dtype == np.uint16 else tokens.view(np.uint16)
+        scores_at[...] = scores
+        return status, result
+
+
 class Card:
     """One opened card: an arena, a staging block, and the table's calls with statuses turned into exceptions."""
 
@@ -199,25 +232,31 @@ class Card:
             self.handle = _card()
 
     # ---- transfers through the staging block ----
+    def call(self, graph, inputs, outputs, staging_offset=0):
+        """One library call on ordinary memory (backend_b200_step_call): inputs, outputs: (arena offset, contiguous
+        array); the graph between them, or None. Everything passes the staging block from staging_offset on."""
+        inputs, outputs = ([pair for pair in pairs if pair[1].nbytes] for pairs in (inputs, outputs))
+
+        def ranges(pairs):
+            return (R.HostRange * max(len(pairs), 1))(*[R.HostRange(offset, array.ctypes.data, array.nbytes)
+                                                        for offset, array in pairs])
+        check(library().backend_b200_step_call(self.handle, R.BACKEND_B200_NO_GRAPH if graph is None else graph,
+                                               ranges(inputs), len(inputs), ranges(outputs), len(outputs),
+                                               self.staging.value + staging_offset, self.staging_bytes - staging_offset),
+              "step_call")
+
+    def fits_staging(self, arrays):
+        return sum(align(array.nbytes, 256) for array in arrays) <= self.staging_bytes
+
     def upload(self, offset, array):
         data = np.ascontiguousarray(array).reshape(-1).view(np.uint8)
         for begin in range(0, data.size, self.staging_bytes):
-            chunk = data[begin:begin + self.staging_bytes]
-            self.staging_view[:chunk.size] = chunk
-            ticket = C.c_uint64()
-            check(self.ops.upload_begin(self.handle, offset + begin, self.staging, chunk.size, C.byref(ticket)),
-                  "upload_begin")
-            check(self.ops.upload_wait(self.handle, ticket.value, WAIT_NANOSECONDS), "upload_wait")
+            self.call(None, [(offset + begin, data[begin:begin + self.staging_bytes])], [])
 
     def download(self, offset, byte_count, dtype=np.uint8):
         out = np.empty(byte_count, dtype=np.uint8)
         for begin in range(0, byte_count, self.staging_bytes):
-            size = min(self.staging_bytes, byte_count - begin)
-            ticket = C.c_uint64()
-            check(self.ops.download_begin(self.handle, offset + begin, self.staging, size, C.byref(ticket)),
-                  "download_begin")
-            check(self.ops.upload_wait(self.handle, ticket.value, WAIT_NANOSECONDS), "download wait")
-            out[begin:begin + size] = self.staging_view[:size]
+            self.call(None, [], [(offset + begin, out[begin:begin + self.staging_bytes])])
         return out.view(dtype)
 
     def upload_async(self, offset, staging_offset, byte_count):

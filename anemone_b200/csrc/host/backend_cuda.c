@@ -15,13 +15,19 @@
 #include <string.h>
 #include <time.h>
 
+#include "copy_pool.h"
 #include "driver_api.h"
 #include "kernel_images.h"
 
-#define CARD_MODULES_MOST 24u
+#define CARD_MODULES_MOST 32u
 #define NANOSECONDS_PER_SECOND 1000000000ull
 #define POLL_NANOSECONDS 20000l
+#define POLL_SPIN_NANOSECONDS 200000ull
 #define SMALL_WRITE_SLOTS 64u
+#define STEP_WORDS 16u /* 64-bit words a graph: a line of 128 bytes of its own */
+#define STEP_COPY_BLOCKS 64u
+#define CALL_PIECE_BYTES (1u << 20) /* 20 us of PCIe, 60 of a core's copy */
+#define STEP_SPIN_NANOSECONDS 2000000ull /* a step's wait looks at its word alone for so long */
 
 struct prepared_kernel {
 	const struct ab_kernel_image *image;
@@ -60,10 +66,15 @@ struct device_card {
 	int shared_memory_most; /* opt-in bytes per block */
 	int threads_most;
 	CUmodule modules[CARD_MODULES_MOST]; /* by image index, loaded at first kernel_prepare of the file */
+	CUdeviceptr wait_words[CARD_MODULES_MOST]; /* the module's exl3_wait_expired; 0: it has none */
+	CUevent piece_events[AB_COPY_BATCH_MOST]; /* of a step call's pieces on their way out */
 	struct prepared_kernel kernels[BACKEND_MAXIMUM_KERNELS];
 	uint32_t kernel_count;
 	CUgraphExec graphs[BACKEND_MAXIMUM_GRAPHS];
 	uint32_t graph_kernel_nodes[BACKEND_MAXIMUM_GRAPHS];
+	bool graph_reports[BACKEND_MAXIMUM_GRAPHS]; /* its copy out stores the run's number in step_words */
+	volatile uint64_t *step_words; /* page-locked: [graph]: the run's number, the number its copy out stored */
+	uint64_t step_ticket;
 	uint32_t graph_count;
 	CUevent marks[BACKEND_MAXIMUM_MARKS];
 	bool mark_set[BACKEND_MAXIMUM_MARKS];
@@ -75,7 +86,7 @@ struct device_card {
 	uint32_t mapping_count;
 	struct peer_word peer_words[PEER_WORDS_MOST]; /* what peer_connect wrote where: a copy launch's places */
 	uint32_t peer_word_count;
-	uint64_t *small_words; /* page-locked: address words written at load */
+	uint64_t *small_words; /* page-locked: address words written at load, then the wait words as they were read */
 	uint32_t small_word_next;
 	uint64_t launches_queued;
 };
@@ -96,10 +107,13 @@ static uint64_t now_nanoseconds(void)
 	return (uint64_t)now.tv_sec * NANOSECONDS_PER_SECOND + (uint64_t)now.tv_nsec;
 }
 
-static void pause_briefly(void)
+/* Between two looks at work the card has queued: at once while the wait is young (a sleep takes 70 us and more, a small
+ * copy ten), asleep later. */
+static void pause_briefly(uint64_t begun)
 {
 	const struct timespec pause = { 0, POLL_NANOSECONDS };
-	(void)nanosleep(&pause, NULL);
+	if (now_nanoseconds() - begun > POLL_SPIN_NANOSECONDS)
+		(void)nanosleep(&pause, NULL);
 }
 
 /* One error line for a driver failure; the card, if any, becomes failed. */
@@ -219,6 +233,9 @@ static void card_release(const struct ab_driver *cu, struct device_card *card)
 		for (uint32_t slot = 0; slot < BACKEND_MAXIMUM_UPLOADS_IN_FLIGHT; slot++)
 			if (card->transfers[slot].done != NULL)
 				(void)cu->cuEventDestroy(card->transfers[slot].done);
+		for (uint32_t piece = 0; piece < AB_COPY_BATCH_MOST; piece++)
+			if (card->piece_events[piece] != NULL)
+				(void)cu->cuEventDestroy(card->piece_events[piece]);
 		if (card->measure_begin_event != NULL)
 			(void)cu->cuEventDestroy(card->measure_begin_event);
 		if (card->measure_end_event != NULL)
@@ -230,6 +247,8 @@ static void card_release(const struct ab_driver *cu, struct device_card *card)
 				(void)cu->cuModuleUnload(card->modules[module]);
 		if (card->small_words != NULL)
 			(void)cu->cuMemFreeHost(card->small_words);
+		if (card->step_words != NULL)
+			(void)cu->cuMemFreeHost((void *)(uintptr_t)card->step_words);
 		if (card->arena != 0)
 			(void)cu->cuMemFree(card->arena);
 		if (card->stream != NULL)
@@ -282,7 +301,8 @@ static result_status cuda_card_open(uint32_t card_index, uint64_t arena_byte_cou
 	if (result == CUDA_SUCCESS)
 		result = cu->cuMemAlloc(&card->arena, arena_byte_count);
 	if (result == CUDA_SUCCESS)
-		result = cu->cuMemHostAlloc((void **)&card->small_words, SMALL_WRITE_SLOTS * sizeof(uint64_t),
+		result = cu->cuMemHostAlloc((void **)&card->small_words,
+					    (SMALL_WRITE_SLOTS + CARD_MODULES_MOST) * sizeof(uint64_t),
 					    CU_MEMHOSTALLOC_PORTABLE);
 	if (result != CUDA_SUCCESS) {
 		status = driver_failure(card, "opening the card", result);
@@ -296,6 +316,7 @@ static result_status cuda_card_open(uint32_t card_index, uint64_t arena_byte_cou
 	}
 	open_cards[card_index] = card;
 	*card_out = card;
+	ab_copy_pool_enter();
 	goto unlock;
 fail:
 	if (pushed) {
@@ -315,10 +336,10 @@ static void cuda_card_close(struct device_card *card, uint64_t wait_limit_nanose
 		return;
 	(void)pthread_mutex_lock(&card->mutex);
 	if (cu->cuCtxPushCurrent(card->context) == CUDA_SUCCESS) {
-		const uint64_t deadline = now_nanoseconds() + wait_limit_nanoseconds;
+		const uint64_t begun = now_nanoseconds(), deadline = begun + wait_limit_nanoseconds;
 		CUresult state;
 		while ((state = cu->cuStreamQuery(card->stream)) == CUDA_ERROR_NOT_READY && now_nanoseconds() < deadline)
-			pause_briefly();
+			pause_briefly(begun);
 		if (state == CUDA_ERROR_NOT_READY) {
 			(void)fprintf(stderr, "anemone_b200: card %u: work still queued at close; draining\n", card->index);
 			state = cu->cuStreamSynchronize(card->stream);
@@ -336,6 +357,7 @@ static void cuda_card_close(struct device_card *card, uint64_t wait_limit_nanose
 	(void)pthread_mutex_lock(&global_mutex);
 	open_cards[card->index] = NULL;
 	(void)pthread_mutex_unlock(&global_mutex);
+	ab_copy_pool_leave();
 	card_release(cu, card);
 }
 
@@ -507,7 +529,7 @@ static result_status cuda_upload_wait(struct device_card *card, uint64_t upload_
 {
 	if (card == NULL || upload_ticket == 0)
 		return STATUS_INVALID_ARGUMENT;
-	const uint64_t deadline = now_nanoseconds() + wait_limit_nanoseconds;
+	const uint64_t begun = now_nanoseconds(), deadline = begun + wait_limit_nanoseconds;
 	for (;;) {
 		CARD_ENTER(card);
 		if (upload_ticket >= card->next_ticket) {
@@ -528,7 +550,7 @@ static result_status cuda_upload_wait(struct device_card *card, uint64_t upload_
 			(void)cu->cuCtxPopCurrent(&popped);
 			(void)pthread_mutex_unlock(&card->mutex);
 		}
-		pause_briefly();
+		pause_briefly(begun);
 	}
 }
 
@@ -629,8 +651,14 @@ static result_status cuda_kernel_prepare(struct device_card *card, const char *k
 		status = STATUS_BUSY_VALUE;
 		goto done;
 	}
-	if (card->modules[image_index] == NULL)
+	if (card->modules[image_index] == NULL) {
 		DRIVER(card, cuModuleLoadData(&card->modules[image_index], image->begin));
+		size_t bytes = 0;
+		CUdeviceptr address = 0;
+		if (cu->cuModuleGetGlobal(&address, &bytes, card->modules[image_index], "exl3_wait_expired") == CUDA_SUCCESS &&
+		    bytes == sizeof(uint32_t))
+			card->wait_words[image_index] = address; /* a kernel file with bounded waits */
+	}
 	CUfunction function;
 	if (cu->cuModuleGetFunction(&function, card->modules[image_index], function_name) != CUDA_SUCCESS) {
 		(void)fprintf(stderr, "anemone_b200: kernel file %s has no function %s\n", kernel_file_name, function_name);
@@ -947,7 +975,7 @@ static result_status cuda_launch_wait(struct device_card *card, uint64_t wait_li
 {
 	if (card == NULL)
 		return STATUS_INVALID_ARGUMENT;
-	const uint64_t deadline = now_nanoseconds() + wait_limit_nanoseconds;
+	const uint64_t begun = now_nanoseconds(), deadline = begun + wait_limit_nanoseconds;
 	for (;;) {
 		CARD_ENTER(card);
 		if (card->failed) {
@@ -965,7 +993,7 @@ static result_status cuda_launch_wait(struct device_card *card, uint64_t wait_li
 			(void)cu->cuCtxPopCurrent(&popped);
 			(void)pthread_mutex_unlock(&card->mutex);
 		}
-		pause_briefly();
+		pause_briefly(begun);
 	}
 }
 
@@ -1176,7 +1204,7 @@ static result_status cuda_measure_elapsed_us(struct device_card *card, uint64_t 
 {
 	if (card == NULL || microseconds_out == NULL)
 		return STATUS_INVALID_ARGUMENT;
-	const uint64_t deadline = now_nanoseconds() + wait_limit_nanoseconds;
+	const uint64_t begun = now_nanoseconds(), deadline = begun + wait_limit_nanoseconds;
 	for (;;) {
 		CARD_ENTER(card);
 		if (card->failed) {
@@ -1208,7 +1236,7 @@ static result_status cuda_measure_elapsed_us(struct device_card *card, uint64_t 
 			(void)cu->cuCtxPopCurrent(&popped);
 			(void)pthread_mutex_unlock(&card->mutex);
 		}
-		pause_briefly();
+		pause_briefly(begun);
 	}
 }
 
@@ -1291,18 +1319,15 @@ result_status backend_b200_waits_expired(struct device_card *card, uint32_t *exp
 		status = STATUS_DEVICE_ERROR;
 		goto done;
 	}
+	/* every file's word behind the queued work, then one wait */
+	for (uint32_t module = 0; module < CARD_MODULES_MOST; module++)
+		if (card->wait_words[module] != 0)
+			DRIVER(card, cuMemcpyDtoHAsync(&card->small_words[SMALL_WRITE_SLOTS + module], card->wait_words[module],
+						       sizeof(uint32_t), card->stream));
 	DRIVER(card, cuStreamSynchronize(card->stream));
-	for (uint32_t module = 0; module < CARD_MODULES_MOST; module++) {
-		CUdeviceptr address = 0;
-		size_t bytes = 0;
-		uint32_t word = 0;
-		if (card->modules[module] == NULL ||
-		    cu->cuModuleGetGlobal(&address, &bytes, card->modules[module], "exl3_wait_expired") != CUDA_SUCCESS ||
-		    bytes != sizeof(word))
-			continue; /* a kernel file without bounded barrier waits */
-		DRIVER(card, cuMemcpyDtoH(&word, address, sizeof(word)));
-		expired |= word;
-	}
+	for (uint32_t module = 0; module < CARD_MODULES_MOST; module++)
+		if (card->wait_words[module] != 0)
+			expired |= *(const volatile uint32_t *)&card->small_words[SMALL_WRITE_SLOTS + module];
 	*expired_out = expired;
 done:
 	CARD_LEAVE(card);
@@ -1342,6 +1367,31 @@ done:
 	CARD_LEAVE(card);
 }
 
+/* whether a step's copy goes by a kernel */
+static bool copy_is_small(uint64_t arena_offset, const void *host, uint64_t byte_count)
+{
+	return byte_count != 0 && byte_count <= BACKEND_B200_STEP_COPY_MOST && arena_offset % 16u == 0 &&
+	       (uintptr_t)host % 16u == 0;
+}
+
+static void step_copy_fill(struct kernel_launch *launch, uint32_t kernel, const void *host, uint64_t arena_offset,
+			   uint64_t byte_count, const volatile uint64_t *words)
+{
+	const struct backend_b200_step_copy_record record = { (uint64_t)(uintptr_t)host, arena_offset, byte_count,
+							      (uint64_t)(uintptr_t)words,
+							      words != NULL ? (uint64_t)(uintptr_t)(words + 1) : 0u };
+	/* a piece of 16 bytes a thread: every load over PCIe is in flight at once */
+	const uint64_t blocks = (byte_count / 16u + BACKEND_B200_STEP_COPY_THREADS) / BACKEND_B200_STEP_COPY_THREADS;
+	memset(launch, 0, sizeof(*launch));
+	launch->kernel = kernel;
+	launch->grid[0] = (uint32_t)(blocks < STEP_COPY_BLOCKS ? blocks : STEP_COPY_BLOCKS);
+	launch->grid[1] = launch->grid[2] = launch->block[1] = launch->block[2] = 1;
+	launch->block[0] = BACKEND_B200_STEP_COPY_THREADS;
+	launch->argument_byte_count = sizeof(record);
+	launch->branch = LAUNCH_CHAIN | LAUNCH_OVERLAPS_PREVIOUS;
+	memcpy(launch->argument, &record, sizeof(record));
+}
+
 result_status backend_b200_step_capture(struct device_card *card, const struct kernel_launch *launches,
 					uint32_t launch_count, uint64_t input_arena_offset, const void *page_locked_input,
 					uint64_t input_byte_count, uint64_t output_arena_offset, void *page_locked_output,
@@ -1355,6 +1405,24 @@ result_status backend_b200_step_capture(struct device_card *card, const struct k
 	     (page_locked_output == NULL || !range_inside(output_arena_offset, output_byte_count, card->arena_byte_count) ||
 	      !inside_one_staging_block(page_locked_output, output_byte_count))))
 		return STATUS_INVALID_ARGUMENT;
+	if (launches == NULL || launch_count == 0 || launch_count > UINT32_MAX - 2u)
+		return STATUS_INVALID_ARGUMENT;
+	/* small copies as kernels of the chain: what they need is prepared before the card is entered */
+	const bool kernel_in = copy_is_small(input_arena_offset, page_locked_input, input_byte_count);
+	const bool kernel_out = copy_is_small(output_arena_offset, page_locked_output, output_byte_count);
+	uint32_t copy_in = BACKEND_NO_KERNEL, copy_out = BACKEND_NO_KERNEL;
+	result_status prepared = STATUS_OK;
+	if (kernel_in)
+		prepared = cuda_kernel_prepare(card, BACKEND_B200_STEP_COPY_KERNEL_FILE, "step_copy_in",
+					       sizeof(struct backend_b200_step_copy_record), &copy_in);
+	if (prepared == STATUS_OK && kernel_out)
+		prepared = cuda_kernel_prepare(card, BACKEND_B200_STEP_COPY_KERNEL_FILE, "step_copy_out",
+					       sizeof(struct backend_b200_step_copy_record), &copy_out);
+	if (prepared != STATUS_OK)
+		return prepared;
+	struct kernel_launch *const chain = calloc((size_t)launch_count + 2u, sizeof(*chain));
+	if (chain == NULL)
+		return STATUS_OUT_OF_MEMORY;
 	CARD_ENTER(card);
 	CUgraph graph = NULL;
 	status = card->failed ? STATUS_DEVICE_ERROR : table_check(card, launches, launch_count);
@@ -1368,15 +1436,30 @@ result_status backend_b200_step_capture(struct device_card *card, const struct k
 		status = STATUS_BUSY_VALUE;
 		goto done;
 	}
+	if (kernel_out && card->step_words == NULL) {
+		void *words = NULL;
+		const size_t bytes = BACKEND_MAXIMUM_GRAPHS * STEP_WORDS * sizeof(uint64_t);
+		DRIVER(card, cuMemHostAlloc(&words, bytes, CU_MEMHOSTALLOC_PORTABLE));
+		memset(words, 0, bytes);
+		card->step_words = words;
+	}
+	uint32_t count = 0;
+	if (kernel_in)
+		step_copy_fill(&chain[count++], copy_in, page_locked_input, input_arena_offset, input_byte_count, NULL);
+	memcpy(&chain[count], launches, launch_count * sizeof(*launches));
+	count += launch_count;
+	if (kernel_out)
+		step_copy_fill(&chain[count++], copy_out, page_locked_output, output_arena_offset, output_byte_count,
+			       card->step_words + (uint64_t)card->graph_count * STEP_WORDS);
 	DRIVER(card, cuStreamBeginCapture(card->stream, CU_STREAM_CAPTURE_MODE_THREAD_LOCAL));
 	{
 		CUresult copied = CUDA_SUCCESS;
-		if (input_byte_count != 0)
+		if (input_byte_count != 0 && !kernel_in)
 			copied = cu->cuMemcpyHtoDAsync(card->arena + input_arena_offset, page_locked_input, input_byte_count,
 						       card->stream);
-		status = copied == CUDA_SUCCESS ? launches_queue(cu, card, launches, launch_count) :
+		status = copied == CUDA_SUCCESS ? launches_queue(cu, card, chain, count) :
 						  driver_failure(card, "capturing the copy in", copied);
-		if (status == STATUS_OK && output_byte_count != 0) {
+		if (status == STATUS_OK && output_byte_count != 0 && !kernel_out) {
 			copied = cu->cuMemcpyDtoHAsync(page_locked_output, card->arena + output_arena_offset, output_byte_count,
 						       card->stream);
 			if (copied != CUDA_SUCCESS)
@@ -1390,11 +1473,35 @@ result_status backend_b200_step_capture(struct device_card *card, const struct k
 		goto done;
 	DRIVER(card, cuGraphInstantiateWithFlags(&card->graphs[card->graph_count], graph, 0));
 	card->graph_kernel_nodes[card->graph_count] = kernel_launches_of(launches, launch_count);
+	card->graph_reports[card->graph_count] = kernel_out;
 	*graph_out = card->graph_count++;
 done:
 	if (graph != NULL)
 		(void)cu->cuGraphDestroy(graph);
+	free(chain);
 	CARD_LEAVE(card);
+}
+
+/* Until the graph's copy out has stored `ticket`: polls the word, and after a while the stream with it, which knows of
+ * a failure. Context current, mutex held. */
+static result_status step_wait(const struct ab_driver *cu, struct device_card *card, const volatile uint64_t *words,
+			       uint64_t ticket)
+{
+	const uint64_t begun = now_nanoseconds();
+	for (uint32_t poll = 1; words[1] != ticket; poll++) {
+		__builtin_ia32_pause();
+		if (poll % 4096u != 0 || now_nanoseconds() - begun < STEP_SPIN_NANOSECONDS)
+			continue;
+		const CUresult state = cu->cuStreamQuery(card->stream);
+		if (state == CUDA_ERROR_NOT_READY)
+			continue;
+		if (state != CUDA_SUCCESS)
+			return driver_failure(card, "a step's graph", state);
+		if (words[1] != ticket) /* everything has run, and the word was not stored */
+			return driver_failure(card, "a step's copy out", CUDA_ERROR_UNKNOWN);
+	}
+	__atomic_thread_fence(__ATOMIC_ACQUIRE);
+	return STATUS_OK;
 }
 
 result_status backend_b200_graph_run_wait(struct device_card *card, uint32_t graph)
@@ -1410,10 +1517,136 @@ result_status backend_b200_graph_run_wait(struct device_card *card, uint32_t gra
 		status = STATUS_INVALID_ARGUMENT;
 		goto done;
 	}
+	const bool reports = card->graph_reports[graph];
+	volatile uint64_t *const words = reports ? card->step_words + (uint64_t)graph * STEP_WORDS : NULL;
+	const uint64_t ticket = ++card->step_ticket;
+	if (reports) {
+		words[0] = ticket;
+		__atomic_thread_fence(__ATOMIC_SEQ_CST);
+	}
 	DRIVER(card, cuGraphLaunch(card->graphs[graph], card->stream));
 	card->launches_queued += card->graph_kernel_nodes[graph];
-	DRIVER(card, cuStreamSynchronize(card->stream));
+	if (reports)
+		status = step_wait(cu, card, words, ticket);
+	else
+		DRIVER(card, cuStreamSynchronize(card->stream));
 done:
+	CARD_LEAVE(card);
+}
+
+/* The ranges as pieces for the copy pool, at most AB_COPY_BATCH_MOST together: of CALL_PIECE_BYTES, or longer where that
+ * would be more. staged[i]: where range i lies in the page-locked block. */
+static uint32_t call_pieces(struct ab_copy_batch *batch, const struct backend_b200_host_range *ranges, uint32_t count,
+			    unsigned char *const *staged, bool out, uint32_t *range_of, uint64_t *within)
+{
+	uint64_t total = 0;
+	for (uint32_t range = 0; range < count; range++)
+		total += ranges[range].byte_count;
+	uint64_t piece = CALL_PIECE_BYTES;
+	while (total / piece + count > AB_COPY_BATCH_MOST)
+		piece *= 2u;
+	uint32_t pieces = 0;
+	for (uint32_t range = 0; range < count; range++)
+		for (uint64_t begin = 0; begin < ranges[range].byte_count; begin += piece, pieces++) {
+			const uint64_t bytes = ranges[range].byte_count - begin < piece ? ranges[range].byte_count - begin : piece;
+			unsigned char *const ordinary = (unsigned char *)ranges[range].memory + begin;
+			unsigned char *const locked = staged[range] + begin;
+			batch->copies[pieces] = (struct ab_copy){ out ? ordinary : locked, out ? locked : ordinary, bytes };
+			range_of[pieces] = range;
+			within[pieces] = begin;
+		}
+	batch->count = pieces;
+	return pieces;
+}
+
+result_status backend_b200_step_call(struct device_card *card, uint32_t graph,
+				     const struct backend_b200_host_range *inputs, uint32_t input_count,
+				     const struct backend_b200_host_range *outputs, uint32_t output_count,
+				     void *page_locked, uint64_t page_locked_byte_count)
+{
+	if (card == NULL || page_locked == NULL || input_count > BACKEND_B200_HOST_RANGES_MOST ||
+	    output_count > BACKEND_B200_HOST_RANGES_MOST || (input_count != 0 && inputs == NULL) ||
+	    (output_count != 0 && outputs == NULL) || !inside_one_staging_block(page_locked, page_locked_byte_count))
+		return STATUS_INVALID_ARGUMENT;
+	unsigned char *staged[2u * BACKEND_B200_HOST_RANGES_MOST];
+	uint64_t used = 0;
+	for (uint32_t index = 0; index < input_count + output_count; index++) {
+		const struct backend_b200_host_range *const range = index < input_count ? &inputs[index] :
+											  &outputs[index - input_count];
+		if (range->memory == NULL || range->byte_count == 0 ||
+		    !range_inside(range->arena_offset, range->byte_count, card->arena_byte_count) ||
+		    !range_inside(used, range->byte_count, page_locked_byte_count))
+			return STATUS_INVALID_ARGUMENT;
+		staged[index] = (unsigned char *)page_locked + used;
+		used += (range->byte_count + 255u) / 256u * 256u;
+	}
+	struct ab_copy_batch batch;
+	uint32_t range_of[AB_COPY_BATCH_MOST];
+	uint64_t within[AB_COPY_BATCH_MOST];
+	CARD_ENTER(card);
+	bool begun = false;
+	if (card->failed) {
+		status = STATUS_DEVICE_ERROR;
+		goto done;
+	}
+	if (graph != BACKEND_B200_NO_GRAPH && graph >= card->graph_count) {
+		status = STATUS_INVALID_ARGUMENT;
+		goto done;
+	}
+	if (input_count != 0) {
+		const uint32_t pieces = call_pieces(&batch, inputs, input_count, staged, false, range_of, within);
+		batch.allowed = pieces;
+		ab_copy_batch_begin(&batch);
+		begun = true;
+		for (uint32_t sent = 0; sent < pieces;) {
+			if (!ab_copy_batch_is_done(&batch, sent)) { /* a piece more while the next to be sent is not there */
+				if (!ab_copy_batch_help(&batch))
+					__builtin_ia32_pause();
+				continue;
+			}
+			DRIVER(card, cuMemcpyHtoDAsync(card->arena + inputs[range_of[sent]].arena_offset + within[sent],
+						       batch.copies[sent].to, batch.copies[sent].byte_count, card->stream));
+			sent++;
+		}
+		ab_copy_batch_end(&batch);
+		begun = false;
+	}
+	if (graph != BACKEND_B200_NO_GRAPH) {
+		DRIVER(card, cuGraphLaunch(card->graphs[graph], card->stream));
+		card->launches_queued += card->graph_kernel_nodes[graph];
+	}
+	if (output_count != 0) {
+		const uint32_t pieces =
+			call_pieces(&batch, outputs, output_count, staged + input_count, true, range_of, within);
+		for (uint32_t piece = 0; piece < pieces; piece++) {
+			if (card->piece_events[piece] == NULL)
+				DRIVER(card, cuEventCreate(&card->piece_events[piece], CU_EVENT_DISABLE_TIMING));
+			DRIVER(card, cuMemcpyDtoHAsync((void *)(uintptr_t)batch.copies[piece].from,
+						       card->arena + outputs[range_of[piece]].arena_offset + within[piece],
+						       batch.copies[piece].byte_count, card->stream));
+			DRIVER(card, cuEventRecord(card->piece_events[piece], card->stream));
+		}
+		batch.allowed = 0;
+		ab_copy_batch_begin(&batch);
+		begun = true;
+		for (uint32_t piece = 0; piece < pieces; piece++) {
+			CUresult state;
+			while ((state = cu->cuEventQuery(card->piece_events[piece])) == CUDA_ERROR_NOT_READY)
+				if (!ab_copy_batch_help(&batch))
+					__builtin_ia32_pause();
+			if (state != CUDA_SUCCESS) {
+				status = driver_failure(card, "a step call", state);
+				batch.count = batch.allowed; /* what has not arrived is not copied on */
+				goto done;
+			}
+			ab_copy_batch_allow(&batch, piece + 1u);
+		}
+	} else {
+		DRIVER(card, cuStreamSynchronize(card->stream)); /* the block is the caller's again */
+	}
+done:
+	if (begun)
+		ab_copy_batch_end(&batch);
 	CARD_LEAVE(card);
 }
 

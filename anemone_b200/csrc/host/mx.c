@@ -82,6 +82,7 @@ result_status mx_route_quantize_prepare(const struct mx_route_quantize_arguments
 	const uint64_t blocks = (tasks + warps - 1u) / warps;
 	prepare_launch_fill(launch_out, kernel, 1u + (uint32_t)(blocks < MX_SMS ? blocks : MX_SMS), 1, 1,
 			    ROUTER_B200_THREADS, 0, arguments, sizeof(*arguments));
+	launch_out->branch = LAUNCH_CHAIN | LAUNCH_OVERLAPS_PREVIOUS; /* behind the copy of the step's inputs */
 	return STATUS_OK;
 }
 

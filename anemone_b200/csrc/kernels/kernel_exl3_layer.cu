@@ -33,6 +33,8 @@ extern "C" __global__ void __launch_bounds__(EXL3_LAYER_ROUTE_THREADS)
 	__shared__ uint64_t candidates[EXL3_LAYER_ROUTE_THREADS / WARP / ROUTER_TEAM_WARPS]
 				      [ROUTER_TEAM_WARPS * ROUTER_B200_MAXIMUM_PICKS];
 	const struct exl3_expert_record &base = record.moe.base;
+	/* the launch before this one may be the copy that brings the step's inputs */
+	asm volatile("griddepcontrol.wait;" ::: "memory");
 	/* the gate/up launch may take its place on the card now: it waits for the whole of this launch before it reads */
 	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 	const struct step_block step = *reinterpret_cast<const struct step_block *>(arena + record.step_offset);

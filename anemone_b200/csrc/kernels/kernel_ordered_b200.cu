@@ -210,6 +210,7 @@ __device__ __forceinline__ void publish_reduce_flags(const struct ordered_publis
 	const struct ordered_collective_arguments &collective = arguments.collective;
 	/* the launch may have been given its place on the card while the down products still run: all of them first */
 	asm volatile("griddepcontrol.wait;" ::: "memory");
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); /* the copy out takes its place; it waits for this launch */
 	const struct step_block step = *reinterpret_cast<const struct step_block *>(arena + collective.step_offset);
 	const uint64_t sequence = step.sequence;
 	if (sequence == 0 || collective.rank_count == 0 || collective.rank_count > ORDERED_COLLECTIVE_MAXIMUM_RANKS)

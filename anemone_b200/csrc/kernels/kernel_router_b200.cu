@@ -86,6 +86,7 @@ extern "C" __global__ void __launch_bounds__(ROUTER_B200_THREADS)
 extern "C" __global__ void __launch_bounds__(ROUTER_B200_THREADS)
 	mx_route_quantize(struct mx_route_quantize_arguments arguments, unsigned char *arena)
 {
+	asm volatile("griddepcontrol.wait;" ::: "memory"); /* for the copy that brings the step's inputs */
 	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 	if (blockIdx.x == 0) {
 		router_select_block(arguments.router, arena);

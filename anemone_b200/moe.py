@@ -211,6 +211,7 @@ class MoeLayer:
         c, L, card, lib = self.config, self.layout, self.card, api.library()
         # which launches stand before the gate/up products, and which launch they are (for callers that time them)
         self.step_graph = None  # step(): the copies and the launches as one graph, captured at its first call
+        self.staged = api.StepStaging(card, L, c)
         self.gate_up_index = 1 if L.reduce_form == "fused" else 2
         self.gate_up_kernel = "exl3_layer_products" if L.reduce_form == "fused" else "exl3_moe_gate_up"
         # the launch at gate_up_index holds the down products too (callers that count a launch's bytes ask)
@@ -319,28 +320,27 @@ class MoeLayer:
     def step(self, tokens, scores):
         """One layer call on host arrays: tokens bfloat16 bits [rows][hidden], scores FP32 [rows][experts].
         Returns bfloat16 bits [rows][hidden]. Raises if the reduction reported a failed wait."""
-        L, card = self.layout, self.card
-        rows = tokens.shape[0]
+        L, card, result_at = self.layout, self.card, self.staged.result_at
         self.sequence += 1
-        result_at = api.align(L.step_input_bytes, 4096)
-        nbytes = rows * self.config.hidden * 2
-        self.stage_step(0, self.sequence, tokens, scores)
+        status, result = self.staged.write(self.sequence, tokens, scores)
         # one library call: inputs in, the graph, status block and result out, wait. The copies are nodes of the
         # step's own graph where its table is a plain chain (one graph launch a step)
         if self.step_graph is None:
-            captured = card.step_capture(self.launches, L.step, 0, L.step_input_bytes, L.status, result_at,
+            launches = [R.KernelLaunch.from_buffer_copy(launch) for launch in self.launches]
+            if L.reduce_form == "fused":  # its first launch waits for the copy in: it may take its place beside it
+                launches[0].branch |= R.LAUNCH_OVERLAPS_PREVIOUS
+            captured = card.step_capture(launches, L.step, 0, L.step_input_bytes, L.status, result_at,
                                          16 + self.config.row_capacity * self.config.hidden * 2)
             self.step_graph = -1 if captured is None else captured
         if self.step_graph >= 0:
             card.graph_run_wait(self.step_graph)
         else:
-            card.step_run(self.graph, L.step, 0, L.step_input_bytes, L.status, result_at, 16 + nbytes)
+            card.step_run(self.graph, L.step, 0, L.step_input_bytes, L.status, result_at, 16 + result.nbytes)
         if L.reduce_form == "push":
             self.check_status()
-        else:
-            self._raise_on(card.staging_view[result_at:result_at + 16].view(np.uint32))
-        return card.staging_view[result_at + 16:result_at + 16 + nbytes].view(np.uint16).reshape(
-            rows, self.config.hidden).copy()
+        elif status[0] != 0:
+            self._raise_on(status)
+        return result.copy()
 
     def check_status(self):
         if self.layout.reduce_form == "push":

@@ -155,6 +155,7 @@ class MxLayer:
         card.upload(L.peer_table, np.frombuffer(bytes(peers), dtype=np.uint8))
         self.sequence = 0
         self.step_graph = None  # step(): the copies and the launches as one graph, captured at its first call
+        self.staged = api.StepStaging(card, L, config)
         if tensor_products(config, L.inner_local, wide, many):
             self._prepare_tensor()
         else:
@@ -467,31 +468,37 @@ class MxLayer:
     def step(self, tokens, scores):
         """One layer call on host arrays; returns bfloat16 bits [rows][hidden]."""
         L, card = self.layout, self.card
-        rows = tokens.shape[0]
         self.sequence += 1
-        result_at = api.align(L.step_input_bytes, 4096)
-        self.stage_step(0, self.sequence, tokens, scores)
-        nbytes = rows * self.config.hidden * 2
-        # one library call: inputs in, the graph, status block and result out, wait. A decode step's copies are nodes of
-        # the step's own graph where its table is a plain chain
+        if L.wide:
+            # one library call on ordinary memory: a prompt's rows in, the graph, status block and result out, wait
+            rows = tokens.shape[0]
+            status, result = np.empty(4, np.uint32), np.empty((rows, self.config.hidden), np.uint16)
+            block = np.array([self.sequence, rows], dtype=np.uint64)
+            card.call(self.graph, [(L.step, block), (L.tokens, np.ascontiguousarray(tokens)),
+                                   (L.scores, np.ascontiguousarray(scores, dtype=np.float32))],
+                      [(L.status, status), (L.result, result)])
+            self._raise_on(status)
+            return result
+        status, result = self.staged.write(self.sequence, tokens, scores)
+        result_at = self.staged.result_at
+        # one library call: inputs in, the graph, status block and result out, wait. The copies are nodes of the step's
+        # own graph where its table is a plain chain
         if self.step_graph is None:
-            captured = None if L.wide else card.step_capture(
-                self.launches, L.step, 0, L.step_input_bytes, L.status, result_at,
-                16 + self.config.row_capacity * self.config.hidden * 2)
+            captured = card.step_capture(self.launches, L.step, 0, L.step_input_bytes, L.status, result_at,
+                                         16 + self.config.row_capacity * self.config.hidden * 2)
             self.step_graph = -1 if captured is None else captured
         if self.step_graph >= 0:
             card.graph_run_wait(self.step_graph)
         else:
-            card.step_run(self.graph, L.step, 0, L.step_input_bytes, L.status, result_at, 16 + nbytes)
-        status = card.staging_view[result_at:result_at + 16].view(np.uint32)
-        if status[0] != 0:
-            raise RuntimeError("ordered reduction failed: code %d (1 timed out, 2 bad sequence), phase %d, rank %d"
-                               % (status[0], status[1], status[2]))
-        return card.staging_view[result_at + 16:result_at + 16 + nbytes].view(np.uint16).reshape(
-            rows, self.config.hidden).copy()
+            card.step_run(self.graph, L.step, 0, L.step_input_bytes, L.status, result_at, 16 + result.nbytes)
+        self._raise_on(status)
+        return result.copy()
 
     def check_status(self):
-        status = self.card.download(self.layout.status, 16, np.uint32)
+        self._raise_on(self.card.download(self.layout.status, 16, np.uint32))
+
+    @staticmethod
+    def _raise_on(status):
         if status[0] != 0:
             raise RuntimeError("ordered reduction failed: code %d (1 timed out, 2 bad sequence), phase %d, rank %d"
                                % (status[0], status[1], status[2]))

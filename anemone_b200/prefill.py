@@ -186,10 +186,13 @@ class PrefillLayer:
         """Place one call's inputs on the card: tokens bfloat16 bits [rows][hidden], scores FP32 [rows][experts]."""
         L, card = self.layout, self.card
         self.sequence += 1
-        block = R.StepBlock(self.sequence, tokens.shape[0], 0)
-        card.upload(L.step, np.frombuffer(bytes(block), dtype=np.uint8))
-        card.upload(L.tokens, tokens)
-        card.upload(L.scores, np.ascontiguousarray(scores, dtype=np.float32))
+        inputs = [(L.step, np.array([self.sequence, tokens.shape[0]], dtype=np.uint64)),
+                  (L.tokens, np.ascontiguousarray(tokens)), (L.scores, np.ascontiguousarray(scores, dtype=np.float32))]
+        if card.fits_staging(array for _, array in inputs):
+            card.call(None, inputs, [])
+        else:
+            for offset, array in inputs:
+                card.upload(offset, array)
 
     def run(self):
         self.card.graph_run(self.graph)
@@ -231,14 +234,19 @@ class PrefillLayer:
 
     def result(self, count):
         """bfloat16 bits [count][hidden]: the ranks' rows added in rank order, of the last run."""
+        L, card, H = self.layout, self.card, self.config.hidden
+        status, result = np.empty(4, np.uint32), np.empty((count, H), np.uint16)
+        if card.fits_staging((status, result)):
+            card.call(None, [], [(L.status, status), (L.result, result)])
+        else:
+            status = card.download(L.status, 16, np.uint32)
+            result = card.download(L.result, count * H * 2, np.uint16).reshape(count, H)
         if self.card.waits_expired():
             raise RuntimeError("a prefill CTA gave up a bounded wait: the result is incomplete")
-        status = self.card.download(self.layout.status, 16, np.uint32)
         if status[0] != 0:
             raise RuntimeError("ordered reduction failed: code %d (1 timed out, 2 bad sequence), phase %d, rank %d"
                                % (status[0], status[1], status[2]))
-        H = self.config.hidden
-        return self.card.download(self.layout.result, count * H * 2, np.uint16).reshape(count, H)
+        return result
 
     def step(self, tokens, scores):
         self.load(tokens, scores)

@@ -385,6 +385,13 @@ LAUNCH_OVERLAPS_PREVIOUS = 0x100
 BACKEND_COPY, EXCHANGE_OWN_ARENA = 0xFFFFFFFE, 0xFFFFFFFFFFFFFFFF
 
 
+BACKEND_B200_NO_GRAPH = 0xFFFFFFFF
+
+
+class HostRange(C.Structure):
+    _fields_ = [("arena_offset", C.c_uint64), ("memory", C.c_void_p), ("byte_count", C.c_uint64)]
+
+
 class ExchangePlace(C.Structure):
     _fields_ = [("address_word_offset", C.c_uint64), ("offset", C.c_uint64)]
 

@@ -239,9 +239,11 @@ MUST_CHECK result_status backend_b200_step_run(struct device_card *card, uint32_
 					       uint64_t input_arena_offset, const void *page_locked_input,
 					       uint64_t input_byte_count, uint64_t output_arena_offset,
 					       void *page_locked_output, uint64_t output_byte_count);
-/* The same step as ONE graph: the copy in, the chain of launches and the copy out are captured together (memcpy nodes
- * at fixed page-locked addresses, read and written when the graph runs), so that a step is a single graph launch and a
- * wait: backend_b200_graph_run_wait. For tables of LAUNCH_CHAIN kernel launches (STATUS_UNSUPPORTED otherwise: such a
+/* The same step as ONE graph: the copy in, the chain of launches and the copy out are captured together (copies
+ * at fixed page-locked addresses, read and written when the graph runs: up to BACKEND_B200_STEP_COPY_MOST bytes each by
+ * kernels that begin while their neighbours run, kernel file "kernel_step_copy", beyond by memcpy nodes), so that a
+ * step is a single graph launch and a wait: backend_b200_graph_run_wait. A first launch whose branch carries
+ * LAUNCH_OVERLAPS_PREVIOUS overlaps the copy in. For tables of LAUNCH_CHAIN kernel launches (STATUS_UNSUPPORTED otherwise: such a
  * table goes through graph_capture and backend_b200_step_run). The caller writes its inputs to the same page-locked
  * range before every run and reads the output range after the wait. */
 MUST_CHECK result_status backend_b200_step_capture(struct device_card *card, const struct kernel_launch *launches,
@@ -249,8 +251,36 @@ MUST_CHECK result_status backend_b200_step_capture(struct device_card *card, con
 						   const void *page_locked_input, uint64_t input_byte_count,
 						   uint64_t output_arena_offset, void *page_locked_output,
 						   uint64_t output_byte_count, uint32_t *graph_out);
-/* graph_run of the table, then the driver's stream wait: returns when the graph has run (any captured graph). */
+/* Half the time of a memcpy node's dispatch is what the kernels save; a megabyte is 20 us of PCIe either way. */
+#define BACKEND_B200_STEP_COPY_MOST (1u << 20)
+#define BACKEND_B200_STEP_COPY_THREADS 256u
+#define BACKEND_B200_STEP_COPY_KERNEL_FILE "kernel_step_copy"
+struct backend_b200_step_copy_record {
+	uint64_t host_address; /* page-locked, 16-byte aligned */
+	uint64_t arena_offset; /* 16-byte aligned */
+	uint64_t byte_count;
+	uint64_t ticket_address; /* copy out: a page-locked word that holds the run's number ... */
+	uint64_t done_address; /* ... and one that is given it when the outputs are in place */
+};
+/* graph_run of the table, then a wait: returns when the graph's outputs are in place (a graph of step_capture whose copy
+ * out is a kernel: the host polls the word that kernel stores; any other graph: the driver's stream wait). */
 MUST_CHECK result_status backend_b200_graph_run_wait(struct device_card *card, uint32_t graph);
+/* A call on ORDINARY host memory in one go: the inputs' bytes through the page-locked block into the arena, the graph
+ * (BACKEND_B200_NO_GRAPH: none), the outputs' bytes through the block into ordinary memory; returns when all of it is
+ * done. A large transfer goes in pieces: pieces are copied on the host by several threads while others cross PCIe. The
+ * block (inside one staging block) holds every input and output at once, each begun on a multiple of 256 bytes;
+ * STATUS_INVALID_ARGUMENT if it is too small. Counts may be 0. */
+#define BACKEND_B200_NO_GRAPH UINT32_MAX
+#define BACKEND_B200_HOST_RANGES_MOST 8u
+struct backend_b200_host_range {
+	uint64_t arena_offset;
+	void *memory;
+	uint64_t byte_count;
+};
+MUST_CHECK result_status backend_b200_step_call(struct device_card *card, uint32_t graph,
+						const struct backend_b200_host_range *inputs, uint32_t input_count,
+						const struct backend_b200_host_range *outputs, uint32_t output_count,
+						void *page_locked, uint64_t page_locked_byte_count);
 /* Kernel launches this card has queued since it was opened, graph launches counted by their kernel nodes. */
 /* The dependencies graph_capture gives every launch of a table (order_out[launch_count]), from the branches alone: no
  * card is needed. STATUS_INVALID_ARGUMENT for a NULL, an empty table, a branch that is none of LAUNCH_* or a table
