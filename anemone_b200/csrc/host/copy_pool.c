@@ -1,6 +1,7 @@
 /* copy_pool.c: host memory copies by a few threads at once (copy_pool.h). */
 #include "copy_pool.h"
 
+#include <emmintrin.h>
 #include <pthread.h>
 #include <sched.h>
 #include <string.h>
@@ -15,9 +16,34 @@ static uint32_t thread_count, users;
 static bool ending;
 static struct ab_copy_batch *current; /* one batch at a time: another caller copies by itself */
 
+/* Stores past the caches: what the device reads next lies in memory and not as dirty lines of some core's cache, which
+ * PCIe reads at half its rate (a prompt of 2048 rows of 4096, 16.8 MB and 2 MB of scores: 1042 us, so 565). */
+static void copy_past_caches(void *to, const void *from, size_t byte_count)
+{
+	unsigned char *out = to;
+	const unsigned char *in = from;
+	const size_t head = (16u - ((uintptr_t)out & 15u)) & 15u;
+	if (byte_count < 64u + head) {
+		memcpy(out, in, byte_count);
+		return;
+	}
+	memcpy(out, in, head);
+	out += head, in += head, byte_count -= head;
+	for (; byte_count >= 64u; out += 64, in += 64, byte_count -= 64u)
+		for (int quarter = 0; quarter < 4; quarter++)
+			_mm_stream_si128((__m128i *)(void *)(out + 16 * quarter),
+					 _mm_loadu_si128((const __m128i *)(const void *)(in + 16 * quarter)));
+	_mm_sfence();
+	memcpy(out, in, byte_count);
+}
+
 static void copy_make(struct ab_copy_batch *batch, uint32_t index)
 {
-	memcpy(batch->copies[index].to, batch->copies[index].from, batch->copies[index].byte_count);
+	const struct ab_copy *const copy = &batch->copies[index];
+	if (batch->to_device)
+		copy_past_caches(copy->to, copy->from, copy->byte_count);
+	else
+		memcpy(copy->to, copy->from, copy->byte_count);
 	__atomic_store_n(&batch->done[index], 1u, __ATOMIC_RELEASE); /* the batch may be gone after this */
 }
 

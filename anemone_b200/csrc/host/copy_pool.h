@@ -24,6 +24,7 @@ struct ab_copy_batch {
 	uint32_t count;
 	uint32_t next, allowed; /* under the pool's mutex */
 	uint32_t done[AB_COPY_BATCH_MOST];
+	bool to_device; /* the copies' targets are read by the device next: written past the caches */
 	bool shared; /* the pool's threads help (else they are busy with another thread's batch) */
 };
 

@@ -93,3 +93,25 @@ def test_side_runs_and_copies(api):
         assert card.ops.launch_run(card.handle, beyond, 1) == R.STATUS_INVALID_ARGUMENT
     finally:
         card.close()
+
+
+@pytest.mark.parametrize("sizes", [(1,), (63, 65, 17), ((1 << 19) - 1, (1 << 19) + 1), (1 << 20, 3, 5 << 20), (40 << 20,)])
+def test_a_call_copies_ordinary_memory(api, sizes):
+    """backend_b200_step_call without a graph: ranges of ordinary memory in and out again, at the edges of the pieces
+    they are cut in (one piece, ragged ones, longer pieces where there would be too many), odd addresses and sizes."""
+    rng = np.random.default_rng(len(sizes) + sizes[0])
+    blocks = [rng.integers(0, 256, size=size + 3, dtype=np.uint8) for size in sizes]
+    offsets = np.cumsum([0] + [api.align(size, 16) + 16 for size in sizes])
+    card = api.Card(0, 64 << 20)
+    try:
+        for lead in (0, 3):
+            card.fill(0, 0xA5, int(offsets[-1]))
+            into = [block[lead:lead + size] for block, size in zip(blocks, sizes)]
+            card.call(None, [(int(at), array) for at, array in zip(offsets, into)], [])
+            back = [np.zeros(size + 3, dtype=np.uint8) for size in sizes]
+            card.call(None, [], [(int(at), array[lead:lead + size]) for at, array, size in zip(offsets, back, sizes)])
+            for array, sent, size, at in zip(back, into, sizes, offsets):
+                assert np.array_equal(array[lead:lead + size], sent) and not array[:lead].any()
+                assert (card.download(int(at) + size, 16) == 0xA5).all()  # nothing past the range
+    finally:
+        card.close()
