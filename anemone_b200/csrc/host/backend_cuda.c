@@ -34,6 +34,7 @@ struct prepared_kernel {
 	char function[96];
 	CUfunction handle;
 	uint32_t argument_byte_count;
+	uint32_t cluster[LAUNCH_DIMENSIONS]; /* blocks of its source's cluster, in which a launch's grid counts; 1, 1, 1: none */
 };
 
 struct transfer_ticket {
@@ -679,7 +680,15 @@ static result_status cuda_kernel_prepare(struct device_card *card, const char *k
 	DRIVER(card, cuFuncGetAttribute(&static_shared, CU_FUNC_ATTRIBUTE_SHARED_SIZE_BYTES, function));
 	DRIVER(card, cuFuncSetAttribute(function, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES,
 					card->shared_memory_most - static_shared));
+	static const CUfunction_attribute cluster_axes[LAUNCH_DIMENSIONS] = { CU_FUNC_ATTRIBUTE_REQUIRED_CLUSTER_WIDTH,
+									      CU_FUNC_ATTRIBUTE_REQUIRED_CLUSTER_HEIGHT,
+									      CU_FUNC_ATTRIBUTE_REQUIRED_CLUSTER_DEPTH };
 	struct prepared_kernel *const prepared = &card->kernels[card->kernel_count];
+	for (uint32_t axis = 0; axis < LAUNCH_DIMENSIONS; axis++) {
+		int width = 0;
+		DRIVER(card, cuFuncGetAttribute(&width, cluster_axes[axis], function));
+		prepared->cluster[axis] = width > 0 ? (uint32_t)width : 1u;
+	}
 	prepared->image = image;
 	prepared->handle = function;
 	prepared->argument_byte_count = argument_byte_count;
@@ -763,6 +772,21 @@ static bool launch_is_valid(const struct device_card *card, const struct kernel_
 	return true;
 }
 
+static bool kernel_has_clusters(const struct prepared_kernel *kernel)
+{
+	return kernel->cluster[0] * kernel->cluster[1] * kernel->cluster[2] != 1u;
+}
+
+static CUlaunchAttributeValue cluster_of(const struct prepared_kernel *kernel)
+{
+	CUlaunchAttributeValue value;
+	memset(&value, 0, sizeof(value));
+	value.clusterDim.x = kernel->cluster[0];
+	value.clusterDim.y = kernel->cluster[1];
+	value.clusterDim.z = kernel->cluster[2];
+	return value;
+}
+
 /* Queue the table on the card's stream (which may be capturing). Context current, mutex held. */
 static result_status launches_queue(const struct ab_driver *cu, struct device_card *card,
 				    const struct kernel_launch *launches, uint32_t launch_count)
@@ -783,25 +807,35 @@ static result_status launches_queue(const struct ab_driver *cu, struct device_ca
 		memcpy(record, launch->argument, launch->argument_byte_count);
 		CUdeviceptr arena = card->arena;
 		void *parameters[] = { record, &arena };
+		const struct prepared_kernel *const prepared = &card->kernels[launch->kernel];
+		CUlaunchAttribute attributes[2];
+		uint32_t attribute_count = 0;
+		memset(attributes, 0, sizeof(attributes));
 		if ((launch->branch & LAUNCH_OVERLAPS_PREVIOUS) != 0 && index != 0) {
 			/* behind the launch before it by a programmatic edge: it may start once that launch lets it */
-			CUlaunchAttribute attribute;
-			memset(&attribute, 0, sizeof(attribute));
-			attribute.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
-			attribute.value.programmaticStreamSerializationAllowed = 1;
+			attributes[attribute_count].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+			attributes[attribute_count++].value.programmaticStreamSerializationAllowed = 1;
+		}
+		if (kernel_has_clusters(prepared)) {
+			attributes[attribute_count].id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+			attributes[attribute_count++].value = cluster_of(prepared);
+		}
+		if (attribute_count != 0) {
 			CUlaunchConfig config;
 			memset(&config, 0, sizeof(config));
-			config.gridDimX = launch->grid[0], config.gridDimY = launch->grid[1], config.gridDimZ = launch->grid[2];
+			config.gridDimX = launch->grid[0] * prepared->cluster[0];
+			config.gridDimY = launch->grid[1] * prepared->cluster[1];
+			config.gridDimZ = launch->grid[2] * prepared->cluster[2];
 			config.blockDimX = launch->block[0], config.blockDimY = launch->block[1];
 			config.blockDimZ = launch->block[2];
 			config.sharedMemBytes = launch->dynamic_shared_byte_count;
 			config.hStream = card->stream;
-			config.attrs = &attribute;
-			config.numAttrs = 1;
-			DRIVER(card, cuLaunchKernelEx(&config, card->kernels[launch->kernel].handle, parameters, NULL));
+			config.attrs = attributes;
+			config.numAttrs = attribute_count;
+			DRIVER(card, cuLaunchKernelEx(&config, prepared->handle, parameters, NULL));
 			continue;
 		}
-		DRIVER(card, cuLaunchKernel(card->kernels[launch->kernel].handle, launch->grid[0], launch->grid[1],
+		DRIVER(card, cuLaunchKernel(prepared->handle, launch->grid[0], launch->grid[1],
 					    launch->grid[2], launch->block[0], launch->block[1], launch->block[2],
 					    launch->dynamic_shared_byte_count, card->stream, parameters, NULL));
 	}
@@ -943,13 +977,19 @@ static result_status graph_build(const struct ab_driver *cu, struct device_card 
 		CUDA_KERNEL_NODE_PARAMS parameters;
 		memset(&parameters, 0, sizeof(parameters));
 		parameters.func = card->kernels[launch->kernel].handle;
-		parameters.gridDimX = launch->grid[0], parameters.gridDimY = launch->grid[1];
-		parameters.gridDimZ = launch->grid[2];
+		const struct prepared_kernel *const prepared = &card->kernels[launch->kernel];
+		parameters.gridDimX = launch->grid[0] * prepared->cluster[0];
+		parameters.gridDimY = launch->grid[1] * prepared->cluster[1];
+		parameters.gridDimZ = launch->grid[2] * prepared->cluster[2];
 		parameters.blockDimX = launch->block[0], parameters.blockDimY = launch->block[1];
 		parameters.blockDimZ = launch->block[2];
 		parameters.sharedMemBytes = launch->dynamic_shared_byte_count;
 		parameters.kernelParams = kernel_parameters; /* copied into the node by the call */
 		DRIVER(card, cuGraphAddKernelNode(&nodes[index], graph, depends, order[index].behind_count, &parameters));
+		if (kernel_has_clusters(prepared)) {
+			const CUlaunchAttributeValue cluster = cluster_of(prepared);
+			DRIVER(card, cuGraphKernelNodeSetAttribute(nodes[index], CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION, &cluster));
+		}
 	}
 done:
 	return status;

@@ -60,6 +60,7 @@
 	X(cuGraphGetNodes)        \
 	X(cuGraphCreate)          \
 	X(cuGraphAddKernelNode)   \
+	X(cuGraphKernelNodeSetAttribute) \
 	X(cuGraphAddMemcpyNode)   \
 	X(cuMemcpyDtoDAsync)      \
 	X(cuMemGetAddressRange)   \

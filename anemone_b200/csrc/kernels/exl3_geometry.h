@@ -82,15 +82,12 @@ AB_INLINE uint64_t exl3_layer_gate_up_product_bytes(uint32_t pair_count, uint32_
 /* ---- prefill (kernel_exl3_prefill) ---- */
 #define EXL3_PREFILL_GEMM_THREADS 576u /* a copy warp, an issuing warp, sixteen decode warps */
 #define EXL3_PREFILL_OPERAND_PARTS 4u /* an operand CTA takes a quarter of a tile's rows */
-#define EXL3_PREFILL_GATE_UP_STEPS 2u /* steps of 16 inputs of one stage: two matrices */
-#define EXL3_PREFILL_DOWN_STEPS 4u /* one matrix */
-/* ring depths: operand blocks (bulk copies, mostly from L2), decoded weights (made on the SM) */
-#define EXL3_PREFILL_A_STAGES 4u
-#define EXL3_PREFILL_B_STAGES 4u
-/* the largest of the product CTAs' forms: a stage is 32 KB of one ring and 16 KB of the other */
-#define EXL3_PREFILL_W_STAGE 8192u /* trellis words of one stage at most: 16 x 16 x 64 weights x 4 bits */
-#define EXL3_PREFILL_DYNAMIC_BYTES \
-	(EXL3_PREFILL_A_STAGES * 32768u + EXL3_PREFILL_B_STAGES * (16384u + EXL3_PREFILL_W_STAGE))
+#define EXL3_PREFILL_STAGE_STEPS 2u /* steps of 16 inputs of one stage */
+/* a stage's turn in the ring (decoded, told to the issuing warp, multiplied, freed) is 3500 cycles and more, its products
+ * 512: as many as fit */
+#define EXL3_PREFILL_STAGES 7u
+#define EXL3_PREFILL_STAGE_BYTES 32768u /* gate/up: two blocks of rows, two of weights; down: one and two */
+#define EXL3_PREFILL_DYNAMIC_BYTES (EXL3_PREFILL_STAGES * EXL3_PREFILL_STAGE_BYTES)
 #define EXL3_PREFILL_STAGING_ROW 132u /* floats of a staged accumulator row */
 
 #endif

@@ -1,16 +1,15 @@
 /*
  * kernel_exl3_prefill.cu: the routed-expert layer for many rows (struct exl3_prefill_record): rows are grouped per
- * expert into tiles of 128 and every (row tile, 128 outputs) is one dense contraction on the fifth-generation tensor
- * cores. The reference's counterpart is its tensor-core prefill family (source/kernel_exl3_tcp.cuh), fixed to its
- * model's shapes and to mma.sync; here a CTA
- *   - streams the row tile's FP16 operand blocks (pre-tiled in the tensor cores' no-swizzle K-major layout) into a ring
- *     of shared-memory stages by bulk asynchronous copies (one warp),
- *   - streams the trellis words of its outputs into a second ring by bulk copies a whole turn of the ring ahead,
- *     decodes them in registers into FP16 and stores them as the B operand block of the stage (sixteen warps in four
- *     teams, a team a stage; the decode's fragment order makes every store a contiguous 128 bytes of the block); two
- *     row tiles of one expert share one decode,
- *   - multiplies with tcgen05.mma (one thread), FP32 accumulators in tensor memory, the stage released by
- *     tcgen05.commit,
+ * expert into tiles of 128 and every (one or two row tiles of an expert, 256 outputs of gate and up or 512 of down) is one
+ * dense contraction on the fifth-generation tensor cores. The reference's counterpart is its tensor-core prefill family
+ * (source/kernel_exl3_tcp.cuh), fixed to its model's shapes and to mma.sync; here a pair of CTAs
+ *   - streams its rows' FP16 operands (pre-tiled in the tensor cores' no-swizzle K-major layout) into a ring of
+ *     shared-memory stages, one bulk asynchronous copy a stage (one warp),
+ *   - loads the trellis words of its outputs into registers a turn of the decode teams ahead, decodes them and stores
+ *     them as the A operand blocks of the stage (sixteen warps in four teams, a team a stage; the decode's fragment order
+ *     makes every store a contiguous 128 bytes of the block),
+ *   - multiplies with tcgen05.mma of cta_group::2 (one thread of the pair), FP32 accumulators in tensor memory, the stage
+ *     released by tcgen05.commit,
  *   - reads the accumulators back with tcgen05.ld and applies the chain's FP32 epilogue (exl3_passes.cuh: Hadamard,
  *     scales, SwiGLU, down-side transform / route weight) a warp a row.
  * Arithmetic per value is the retained chain's; only the association of the FP32 sums over K is the tensor cores'.
@@ -22,23 +21,18 @@
 
 #define PREFILL_FIRST_DECODE_WARP 2u /* behind the copy warp and the issuing warp */
 #define PREFILL_DECODE_WARPS 16u
-#define PREFILL_GROUPS 2u /* groups of 128 outputs of one product CTA */
 #define PREFILL_DECODE_THREADS (PREFILL_DECODE_WARPS * EXL3_WARP)
-#define PREFILL_COLUMNS 128u /* tensor-memory columns of one accumulator tile */
+#define PREFILL_TEAMS 4u /* of four decode warps */
 #define PREFILL_GROUP_THREADS 256u
 
 struct prefill_shared {
-	uint64_t a_full[EXL3_PREFILL_A_STAGES]; /* the stage's operand blocks have landed */
-	uint64_t a_free[EXL3_PREFILL_A_STAGES]; /* the products that read them are done */
-	uint64_t b_full[EXL3_PREFILL_B_STAGES]; /* the stage's decoded weights are written */
-	uint64_t b_free[EXL3_PREFILL_B_STAGES]; /* the products that read them are done */
-	uint64_t w_full[EXL3_PREFILL_B_STAGES]; /* the stage's trellis words have landed */
-	uint64_t done; /* every product of the CTA is done */
+	uint64_t full[EXL3_PREFILL_STAGES]; /* the stage's weights are decoded and its rows have landed; rank 0: the other CTA's too */
+	uint64_t free[EXL3_PREFILL_STAGES]; /* the products that read it are done */
+	uint64_t done; /* every product of the pair is done */
 	uint32_t tensor_memory;
 	volatile uint32_t failed;
-	uint32_t armed_a; /* K blocks whose operand copies were started */
-	uint32_t armed_w[EXL3_PREFILL_B_STAGES]; /* a team's stages whose trellis copies were started */
-	uint32_t issued; /* 1: products were issued and `done` will complete */
+	uint32_t expired; /* an earlier wait had run out when the CTA began */
+	uint32_t armed; /* stages whose row copies were started */
 };
 
 struct prefill_view {
@@ -180,11 +174,44 @@ __device__ __forceinline__ uint32_t prefill_inner_of(const struct exl3_prefill_r
 	return expert < record.local_count ? record.inner_size : record.shared_inner_size;
 }
 
-/* byte of (row, input) inside an operand block of 128 rows x 64 inputs: 16-byte pieces of eight inputs, the pieces of
- * eight rows adjacent, the 16 row groups adjacent, then the next eight inputs */
-__device__ __forceinline__ uint32_t prefill_block_byte(uint32_t row, uint32_t input)
+/* A unit's rows: one row tile, or two of one expert (0: the second of two). An expert's row tiles are taken two at a time: the pair of an
+ * even-numbered tile that has a successor also takes the successor's rows, so that every decoded weight is multiplied
+ * with 256 rows; the pair of an odd-numbered tile returns. */
+__device__ __forceinline__ uint32_t prefill_tiles_of_unit(const prefill_view &view, const struct exl3_prefill_tile &tile,
+							  uint32_t tile_index, uint32_t tile_count)
 {
-	return (input / 8u) * 2048u + (row / 8u) * 128u + (row % 8u) * 16u + (input % 8u) * 2u;
+	if ((tile.first_entry / EXL3_PREFILL_TILE_ROWS) % 2u != 0u)
+		return 0;
+	const struct exl3_prefill_tile *const tiles =
+		reinterpret_cast<const struct exl3_prefill_tile *>(view.workspace + view.parts.tiles);
+	return tile_index + 1u < tile_count && tiles[tile_index + 1u].expert == tile.expert ? 2u : 1u;
+}
+
+/* Where a tile's operands lie: what a CTA of the pair takes for one stage of 32 inputs is ONE run of bytes, [matrix][four
+ * pieces of eight inputs][half rows][16 bytes], the stages one behind the other. The second CTA's runs are in the second
+ * tile's region, or behind the first CTA's for a single tile. (With a fixed place for each of 128 rows a stage of fewer
+ * rows was up to eight copies, and their issue, 1070 cycles a stage, was what bounded the products.) */
+struct prefill_rows {
+	uint32_t half; /* rows a CTA takes, whole sixteens */
+	uint64_t second; /* from a single tile's first run to the second CTA's */
+};
+
+__device__ __forceinline__ prefill_rows prefill_rows_of(uint32_t count, uint32_t row_count, uint32_t matrices, uint32_t inputs)
+{
+	prefill_rows rows;
+	/* a tile of two has a CTA for itself: all of its rows count as the first half */
+	rows.half = count == 1u ? (row_count + 31u) / 32u * 16u : EXL3_PREFILL_TILE_ROWS;
+	rows.second = (uint64_t)inputs * matrices * rows.half * 2u;
+	return rows;
+}
+
+/* byte of (row, input) of matrix m inside the tile's region */
+__device__ __forceinline__ uint64_t prefill_operand_byte(const prefill_rows &rows, uint32_t matrices, uint32_t m, uint32_t row,
+							 uint32_t input)
+{
+	const uint32_t rank = row / rows.half, piece = input / 8u;
+	return rank * rows.second + (uint64_t)((piece / 4u * matrices + m) * 4u + piece % 4u) * (rows.half * 16u) +
+	       (row - rank * rows.half) * 16u + input % 8u * 2u;
 }
 
 /* grid (tile capacity, ceil(H / 128 / 4) x EXL3_PREFILL_OPERAND_PARTS, 2) x 128: x . suh, Hadamard, FP16 operands of
@@ -223,12 +250,10 @@ extern "C" __global__ void __launch_bounds__(EXL3_TRANSFORM_THREADS)
 		reinterpret_cast<const struct exl3_prefill_entry *>(view.workspace + view.parts.entries) +
 		(uint64_t)tile.expert * record.row_capacity + tile.first_entry;
 	const __nv_bfloat16 *const input = reinterpret_cast<const __nv_bfloat16 *>(arena + record.input_offset);
-	/* the two operand blocks (64 inputs each) this warp's 128 channels fall in */
-	unsigned char *const blocks = view.workspace + view.parts.gate_up_operands +
-				      (((uint64_t)blockIdx.z * view.parts.tile_capacity + tile_index) *
-					       (H / EXL3_PREFILL_BLOCK_INPUTS) +
-				       2u * block) *
-					      EXL3_PREFILL_BLOCK_BYTES;
+	const uint32_t count = prefill_tiles_of_unit(
+		view, tile, tile_index, reinterpret_cast<const uint32_t *>(view.workspace + view.parts.counts)[view.experts]);
+	const prefill_rows rows = prefill_rows_of(count, tile.row_count, EXL3_PROJECTIONS, H);
+	unsigned char *const region = view.workspace + view.parts.gate_up_operands + (uint64_t)tile_index * H * 512u;
 	unsigned char *const mine = staged[warp];
 	for (uint32_t first = part * part_rows; first < (part + 1u) * part_rows && first < tile.row_count; first += 8u) {
 		uint2 raw[8];
@@ -259,8 +284,8 @@ extern "C" __global__ void __launch_bounds__(EXL3_TRANSFORM_THREADS)
 		for (uint32_t turn = 0; turn < 4; turn++) {
 			const uint32_t piece = turn * 4u + lane / 8u, row = lane % 8u;
 			const uint4 value = *reinterpret_cast<const uint4 *>(mine + row * OPERAND_ROW_BYTES + piece * 16u);
-			*reinterpret_cast<uint4 *>(blocks + (piece / 8u) * EXL3_PREFILL_BLOCK_BYTES + (piece % 8u) * 2048u +
-						   (first / 8u) * 128u + row * 16u) = value;
+			*reinterpret_cast<uint4 *>(region + prefill_operand_byte(rows, EXL3_PROJECTIONS, blockIdx.z, first + row,
+										 block * EXL3_TRANSFORM + piece * 8u)) = value;
 		}
 		__syncwarp();
 	}
@@ -268,19 +293,31 @@ extern "C" __global__ void __launch_bounds__(EXL3_TRANSFORM_THREADS)
 
 /* ------------------------------------------------------------------ tensor-core products */
 
-/* shared-memory matrix descriptor of an operand block at a 16-byte aligned address: no swizzle, K-major;
- * piece_bytes between the two 16-byte K pieces of a K = 16 step (128 bytes a group of eight rows: 2048 for 128 rows,
- * 4096 for 256), 128 bytes between groups of eight rows */
-__device__ __forceinline__ uint64_t prefill_descriptor(uint32_t shared_address, uint32_t piece_bytes)
+/* A product unit belongs to a CTA PAIR (tcgen05 cta_group::2, one instruction over two SMs): the weights are the
+ * instruction's M side, 256 outputs of which each CTA decodes its own 128, and the rows are its N side, up to two row
+ * tiles of one expert (256 rows) of which each CTA brings its own half. So a decoded weight meets 256 rows, a row's
+ * operands meet 256 outputs (gate/up; down: 512), and each SM's shared memory gives an instruction 64 bytes a cycle
+ * (its 128 outputs and its 128 rows per 128 cycles). One CTA on its own with two row tiles of 128 x 128 products needs
+ * 128 bytes a cycle for the instructions alone, all there is, and takes every row's operands from L2 twice as often.
+ * The rows' number is the instruction's N, so a last tile of few rows costs the tensor cores little; the decode is the
+ * same for any. 4096 rows of H 4096, I 2048, 256 experts of 8: gate/up 2202 us with single CTAs, 1880 so; down 1211,
+ * 1137. Bound by issue: the decode of a stage alone is about 500 cycles of its 600. */
+#define PREFILL_PAIR 2u /* CTAs of a unit */
+#define PREFILL_SUM_COLUMNS 256u /* tensor-memory columns of one accumulator: a row a column */
+
+/* Shared-memory matrix descriptor of operands at a 16-byte aligned address, in two words, the second constant: no
+ * swizzle, K-major, piece_bytes between the two 16-byte K pieces of a K = 16 step, 128 bytes between groups of eight rows
+ * (or outputs). Places in the rings are constant numbers of 16-byte units apart. */
+#define PREFILL_DESCRIPTOR_HIGH ((128u >> 4) | 1u << 14)
+__device__ __forceinline__ uint32_t prefill_descriptor_low(const void *operands, uint32_t piece_bytes)
 {
-	return (uint64_t)((shared_address >> 4) & 0x3FFFu) | (uint64_t)(piece_bytes >> 4) << 16 |
-	       (uint64_t)(128u >> 4) << 32 | (uint64_t)1 << 46;
+	return smem_address(operands) >> 4 | (piece_bytes >> 4) << 16;
 }
 
-/* FP16 A and B, both K-major, FP32 accumulators, M = 128, N = 128 x groups */
-__device__ __forceinline__ uint32_t prefill_instruction(uint32_t groups)
+/* FP16 A and B, both K-major, FP32 accumulators, M = 256, N = the pair's rows (a multiple of 32) */
+__device__ __forceinline__ uint32_t prefill_instruction(uint32_t rows)
 {
-	return (1u << 4) | ((groups * 128u >> 3) << 17) | ((128u >> 4) << 24);
+	return (1u << 4) | ((rows >> 3) << 17) | ((256u >> 4) << 24);
 }
 
 __device__ __forceinline__ void tensor_fence_before()
@@ -293,10 +330,24 @@ __device__ __forceinline__ void tensor_fence_after()
 	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-__device__ __forceinline__ void tensor_commit(uint64_t *barrier)
+/* accumulate 0: the sums begin with this product */
+__device__ __forceinline__ void tensor_multiply(uint32_t sums, uint32_t a, uint32_t b, uint32_t instruction, uint32_t accumulate)
 {
-	asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-			     smem_address(barrier))
+	asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+		     "setp.ne.b32 p, %4, 0;\n\t"
+		     "mov.b64 a, {%1, %5};\n\t"
+		     "mov.b64 b, {%2, %5};\n\t"
+		     "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(sums),
+		     "r"(a), "r"(b), "r"(instruction), "r"(accumulate), "n"(PREFILL_DESCRIPTOR_HIGH)
+		     : "memory");
+}
+
+/* arrives at this barrier of the CTAs of `ranks` (a bit each) once the products this thread issued so far are done */
+__device__ __forceinline__ void tensor_commit(uint64_t *barrier, uint32_t ranks)
+{
+	asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+			     smem_address(barrier)),
+		     "h"((uint16_t)ranks)
 		     : "memory");
 }
 
@@ -305,244 +356,242 @@ __device__ __forceinline__ void decode_sync()
 	asm volatile("bar.sync 1, %0;" ::"n"(PREFILL_DECODE_THREADS) : "memory");
 }
 
-/* Dynamic shared memory of a product CTA, for TILES row tiles of one expert, MATRICES matrices, GROUPS groups of 128
- * outputs and stages of KSTEPS steps of 16 inputs. Three rings:
- *   A ring        EXL3_PREFILL_A_STAGES x [tile][matrix] operand blocks (128 rows x 16 KSTEPS FP16 in the tensor cores'
- *                 layout, KSTEPS x 4096 bytes): bulk copies, mostly from L2
- *   B ring        EXL3_PREFILL_B_STAGES x [matrix] blocks of decoded weights, 128 GROUPS outputs x 16 KSTEPS FP16 in
- *                 the same layout (one instruction multiplies all groups and reads the operand rows once): written by
- *                 the decode warps, read by the products of EVERY row tile
- *   W ring        EXL3_PREFILL_B_STAGES x EXL3_PREFILL_W_STAGE bytes: the stage's trellis words as they lie in the
- *                 matrix, one run of GROUPS x 8 tiles for every (matrix, step): bulk copies by the copy warp, read by the
- *                 decode warps with shared-memory loads. The team that owns a stage starts the copies of its next use
- *                 as soon as its four warps have read this one, a whole turn of the ring before it needs them. */
-template <uint32_t MATRICES, uint32_t KSTEPS, uint32_t TILES, uint32_t GROUPS> struct prefill_rings {
-	static constexpr uint32_t block_bytes = KSTEPS * 4096u;
-	static constexpr uint32_t a_stage = TILES * MATRICES * block_bytes;
-	static constexpr uint32_t b_piece = GROUPS * 2048u; /* eight inputs of 128 GROUPS outputs */
-	static constexpr uint32_t b_block = GROUPS * block_bytes; /* of one matrix */
-	static constexpr uint32_t b_stage = MATRICES * b_block;
-	static constexpr uint32_t b_at = EXL3_PREFILL_A_STAGES * a_stage;
-	static constexpr uint32_t w_at = b_at + EXL3_PREFILL_B_STAGES * b_stage;
-	static constexpr uint32_t bytes = w_at + EXL3_PREFILL_B_STAGES * EXL3_PREFILL_W_STAGE;
-	static constexpr uint32_t columns = TILES * MATRICES * GROUPS * PREFILL_COLUMNS; /* of tensor memory */
-	static_assert(bytes <= EXL3_PREFILL_DYNAMIC_BYTES, "the host sizes the rings");
-	static_assert(columns <= 512u, "tensor memory has 512 columns");
-	/* first column of the accumulator of (row tile, matrix, group) */
-	__device__ static constexpr uint32_t column(uint32_t tile, uint32_t m, uint32_t g)
-	{
-		return ((tile * MATRICES + m) * GROUPS + g) * PREFILL_COLUMNS;
-	}
+/* one lane of a converged warp, the same one every time */
+__device__ __forceinline__ bool prefill_elected()
+{
+	uint32_t elected;
+	asm volatile("{\n\t.reg .pred p;\n\t"
+		     "elect.sync _|p, 0xFFFFFFFF;\n\t"
+		     "selp.u32 %0, 1, 0, p;\n\t}"
+		     : "=r"(elected));
+	return elected != 0;
+}
+
+/* a whole warp's wait: its lanes go on, or give up, together */
+__device__ __forceinline__ bool warp_wait(uint64_t *barrier, uint32_t parity)
+{
+	return __all_sync(0xFFFFFFFFu, barrier_wait(barrier, parity)) != 0;
+}
+
+/* whether the phase has completed by now, without a wait */
+__device__ __forceinline__ uint32_t barrier_test(uint32_t barrier, uint32_t parity)
+{
+	uint32_t complete;
+	asm volatile("{\n\t.reg .pred p;\n\t"
+		     "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+		     "selp.u32 %0, 1, 0, p;\n\t}"
+		     : "=r"(complete)
+		     : "r"(barrier), "r"(parity)
+		     : "memory");
+	return complete;
+}
+
+/* a value every lane holds, as one the compiler knows to be the warp's (an operand of the tensor cores' instructions) */
+__device__ __forceinline__ uint32_t warp_value(uint32_t value)
+{
+	return __shfl_sync(0xFFFFFFFFu, value, 0);
+}
+
+__device__ __forceinline__ void pair_sync()
+{
+	asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+/* the other CTA's (rank's) address of a variable of this one's */
+__device__ __forceinline__ uint32_t pair_address(const volatile void *here, uint32_t rank)
+{
+	uint32_t there;
+	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+		     : "=r"(there)
+		     : "r"((uint32_t)__cvta_generic_to_shared(const_cast<const void *>(here))), "r"(rank));
+	return there;
+}
+
+/* Dynamic shared memory of a product CTA: MATRICES x GROUPS = 2 accumulators, gate and up of 128 outputs or down of
+ * 2 x 128; a ring of EXL3_PREFILL_STAGES stages of 32 inputs, each
+ *   [matrix] the CTA's rows (up to 128 x 32 FP16, 8 KB): one bulk copy, mostly from L2
+ *   [matrix x group] decoded weights, 128 outputs x 32 FP16, 8 KB in the same layout: written by the decode warps
+ * Rows and weights share the stage so that the issuing warp waits for ONE barrier a stage: a wait on a barrier that is
+ * long complete takes it 150 cycles, three of them and the issue of four products 730, where the products of 256 rows
+ * last 512. The trellis words do not pass here: the start of a bulk copy takes a warp 300 to 500 cycles, whatever the
+ * bytes, and a stage's words were four runs (5 copies a stage: 650 cycles a stage; 12: 900). */
+#define PREFILL_STEPS EXL3_PREFILL_STAGE_STEPS
+#define PREFILL_BLOCK (PREFILL_STEPS * 4096u) /* 512 units of 16 bytes, 256 a step */
+template <uint32_t MATRICES, uint32_t GROUPS> struct prefill_rings {
+	static constexpr uint32_t weights_at = MATRICES * PREFILL_BLOCK; /* in a stage, behind the rows */
+	static constexpr uint32_t stage = EXL3_PREFILL_STAGE_BYTES;
+	static constexpr uint32_t bytes = EXL3_PREFILL_STAGES * stage;
+	static_assert(weights_at + MATRICES * GROUPS * PREFILL_BLOCK <= stage, "a stage holds its blocks");
+	static_assert(MATRICES * GROUPS * PREFILL_SUM_COLUMNS == 512u, "tensor memory has 512 columns");
+	static_assert(bytes == EXL3_PREFILL_DYNAMIC_BYTES, "the host sizes the rings");
 };
 
-/* The K loop of one CTA. matrices[m]: the codes of matrix m (`outputs` outputs), of which the CTA takes the `groups`
- * (1 .. GROUPS) groups of 128 outputs from group `first_group`; operand_blocks[tile * MATRICES + m]: row tile `tile`'s
- * operand blocks for matrix m; `blocks` stages of 16 KSTEPS inputs. Warp 0 copies operand blocks, one thread of warp 1
- * issues the products, warps 2 .. copy trellis words and decode. On return the decode warps know whether the
- * accumulators (prefill_rings::column from shared->tensor_memory) are complete; the other warps return false.
- * All threads call. */
-template <uint32_t BX2, uint32_t MATRICES, uint32_t KSTEPS, uint32_t TILES, uint32_t GROUPS>
+/* The K loop of one CTA of the pair. matrices[m]: the codes of matrix m (`outputs` outputs), of which this CTA decodes
+ * the `groups` (0 .. GROUPS) groups of 128 outputs from group `first_group`; `sums`: GROUPS, or the groups either CTA
+ * decodes if that is less; row_runs: this CTA's `half` rows (half the pair's, a multiple of 16) of the operands, a run a
+ * stage; `blocks` stages. Warp 0 copies the rows' operands; warp 1 issues the products (rank 0) or
+ * tells rank 0 which of this CTA's stages are in place (rank 1); warps 2 .. copy trellis words and decode. On return
+ * the decode warps know whether the accumulators (PREFILL_SUM_COLUMNS apart from shared->tensor_memory; lane: output,
+ * column: row of the pair) are complete; the other warps return false. All threads of both CTAs call. */
+template <uint32_t BX2, uint32_t MATRICES, uint32_t GROUPS>
 __device__ __forceinline__ bool prefill_products(const unsigned char *const (&matrices)[MATRICES], uint32_t outputs,
-						 uint32_t first_group, uint32_t groups,
-						 const unsigned char *const (&operand_blocks)[TILES * MATRICES],
-						 uint32_t blocks, unsigned char *dynamic_shared, prefill_shared *shared)
+						 uint32_t first_group, uint32_t groups, uint32_t sums,
+						 const unsigned char *row_runs, uint32_t half,
+						 uint32_t blocks, uint32_t rank, unsigned char *dynamic_shared,
+						 prefill_shared *shared)
 {
 	typedef exl3_ring<BX2> ring;
-	typedef prefill_rings<MATRICES, KSTEPS, TILES, GROUPS> rings;
-	constexpr uint32_t AS = EXL3_PREFILL_A_STAGES, BS = EXL3_PREFILL_B_STAGES;
-	/* the trellis words of one (matrix, step) of a stage: GROUPS groups of eight tiles, adjacent in the matrix */
-	constexpr uint32_t w_chunk = GROUPS * EXL3_GROUP_TILES * ring::words * 4u;
-	static_assert(MATRICES * KSTEPS * w_chunk <= EXL3_PREFILL_W_STAGE, "the W ring holds a stage");
-	static_assert(MATRICES <= 2u && MATRICES * KSTEPS <= EXL3_WARP && w_chunk % 16u == 0u, "a lane a copy, whole 16 bytes");
+	typedef prefill_rings<MATRICES, GROUPS> rings;
+	constexpr uint32_t S = EXL3_PREFILL_STAGES;
 	const uint32_t lane = threadIdx.x % EXL3_WARP, warp = threadIdx.x / EXL3_WARP;
 	const uint64_t step_words = (uint64_t)(outputs / EXL3_TILE) * ring::words; /* of one step of 16 inputs */
-
-	if (threadIdx.x == 0) {
-		for (uint32_t stage = 0; stage < AS; stage++) {
-			barrier_init(&shared->a_full[stage], 1);
-			barrier_init(&shared->a_free[stage], 1);
-		}
-		for (uint32_t stage = 0; stage < BS; stage++) {
-			barrier_init(&shared->b_full[stage], 4u); /* the four warps of the team that decodes the stage */
-			barrier_init(&shared->b_free[stage], 1);
-			barrier_init(&shared->w_full[stage], 1);
-		}
-		barrier_init(&shared->done, 1);
-		shared->failed = 0;
-		shared->armed_a = 0;
-		for (uint32_t stage = 0; stage < BS; stage++)
-			shared->armed_w[stage] = 0;
-		shared->issued = 0;
-		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-	}
-	if (warp == 1) {
-		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-				     smem_address(&shared->tensor_memory)),
-			     "r"(rings::columns)
-			     : "memory");
-		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-	}
-	tensor_fence_before();
-	__syncthreads();
-	tensor_fence_after();
 	const uint32_t accumulators = shared->tensor_memory;
 
 	if (warp == 0) {
-		/* operand copies: lane (tile, m) copies that block */
-		uint32_t block = 0;
-		for (; block < blocks; block++) {
-			const uint32_t stage = block % AS, use = block / AS;
-			uint32_t good = 1;
-			if (lane == 0) {
-				if (use > 0 && !barrier_wait(&shared->a_free[stage], (use - 1u) & 1u))
-					good = 0;
-				else
-					barrier_expect(&shared->a_full[stage], rings::a_stage);
-			}
-			good = __shfl_sync(0xFFFFFFFFu, good, 0);
-			if (good == 0)
-				break;
-			if (lane < TILES * MATRICES)
-				bulk_load(dynamic_shared + stage * rings::a_stage + lane * rings::block_bytes,
-					  operand_blocks[lane] + (uint64_t)block * rings::block_bytes, rings::block_bytes,
-					  &shared->a_full[stage]);
-		}
+		/* the rows' operands: a copy a stage */
 		if (lane == 0) {
-			shared->armed_a = block;
+			const uint32_t bytes = MATRICES * PREFILL_STEPS * 32u * half;
+			uint32_t block = 0;
+			for (; block < blocks; block++) {
+				const uint32_t stage = block % S;
+				if (block >= S && !barrier_wait(&shared->free[stage], (block / S - 1u) & 1u))
+					break;
+				barrier_expect(&shared->full[stage], bytes);
+				bulk_load(dynamic_shared + stage * rings::stage, row_runs + (uint64_t)block * bytes, bytes,
+					  &shared->full[stage]);
+			}
+			shared->armed = block;
 			if (block < blocks)
 				shared->failed = 1;
 		}
 		return false;
 	}
+	if (warp == 1 && rank != 0) {
+		/* rank 0 issues for both: a stage's arrival there says that this CTA's part of it is in place. The decode warps
+		 * do not tell rank 0 themselves: their arrival across the pair would wait for their stores. */
+		bool good = true;
+		for (uint32_t block = 0; block < blocks && good; block++) {
+			good = warp_wait(&shared->full[block % S], (block / S) & 1u);
+			if (good && prefill_elected())
+				tensor_commit(&shared->full[block % S], 1u);
+			__syncwarp();
+		}
+		if (!good)
+			shared->failed = 1;
+		return false;
+	}
 	if (warp == 1) {
-		/* products: one thread; every row tile's products read the same decoded weights */
-		if (lane == 0) {
-			bool good = true;
-			const uint32_t instruction = prefill_instruction(groups);
-			for (uint32_t block = 0; block < blocks && good; block++) {
-				const uint32_t sa = block % AS, sb = block % BS;
-				good = barrier_wait(&shared->a_full[sa], (block / AS) & 1u) &&
-				       barrier_wait(&shared->b_full[sb], (block / BS) & 1u);
+		/* This warp bounds the products where the rows are few. It has one issue slot in five or six beside the decode
+		 * warps of its scheduler, so what counts is how many instructions a stage takes: counters instead of remainders,
+		 * sums of descriptors made once, and the next stage's barrier asked for before this stage's products go out. */
+		bool good = true;
+		uint32_t ready = 0, stage = 0, parity = 0, accumulate = 0;
+		const uint32_t instruction = warp_value(prefill_instruction(PREFILL_PAIR * half));
+		const uint32_t r_low = warp_value(prefill_descriptor_low(dynamic_shared, half * 16u));
+		const uint32_t w_low = warp_value(prefill_descriptor_low(dynamic_shared + rings::weights_at, 2048u));
+		const uint32_t r_step = warp_value(2u * half), columns = warp_value(accumulators), live = warp_value(sums);
+		const uint32_t full = warp_value(smem_address(shared->full)), r_second = MATRICES > 1u ? 2u * r_step : 0u;
+		for (uint32_t left = blocks; left != 0; left--) {
+			if (ready == 0) {
+				good = warp_wait(&shared->full[stage], parity);
 				if (!good)
 					break;
-				tensor_fence_after();
-				/* the stage's first descriptors; every other one lies a constant number of 16-byte units behind */
-				const uint64_t a_first =
-					prefill_descriptor(smem_address(dynamic_shared + sa * rings::a_stage), 2048u);
-				const uint64_t b_first = prefill_descriptor(
-					smem_address(dynamic_shared + rings::b_at + sb * rings::b_stage), rings::b_piece);
-#pragma unroll
-				for (uint32_t tile = 0; tile < TILES; tile++)
-#pragma unroll
-					for (uint32_t m = 0; m < MATRICES; m++)
-#pragma unroll
-						for (uint32_t step = 0; step < KSTEPS; step++) {
-							const uint64_t a =
-								a_first + (((tile * MATRICES + m) * rings::block_bytes + step * 2u * 2048u) >> 4);
-							const uint64_t b = b_first + ((m * rings::b_block + step * 2u * rings::b_piece) >> 4);
-							const uint32_t accumulate = block > 0 || step > 0 ? 1u : 0u;
-							asm volatile("{\n\t.reg .pred p;\n\t"
-								     "setp.ne.b32 p, %4, 0;\n\t"
-								     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(
-									     accumulators + rings::column(tile, m, 0)),
-								     "l"(a), "l"(b), "r"(instruction), "r"(accumulate)
-								     : "memory");
-						}
-				tensor_commit(&shared->a_free[sa]);
-				tensor_commit(&shared->b_free[sb]);
-				shared->issued = 1;
 			}
-			if (!good) {
-				shared->failed = 1;
-				__threadfence_block();
+			const uint32_t r = r_low + stage * (rings::stage >> 4), w = w_low + stage * (rings::stage >> 4);
+			uint64_t *const freed = &shared->free[stage];
+			stage++;
+			if (stage == S)
+				stage = 0, parity ^= 1u;
+			ready = barrier_test(full + stage * 8u, parity);
+			tensor_fence_after();
+			if (prefill_elected()) {
+				tensor_multiply(columns, w, r, instruction, accumulate);
+				tensor_multiply(columns, w + 256u, r + r_step, instruction, 1u);
+				if (GROUPS == 1u || live > 1u) {
+					tensor_multiply(columns + PREFILL_SUM_COLUMNS, w + 512u, r + r_second, instruction, accumulate);
+					tensor_multiply(columns + PREFILL_SUM_COLUMNS, w + 768u, r + r_second + r_step, instruction, 1u);
+				}
+				tensor_commit(freed, 3u);
+				if (left == 1u)
+					tensor_commit(&shared->done, 3u);
 			}
-			if (shared->issued != 0) /* the decode warps and the release wait on this */
-				tensor_commit(&shared->done);
+			accumulate = 1u;
+			ready = __all_sync(0xFFFFFFFFu, left != 1u && ready != 0) ? 1u : 0u;
 		}
+		if (!good) {
+			/* neither CTA stores anything; what was issued is waited for before either goes */
+			if (lane == 0) {
+				shared->failed = 1;
+				asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(pair_address(&shared->failed, 1)), "r"(1u)
+					     : "memory");
+			}
+			__syncwarp();
+			if (prefill_elected())
+				tensor_commit(&shared->done, 3u);
+			__syncwarp();
+		}
+		(void)warp_wait(&shared->done, 0u);
 		return false;
 	}
 
-	/* decode: the sixteen warps are four teams of four; team q decodes the WHOLE stages q, q + 4, ... (with four
-	 * decoded-weights stages in the ring a team owns one of them, and the W stage of the same number), so that the
-	 * teams work on four different stages at once and a warp crosses a barrier and a proxy fence once per stage of 8
-	 * or 16 tiles, not once per 2 or 4. Warp r of a team takes the stage's units r * units_a_warp .. : a unit is the
-	 * eight adjacent tiles of one (matrix, group, step), whose ring words the lane reads from the W ring. */
+	/* decode: the sixteen warps are four teams of four; team q decodes the WHOLE stages q, q + 4, ..., so that the
+	 * teams work on four different stages at once and a warp crosses a barrier and a proxy fence once per stage of
+	 * eight tiles. A warp's part of a stage is the eight adjacent tiles of one (matrix, group, step). A lane loads
+	 * its ring words straight into registers, a tile's words for the team's next stage as soon as this one's are decoded: four
+	 * stages, two microseconds, ahead. */
 	{
-		static_assert(EXL3_PREFILL_B_STAGES == 4u && PREFILL_DECODE_WARPS == 16u, "a team of four warps a stage");
-		constexpr uint32_t units = MATRICES * GROUPS * KSTEPS, units_a_warp = units / 4u;
-		static_assert(units % 4u == 0u, "whole units a warp");
+		static_assert(MATRICES * GROUPS * PREFILL_STEPS == 4u && PREFILL_DECODE_WARPS == 4u * PREFILL_TEAMS, "a part a warp");
 		const uint32_t decoder = warp - PREFILL_FIRST_DECODE_WARP, team = decoder / 4u, member = decoder % 4u;
+		const uint32_t step = member % PREFILL_STEPS, g = GROUPS > 1u ? member / PREFILL_STEPS : 0u;
+		const uint32_t m = MATRICES > 1u ? member / PREFILL_STEPS : 0u;
 		const uint32_t begin = ring::begin(lane);
 		const uint32_t word_index = begin / 32u, shift = begin % 32u, next_index = (word_index + 1u) % ring::words;
-		const uint32_t *const words_at =
-			reinterpret_cast<const uint32_t *>(dynamic_shared + rings::w_at + team * EXL3_PREFILL_W_STAGE);
-		unsigned char *const b_at = dynamic_shared + rings::b_at + team * rings::b_stage + lane * 4u;
-		/* the team's first warp copies the stage's trellis words: lane (m, step) the run of that matrix and step */
-		const uint32_t w_bytes = groups * EXL3_GROUP_TILES * ring::words * 4u;
-		const unsigned char *const w_from =
-			(MATRICES > 1u && lane >= KSTEPS ? matrices[MATRICES - 1u] : matrices[0]) +
-			((uint64_t)(lane % KSTEPS) * step_words + (uint64_t)first_group * EXL3_GROUP_TILES * ring::words) * 4u;
-		unsigned char *const w_to = dynamic_shared + rings::w_at + team * EXL3_PREFILL_W_STAGE + lane * w_chunk;
-#define PREFILL_WORDS_COPY(block)                                                                             \
-	do {                                                                                                  \
-		if (lane == 0) {                                                                              \
-			barrier_expect(&shared->w_full[team], MATRICES * KSTEPS * w_bytes);                   \
-			shared->armed_w[team] = (block) / BS + 1u;                                            \
-		}                                                                                             \
-		__syncwarp();                                                                                 \
-		if (lane < MATRICES * KSTEPS)                                                                 \
-			bulk_load(w_to, w_from + (uint64_t)(block) * KSTEPS * step_words * 4u, w_bytes,      \
-				  &shared->w_full[team]);                                                     \
-	} while (0)
+		const bool taken = g < groups; /* the CTA has this group */
+		unsigned char *const to_part = dynamic_shared + rings::weights_at + (m + g) * PREFILL_BLOCK + step * 4096u + lane * 4u;
+		const uint32_t *words_at =
+			reinterpret_cast<const uint32_t *>(MATRICES > 1u && m != 0u ? matrices[MATRICES - 1u] : matrices[0]) +
+			(uint64_t)(team * PREFILL_STEPS + step) * step_words +
+			(uint64_t)(first_group + g) * EXL3_GROUP_TILES * ring::words;
+		const uint64_t turn_words = (uint64_t)(PREFILL_TEAMS * PREFILL_STEPS) * step_words;
 		bool good = true;
-		if (member == 0u && team < blocks)
-			PREFILL_WORDS_COPY(team);
-		for (uint32_t block = team; block < blocks; block += 4u) {
-			const uint32_t use = block / BS;
-			if (use > 0u)
-				good = barrier_wait(&shared->b_free[team], (use - 1u) & 1u);
-			if (good)
-				good = barrier_wait(&shared->w_full[team], use & 1u);
-			if (!good)
-				break;
+		uint32_t words[EXL3_GROUP_TILES][2];
+		if (taken && team < blocks)
 #pragma unroll
-			for (uint32_t turn = 0; turn < units_a_warp; turn++) {
-				/* unit = (matrix m, group g, step) in that order of significance */
-				const uint32_t unit = member * units_a_warp + turn;
-				const uint32_t step = unit % KSTEPS, g = unit / KSTEPS % GROUPS, m = unit / (KSTEPS * GROUPS);
-				if (g >= groups)
+			for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++) {
+				words[tile][0] = __ldg(words_at + tile * ring::words + word_index);
+				words[tile][1] = __ldg(words_at + tile * ring::words + next_index);
+			}
+		for (uint32_t block = team; block < blocks; block += PREFILL_TEAMS) {
+			const uint32_t stage = block % S;
+			if (block + PREFILL_TEAMS < blocks)
+				words_at += turn_words; /* of the next turn; the last loads its own once more */
+			if (block >= S) {
+				good = warp_wait(&shared->free[stage], (block / S - 1u) & 1u);
+				if (!good)
+					break;
+			}
+			unsigned char *const to_stage = to_part + stage * rings::stage;
+#pragma unroll
+			for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++) {
+				if (!taken)
 					continue;
-				const uint32_t *const from =
-					words_at + (m * KSTEPS + step) * (w_chunk / 4u) + g * EXL3_GROUP_TILES * ring::words;
-				unsigned char *const to_unit = b_at + m * rings::b_block + step * 2u * rings::b_piece +
-							       g * EXL3_GROUP_TILES * 2u * 128u;
-#pragma unroll
-				for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++) {
-					uint32_t fragment[4];
-					exl3_decode_fragment<BX2>(from[tile * ring::words + word_index],
-								  from[tile * ring::words + next_index], shift, fragment);
-					/* fragment f: outputs 16 tile + g + 8 (f % 2), inputs 16 step + 2 t + 8 (f / 2): the warp's 32
-					 * words are the 128 bytes of one K piece of one group of eight outputs */
-					uint32_t *const to = reinterpret_cast<uint32_t *>(to_unit + tile * 2u * 128u);
-					to[0] = fragment[0];
-					to[128u / 4u] = fragment[1];
-					to[rings::b_piece / 4u] = fragment[2];
-					to[(rings::b_piece + 128u) / 4u] = fragment[3];
-				}
+				uint32_t fragment[4];
+				exl3_decode_fragment<BX2>(words[tile][0], words[tile][1], shift, fragment);
+				words[tile][0] = __ldg(words_at + tile * ring::words + word_index);
+				words[tile][1] = __ldg(words_at + tile * ring::words + next_index);
+				/* fragment f: outputs 16 tile + g + 8 (f % 2), inputs 16 step + 2 t + 8 (f / 2): the warp's 32
+				 * words are the 128 bytes of one K piece of one group of eight outputs */
+				uint32_t *const to = reinterpret_cast<uint32_t *>(to_stage + tile * 2u * 128u);
+				to[0] = fragment[0];
+				to[128u / 4u] = fragment[1];
+				to[2048u / 4u] = fragment[2];
+				to[(2048u + 128u) / 4u] = fragment[3];
 			}
 			asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 			__syncwarp();
 			if (lane == 0)
-				barrier_arrive(&shared->b_full[team]);
-			/* the stage's next use: its words may be overwritten once all four warps have read these */
-			if (member == 0u && block + 4u < blocks) {
-				good = barrier_wait(&shared->b_full[team], use & 1u);
-				if (!good)
-					break;
-				PREFILL_WORDS_COPY(block + 4u);
-			}
+				barrier_arrive(&shared->full[stage]);
 		}
-#undef PREFILL_WORDS_COPY
 		if (good)
 			good = barrier_wait(&shared->done, 0u);
 		if (!good)
@@ -553,64 +602,92 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 	}
 }
 
-/* `matrices` accumulator tiles (first columns first_column, first_column + column_stride, ...) into shared memory,
- * FP32 [matrix][128 rows][EXL3_PREFILL_STAGING_ROW]. A warp reads the 32 tensor-memory lanes of its quarter (warp % 4)
- * and one quarter of the columns. Decode warps only; ends with their barrier. */
-__device__ __forceinline__ void prefill_stage_out(uint32_t accumulators, uint32_t matrices, uint32_t first_column,
-						  uint32_t column_stride, float *staging)
+/* Begins a product CTA: barriers, tensor memory, and the pair's agreement on whether to run. All threads of both CTAs
+ * call; false: an earlier wait ran out, the pair is to go (the flag is never cleared while the kernel file stays loaded:
+ * later CTAs do not queue up behind the same fault, the host reads the flag and rejects the result). */
+__device__ __forceinline__ bool prefill_begin(prefill_shared *shared, uint32_t rank)
+{
+	const uint32_t warp = threadIdx.x / EXL3_WARP;
+	if (threadIdx.x == 0) {
+		for (uint32_t stage = 0; stage < EXL3_PREFILL_STAGES; stage++) {
+			/* the four warps of the team that decodes the stage, the rows' copies, at rank 0 the other CTA */
+			barrier_init(&shared->full[stage], rank == 0 ? 6u : 5u);
+			barrier_init(&shared->free[stage], 1);
+		}
+		barrier_init(&shared->done, 1);
+		shared->failed = 0;
+		shared->armed = 0;
+		shared->expired = *reinterpret_cast<volatile unsigned int *>(&exl3_wait_expired);
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	}
+	if (warp == 1) {
+		asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+				     smem_address(&shared->tensor_memory))
+			     : "memory");
+		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+	}
+	tensor_fence_before();
+	__syncthreads();
+	pair_sync();
+	tensor_fence_after();
+	uint32_t other;
+	asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(other) : "r"(pair_address(&shared->expired, rank ^ 1u)) : "memory");
+	return (shared->expired | other) == 0;
+}
+
+/* `sums` accumulators of one row tile (first columns first_column, + PREFILL_SUM_COLUMNS, ...) into shared memory, FP32
+ * [accumulator][row][EXL3_PREFILL_STAGING_ROW outputs]. A warp reads the 32 outputs of its quarter (warp % 4) and 32 of
+ * the `rows` rows. Decode warps only; ends with their barrier. */
+__device__ __forceinline__ void prefill_stage_out(uint32_t accumulators, uint32_t sums, uint32_t first_column, uint32_t rows,
+						  float *staging)
 {
 	const uint32_t lane = threadIdx.x % EXL3_WARP, warp = threadIdx.x / EXL3_WARP;
 	const uint32_t quarter = warp % 4u, column = (warp - PREFILL_FIRST_DECODE_WARP) / 4u * 32u;
 	__syncwarp();
-	for (uint32_t m = 0; m < matrices; m++) {
-		uint32_t r[32];
-		asm volatile(
-			"tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-			"{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,"
-			"%26,%27,%28,%29,%30,%31}, [%32];"
-			: "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-			  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-			  "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
-			  "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
-			  "=r"(r[30]), "=r"(r[31])
-			: "r"(accumulators + ((quarter * 32u) << 16) + first_column + m * column_stride + column)
-			: "memory");
-		asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-		uint4 *const to = reinterpret_cast<uint4 *>(
-			staging + ((uint64_t)m * EXL3_PREFILL_TILE_ROWS + quarter * 32u + lane) * EXL3_PREFILL_STAGING_ROW +
-			column);
+	if (column < rows)
+		for (uint32_t m = 0; m < sums; m++) {
+			uint32_t r[32];
+			asm volatile(
+				"tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+				"{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,"
+				"%26,%27,%28,%29,%30,%31}, [%32];"
+				: "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+				  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+				  "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
+				  "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
+				  "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+				: "r"(accumulators + ((quarter * 32u) << 16) + first_column + m * PREFILL_SUM_COLUMNS + column)
+				: "memory");
+			asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+			/* a lane an output: the 32 lanes of a row's store are 32 adjacent floats */
+			float *const to = staging + (m * EXL3_PREFILL_TILE_ROWS + column) * EXL3_PREFILL_STAGING_ROW + quarter * 32u + lane;
 #pragma unroll
-		for (uint32_t index = 0; index < 8; index++)
-			to[index] = make_uint4(r[4 * index], r[4 * index + 1], r[4 * index + 2], r[4 * index + 3]);
-	}
+			for (uint32_t index = 0; index < 32; index++)
+				to[index * EXL3_PREFILL_STAGING_ROW] = __uint_as_float(r[index]);
+		}
 	tensor_fence_before();
 	decode_sync();
 }
 
-/* All threads, at the end of a product CTA: wait (bounded) for what a failed CTA still has in flight, then free the
- * tensor memory. */
-template <uint32_t COLUMNS> __device__ __forceinline__ void prefill_release(prefill_shared *shared)
+/* All threads of both CTAs, at the end: wait (bounded) for what a failed CTA still has in flight, and for the other CTA,
+ * whose products read this one's shared memory, then free the tensor memory. */
+__device__ __forceinline__ void prefill_release(prefill_shared *shared)
 {
 	tensor_fence_before();
 	__syncthreads();
 	if (shared->failed != 0 && threadIdx.x == 0) {
-		for (uint32_t back = 0; back < EXL3_PREFILL_A_STAGES && back < shared->armed_a; back++) {
-			const uint32_t block = shared->armed_a - 1u - back;
-			(void)barrier_wait(&shared->a_full[block % EXL3_PREFILL_A_STAGES], (block / EXL3_PREFILL_A_STAGES) & 1u);
+		/* a stage whose other arrivals are missing holds this thread up to the bound, long past its copies' end */
+		for (uint32_t back = 0; back < EXL3_PREFILL_STAGES && back < shared->armed; back++) {
+			const uint32_t block = shared->armed - 1u - back;
+			(void)barrier_wait(&shared->full[block % EXL3_PREFILL_STAGES], (block / EXL3_PREFILL_STAGES) & 1u);
 		}
-		for (uint32_t team = 0; team < EXL3_PREFILL_B_STAGES; team++)
-			if (shared->armed_w[team] != 0)
-				(void)barrier_wait(&shared->w_full[team], (shared->armed_w[team] - 1u) & 1u);
-		if (shared->issued != 0)
-			(void)barrier_wait(&shared->done, 0u);
 	}
 	__syncthreads();
+	pair_sync();
 	if (threadIdx.x / EXL3_WARP == 1u) {
 		tensor_fence_after();
 		__syncwarp();
-		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(shared->tensor_memory),
-			     "r"(COLUMNS)
-			     : "memory");
+		asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(shared->tensor_memory) : "memory");
 	}
 }
 
@@ -635,28 +712,13 @@ __device__ __forceinline__ prefill_tile_view prefill_tile_of(const struct exl3_p
 	return out;
 }
 
-/* An expert's row tiles are taken two at a time: the CTAs of an even-numbered tile that has a successor also take the
- * successor's rows, so that every decoded weight is multiplied with 256 rows; the CTAs of an odd-numbered tile return. */
-#define PREFILL_SINGLE 0u
-#define PREFILL_FIRST_OF_TWO 1u
-#define PREFILL_SECOND_OF_TWO 2u
-__device__ __forceinline__ uint32_t prefill_pairing(const prefill_view &view, const struct exl3_prefill_tile &tile,
-						    uint32_t tile_index, uint32_t tile_count)
-{
-	if ((tile.first_entry / EXL3_PREFILL_TILE_ROWS) % 2u != 0u)
-		return PREFILL_SECOND_OF_TWO;
-	const struct exl3_prefill_tile *const tiles =
-		reinterpret_cast<const struct exl3_prefill_tile *>(view.workspace + view.parts.tiles);
-	return tile_index + 1u < tile_count && tiles[tile_index + 1u].expert == tile.expert ? PREFILL_FIRST_OF_TWO :
-											       PREFILL_SINGLE;
-}
-
 /* The gate/up epilogue of one row tile and one group of 128 outputs, from the staged accumulators (gate rows, then up
  * rows): Hadamard, scales, SwiGLU, down-side transform, FP16 down operand blocks. Decode warps; a warp a row. */
 template <uint32_t BX2>
 __device__ __forceinline__ void prefill_gate_up_rows(const struct exl3_prefill_record &record, unsigned char *arena,
 						     const prefill_view &view, const prefill_tile_view &tile,
-						     uint32_t tile_index, uint32_t group, const float *staging)
+						     uint32_t tile_index, uint32_t count, uint32_t group,
+						     const float *staging)
 {
 	const uint32_t H = record.input_size, I = prefill_inner_of(record, tile.tile.expert);
 	const uint32_t lane = threadIdx.x % EXL3_WARP, warp = threadIdx.x / EXL3_WARP;
@@ -666,10 +728,8 @@ __device__ __forceinline__ void prefill_gate_up_rows(const struct exl3_prefill_r
 	load_half4(reinterpret_cast<const __half *>(arena + tile.gate + codes) + H + channel, gate_scale);
 	load_half4(reinterpret_cast<const __half *>(arena + tile.up + codes) + H + channel, up_scale);
 	load_half4(reinterpret_cast<const __half *>(arena + tile.down + exl3_code_bytes(I, H, BX2)) + channel, down_scale);
-	unsigned char *const blocks = view.workspace + view.parts.down_operands +
-				      ((uint64_t)tile_index * (view.widest / EXL3_PREFILL_BLOCK_INPUTS) +
-				       channel / EXL3_PREFILL_BLOCK_INPUTS) *
-					      EXL3_PREFILL_BLOCK_BYTES;
+	const prefill_rows rows = prefill_rows_of(count, tile.tile.row_count, 1u, I);
+	unsigned char *const region = view.workspace + view.parts.down_operands + (uint64_t)tile_index * view.widest * 256u;
 	for (uint32_t row = warp - PREFILL_FIRST_DECODE_WARP; row < tile.tile.row_count; row += PREFILL_DECODE_WARPS) {
 		const float4 gate_raw = *reinterpret_cast<const float4 *>(staging + row * EXL3_PREFILL_STAGING_ROW + lane * 4u);
 		const float4 up_raw = *reinterpret_cast<const float4 *>(
@@ -687,89 +747,74 @@ __device__ __forceinline__ void prefill_gate_up_rows(const struct exl3_prefill_r
 #pragma unroll
 		for (uint32_t i = 0; i < 4; i++)
 			fed[i] = __fmul_rn(fed[i], EXL3_NORMALIZATION);
-		store_half4(reinterpret_cast<__half *>(blocks + prefill_block_byte(row, channel % EXL3_PREFILL_BLOCK_INPUTS)),
-			    fed);
+		store_half4(reinterpret_cast<__half *>(region + prefill_operand_byte(rows, 1u, 0u, row, channel)), fed);
 	}
 }
 
-/* TILES row tiles (tile_index, tile_index + 1) of one expert by GROUPS groups of 128 outputs from first_group */
-template <uint32_t BX2, uint32_t TILES, uint32_t GROUPS>
+/* gate and up of a unit's `count` row tiles (tile_index, + 1) by 256 outputs: this CTA's group is `group` */
+template <uint32_t BX2>
 __device__ __forceinline__ void prefill_gate_up(const struct exl3_prefill_record &record, unsigned char *arena,
-						const prefill_view &view, uint32_t tile_index, uint32_t first_group,
-						unsigned char *dynamic_shared, prefill_shared *shared)
+						const prefill_view &view, uint32_t tile_index, uint32_t count, uint32_t group,
+						uint32_t rank, unsigned char *dynamic_shared, prefill_shared *shared)
 {
-	typedef prefill_rings<2, EXL3_PREFILL_GATE_UP_STEPS, TILES, GROUPS> rings;
-	prefill_tile_view tiles[TILES];
-#pragma unroll
-	for (uint32_t tile = 0; tile < TILES; tile++)
-		tiles[tile] = prefill_tile_of(record, arena, view, tile_index + tile);
-	const uint32_t H = record.input_size, I = prefill_inner_of(record, tiles[0].tile.expert);
-	const uint32_t groups = min(GROUPS, I / EXL3_TRANSFORM - first_group);
-	const uint32_t warp = threadIdx.x / EXL3_WARP;
-	const unsigned char *const matrices[2] = { arena + tiles[0].gate, arena + tiles[0].up };
-	const uint64_t tile_bytes = (uint64_t)(H / EXL3_PREFILL_BLOCK_INPUTS) * EXL3_PREFILL_BLOCK_BYTES;
-	const unsigned char *operands[TILES * 2];
-#pragma unroll
-	for (uint32_t tile = 0; tile < TILES; tile++) {
-		operands[tile * 2u] = view.workspace + view.parts.gate_up_operands + (tile_index + tile) * tile_bytes;
-		operands[tile * 2u + 1u] = view.workspace + view.parts.gate_up_operands +
-					   ((uint64_t)view.parts.tile_capacity + tile_index + tile) * tile_bytes;
-	}
-	const bool complete = prefill_products<BX2, 2, EXL3_PREFILL_GATE_UP_STEPS, TILES, GROUPS>(
-		matrices, I, first_group, groups, operands, H / (EXL3_PREFILL_GATE_UP_STEPS * EXL3_TILE), dynamic_shared,
-		shared);
-	if (warp >= PREFILL_FIRST_DECODE_WARP && complete) {
+	const prefill_tile_view first = prefill_tile_of(record, arena, view, tile_index);
+	const uint32_t H = record.input_size, I = prefill_inner_of(record, first.tile.expert);
+	const uint32_t mine = group < I / EXL3_TRANSFORM ? 1u : 0u;
+	const unsigned char *const matrices[2] = { arena + first.gate, arena + first.up };
+	const prefill_rows rows = prefill_rows_of(count, first.tile.row_count, 2u, H);
+	const unsigned char *const row_runs = view.workspace + view.parts.gate_up_operands +
+					      (uint64_t)(tile_index + (count == 2u ? rank : 0u)) * H * 512u +
+					      (count == 2u ? 0u : rank * rows.second);
+	const bool complete = prefill_products<BX2, 2, 1>(matrices, I, group, mine, 1, row_runs, rows.half,
+							  H / (PREFILL_STEPS * EXL3_TILE), rank, dynamic_shared, shared);
+	if (threadIdx.x / EXL3_WARP >= PREFILL_FIRST_DECODE_WARP && complete && mine != 0) {
 		float *const staging = reinterpret_cast<float *>(dynamic_shared);
-		for (uint32_t tile = 0; tile < TILES; tile++)
-			for (uint32_t g = 0; g < groups; g++) {
-				prefill_stage_out(shared->tensor_memory, 2, rings::column(tile, 0, g), rings::column(0, 1, 0),
-						  staging);
-				prefill_gate_up_rows<BX2>(record, arena, view, tiles[tile], tile_index + tile, first_group + g,
-							  staging);
-				decode_sync(); /* the staging rows are read: the next tile may overwrite them */
-			}
+		for (uint32_t tile = 0; tile < count; tile++) {
+			const prefill_tile_view rows_of = prefill_tile_of(record, arena, view, tile_index + tile);
+			prefill_stage_out(shared->tensor_memory, 2, tile * EXL3_PREFILL_TILE_ROWS, rows_of.tile.row_count, staging);
+			prefill_gate_up_rows<BX2>(record, arena, view, rows_of, tile_index + tile, count, group, staging);
+			decode_sync(); /* the staging rows are read: the next tile may overwrite them */
+		}
 	}
-	prefill_release<rings::columns>(shared);
+	prefill_release(shared);
 }
 
-template <uint32_t BX2, uint32_t TILES, uint32_t KSTEPS>
+/* down of a unit's `count` row tiles by 512 outputs: this CTA's groups are first_group, + 1; `sums`: 2, or 1 where the
+ * last unit has no second group for either CTA */
+template <uint32_t BX2>
 __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &record, unsigned char *arena,
-					     const prefill_view &view, uint32_t tile_index, uint32_t first_group,
-					     unsigned char *dynamic_shared, prefill_shared *shared)
+					     const prefill_view &view, uint32_t tile_index, uint32_t count,
+					     uint32_t first_group, uint32_t sums, uint32_t rank, unsigned char *dynamic_shared,
+					     prefill_shared *shared)
 {
-	typedef prefill_rings<1, KSTEPS, TILES, PREFILL_GROUPS> rings;
-	prefill_tile_view tiles[TILES];
-#pragma unroll
-	for (uint32_t tile = 0; tile < TILES; tile++)
-		tiles[tile] = prefill_tile_of(record, arena, view, tile_index + tile);
-	const uint32_t H = record.input_size, I = prefill_inner_of(record, tiles[0].tile.expert);
-	const uint32_t groups = min(PREFILL_GROUPS, H / EXL3_TRANSFORM - first_group);
+	const prefill_tile_view first = prefill_tile_of(record, arena, view, tile_index);
+	const uint32_t H = record.input_size, I = prefill_inner_of(record, first.tile.expert);
+	const uint32_t groups = first_group < H / EXL3_TRANSFORM ? min(2u, H / EXL3_TRANSFORM - first_group) : 0u;
 	const uint32_t lane = threadIdx.x % EXL3_WARP, warp = threadIdx.x / EXL3_WARP;
-	const unsigned char *const matrices[1] = { arena + tiles[0].down };
-	const unsigned char *operands[TILES];
-#pragma unroll
-	for (uint32_t tile = 0; tile < TILES; tile++)
-		operands[tile] = view.workspace + view.parts.down_operands +
-				 (uint64_t)(tile_index + tile) * (view.widest / EXL3_PREFILL_BLOCK_INPUTS) *
-					 EXL3_PREFILL_BLOCK_BYTES;
-	const bool complete = prefill_products<BX2, 1, KSTEPS, TILES, PREFILL_GROUPS>(
-		matrices, H, first_group, groups, operands, I / (KSTEPS * EXL3_TILE), dynamic_shared, shared);
+	const unsigned char *const matrices[1] = { arena + first.down };
+	const prefill_rows rows = prefill_rows_of(count, first.tile.row_count, 1u, I);
+	const unsigned char *const row_runs = view.workspace + view.parts.down_operands +
+					      (uint64_t)(tile_index + (count == 2u ? rank : 0u)) * view.widest * 256u +
+					      (count == 2u ? 0u : rank * rows.second);
+	const bool complete = prefill_products<BX2, 1, 2>(matrices, H, first_group, groups, sums, row_runs, rows.half,
+							  I / (PREFILL_STEPS * EXL3_TILE), rank, dynamic_shared, shared);
 	if (warp >= PREFILL_FIRST_DECODE_WARP && complete) {
 		float *const staging = reinterpret_cast<float *>(dynamic_shared);
 		float *const outputs = reinterpret_cast<float *>(arena + record.pair_output_offset);
-		for (uint32_t tile = 0; tile < TILES; tile++)
+		for (uint32_t tile = 0; tile < count && groups != 0; tile++) {
+			const prefill_tile_view rows_of = prefill_tile_of(record, arena, view, tile_index + tile);
+			prefill_stage_out(shared->tensor_memory, groups, tile * EXL3_PREFILL_TILE_ROWS, rows_of.tile.row_count,
+					  staging);
 			for (uint32_t g = 0; g < groups; g++) {
-				prefill_stage_out(shared->tensor_memory, 1, rings::column(tile, 0, g), 0, staging);
 				const uint32_t channel = (first_group + g) * EXL3_TRANSFORM + lane * 4u;
 				float scale[4];
-				load_half4(reinterpret_cast<const __half *>(arena + tiles[tile].down + exl3_code_bytes(I, H, BX2)) +
-						   I + channel,
+				load_half4(reinterpret_cast<const __half *>(arena + first.down + exl3_code_bytes(I, H, BX2)) + I + channel,
 					   scale);
-				for (uint32_t row = warp - PREFILL_FIRST_DECODE_WARP; row < tiles[tile].tile.row_count;
+				for (uint32_t row = warp - PREFILL_FIRST_DECODE_WARP; row < rows_of.tile.row_count;
 				     row += PREFILL_DECODE_WARPS) {
-					const struct exl3_prefill_entry entry = tiles[tile].entries[row];
+					const struct exl3_prefill_entry entry = rows_of.entries[row];
 					const float4 raw = *reinterpret_cast<const float4 *>(
-						staging + row * EXL3_PREFILL_STAGING_ROW + lane * 4u);
+						staging + (g * EXL3_PREFILL_TILE_ROWS + row) * EXL3_PREFILL_STAGING_ROW + lane * 4u);
 					float v[4] = { raw.x, raw.y, raw.z, raw.w };
 					hadamard128_warp(v, lane);
 #pragma unroll
@@ -779,10 +824,11 @@ __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &r
 					*reinterpret_cast<float4 *>(outputs + (uint64_t)entry.pair * H + channel) =
 						make_float4(v[0], v[1], v[2], v[3]);
 				}
-				decode_sync();
 			}
+			decode_sync();
+		}
 	}
-	prefill_release<rings::columns>(shared);
+	prefill_release(shared);
 }
 
 #define PREFILL_WIDTH_SWITCH(call)                                                                     \
@@ -804,60 +850,57 @@ __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &r
 		call;                                                                                  \
 	} break;                                                                                       \
 	default:                                                                                       \
+		prefill_release(&shared);                                                           \
 		break;                                                                                 \
 	}
 
-/* grid (widest I / 128, tile capacity) x 576: a single row tile is taken by the CTAs of even x with two groups of 128
- * outputs each; two row tiles of one expert by every x with one group each (tensor memory holds 512 columns) */
-extern "C" __global__ void __launch_bounds__(EXL3_PREFILL_GEMM_THREADS, 1)
+/* grid (ceil(widest I / 256), tile capacity) CTA pairs x 576 */
+extern "C" __global__ void __cluster_dims__(PREFILL_PAIR, 1, 1) __launch_bounds__(EXL3_PREFILL_GEMM_THREADS, 1)
 	exl3_prefill_gate_up(struct exl3_prefill_record record, unsigned char *arena)
 {
 	extern __shared__ __align__(1024) unsigned char dynamic_shared[];
 	__shared__ prefill_shared shared;
 	const prefill_view view = prefill_view_of(record, arena);
 	const uint32_t tile_count = reinterpret_cast<const uint32_t *>(view.workspace + view.parts.counts)[view.experts];
-	/* once a wait has run out (the flag is never cleared while the kernel file stays loaded), later CTAs do not
-	 * queue up behind the same fault: the host reads the flag and rejects the result */
-	if (*reinterpret_cast<volatile unsigned int *>(&exl3_wait_expired) != 0u || blockIdx.y >= tile_count)
+	const uint32_t tile_index = blockIdx.y, rank = blockIdx.x % PREFILL_PAIR, first_group = blockIdx.x / PREFILL_PAIR * 2u;
+	if (tile_index >= tile_count)
 		return;
 	const struct exl3_prefill_tile tile =
-		reinterpret_cast<const struct exl3_prefill_tile *>(view.workspace + view.parts.tiles)[blockIdx.y];
-	const uint32_t pairing = prefill_pairing(view, tile, blockIdx.y, tile_count);
-	const uint32_t group_count = prefill_inner_of(record, tile.expert) / EXL3_TRANSFORM;
-	if (pairing == PREFILL_SECOND_OF_TWO || blockIdx.x >= group_count ||
-	    (pairing == PREFILL_SINGLE && blockIdx.x % PREFILL_GROUPS != 0u))
+		reinterpret_cast<const struct exl3_prefill_tile *>(view.workspace + view.parts.tiles)[tile_index];
+	const uint32_t count = prefill_tiles_of_unit(view, tile, tile_index, tile_count);
+	if (count == 0 || first_group >= prefill_inner_of(record, tile.expert) / EXL3_TRANSFORM)
 		return;
-	if (pairing == PREFILL_FIRST_OF_TWO) {
-		PREFILL_WIDTH_SWITCH((prefill_gate_up<BX2, 2, 1>(record, arena, view, blockIdx.y, blockIdx.x, dynamic_shared,
-								 &shared)))
-	} else {
-		PREFILL_WIDTH_SWITCH((prefill_gate_up<BX2, 1, PREFILL_GROUPS>(record, arena, view, blockIdx.y, blockIdx.x,
-									      dynamic_shared, &shared)))
+	if (!prefill_begin(&shared, rank)) {
+		prefill_release(&shared);
+		return;
 	}
+	PREFILL_WIDTH_SWITCH((prefill_gate_up<BX2>(record, arena, view, tile_index, count, first_group + rank, rank,
+						   dynamic_shared, &shared)))
 }
 
-/* grid (ceil(H / 256), tile capacity) x 576: two groups of 128 outputs a CTA, for one row tile or for two of one expert */
-extern "C" __global__ void __launch_bounds__(EXL3_PREFILL_GEMM_THREADS, 1)
+/* grid (ceil(H / 512), tile capacity) CTA pairs x 576 */
+extern "C" __global__ void __cluster_dims__(PREFILL_PAIR, 1, 1) __launch_bounds__(EXL3_PREFILL_GEMM_THREADS, 1)
 	exl3_prefill_down(struct exl3_prefill_record record, unsigned char *arena)
 {
 	extern __shared__ __align__(1024) unsigned char dynamic_shared[];
 	__shared__ prefill_shared shared;
 	const prefill_view view = prefill_view_of(record, arena);
 	const uint32_t tile_count = reinterpret_cast<const uint32_t *>(view.workspace + view.parts.counts)[view.experts];
-	if (*reinterpret_cast<volatile unsigned int *>(&exl3_wait_expired) != 0u || blockIdx.y >= tile_count)
+	const uint32_t tile_index = blockIdx.y, rank = blockIdx.x % PREFILL_PAIR, first_group = blockIdx.x / PREFILL_PAIR * 4u;
+	if (tile_index >= tile_count)
 		return;
 	const struct exl3_prefill_tile tile =
-		reinterpret_cast<const struct exl3_prefill_tile *>(view.workspace + view.parts.tiles)[blockIdx.y];
-	const uint32_t pairing = prefill_pairing(view, tile, blockIdx.y, tile_count);
-	if (pairing == PREFILL_SECOND_OF_TWO)
+		reinterpret_cast<const struct exl3_prefill_tile *>(view.workspace + view.parts.tiles)[tile_index];
+	const uint32_t count = prefill_tiles_of_unit(view, tile, tile_index, tile_count);
+	if (count == 0)
 		return;
-	if (pairing == PREFILL_FIRST_OF_TWO) {
-		PREFILL_WIDTH_SWITCH((prefill_down<BX2, 2, EXL3_PREFILL_GATE_UP_STEPS>(
-			record, arena, view, blockIdx.y, blockIdx.x * PREFILL_GROUPS, dynamic_shared, &shared)))
-	} else {
-		PREFILL_WIDTH_SWITCH((prefill_down<BX2, 1, EXL3_PREFILL_DOWN_STEPS>(
-			record, arena, view, blockIdx.y, blockIdx.x * PREFILL_GROUPS, dynamic_shared, &shared)))
+	if (!prefill_begin(&shared, rank)) {
+		prefill_release(&shared);
+		return;
 	}
+	PREFILL_WIDTH_SWITCH((prefill_down<BX2>(record, arena, view, tile_index, count, first_group + 2u * rank,
+						min(2u, record.input_size / EXL3_TRANSFORM - first_group), rank, dynamic_shared,
+						&shared)))
 }
 
 /* grid (ceil(H / 512), row capacity) x 128: FP32 row sums over the row's local pairs from +0 in ascending slot order,

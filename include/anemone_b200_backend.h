@@ -110,6 +110,7 @@ struct device_card; /* opaque to every caller */
  * node runs the launch behind the whole of the launch before it. The bit is set only in launches this library's own layer preparers write; the
  * reference's backend would refuse it as a branch it does not know. */
 #define LAUNCH_OVERLAPS_PREVIOUS 0x100u
+/* grid: blocks, or clusters for a kernel whose source names its cluster's dimensions (__cluster_dims__) */
 struct kernel_launch {
 	uint32_t kernel;
 	uint32_t grid[LAUNCH_DIMENSIONS];

@@ -674,17 +674,20 @@ struct router_select_b200_arguments {
  *                          ascending row order, and their count
  *   exl3_prefill_tiles     grid 1 x 1024: the tile table: (expert, first entry, rows) per 128-row tile, tile count
  *   exl3_prefill_operands  grid (tile capacity, 4 ceil(H / 512), 2) x 128: FP16 gate and up operands of every tile row
- *   exl3_prefill_gate_up   grid (max(I, shared I) / 128, tile capacity) x 576: both products, SwiGLU, FP16 down operands
- *   exl3_prefill_down      grid (ceil(H / 256), tile capacity) x 576: down product, output transform: FP32 pair outputs
+ *   exl3_prefill_gate_up   grid (ceil(max(I, shared I) / 256), tile capacity) pairs of CTAs x 576: both products, SwiGLU,
+ *                          FP16 down operands
+ *   exl3_prefill_down      grid (ceil(H / 512), tile capacity) pairs of CTAs x 576: down product, output transform: FP32
+ *                          pair outputs
  *   exl3_prefill_row_sum   grid (ceil(H / 512), rows) x 128: FP32 row sums over the row's LOCAL pairs, ascending slots
  *                          from +0
  * Workspace at workspace_offset, parts in this order, each aligned to 1024 bytes (exl3_prefill_sizes gives them):
  *   counts uint32 [local + shared + 1] (the last: tile count) | tiles struct exl3_prefill_tile [tile capacity] |
  *   entries struct exl3_prefill_entry [local + shared][row_capacity] |
- *   gate/up operands FP16 [2][tile capacity][H / 64][128 x 64 block] |
- *   down operands FP16 [tile capacity][max(I, shared I) / 64][block]
- * where a 128 x 64 block is stored as the tensor cores read it without swizzling: the 16 bytes of row r, inputs
- * 8 c .. 8 c + 7 lie at byte 2048 c + 128 (r / 8) + 16 (r % 8).
+ *   gate/up operands FP16, H * 512 bytes a tile | down operands FP16, max(I, shared I) * 256 bytes a tile
+ * stored as the tensor cores read them without swizzling, and so that what a CTA of a pair reads for 32 inputs is one
+ * run of bytes: [H / 32][gate, up][4 pieces of eight inputs][rows][16 bytes] (down: without the second part), the rows
+ * being the tile's 128, or, for an expert's last tile if its number is even (counted from 0), half its rows rounded up
+ * to whole sixteens, the other half's runs behind them.
  * tile capacity = ceil(row_capacity * (picks + shared) / 128) + local + shared; exl3_prefill_parts_of takes the local
  * expert count and the larger of the two intermediate widths.
  * Rows at or beyond step.row_count are not read and nothing is written for them; a pair output is written only for

@@ -304,3 +304,22 @@ def test_prefill_empty_and_full_calls(api, oracle):
         assert np.array_equal(again.view(np.uint32), first[:130].view(np.uint32))
     finally:
         card.close()
+
+
+@pytest.mark.parametrize("rows", [16, 17, 33, 128, 129, 161, 257, 385])
+def test_prefill_units_at_their_edges(api, oracle, rows):
+    """A unit of the products is one or two row tiles (halves of whole sixteens) by 256 outputs of gate and up or 512 of
+    down, a CTA half of them: an odd number of groups of 128 in both widths, every stored width, every row's tail. With two
+    picks of two experts and an always-on one, every expert sees every row."""
+    config = MoeConfig(hidden=640, inner=384, experts=2, shared=1, picks=2, row_capacity=rows)
+    for width in (2, 3, 4, 40):
+        widths, matrices, tokens, scores = make_inputs(500 + rows, config, rows, width)
+        experts, weights = moe_reference.route(oracle, config, scores)
+        expected = moe_reference.rank_partial(oracle, config, widths, matrices, tokens, experts, weights, 1, 0)[0]
+        layout = PrefillLayout(config, widths)
+        card = api.Card(0, layout.arena_bytes)
+        try:
+            got = PrefillLayer(card, config, widths, matrices).step(tokens, scores)
+        finally:
+            card.close()
+        assert np.abs(got - expected).max() <= MAX_ABS and cosine(got, expected) >= COSINE, width
