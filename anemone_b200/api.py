@@ -94,6 +94,7 @@ def library():
                                                   C.c_uint64, C.c_uint64, C.c_void_p, C.c_uint64,
                                                   C.POINTER(C.c_uint32)]
         lib.backend_b200_graph_run_wait.argtypes = [_card, C.c_uint32]
+        lib.backend_b200_step_pieces.argtypes = [_card, C.POINTER(R.StepPiece), C.c_uint32]
         lib.backend_b200_step_call.argtypes = [_card, C.c_uint32, C.POINTER(R.HostRange), C.c_uint32,
                                                C.POINTER(R.HostRange), C.c_uint32, C.c_void_p, C.c_uint64]
         lib.backend_b200_ipc_export.argtypes = [_card, C.c_char_p]
@@ -309,6 +310,17 @@ class Card:
                                               output_offset,
                                               C.c_void_p(self.staging.value + output_staging_offset), output_bytes),
               "step_run")
+
+    def step_pieces(self, pieces):
+        """One call in pieces (backend_b200_step_pieces): pieces: (graph, inputs, outputs), inputs and outputs up to two
+        (arena offset, staging offset, bytes) each."""
+        table = (R.StepPiece * len(pieces))()
+        for piece, (graph, inputs, outputs) in zip(table, pieces):
+            piece.graph, piece.input_count, piece.output_count = graph, len(inputs), len(outputs)
+            for ranges, given in ((piece.inputs, inputs), (piece.outputs, outputs)):
+                for index, (offset, staging_offset, nbytes) in enumerate(given):
+                    ranges[index] = R.HostRange(offset, self.staging.value + staging_offset, nbytes)
+        check(library().backend_b200_step_pieces(self.handle, table, len(table)), "step_pieces")
 
     def step_capture(self, launches, input_offset, input_staging_offset, input_bytes, output_offset,
                      output_staging_offset, output_bytes):

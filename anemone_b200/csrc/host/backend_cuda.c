@@ -68,7 +68,8 @@ struct device_card {
 	int threads_most;
 	CUmodule modules[CARD_MODULES_MOST]; /* by image index, loaded at first kernel_prepare of the file */
 	CUdeviceptr wait_words[CARD_MODULES_MOST]; /* the module's exl3_wait_expired; 0: it has none */
-	CUevent piece_events[AB_COPY_BATCH_MOST]; /* of a step call's pieces on their way out */
+	CUevent piece_events[AB_COPY_BATCH_MOST]; /* of a step call's pieces on their way out, or between the streams below */
+	CUstream in_stream, out_stream; /* of backend_b200_step_pieces: the copies beside the card's stream */
 	struct prepared_kernel kernels[BACKEND_MAXIMUM_KERNELS];
 	uint32_t kernel_count;
 	CUgraphExec graphs[BACKEND_MAXIMUM_GRAPHS];
@@ -237,6 +238,10 @@ static void card_release(const struct ab_driver *cu, struct device_card *card)
 		for (uint32_t piece = 0; piece < AB_COPY_BATCH_MOST; piece++)
 			if (card->piece_events[piece] != NULL)
 				(void)cu->cuEventDestroy(card->piece_events[piece]);
+		if (card->in_stream != NULL)
+			(void)cu->cuStreamDestroy(card->in_stream);
+		if (card->out_stream != NULL)
+			(void)cu->cuStreamDestroy(card->out_stream);
 		if (card->measure_begin_event != NULL)
 			(void)cu->cuEventDestroy(card->measure_begin_event);
 		if (card->measure_end_event != NULL)
@@ -1688,6 +1693,78 @@ result_status backend_b200_step_call(struct device_card *card, uint32_t graph,
 done:
 	if (begun)
 		ab_copy_batch_end(&batch);
+	CARD_LEAVE(card);
+}
+
+static bool piece_ranges_are_valid(const struct device_card *card, const struct backend_b200_host_range *ranges,
+				   uint32_t count)
+{
+	if (count > BACKEND_B200_PIECE_RANGES_MOST)
+		return false;
+	for (uint32_t range = 0; range < count; range++)
+		if (ranges[range].memory == NULL || ranges[range].byte_count == 0 ||
+		    !range_inside(ranges[range].arena_offset, ranges[range].byte_count, card->arena_byte_count) ||
+		    !inside_one_staging_block(ranges[range].memory, ranges[range].byte_count))
+			return false;
+	return true;
+}
+
+result_status backend_b200_step_pieces(struct device_card *card, const struct backend_b200_step_piece *pieces,
+				       uint32_t piece_count)
+{
+	if (card == NULL || pieces == NULL || piece_count == 0 || piece_count > BACKEND_B200_PIECES_MOST)
+		return STATUS_INVALID_ARGUMENT;
+	for (uint32_t piece = 0; piece < piece_count; piece++)
+		if (pieces[piece].reserved_zero != 0 ||
+		    !piece_ranges_are_valid(card, pieces[piece].inputs, pieces[piece].input_count) ||
+		    !piece_ranges_are_valid(card, pieces[piece].outputs, pieces[piece].output_count))
+			return STATUS_INVALID_ARGUMENT;
+	CARD_ENTER(card);
+	bool queued = false;
+	if (card->failed) {
+		status = STATUS_DEVICE_ERROR;
+		goto done;
+	}
+	for (uint32_t piece = 0; piece < piece_count; piece++)
+		if (pieces[piece].graph >= card->graph_count) {
+			status = STATUS_INVALID_ARGUMENT;
+			goto done;
+		}
+	if (card->in_stream == NULL)
+		DRIVER(card, cuStreamCreate(&card->in_stream, CU_STREAM_NON_BLOCKING));
+	if (card->out_stream == NULL)
+		DRIVER(card, cuStreamCreate(&card->out_stream, CU_STREAM_NON_BLOCKING));
+	for (uint32_t event = 0; event < 1u + 2u * piece_count; event++)
+		if (card->piece_events[event] == NULL)
+			DRIVER(card, cuEventCreate(&card->piece_events[event], CU_EVENT_DISABLE_TIMING));
+	queued = true;
+	DRIVER(card, cuEventRecord(card->piece_events[0], card->stream));
+	DRIVER(card, cuStreamWaitEvent(card->in_stream, card->piece_events[0], 0));
+	for (uint32_t piece = 0; piece < piece_count; piece++) {
+		const struct backend_b200_step_piece *const step = &pieces[piece];
+		const CUevent arrived = card->piece_events[1u + 2u * piece], computed = card->piece_events[2u + 2u * piece];
+		for (uint32_t range = 0; range < step->input_count; range++)
+			DRIVER(card, cuMemcpyHtoDAsync(card->arena + step->inputs[range].arena_offset,
+						       step->inputs[range].memory, step->inputs[range].byte_count,
+						       card->in_stream));
+		DRIVER(card, cuEventRecord(arrived, card->in_stream));
+		DRIVER(card, cuStreamWaitEvent(card->stream, arrived, 0));
+		DRIVER(card, cuGraphLaunch(card->graphs[step->graph], card->stream));
+		card->launches_queued += card->graph_kernel_nodes[step->graph];
+		DRIVER(card, cuEventRecord(computed, card->stream));
+		DRIVER(card, cuStreamWaitEvent(card->out_stream, computed, 0));
+		for (uint32_t range = 0; range < step->output_count; range++)
+			DRIVER(card, cuMemcpyDtoHAsync(step->outputs[range].memory,
+						       card->arena + step->outputs[range].arena_offset,
+						       step->outputs[range].byte_count, card->out_stream));
+	}
+	DRIVER(card, cuStreamSynchronize(card->out_stream)); /* behind the last graph, and that behind the last copy in */
+	queued = false;
+done:
+	if (queued) { /* the caller's memory is not read or written after the call */
+		(void)cu->cuStreamSynchronize(card->in_stream);
+		(void)cu->cuStreamSynchronize(card->out_stream);
+	}
 	CARD_LEAVE(card);
 }
 

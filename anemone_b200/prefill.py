@@ -22,6 +22,33 @@ from . import synthetic
 from .moe import LINE, SIGNAL_BYTES, rank_columns
 
 
+PIECE_ROWS = 128  # a staged call's pieces begin on whole row tiles
+STEP_SPACE = 48  # a piece's step block and its status, behind the call's own in the 256 bytes of the step's space
+PCIE_BYTES, WEIGHT_RATE = 53e9, 2.4e12  # a second: measured copies; weights decoded and multiplied with up to 256 rows
+PIECE_SECONDS = 1e-4  # routing, grouping, the reduction and the gaps between their launches, whatever the rows
+
+
+def call_pieces(config, share, rank_count):
+    """In how many pieces a staged call takes its rows: 1, 2 or 4, by an estimate of the call's time. More pieces hide more
+    of the copies, but each decodes every expert's weights again, so few rows of many experts stay whole. 4096 rows of
+    H 4096, I 2048 on 32 of 256 experts: 1.35 ms of copies, 0.5 of products; two pieces. All 256: 3.5 ms of products
+    against 5 in two pieces; one. The ranks of a reduction must agree: theirs is the largest share of equal ones."""
+    rows, H = config.row_capacity, config.hidden
+    if rank_count > 1:
+        matrices, pairs = -(-config.experts // rank_count), config.picks / rank_count
+        inner, always_on = config.inner, config.shared * config.inner / rank_count
+    else:
+        matrices, pairs, inner = share.local_count, config.picks * share.local_count / config.experts, share.inner
+        always_on = share.shared_count(config) * share.shared_inner
+    taken, returned = rows * (H * 2 + config.experts * 4) / PCIE_BYTES, rows * H * 2 / PCIE_BYTES
+
+    def estimate(count):
+        weights = 3 * H * (inner * (count * matrices + rows * pairs / 256) + always_on * (count + rows / 256))
+        hidden = (count - 1) / count
+        return taken / count + max(count * PIECE_SECONDS + weights / WEIGHT_RATE, taken * hidden, returned * hidden) + returned / count
+    return min((count for count in (1, 2, 4) if rows >= 2 * PIECE_ROWS * count), key=estimate, default=1)
+
+
 @dataclass
 class Share:
     """What one rank holds of the layer's experts."""
@@ -143,31 +170,48 @@ class PrefillLayer:
         for peer in range(rank_count):
             peers[peer].region_offset = L.region
         card.upload(L.peer_table, np.frombuffer(bytes(peers), dtype=np.uint8))
-        c = config
-        self.record = R.Exl3Prefill(L.scores, L.tokens, L.expert_table, L.widths, L.picks, L.weights, L.workspace,
-                                    L.pair_outputs, L.row_output, L.step, c.hidden, share.inner, share.shared_inner,
-                                    c.experts, share.local_first, share.local_count, L.shared_count, c.picks,
-                                    c.row_capacity, c.scoring, c.route_scale, c.activation_limit)
-        self.launches = (R.KernelLaunch * 7)()
-        api.check(api.library().exl3_prefill_prepare(C.byref(self.record), card.arena_bytes, card.ops_pointer,
-                                                     card.handle, self.launches), "exl3_prefill_prepare")
         lib = api.library()
-        reduce = R.OrderedReduceBf16Description()
-        reduce.reduce.collective = R.OrderedCollective(L.peer_table, L.region, L.slot_input, L.result, 0, L.step,
-                                                       L.parity_stride, c.deadline_cycles, c.row_capacity * c.hidden,
-                                                       rank_count, rank, 0)
-        reduce.reduce.status_offset, reduce.reduce.width, reduce.reduce.mode = L.status, c.hidden, reduce_mode
-        # the rows are already summed over the pairs: one "pair" a row
-        reduce.pair_output_offset, reduce.arena_byte_count = L.row_output, card.arena_bytes
-        reduce.pairs_per_row, reduce.row_capacity = 1, c.row_capacity
         lib.ordered_reduce_bf16_prepare.argtypes = [C.POINTER(R.OrderedReduceBf16Description),
                                                     C.POINTER(api.BackendOperations), C.c_void_p,
                                                     C.POINTER(R.KernelLaunch)]
-        self.reduce_launches = (R.KernelLaunch * 2)()
-        api.check(lib.ordered_reduce_bf16_prepare(C.byref(reduce), card.ops_pointer, card.handle,
-                                                  self.reduce_launches), "ordered_reduce_bf16_prepare")
+        self.reduce_mode = reduce_mode
+        self.record, self.launches, self.reduce_launches = self._prepare(0, config.row_capacity, 0)
         self.graph = card.graph(list(self.launches) + list(self.reduce_launches))
         self.sequence = 0
+        # a staged call's pieces: (first row, rows, graph)
+        count = call_pieces(config, share, rank_count)
+        bounds = [config.row_capacity * piece // count // PIECE_ROWS * PIECE_ROWS for piece in range(count)]
+        bounds.append(config.row_capacity)
+        self.pieces = []
+        for piece in range(count if count > 1 else 0):
+            _, launches, reduce = self._prepare(bounds[piece], bounds[piece + 1] - bounds[piece], (piece + 1) * STEP_SPACE)
+            self.pieces.append((bounds[piece], bounds[piece + 1] - bounds[piece],
+                                card.graph(list(launches) + list(reduce))))
+
+    def _prepare(self, first, rows, step_at):
+        """The launches for rows first .. first + rows - 1 of the arrays, with the step block at `step_at` of its space."""
+        L, c, card, lib, share = self.layout, self.config, self.card, api.library(), self.layout.share
+        H, step = c.hidden, L.step + step_at
+        record = R.Exl3Prefill(L.scores + first * c.experts * 4, L.tokens + first * H * 2, L.expert_table, L.widths,
+                               L.picks + first * c.picks * 4, L.weights + first * c.picks * 4, L.workspace,
+                               L.pair_outputs + first * L.pairs_per_row * H * 4, L.row_output + first * H * 4, step, H,
+                               share.inner, share.shared_inner, c.experts, share.local_first, share.local_count,
+                               L.shared_count, c.picks, rows, c.scoring, c.route_scale, c.activation_limit)
+        launches = (R.KernelLaunch * 7)()
+        api.check(lib.exl3_prefill_prepare(C.byref(record), card.arena_bytes, card.ops_pointer, card.handle, launches),
+                  "exl3_prefill_prepare")
+        reduce = R.OrderedReduceBf16Description()
+        reduce.reduce.collective = R.OrderedCollective(L.peer_table, L.region, L.slot_input, L.result + first * H * 2, 0,
+                                                       step, L.parity_stride, c.deadline_cycles, rows * H,
+                                                       self.rank_count, self.rank, 0)
+        reduce.reduce.status_offset, reduce.reduce.width, reduce.reduce.mode = L.status, H, self.reduce_mode
+        # the rows are already summed over the pairs: one "pair" a row
+        reduce.pair_output_offset, reduce.arena_byte_count = L.row_output + first * H * 4, card.arena_bytes
+        reduce.pairs_per_row, reduce.row_capacity = 1, rows
+        reduce_launches = (R.KernelLaunch * 2)()
+        api.check(lib.ordered_reduce_bf16_prepare(C.byref(reduce), card.ops_pointer, card.handle, reduce_launches),
+                  "ordered_reduce_bf16_prepare")
+        return record, launches, reduce_launches
 
     def connect_local(self, layers):
         """All ranks in this process: peer_connect every card to every card."""
@@ -213,17 +257,47 @@ class PrefillLayer:
         """One whole call on staged inputs in ONE library call: inputs in, the graph, status block and bfloat16 result
         out, wait. Returns the result as a view of the staging block (bfloat16 bits [rows][hidden])."""
         L, card, rows = self.layout, self.card, self.config.row_capacity
+        if self.pieces:
+            return self._call_pieces(staging_offset, result_staging_offset)
         self.sequence += 1
         block = R.StepBlock(self.sequence, rows, 0)
         card.staging_view[staging_offset:staging_offset + 16] = np.frombuffer(bytes(block), dtype=np.uint8)
         nbytes = rows * self.config.hidden * 2
         card.step_run(self.graph, L.step, staging_offset, L.input_bytes, L.status, result_staging_offset, 16 + nbytes)
-        status = card.staging_view[result_staging_offset:result_staging_offset + 16].view(np.uint32)
-        if status[0] != 0:
-            raise RuntimeError("ordered reduction failed: code %d (1 timed out, 2 bad sequence), phase %d, rank %d"
-                               % (status[0], status[1], status[2]))
-        return card.staging_view[result_staging_offset + 16:result_staging_offset + 16 + nbytes].view(
-            np.uint16).reshape(rows, self.config.hidden)
+        return self._staged_result([result_staging_offset], result_staging_offset)
+
+    def _call_pieces(self, staging_offset, result_at):
+        """call in pieces of the rows: while one is computed the next one's inputs and the last one's results cross PCIe."""
+        L, c, view = self.layout, self.config, self.card.staging_view
+        token_bytes, score_bytes = c.hidden * 2, c.experts * 4
+        tokens_at, scores_at = staging_offset + (L.tokens - L.step), staging_offset + (L.scores - L.step)
+        pieces, statuses = [], []
+        for piece, (first, rows, graph) in enumerate(self.pieces):
+            self.sequence += 1
+            space = (piece + 1) * STEP_SPACE
+            view[staging_offset + space:staging_offset + space + 16] = np.frombuffer(
+                bytes(R.StepBlock(self.sequence, rows, 0)), dtype=np.uint8)
+            # the step blocks of all pieces stand in front of the first one's tokens
+            begin = tokens_at + first * token_bytes if piece else staging_offset
+            inputs = [(L.step + begin - staging_offset, begin, tokens_at + (first + rows) * token_bytes - begin),
+                      (L.scores + first * score_bytes, scores_at + first * score_bytes, rows * score_bytes)]
+            # a piece's status returns to a place of its own, behind the step block it has used
+            statuses.append(staging_offset + space + 16)
+            outputs = [(L.status, statuses[-1], 16),
+                       (L.result + first * token_bytes, result_at + 16 + first * token_bytes, rows * token_bytes)]
+            pieces.append((graph, inputs, outputs))
+        self.card.step_pieces(pieces)
+        view[result_at:result_at + 16] = view[statuses[-1]:statuses[-1] + 16]
+        return self._staged_result(statuses, result_at)
+
+    def _staged_result(self, statuses, result_at):
+        view, rows, hidden = self.card.staging_view, self.config.row_capacity, self.config.hidden
+        for at in statuses:
+            status = view[at:at + 16].view(np.uint32)
+            if status[0] != 0:
+                raise RuntimeError("ordered reduction failed: code %d (1 timed out, 2 bad sequence), phase %d, rank %d"
+                                   % (status[0], status[1], status[2]))
+        return view[result_at + 16:result_at + 16 + rows * hidden * 2].view(np.uint16).reshape(rows, hidden)
 
     def rows(self, count):
         """FP32 [count][hidden] row sums of the last run. Raises if a CTA gave up a bounded wait."""

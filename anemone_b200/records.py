@@ -392,6 +392,11 @@ class HostRange(C.Structure):
     _fields_ = [("arena_offset", C.c_uint64), ("memory", C.c_void_p), ("byte_count", C.c_uint64)]
 
 
+class StepPiece(C.Structure):
+    _fields_ = [("graph", C.c_uint32), ("input_count", C.c_uint32), ("output_count", C.c_uint32),
+                ("reserved_zero", C.c_uint32), ("inputs", HostRange * 2), ("outputs", HostRange * 2)]
+
+
 class ExchangePlace(C.Structure):
     _fields_ = [("address_word_offset", C.c_uint64), ("offset", C.c_uint64)]
 

@@ -282,6 +282,18 @@ MUST_CHECK result_status backend_b200_step_call(struct device_card *card, uint32
 						const struct backend_b200_host_range *inputs, uint32_t input_count,
 						const struct backend_b200_host_range *outputs, uint32_t output_count,
 						void *page_locked, uint64_t page_locked_byte_count);
+/* One call on page-locked memory whose work comes in pieces: piece by piece the copies in, the graph and the copies out,
+ * on a stream each, so that a piece's graph runs while the next piece's inputs and the last one's outputs cross PCIe;
+ * returns when all of it is done. What is queued on the card before comes first. A range's memory lies inside one staging
+ * block; inputs of a piece must not be what an earlier piece's graph still reads. STATUS_INVALID_ARGUMENT otherwise. */
+#define BACKEND_B200_PIECES_MOST 8u
+#define BACKEND_B200_PIECE_RANGES_MOST 2u
+struct backend_b200_step_piece {
+	uint32_t graph, input_count, output_count, reserved_zero;
+	struct backend_b200_host_range inputs[BACKEND_B200_PIECE_RANGES_MOST], outputs[BACKEND_B200_PIECE_RANGES_MOST];
+};
+MUST_CHECK result_status backend_b200_step_pieces(struct device_card *card, const struct backend_b200_step_piece *pieces,
+						  uint32_t piece_count);
 /* Kernel launches this card has queued since it was opened, graph launches counted by their kernel nodes. */
 /* The dependencies graph_capture gives every launch of a table (order_out[launch_count]), from the branches alone: no
  * card is needed. STATUS_INVALID_ARGUMENT for a NULL, an empty table, a branch that is none of LAUNCH_* or a table

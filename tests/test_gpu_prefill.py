@@ -4,6 +4,7 @@ grouping tables checked for their invariants, and the decode launches on the sam
 import numpy as np
 import pytest
 
+from anemone_b200 import prefill
 from anemone_b200 import records as R
 from anemone_b200 import synthetic
 from anemone_b200.moe import MoeConfig, MoeLayer, MoeLayout
@@ -323,3 +324,36 @@ def test_prefill_units_at_their_edges(api, oracle, rows):
         finally:
             card.close()
         assert np.abs(got - expected).max() <= MAX_ABS and cosine(got, expected) >= COSINE, width
+
+
+@pytest.mark.parametrize("rows,count", [(519, 2), (1100, 4)])
+def test_staged_call_in_pieces(api, monkeypatch, rows, count):
+    """A staged call that takes its rows in pieces (beside the copies) against the whole: the same bits, call after call,
+    with a call of the other form in between, and the tail rows in the last piece."""
+    config = MoeConfig(hidden=512, inner=128, experts=16, shared=1, picks=2, row_capacity=rows)
+    widths, matrices, tokens, scores = make_inputs(rows, config, rows)
+    monkeypatch.setattr(prefill, "call_pieces", lambda *_: count)
+    layout = PrefillLayout(config, widths)
+    card = api.Card(0, layout.arena_bytes)
+    try:
+        layer = PrefillLayer(card, config, widths, matrices)
+        layer.connect_local([layer])
+        card.wait()
+        assert len(layer.pieces) == count
+        result_at = api.align(layout.input_bytes, 4096)
+        for turn in range(3):
+            given, turned = np.roll(tokens, turn, axis=0), np.roll(scores, turn, axis=0)
+            layer.stage(0, given, turned)
+            staged = layer.call(0, result_at).copy()
+            sums = layer.rows(rows)
+            layer.load(given, turned)
+            layer.run()
+            assert np.array_equal(layer.result(rows), staged) and np.array_equal(layer.rows(rows), sums)
+        with pytest.raises(api.StatusError):
+            card.step_pieces([])
+        with pytest.raises(api.StatusError):
+            card.step_pieces([(1 << 20, [], [])])
+        with pytest.raises(api.StatusError):
+            card.step_pieces([(layer.graph, [(card.arena_bytes, 0, 16)], [])])
+    finally:
+        card.close()
