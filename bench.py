@@ -51,11 +51,11 @@ SEED = 20261125
 # one ncu capture of a 64-expert, 8-row launch over that launch's algorithmic bytes (the capture is too large for the
 # full workload; traffic grows in proportion to the experts streamed)
 GATE_UP_TRAFFIC_RATIO = 1.03
-# the same for the prefill's gate/up products (one capture at 32 experts and 1024 rows: 401.3 MB read and 45.0 MB
-# written against 444 MB of codes, scales, operand blocks read and down operand blocks written) and for the
-# original-weights gate/up products (one capture of the mma.sync launch at 64 experts: 360.1 MB against 356.8 MB)
-PREFILL_TRAFFIC_RATIO = 1.00
-MX_GATE_UP_TRAFFIC_RATIO = 1.01
+# the same for the prefill's gate/up products (one capture at 32 experts and 1024 rows: 378.0 MB read and 27.0 MB
+# written against 418.8 MB of codes, scales, operands read and down operands written, some of which stay in L2) and for
+# the original-weights gate/up products (one capture at 64 experts: 427.1 MB against 427.0 MB)
+PREFILL_TRAFFIC_RATIO = 0.97
+MX_GATE_UP_TRAFFIC_RATIO = 1.00
 
 
 def parse():
@@ -269,13 +269,15 @@ def run_prefill(args, api, base, widths, draw, rank, world, local_rank, dist, ba
                     for local, expert in enumerate(held))
         peak, source = measured_tensor_peak()
         achieved = flops / us / 1e6  # TFLOP/s
-        # bytes of the launch: gate and up of every expert that has a row; a row tile's operand blocks of both in, its
-        # down operand blocks out (whole tiles of 128 rows move, filled or not)
+        # bytes of the launch: gate and up of every expert that has a row; a row tile's operands of both in, its down
+        # operands out (whole tiles of 128 rows move, filled or not, but of an odd last one whole thirty-twos)
         tiles_of = [(int(counts[local]) + 127) // 128 for local in range(len(held))]
+        moved = [(tiles - tiles % 2) * 128 + tiles % 2 * ((int(counts[local]) - (tiles - 1) * 128 + 31) // 32 * 32)
+                 for local, tiles in enumerate(tiles_of)]
         byte_total = sum((2 * synthetic.matrix_bytes(config.hidden, share.inner if expert < config.experts else
                                                      share.shared_inner, int(widths[expert])) if tiles else 0) +
-                         tiles * 128 * (2 * config.hidden * 2 +
-                                        (share.inner if expert < config.experts else share.shared_inner) * 2)
+                         moved[local] * (2 * config.hidden * 2 +
+                                         (share.inner if expert < config.experts else share.shared_inner) * 2)
                          for (local, expert), tiles in zip(enumerate(held), tiles_of))
         roofline = {"kernel": "exl3_prefill_gate_up", "bound": "tensor", "achieved": achieved, "peak": peak,
                     "unit": "TFLOP/s", "frac": achieved / peak, "peak_source": source,
