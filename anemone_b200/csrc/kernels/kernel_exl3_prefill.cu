@@ -301,7 +301,9 @@ extern "C" __global__ void __launch_bounds__(EXL3_TRANSFORM_THREADS)
  * 128 bytes a cycle for the instructions alone, all there is, and takes every row's operands from L2 twice as often.
  * The rows' number is the instruction's N, so a last tile of few rows costs the tensor cores little; the decode is the
  * same for any. 4096 rows of H 4096, I 2048, 256 experts of 8: gate/up 2202 us with single CTAs, 1880 so; down 1211,
- * 1137. Bound by issue: the decode of a stage alone is about 500 cycles of its 600. */
+ * 1137. Neither end is full (1024 rows of 32 experts: 67 % of the issue slots, the tensor cores 43 % of the cycles): a
+ * stage's turn in the ring, about 600 cycles of which the products take 512 at most, and a unit's beginning and epilogue,
+ * a sixth of gate/up and a quarter of down, lie between them. */
 #define PREFILL_PAIR 2u /* CTAs of a unit */
 #define PREFILL_SUM_COLUMNS 256u /* tensor-memory columns of one accumulator: a row a column */
 
