@@ -24,7 +24,7 @@
 #define POLL_NANOSECONDS 20000l
 #define POLL_SPIN_NANOSECONDS 200000ull
 #define SMALL_WRITE_SLOTS 64u
-#define STEP_WORDS 16u /* 64-bit words a graph: a line of 128 bytes of its own */
+#define STEP_WORDS 16u /* 64-bit words a graph: a line of 128 bytes of its own, the first one used */
 #define STEP_COPY_BLOCKS 64u
 #define CALL_PIECE_BYTES (1u << 19) /* 10 us of PCIe, 30 of a core's copy */
 #define STEP_SPIN_NANOSECONDS 2000000ull /* a step's wait looks at its word alone for so long */
@@ -75,8 +75,8 @@ struct device_card {
 	CUgraphExec graphs[BACKEND_MAXIMUM_GRAPHS];
 	uint32_t graph_kernel_nodes[BACKEND_MAXIMUM_GRAPHS];
 	bool graph_reports[BACKEND_MAXIMUM_GRAPHS]; /* its copy out stores the run's number in step_words */
-	volatile uint64_t *step_words; /* page-locked: [graph]: the run's number, the number its copy out stored */
-	uint64_t step_ticket;
+	uint64_t graph_runs[BACKEND_MAXIMUM_GRAPHS]; /* queued so far; the copy out counts the same runs on the card */
+	volatile uint64_t *step_words; /* page-locked: [graph]: the number of its last run whose outputs are in place */
 	uint32_t graph_count;
 	CUevent marks[BACKEND_MAXIMUM_MARKS];
 	bool mark_set[BACKEND_MAXIMUM_MARKS];
@@ -1104,20 +1104,28 @@ done:
 	CARD_LEAVE(card);
 }
 
+/* Queue one run of a graph on the card's stream: every run is counted. Context current, mutex held. */
+static result_status graph_queue(const struct ab_driver *cu, struct device_card *card, uint32_t graph)
+{
+	result_status status = STATUS_OK;
+	DRIVER(card, cuGraphLaunch(card->graphs[graph], card->stream));
+	card->launches_queued += card->graph_kernel_nodes[graph];
+	card->graph_runs[graph]++;
+done:
+	return status;
+}
+
 static result_status cuda_graph_run(struct device_card *card, uint32_t graph)
 {
 	if (card == NULL)
 		return STATUS_INVALID_ARGUMENT;
 	CARD_ENTER(card);
-	if (card->failed) {
+	if (card->failed)
 		status = STATUS_DEVICE_ERROR;
-	} else if (graph >= card->graph_count) {
+	else if (graph >= card->graph_count)
 		status = STATUS_INVALID_ARGUMENT;
-	} else {
-		DRIVER(card, cuGraphLaunch(card->graphs[graph], card->stream));
-		card->launches_queued += card->graph_kernel_nodes[graph];
-	}
-done:
+	else
+		status = graph_queue(cu, card, graph);
 	CARD_LEAVE(card);
 }
 
@@ -1402,8 +1410,9 @@ result_status backend_b200_step_run(struct device_card *card, uint32_t graph, ui
 	if (input_byte_count != 0)
 		DRIVER(card, cuMemcpyHtoDAsync(card->arena + input_arena_offset, page_locked_input, input_byte_count,
 					       card->stream));
-	DRIVER(card, cuGraphLaunch(card->graphs[graph], card->stream));
-	card->launches_queued += card->graph_kernel_nodes[graph];
+	status = graph_queue(cu, card, graph);
+	if (status != STATUS_OK)
+		goto done;
 	if (output_byte_count != 0)
 		DRIVER(card, cuMemcpyDtoHAsync(page_locked_output, card->arena + output_arena_offset, output_byte_count,
 					       card->stream));
@@ -1420,11 +1429,10 @@ static bool copy_is_small(uint64_t arena_offset, const void *host, uint64_t byte
 }
 
 static void step_copy_fill(struct kernel_launch *launch, uint32_t kernel, const void *host, uint64_t arena_offset,
-			   uint64_t byte_count, const volatile uint64_t *words)
+			   uint64_t byte_count, const volatile uint64_t *done, uint32_t graph)
 {
 	const struct backend_b200_step_copy_record record = { (uint64_t)(uintptr_t)host, arena_offset, byte_count,
-							      (uint64_t)(uintptr_t)words,
-							      words != NULL ? (uint64_t)(uintptr_t)(words + 1) : 0u };
+							      (uint64_t)(uintptr_t)done, graph, 0u };
 	/* a piece of 16 bytes a thread: every load over PCIe is in flight at once */
 	const uint64_t blocks = (byte_count / 16u + BACKEND_B200_STEP_COPY_THREADS) / BACKEND_B200_STEP_COPY_THREADS;
 	memset(launch, 0, sizeof(*launch));
@@ -1490,12 +1498,12 @@ result_status backend_b200_step_capture(struct device_card *card, const struct k
 	}
 	uint32_t count = 0;
 	if (kernel_in)
-		step_copy_fill(&chain[count++], copy_in, page_locked_input, input_arena_offset, input_byte_count, NULL);
+		step_copy_fill(&chain[count++], copy_in, page_locked_input, input_arena_offset, input_byte_count, NULL, 0u);
 	memcpy(&chain[count], launches, launch_count * sizeof(*launches));
 	count += launch_count;
 	if (kernel_out)
 		step_copy_fill(&chain[count++], copy_out, page_locked_output, output_arena_offset, output_byte_count,
-			       card->step_words + (uint64_t)card->graph_count * STEP_WORDS);
+			       card->step_words + (uint64_t)card->graph_count * STEP_WORDS, card->graph_count);
 	DRIVER(card, cuStreamBeginCapture(card->stream, CU_STREAM_CAPTURE_MODE_THREAD_LOCAL));
 	{
 		CUresult copied = CUDA_SUCCESS;
@@ -1527,13 +1535,13 @@ done:
 	CARD_LEAVE(card);
 }
 
-/* Until the graph's copy out has stored `ticket`: polls the word, and after a while the stream with it, which knows of
- * a failure. Context current, mutex held. */
-static result_status step_wait(const struct ab_driver *cu, struct device_card *card, const volatile uint64_t *words,
-			       uint64_t ticket)
+/* Until the graph's copy out has stored the number `run`: polls the word, and after a while the stream with it, which
+ * knows of a failure. Context current, mutex held. */
+static result_status step_wait(const struct ab_driver *cu, struct device_card *card, const volatile uint64_t *done,
+			       uint64_t run)
 {
 	const uint64_t begun = now_nanoseconds();
-	for (uint32_t poll = 1; words[1] != ticket; poll++) {
+	for (uint32_t poll = 1; *done != run; poll++) {
 		__builtin_ia32_pause();
 		if (poll % 4096u != 0 || now_nanoseconds() - begun < STEP_SPIN_NANOSECONDS)
 			continue;
@@ -1542,7 +1550,7 @@ static result_status step_wait(const struct ab_driver *cu, struct device_card *c
 			continue;
 		if (state != CUDA_SUCCESS)
 			return driver_failure(card, "a step's graph", state);
-		if (words[1] != ticket) /* everything has run, and the word was not stored */
+		if (*done != run) /* everything has run, and the word was not stored */
 			return driver_failure(card, "a step's copy out", CUDA_ERROR_UNKNOWN);
 	}
 	__atomic_thread_fence(__ATOMIC_ACQUIRE);
@@ -1562,17 +1570,11 @@ result_status backend_b200_graph_run_wait(struct device_card *card, uint32_t gra
 		status = STATUS_INVALID_ARGUMENT;
 		goto done;
 	}
-	const bool reports = card->graph_reports[graph];
-	volatile uint64_t *const words = reports ? card->step_words + (uint64_t)graph * STEP_WORDS : NULL;
-	const uint64_t ticket = ++card->step_ticket;
-	if (reports) {
-		words[0] = ticket;
-		__atomic_thread_fence(__ATOMIC_SEQ_CST);
-	}
-	DRIVER(card, cuGraphLaunch(card->graphs[graph], card->stream));
-	card->launches_queued += card->graph_kernel_nodes[graph];
-	if (reports)
-		status = step_wait(cu, card, words, ticket);
+	status = graph_queue(cu, card, graph);
+	if (status != STATUS_OK)
+		goto done;
+	if (card->graph_reports[graph])
+		status = step_wait(cu, card, card->step_words + (uint64_t)graph * STEP_WORDS, card->graph_runs[graph]);
 	else
 		DRIVER(card, cuStreamSynchronize(card->stream));
 done:
@@ -1658,8 +1660,9 @@ result_status backend_b200_step_call(struct device_card *card, uint32_t graph,
 		begun = false;
 	}
 	if (graph != BACKEND_B200_NO_GRAPH) {
-		DRIVER(card, cuGraphLaunch(card->graphs[graph], card->stream));
-		card->launches_queued += card->graph_kernel_nodes[graph];
+		status = graph_queue(cu, card, graph);
+		if (status != STATUS_OK)
+			goto done;
 	}
 	if (output_count != 0) {
 		const uint32_t pieces =
@@ -1749,8 +1752,9 @@ result_status backend_b200_step_pieces(struct device_card *card, const struct ba
 						       card->in_stream));
 		DRIVER(card, cuEventRecord(arrived, card->in_stream));
 		DRIVER(card, cuStreamWaitEvent(card->stream, arrived, 0));
-		DRIVER(card, cuGraphLaunch(card->graphs[step->graph], card->stream));
-		card->launches_queued += card->graph_kernel_nodes[step->graph];
+		status = graph_queue(cu, card, step->graph);
+		if (status != STATUS_OK)
+			goto done;
 		DRIVER(card, cuEventRecord(computed, card->stream));
 		DRIVER(card, cuStreamWaitEvent(card->out_stream, computed, 0));
 		for (uint32_t range = 0; range < step->output_count; range++)

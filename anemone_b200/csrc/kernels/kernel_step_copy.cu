@@ -39,14 +39,16 @@ extern "C" __global__ void __launch_bounds__(BACKEND_B200_STEP_COPY_THREADS)
 }
 
 __device__ unsigned int step_copy_arrived; /* blocks of the launch that have stored their part; zero between launches */
-__device__ uint64_t step_copy_ticket; /* the run's number, as block 0 read it */
+__device__ uint64_t step_copy_runs[BACKEND_MAXIMUM_GRAPHS]; /* of a graph: the number of its last run that is done */
 
 extern "C" __global__ void __launch_bounds__(BACKEND_B200_STEP_COPY_THREADS)
 	step_copy_out(struct backend_b200_step_copy_record record, unsigned char *arena)
 {
-	/* the number of this run, written before the graph was launched; its trip overlaps the launch before this one */
-	if (blockIdx.x == 0 && threadIdx.x == 0)
-		step_copy_ticket = *reinterpret_cast<const volatile uint64_t *>(record.ticket_address);
+	/* this run's number: the runs of a graph follow one another on the card's stream, and the host counts them as it
+	 * queues them. (A number the host wrote before each launch would be read by every run still queued.) */
+	uint64_t run = 0;
+	if (threadIdx.x == 0)
+		run = *reinterpret_cast<volatile uint64_t *>(&step_copy_runs[record.graph]) + 1u;
 	asm volatile("griddepcontrol.wait;" ::: "memory");
 	unsigned char *const to = reinterpret_cast<unsigned char *>(record.host_address);
 	const unsigned char *const from = arena + record.arena_offset;
@@ -62,9 +64,9 @@ extern "C" __global__ void __launch_bounds__(BACKEND_B200_STEP_COPY_THREADS)
 		__threadfence();
 		if (atomicAdd(&step_copy_arrived, 1u) == gridDim.x - 1u) {
 			step_copy_arrived = 0u;
+			step_copy_runs[record.graph] = run;
 			__threadfence_system();
-			*reinterpret_cast<volatile uint64_t *>(record.done_address) =
-				*reinterpret_cast<volatile uint64_t *>(&step_copy_ticket);
+			*reinterpret_cast<volatile uint64_t *>(record.done_address) = run;
 		}
 	}
 }

@@ -260,11 +260,13 @@ struct backend_b200_step_copy_record {
 	uint64_t host_address; /* page-locked, 16-byte aligned */
 	uint64_t arena_offset; /* 16-byte aligned */
 	uint64_t byte_count;
-	uint64_t ticket_address; /* copy out: a page-locked word that holds the run's number ... */
-	uint64_t done_address; /* ... and one that is given it when the outputs are in place */
+	uint64_t done_address; /* copy out: a page-locked word that is given the run's number when the outputs are in place */
+	uint32_t graph; /* copy out: whose runs it counts */
+	uint32_t reserved_zero;
 };
-/* graph_run of the table, then a wait: returns when the graph's outputs are in place (a graph of step_capture whose copy
- * out is a kernel: the host polls the word that kernel stores; any other graph: the driver's stream wait). */
+/* graph_run of the table, then a wait: returns when the outputs of this run are in place (a graph of step_capture whose
+ * copy out is a kernel: that kernel counts the graph's runs and stores the count in a word the host polls, so that runs
+ * still queued from graph_run are not taken for this one; any other graph: the driver's stream wait). */
 MUST_CHECK result_status backend_b200_graph_run_wait(struct device_card *card, uint32_t graph);
 /* A call on ORDINARY host memory in one go: the inputs' bytes through the page-locked block into the arena, the graph
  * (BACKEND_B200_NO_GRAPH: none), the outputs' bytes through the block into ordinary memory; returns when all of it is

@@ -115,3 +115,38 @@ def test_a_call_copies_ordinary_memory(api, sizes):
                 assert (card.download(int(at) + size, 16) == 0xA5).all()  # nothing past the range
     finally:
         card.close()
+
+
+def test_a_wait_is_for_its_own_run(api):
+    """backend_b200_graph_run_wait behind runs of the same graph that graph_run left in the queue: it
+    returns when ITS run's outputs are in place. Every run brings the pool's next entry, so the outputs say whose they
+    are; the fills in front keep the earlier runs queued until the waiting one is."""
+    entries, entry_bytes, earlier = 8, 4096, 5
+    layout = api.Layout()
+    pool, step, cursor = layout.take(entries * entry_bytes), layout.take(entry_bytes), layout.take(16)
+    space_bytes = 1 << 30
+    space = layout.take(space_bytes, 4096)
+    card, lib = api.Card(0, layout.take(0, 4096) + 4096), api.library()
+    try:
+        for entry in range(entries):
+            card.upload(pool + entry * entry_bytes, np.full(entry_bytes // 4, entry + 1, dtype=np.uint32))
+        select, launch = R.StepInputSelect(pool, entry_bytes, step, cursor, entries, entry_bytes), R.KernelLaunch()
+        lib.step_input_select_prepare.argtypes = [C.POINTER(R.StepInputSelect), C.c_uint64,
+                                                  C.POINTER(api.BackendOperations), C.c_void_p,
+                                                  C.POINTER(R.KernelLaunch)]
+        api.check(lib.step_input_select_prepare(C.byref(select), card.arena_bytes, card.ops_pointer, card.handle,
+                                                C.byref(launch)), "step_input_select_prepare")
+        graphs = [card.step_capture([launch], 0, 0, 0, step, 4096 * which, entry_bytes) for which in (1, 3)]
+        seen = [card.staging_view[4096 * which:4096 * which + entry_bytes].view(np.uint32) for which in (1, 3)]
+        for turn in range(3):
+            card.fill(cursor, 0, 16)
+            for _ in range(20):  # several milliseconds
+                card.fill(space, turn, space_bytes)
+            for run in range(earlier):  # runs of both graphs among one another: a number is a graph's own
+                card.graph_run(graphs[run % 2])
+            card.graph_run_wait(graphs[0])
+            assert (seen[0] == earlier + 1).all(), (turn, seen[0][0])
+            card.graph_run_wait(graphs[1])
+            assert (seen[1] == earlier + 2).all(), (turn, seen[1][0])
+    finally:
+        card.close()
