@@ -212,6 +212,9 @@ class StepStaging:
         return status, result
 
 
+EXPIRED_BITS = "bits %d (1 a wait ran out, 2 bad sequence, 4 too many rows)"
+
+
 class Card:
     """One opened card: an arena, a staging block, and the table's calls with statuses turned into exceptions."""
 
@@ -232,6 +235,13 @@ class Card:
             self.ops.staging_free(self.staging)
             self.handle = _card()
 
+    def ran(self, status, what):
+        """The status of a call that ran a graph: also raises where one of the graph's kernels gave up a bounded wait."""
+        if status == R.STATUS_TIMED_OUT:
+            raise StatusError("%s: a kernel gave up, the outputs are incomplete: %s"
+                              % (what, EXPIRED_BITS % self.expired_bits()), status)
+        check(status, what)
+
     # ---- transfers through the staging block ----
     def call(self, graph, inputs, outputs, staging_offset=0):
         """One library call on ordinary memory (backend_b200_step_call): inputs, outputs: (arena offset, contiguous
@@ -241,10 +251,10 @@ class Card:
         def ranges(pairs):
             return (R.HostRange * max(len(pairs), 1))(*[R.HostRange(offset, array.ctypes.data, array.nbytes)
                                                         for offset, array in pairs])
-        check(library().backend_b200_step_call(self.handle, R.BACKEND_B200_NO_GRAPH if graph is None else graph,
-                                               ranges(inputs), len(inputs), ranges(outputs), len(outputs),
-                                               self.staging.value + staging_offset, self.staging_bytes - staging_offset),
-              "step_call")
+        self.ran(library().backend_b200_step_call(self.handle, R.BACKEND_B200_NO_GRAPH if graph is None else graph,
+                                                  ranges(inputs), len(inputs), ranges(outputs), len(outputs),
+                                                  self.staging.value + staging_offset,
+                                                  self.staging_bytes - staging_offset), "step_call")
 
     def fits_staging(self, arrays):
         return sum(align(array.nbytes, 256) for array in arrays) <= self.staging_bytes
@@ -305,11 +315,11 @@ class Card:
     def step_run(self, graph, input_offset, input_staging_offset, input_bytes, output_offset, output_staging_offset,
                  output_bytes):
         """Copy in, run the graph, copy out and wait, in one call of the library (backend_b200_step_run)."""
-        check(library().backend_b200_step_run(self.handle, graph, input_offset,
-                                              C.c_void_p(self.staging.value + input_staging_offset), input_bytes,
-                                              output_offset,
-                                              C.c_void_p(self.staging.value + output_staging_offset), output_bytes),
-              "step_run")
+        self.ran(library().backend_b200_step_run(self.handle, graph, input_offset,
+                                                 C.c_void_p(self.staging.value + input_staging_offset), input_bytes,
+                                                 output_offset,
+                                                 C.c_void_p(self.staging.value + output_staging_offset), output_bytes),
+                 "step_run")
 
     def step_pieces(self, pieces):
         """One call in pieces (backend_b200_step_pieces): pieces: (graph, inputs, outputs), inputs and outputs up to two
@@ -320,7 +330,7 @@ class Card:
             for ranges, given in ((piece.inputs, inputs), (piece.outputs, outputs)):
                 for index, (offset, staging_offset, nbytes) in enumerate(given):
                     ranges[index] = R.HostRange(offset, self.staging.value + staging_offset, nbytes)
-        check(library().backend_b200_step_pieces(self.handle, table, len(table)), "step_pieces")
+        self.ran(library().backend_b200_step_pieces(self.handle, table, len(table)), "step_pieces")
 
     def step_capture(self, launches, input_offset, input_staging_offset, input_bytes, output_offset,
                      output_staging_offset, output_bytes):
@@ -339,7 +349,7 @@ class Card:
         return graph.value
 
     def graph_run_wait(self, graph):
-        check(library().backend_b200_graph_run_wait(self.handle, graph), "graph_run_wait")
+        self.ran(library().backend_b200_graph_run_wait(self.handle, graph), "graph_run_wait")
 
     def measure_begin(self):
         check(self.ops.measure_begin(self.handle), "measure_begin")
@@ -362,6 +372,11 @@ class Card:
     def waits_expired(self):
         """Waits for the queue; True if a kernel gave up a bounded wait (its CTA then stored nothing more)."""
         return self.expired_bits() != 0
+
+    def check_waits(self):
+        bits = self.expired_bits()
+        if bits != 0:
+            raise RuntimeError("a kernel gave up: " + EXPIRED_BITS % bits)
 
     def launch_count(self):
         return library().backend_b200_launch_count(self.handle)

@@ -24,13 +24,14 @@
 #define POLL_NANOSECONDS 20000l
 #define POLL_SPIN_NANOSECONDS 200000ull
 #define SMALL_WRITE_SLOTS 64u
-#define STEP_WORDS 16u /* 64-bit words a graph: a line of 128 bytes of its own, the first one used */
+#define STEP_WORDS 16u /* 64-bit words a graph: a line of 128 bytes of its own, the first two used */
 #define STEP_COPY_BLOCKS 64u
 #define CALL_PIECE_BYTES (1u << 19) /* 10 us of PCIe, 30 of a core's copy */
 #define STEP_SPIN_NANOSECONDS 2000000ull /* a step's wait looks at its word alone for so long */
 
 struct prepared_kernel {
 	const struct ab_kernel_image *image;
+	uint32_t module; /* its index */
 	char function[96];
 	CUfunction handle;
 	uint32_t argument_byte_count;
@@ -72,11 +73,15 @@ struct device_card {
 	CUstream in_stream, out_stream; /* of backend_b200_step_pieces: the copies beside the card's stream */
 	struct prepared_kernel kernels[BACKEND_MAXIMUM_KERNELS];
 	uint32_t kernel_count;
+	uint32_t wait_kernel; /* reads wait words for the calls that wait */
+	bool wait_kernel_is_there;
 	CUgraphExec graphs[BACKEND_MAXIMUM_GRAPHS];
 	uint32_t graph_kernel_nodes[BACKEND_MAXIMUM_GRAPHS];
 	bool graph_reports[BACKEND_MAXIMUM_GRAPHS]; /* its copy out stores the run's number in step_words */
 	uint64_t graph_runs[BACKEND_MAXIMUM_GRAPHS]; /* queued so far; the copy out counts the same runs on the card */
-	volatile uint64_t *step_words; /* page-locked: [graph]: the number of its last run whose outputs are in place */
+	uint32_t graph_wait_modules[BACKEND_MAXIMUM_GRAPHS]; /* a bit a module of its launches that has a wait word */
+	/* page-locked: [graph]: the number of its last run whose outputs are in place, the wait words' bits as it saw them */
+	volatile uint64_t *step_words;
 	uint32_t graph_count;
 	CUevent marks[BACKEND_MAXIMUM_MARKS];
 	bool mark_set[BACKEND_MAXIMUM_MARKS];
@@ -308,7 +313,7 @@ static result_status cuda_card_open(uint32_t card_index, uint64_t arena_byte_cou
 		result = cu->cuMemAlloc(&card->arena, arena_byte_count);
 	if (result == CUDA_SUCCESS)
 		result = cu->cuMemHostAlloc((void **)&card->small_words,
-					    (SMALL_WRITE_SLOTS + CARD_MODULES_MOST) * sizeof(uint64_t),
+					    (SMALL_WRITE_SLOTS + CARD_MODULES_MOST + 1u) * sizeof(uint64_t),
 					    CU_MEMHOSTALLOC_PORTABLE);
 	if (result != CUDA_SUCCESS) {
 		status = driver_failure(card, "opening the card", result);
@@ -695,6 +700,7 @@ static result_status cuda_kernel_prepare(struct device_card *card, const char *k
 		prepared->cluster[axis] = width > 0 ? (uint32_t)width : 1u;
 	}
 	prepared->image = image;
+	prepared->module = image_index;
 	prepared->handle = function;
 	prepared->argument_byte_count = argument_byte_count;
 	(void)snprintf(prepared->function, sizeof(prepared->function), "%s", function_name);
@@ -1056,11 +1062,79 @@ static bool cuda_format_supported(uint32_t card_index, enum weight_format_code f
 
 /* ------------------------------------------------------------------ graphs, marks, peers, timing */
 
+/* The modules of a table's launches whose kernels may give up a bounded wait, a bit each. */
+static uint32_t wait_modules_of(const struct device_card *card, const struct kernel_launch *launches, uint32_t launch_count)
+{
+	_Static_assert(CARD_MODULES_MOST <= 32u, "a bit a module");
+	uint32_t modules = 0;
+	for (uint32_t index = 0; index < launch_count; index++)
+		if (launches[index].kernel != BACKEND_COPY && card->wait_words[card->kernels[launches[index].kernel].module] != 0)
+			modules |= 1u << card->kernels[launches[index].kernel].module;
+	return modules;
+}
+
+/* The kernel that reads wait words, where the card has room for it; graph_capture asks, before it enters the card. */
+static void wait_kernel_prepare(struct device_card *card)
+{
+	uint32_t kernel = BACKEND_NO_KERNEL;
+	(void)pthread_mutex_lock(&card->mutex);
+	const bool wanted = !card->failed && !card->wait_kernel_is_there && card->kernel_count < BACKEND_MAXIMUM_KERNELS;
+	(void)pthread_mutex_unlock(&card->mutex);
+	if (!wanted || cuda_kernel_prepare(card, BACKEND_B200_STEP_COPY_KERNEL_FILE, "step_wait_words",
+					   sizeof(struct backend_b200_wait_words_record), &kernel) != STATUS_OK)
+		return;
+	(void)pthread_mutex_lock(&card->mutex);
+	card->wait_kernel = kernel;
+	card->wait_kernel_is_there = true;
+	(void)pthread_mutex_unlock(&card->mutex);
+}
+
+/* Queue the reading of these modules' wait words; wait_words_seen has them once the stream has come that far. Context
+ * current, mutex held from here to there. By a kernel that stores them in page-locked memory: copies of two such words
+ * cost a prompt of 4096 rows 10 to 13 us, the kernel 5. */
+static result_status wait_words_queue(const struct ab_driver *cu, struct device_card *card, uint32_t modules, CUstream stream)
+{
+	result_status status = STATUS_OK;
+	volatile uint64_t *const seen = card->small_words + SMALL_WRITE_SLOTS;
+	struct backend_b200_wait_words_record record;
+	uint32_t count = 0;
+	memset(&record, 0, sizeof(record));
+	for (uint32_t module = 0; module <= CARD_MODULES_MOST; module++)
+		seen[module] = 0;
+	for (uint32_t module = 0; module < CARD_MODULES_MOST; module++) {
+		if ((modules >> module & 1u) == 0 || card->wait_words[module] == 0)
+			continue;
+		if (card->wait_kernel_is_there && count < BACKEND_B200_WAIT_WORDS_MOST)
+			record.wait_words[count++] = card->wait_words[module];
+		else
+			DRIVER(card, cuMemcpyDtoHAsync((void *)(uintptr_t)&seen[module], card->wait_words[module],
+						       sizeof(uint32_t), stream));
+	}
+	if (count != 0) {
+		record.host_address = (uint64_t)(uintptr_t)&seen[CARD_MODULES_MOST];
+		CUdeviceptr arena = card->arena;
+		void *parameters[] = { &record, &arena };
+		DRIVER(card, cuLaunchKernel(card->kernels[card->wait_kernel].handle, 1, 1, 1, 32, 1, 1, 0, stream, parameters,
+					    NULL));
+	}
+done:
+	return status;
+}
+
+static uint32_t wait_words_seen(const struct device_card *card)
+{
+	uint64_t expired = 0;
+	for (uint32_t module = 0; module <= CARD_MODULES_MOST; module++)
+		expired |= *(const volatile uint64_t *)&card->small_words[SMALL_WRITE_SLOTS + module];
+	return (uint32_t)expired;
+}
+
 static result_status cuda_graph_capture(struct device_card *card, const struct kernel_launch *launches,
 					uint32_t launch_count, uint32_t *graph_out)
 {
 	if (card == NULL || graph_out == NULL)
 		return STATUS_INVALID_ARGUMENT;
+	wait_kernel_prepare(card);
 	CARD_ENTER(card);
 	CUgraph graph = NULL;
 	struct launch_order *order = NULL;
@@ -1095,6 +1169,7 @@ static result_status cuda_graph_capture(struct device_card *card, const struct k
 		goto done;
 	DRIVER(card, cuGraphInstantiateWithFlags(&card->graphs[card->graph_count], graph, 0));
 	card->graph_kernel_nodes[card->graph_count] = kernel_launches_of(launches, launch_count);
+	card->graph_wait_modules[card->graph_count] = wait_modules_of(card, launches, launch_count);
 	*graph_out = card->graph_count++;
 done:
 	if (graph != NULL)
@@ -1373,14 +1448,11 @@ result_status backend_b200_waits_expired(struct device_card *card, uint32_t *exp
 		goto done;
 	}
 	/* every file's word behind the queued work, then one wait */
-	for (uint32_t module = 0; module < CARD_MODULES_MOST; module++)
-		if (card->wait_words[module] != 0)
-			DRIVER(card, cuMemcpyDtoHAsync(&card->small_words[SMALL_WRITE_SLOTS + module], card->wait_words[module],
-						       sizeof(uint32_t), card->stream));
+	status = wait_words_queue(cu, card, UINT32_MAX, card->stream);
+	if (status != STATUS_OK)
+		goto done;
 	DRIVER(card, cuStreamSynchronize(card->stream));
-	for (uint32_t module = 0; module < CARD_MODULES_MOST; module++)
-		if (card->wait_words[module] != 0)
-			expired |= *(const volatile uint32_t *)&card->small_words[SMALL_WRITE_SLOTS + module];
+	expired = wait_words_seen(card);
 	*expired_out = expired;
 done:
 	CARD_LEAVE(card);
@@ -1416,7 +1488,12 @@ result_status backend_b200_step_run(struct device_card *card, uint32_t graph, ui
 	if (output_byte_count != 0)
 		DRIVER(card, cuMemcpyDtoHAsync(page_locked_output, card->arena + output_arena_offset, output_byte_count,
 					       card->stream));
+	status = wait_words_queue(cu, card, card->graph_wait_modules[graph], card->stream);
+	if (status != STATUS_OK)
+		goto done;
 	DRIVER(card, cuStreamSynchronize(card->stream));
+	if (wait_words_seen(card) != 0)
+		status = STATUS_TIMED_OUT;
 done:
 	CARD_LEAVE(card);
 }
@@ -1429,10 +1506,20 @@ static bool copy_is_small(uint64_t arena_offset, const void *host, uint64_t byte
 }
 
 static void step_copy_fill(struct kernel_launch *launch, uint32_t kernel, const void *host, uint64_t arena_offset,
-			   uint64_t byte_count, const volatile uint64_t *done, uint32_t graph)
+			   uint64_t byte_count, const struct device_card *card, uint32_t modules)
 {
-	const struct backend_b200_step_copy_record record = { (uint64_t)(uintptr_t)host, arena_offset, byte_count,
-							      (uint64_t)(uintptr_t)done, graph, 0u };
+	struct backend_b200_step_copy_record record = { .host_address = (uint64_t)(uintptr_t)host,
+							.arena_offset = arena_offset, .byte_count = byte_count };
+	if (card != NULL) { /* the copy out of the card's next graph, whose launches are these modules' */
+		const volatile uint64_t *const words = card->step_words + (uint64_t)card->graph_count * STEP_WORDS;
+		record.done_address = (uint64_t)(uintptr_t)words;
+		record.expired_address = (uint64_t)(uintptr_t)(words + 1);
+		record.graph = card->graph_count;
+		uint32_t word = 0;
+		for (uint32_t module = 0; module < CARD_MODULES_MOST; module++)
+			if ((modules >> module & 1u) != 0)
+				record.wait_words[word++] = card->wait_words[module];
+	}
 	/* a piece of 16 bytes a thread: every load over PCIe is in flight at once */
 	const uint64_t blocks = (byte_count / 16u + BACKEND_B200_STEP_COPY_THREADS) / BACKEND_B200_STEP_COPY_THREADS;
 	memset(launch, 0, sizeof(*launch));
@@ -1462,7 +1549,7 @@ result_status backend_b200_step_capture(struct device_card *card, const struct k
 		return STATUS_INVALID_ARGUMENT;
 	/* small copies as kernels of the chain: what they need is prepared before the card is entered */
 	const bool kernel_in = copy_is_small(input_arena_offset, page_locked_input, input_byte_count);
-	const bool kernel_out = copy_is_small(output_arena_offset, page_locked_output, output_byte_count);
+	bool kernel_out = copy_is_small(output_arena_offset, page_locked_output, output_byte_count);
 	uint32_t copy_in = BACKEND_NO_KERNEL, copy_out = BACKEND_NO_KERNEL;
 	result_status prepared = STATUS_OK;
 	if (kernel_in)
@@ -1489,6 +1576,9 @@ result_status backend_b200_step_capture(struct device_card *card, const struct k
 		status = STATUS_BUSY_VALUE;
 		goto done;
 	}
+	const uint32_t modules = wait_modules_of(card, launches, launch_count);
+	if ((uint32_t)__builtin_popcount(modules) > BACKEND_B200_STEP_COPY_WAIT_WORDS)
+		kernel_out = false;
 	if (kernel_out && card->step_words == NULL) {
 		void *words = NULL;
 		const size_t bytes = BACKEND_MAXIMUM_GRAPHS * STEP_WORDS * sizeof(uint64_t);
@@ -1498,12 +1588,12 @@ result_status backend_b200_step_capture(struct device_card *card, const struct k
 	}
 	uint32_t count = 0;
 	if (kernel_in)
-		step_copy_fill(&chain[count++], copy_in, page_locked_input, input_arena_offset, input_byte_count, NULL, 0u);
+		step_copy_fill(&chain[count++], copy_in, page_locked_input, input_arena_offset, input_byte_count, NULL, 0);
 	memcpy(&chain[count], launches, launch_count * sizeof(*launches));
 	count += launch_count;
 	if (kernel_out)
-		step_copy_fill(&chain[count++], copy_out, page_locked_output, output_arena_offset, output_byte_count,
-			       card->step_words + (uint64_t)card->graph_count * STEP_WORDS, card->graph_count);
+		step_copy_fill(&chain[count++], copy_out, page_locked_output, output_arena_offset, output_byte_count, card,
+			       modules);
 	DRIVER(card, cuStreamBeginCapture(card->stream, CU_STREAM_CAPTURE_MODE_THREAD_LOCAL));
 	{
 		CUresult copied = CUDA_SUCCESS;
@@ -1526,6 +1616,7 @@ result_status backend_b200_step_capture(struct device_card *card, const struct k
 		goto done;
 	DRIVER(card, cuGraphInstantiateWithFlags(&card->graphs[card->graph_count], graph, 0));
 	card->graph_kernel_nodes[card->graph_count] = kernel_launches_of(launches, launch_count);
+	card->graph_wait_modules[card->graph_count] = wait_modules_of(card, launches, launch_count);
 	card->graph_reports[card->graph_count] = kernel_out;
 	*graph_out = card->graph_count++;
 done:
@@ -1554,7 +1645,7 @@ static result_status step_wait(const struct ab_driver *cu, struct device_card *c
 			return driver_failure(card, "a step's copy out", CUDA_ERROR_UNKNOWN);
 	}
 	__atomic_thread_fence(__ATOMIC_ACQUIRE);
-	return STATUS_OK;
+	return done[1] != 0 ? STATUS_TIMED_OUT : STATUS_OK; /* a kernel of the graph's files gave up a bounded wait */
 }
 
 result_status backend_b200_graph_run_wait(struct device_card *card, uint32_t graph)
@@ -1573,10 +1664,16 @@ result_status backend_b200_graph_run_wait(struct device_card *card, uint32_t gra
 	status = graph_queue(cu, card, graph);
 	if (status != STATUS_OK)
 		goto done;
-	if (card->graph_reports[graph])
+	if (card->graph_reports[graph]) {
 		status = step_wait(cu, card, card->step_words + (uint64_t)graph * STEP_WORDS, card->graph_runs[graph]);
-	else
-		DRIVER(card, cuStreamSynchronize(card->stream));
+		goto done;
+	}
+	status = wait_words_queue(cu, card, card->graph_wait_modules[graph], card->stream);
+	if (status != STATUS_OK)
+		goto done;
+	DRIVER(card, cuStreamSynchronize(card->stream));
+	if (wait_words_seen(card) != 0)
+		status = STATUS_TIMED_OUT;
 done:
 	CARD_LEAVE(card);
 }
@@ -1659,7 +1756,9 @@ result_status backend_b200_step_call(struct device_card *card, uint32_t graph,
 		ab_copy_batch_end(&batch);
 		begun = false;
 	}
+	uint32_t modules = 0;
 	if (graph != BACKEND_B200_NO_GRAPH) {
+		modules = card->graph_wait_modules[graph];
 		status = graph_queue(cu, card, graph);
 		if (status != STATUS_OK)
 			goto done;
@@ -1675,6 +1774,9 @@ result_status backend_b200_step_call(struct device_card *card, uint32_t graph,
 						       batch.copies[piece].byte_count, card->stream));
 			DRIVER(card, cuEventRecord(card->piece_events[piece], card->stream));
 		}
+		status = wait_words_queue(cu, card, modules, card->stream); /* they cross beside the host's last copies */
+		if (status != STATUS_OK)
+			goto done;
 		batch.allowed = 0;
 		ab_copy_batch_begin(&batch);
 		begun = true;
@@ -1690,9 +1792,17 @@ result_status backend_b200_step_call(struct device_card *card, uint32_t graph,
 			}
 			ab_copy_batch_allow(&batch, piece + 1u);
 		}
+		ab_copy_batch_end(&batch);
+		begun = false;
 	} else {
-		DRIVER(card, cuStreamSynchronize(card->stream)); /* the block is the caller's again */
+		status = wait_words_queue(cu, card, modules, card->stream);
+		if (status != STATUS_OK)
+			goto done;
 	}
+	if (modules != 0 || output_count == 0) /* the block is the caller's again, the words are in */
+		DRIVER(card, cuStreamSynchronize(card->stream));
+	if (modules != 0 && wait_words_seen(card) != 0)
+		status = STATUS_TIMED_OUT;
 done:
 	if (begun)
 		ab_copy_batch_end(&batch);
@@ -1724,6 +1834,7 @@ result_status backend_b200_step_pieces(struct device_card *card, const struct ba
 			return STATUS_INVALID_ARGUMENT;
 	CARD_ENTER(card);
 	bool queued = false;
+	uint32_t modules = 0;
 	if (card->failed) {
 		status = STATUS_DEVICE_ERROR;
 		goto done;
@@ -1762,8 +1873,16 @@ result_status backend_b200_step_pieces(struct device_card *card, const struct ba
 						       card->arena + step->outputs[range].arena_offset,
 						       step->outputs[range].byte_count, card->out_stream));
 	}
+	for (uint32_t piece = 0; piece < piece_count; piece++)
+		modules |= card->graph_wait_modules[pieces[piece].graph];
+	status = wait_words_queue(cu, card, modules, card->stream); /* beside the last piece's way out */
+	if (status != STATUS_OK)
+		goto done;
 	DRIVER(card, cuStreamSynchronize(card->out_stream)); /* behind the last graph, and that behind the last copy in */
+	DRIVER(card, cuStreamSynchronize(card->stream));
 	queued = false;
+	if (wait_words_seen(card) != 0)
+		status = STATUS_TIMED_OUT;
 done:
 	if (queued) { /* the caller's memory is not read or written after the call */
 		(void)cu->cuStreamSynchronize(card->in_stream);

@@ -22,6 +22,13 @@ __device__ __forceinline__ uint4 load_host(const uint4 *address)
 	return value;
 }
 
+/* a warp: the bits of up to 32 of these words (device addresses, 0: none) or-ed */
+__device__ __forceinline__ unsigned int wait_bits(const uint64_t *words, uint32_t count)
+{
+	const uint64_t word = threadIdx.x < count ? words[threadIdx.x] : 0u;
+	return __reduce_or_sync(0xFFFFFFFFu, word != 0 ? *reinterpret_cast<const volatile unsigned int *>(word) : 0u);
+}
+
 /* grid (blocks) x BACKEND_B200_STEP_COPY_THREADS */
 extern "C" __global__ void __launch_bounds__(BACKEND_B200_STEP_COPY_THREADS)
 	step_copy_in(struct backend_b200_step_copy_record record, unsigned char *arena)
@@ -42,7 +49,7 @@ __device__ unsigned int step_copy_arrived; /* blocks of the launch that have sto
 __device__ uint64_t step_copy_runs[BACKEND_MAXIMUM_GRAPHS]; /* of a graph: the number of its last run that is done */
 
 extern "C" __global__ void __launch_bounds__(BACKEND_B200_STEP_COPY_THREADS)
-	step_copy_out(struct backend_b200_step_copy_record record, unsigned char *arena)
+	step_copy_out(const __grid_constant__ struct backend_b200_step_copy_record record, unsigned char *arena)
 {
 	/* this run's number: the runs of a graph follow one another on the card's stream, and the host counts them as it
 	 * queues them. (A number the host wrote before each launch would be read by every run still queued.) */
@@ -50,6 +57,12 @@ extern "C" __global__ void __launch_bounds__(BACKEND_B200_STEP_COPY_THREADS)
 	if (threadIdx.x == 0)
 		run = *reinterpret_cast<volatile uint64_t *>(&step_copy_runs[record.graph]) + 1u;
 	asm volatile("griddepcontrol.wait;" ::: "memory");
+	/* whether a kernel of the graph's files gave up a bounded wait: beside the copy, a word is an L2 read */
+	if (blockIdx.x == 0 && threadIdx.x < 32u) {
+		const unsigned int bits = wait_bits(record.wait_words, BACKEND_B200_STEP_COPY_WAIT_WORDS);
+		if (threadIdx.x == 0 && bits != 0)
+			*reinterpret_cast<volatile uint64_t *>(record.expired_address) = bits;
+	}
 	unsigned char *const to = reinterpret_cast<unsigned char *>(record.host_address);
 	const unsigned char *const from = arena + record.arena_offset;
 	const uint64_t pieces = record.byte_count / 16u;
@@ -69,4 +82,14 @@ extern "C" __global__ void __launch_bounds__(BACKEND_B200_STEP_COPY_THREADS)
 			*reinterpret_cast<volatile uint64_t *>(record.done_address) = run;
 		}
 	}
+}
+
+/* grid (1) x 32: behind a graph, for the calls whose outputs go by memcpy */
+extern "C" __global__ void __launch_bounds__(32)
+	step_wait_words(const __grid_constant__ struct backend_b200_wait_words_record record, unsigned char *arena)
+{
+	(void)arena;
+	const unsigned int bits = wait_bits(record.wait_words, BACKEND_B200_WAIT_WORDS_MOST);
+	if (threadIdx.x == 0 && bits != 0)
+		*reinterpret_cast<volatile uint64_t *>(record.host_address) = bits;
 }

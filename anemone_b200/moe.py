@@ -319,7 +319,7 @@ class MoeLayer:
 
     def step(self, tokens, scores):
         """One layer call on host arrays: tokens bfloat16 bits [rows][hidden], scores FP32 [rows][experts].
-        Returns bfloat16 bits [rows][hidden]. Raises if the reduction reported a failed wait."""
+        Returns bfloat16 bits [rows][hidden]. Raises if a kernel of the step gave up a wait."""
         L, card, result_at = self.layout, self.card, self.staged.result_at
         self.sequence += 1
         status, result = self.staged.write(self.sequence, tokens, scores)
@@ -336,19 +336,12 @@ class MoeLayer:
             card.graph_run_wait(self.step_graph)
         else:
             card.step_run(self.graph, L.step, 0, L.step_input_bytes, L.status, result_at, 16 + result.nbytes)
-        if L.reduce_form == "push":
-            self.check_status()
-        elif status[0] != 0:
-            self._raise_on(status)
+        self._raise_on(status)  # the push form has no status block: its words are among those the call has read
         return result.copy()
 
     def check_status(self):
-        if self.layout.reduce_form == "push":
-            bits = self.card.expired_bits()
-            if bits != 0:
-                raise RuntimeError("ordered reduction failed: bits %d (1 a wait ran out, 2 bad sequence, 4 too many "
-                                   "rows)" % bits)
-            return
+        """What step raises, of the steps that were submitted (it waits for them)."""
+        self.card.check_waits()
         self._raise_on(self.card.download(self.layout.status, 16, np.uint32))
 
     @staticmethod

@@ -466,7 +466,7 @@ class MxLayer:
         return card.download_async(L.result, result_staging_offset, rows * self.config.hidden * 2)
 
     def step(self, tokens, scores):
-        """One layer call on host arrays; returns bfloat16 bits [rows][hidden]."""
+        """One layer call on host arrays; returns bfloat16 bits [rows][hidden]. Raises if a kernel of it gave up a wait."""
         L, card = self.layout, self.card
         self.sequence += 1
         if L.wide:
@@ -495,6 +495,8 @@ class MxLayer:
         return result.copy()
 
     def check_status(self):
+        """What step raises, of the steps that were submitted (it waits for them)."""
+        self.card.check_waits()
         self._raise_on(self.card.download(self.layout.status, 16, np.uint32))
 
     @staticmethod

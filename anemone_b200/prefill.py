@@ -255,7 +255,8 @@ class PrefillLayer:
 
     def call(self, staging_offset, result_staging_offset):
         """One whole call on staged inputs in ONE library call: inputs in, the graph, status block and bfloat16 result
-        out, wait. Returns the result as a view of the staging block (bfloat16 bits [rows][hidden])."""
+        out, wait. Returns the result as a view of the staging block (bfloat16 bits [rows][hidden]). Raises if a kernel of
+        it gave up a wait."""
         L, card, rows = self.layout, self.card, self.config.row_capacity
         if self.pieces:
             return self._call_pieces(staging_offset, result_staging_offset)

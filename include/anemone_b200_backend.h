@@ -230,6 +230,11 @@ MUST_CHECK result_status backend_b200_image_register(const char *kernel_file_nam
  * exchange, whose kernels also report a replayed sequence, 2, and a row count beyond the prepared rows, 4). Such a CTA
  * stores nothing more and returns; nothing traps. *expired_out is 0, or the kernels' bits or-ed. */
 MUST_CHECK result_status backend_b200_waits_expired(struct device_card *card, uint32_t *expired_out);
+/* The calls below that run a graph and wait for it (backend_b200_step_run, _graph_run_wait, _step_call, _step_pieces) ask
+ * this themselves, of the kernel files of the graph's launches alone: STATUS_TIMED_OUT where one of their kernels gave up
+ * since the file was loaded. The outputs are then incomplete and not to be used, and the file's kernels may do nothing more
+ * until the card is opened again. (The other ranks of a reduction see their own kernels alone: they learn of it from the
+ * rank that was told.) */
 /* One step in ONE call, for a serving loop that must not pay a foreign-function call, a ticket and a polled wait per
  * transfer: queue the copy of input_byte_count bytes from page-locked memory to the arena, the captured graph, the
  * copy of output_byte_count arena bytes back to page-locked memory, then block (the driver's stream wait, which
@@ -256,6 +261,7 @@ MUST_CHECK result_status backend_b200_step_capture(struct device_card *card, con
 #define BACKEND_B200_STEP_COPY_MOST (1u << 20)
 #define BACKEND_B200_STEP_COPY_THREADS 256u
 #define BACKEND_B200_STEP_COPY_KERNEL_FILE "kernel_step_copy"
+#define BACKEND_B200_STEP_COPY_WAIT_WORDS 8u /* a graph of more such kernel files goes out by a memcpy node */
 struct backend_b200_step_copy_record {
 	uint64_t host_address; /* page-locked, 16-byte aligned */
 	uint64_t arena_offset; /* 16-byte aligned */
@@ -263,6 +269,14 @@ struct backend_b200_step_copy_record {
 	uint64_t done_address; /* copy out: a page-locked word that is given the run's number when the outputs are in place */
 	uint32_t graph; /* copy out: whose runs it counts */
 	uint32_t reserved_zero;
+	uint64_t expired_address; /* copy out: a page-locked word that is given the bits of the wait words below, if any is set */
+	uint64_t wait_words[BACKEND_B200_STEP_COPY_WAIT_WORDS]; /* device addresses, 0 behind the last */
+};
+/* Entry "step_wait_words" of the same file (one warp): the bits of these words or-ed, into page-locked memory. */
+#define BACKEND_B200_WAIT_WORDS_MOST 20u
+struct backend_b200_wait_words_record {
+	uint64_t host_address;
+	uint64_t wait_words[BACKEND_B200_WAIT_WORDS_MOST]; /* device addresses, 0 behind the last */
 };
 /* graph_run of the table, then a wait: returns when the outputs of this run are in place (a graph of step_capture whose
  * copy out is a kernel: that kernel counts the graph's runs and stores the count in a word the host polls, so that runs
