@@ -55,19 +55,28 @@ __device__ __forceinline__ void barrier_arrive(uint64_t *barrier)
 
 /* true once the phase of the given parity has completed; false if the bounded wait ran out. The wait spins on
  * try_wait (which itself suspends the thread for a short, hardware-chosen time) and never sleeps: a sleep's wake-up
- * is far coarser than the hand-offs of a pipeline stage. The bound is a count of device clock cycles. */
-__device__ __forceinline__ bool barrier_wait(uint64_t *barrier, uint32_t parity)
+ * is far coarser than the hand-offs of a pipeline stage. The bound is a count of device clock cycles. ACROSS: the phase
+ * has arrivals of the cluster's other CTAs; the wait orders nothing by itself, a fence at cluster scope follows it. */
+template <bool ACROSS = false> __device__ __forceinline__ bool barrier_wait(uint64_t *barrier, uint32_t parity)
 {
 	const uint32_t address = smem_address(barrier);
 	long long begun = 0;
 	for (uint32_t poll = 1;; poll++) {
 		uint32_t complete;
-		asm volatile("{\n\t.reg .pred p;\n\t"
-			     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-			     "selp.u32 %0, 1, 0, p;\n\t}"
-			     : "=r"(complete)
-			     : "r"(address), "r"(parity)
-			     : "memory");
+		if (ACROSS)
+			asm volatile("{\n\t.reg .pred p;\n\t"
+				     "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+				     "selp.u32 %0, 1, 0, p;\n\t}"
+				     : "=r"(complete)
+				     : "r"(address), "r"(parity)
+				     : "memory");
+		else
+			asm volatile("{\n\t.reg .pred p;\n\t"
+				     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+				     "selp.u32 %0, 1, 0, p;\n\t}"
+				     : "=r"(complete)
+				     : "r"(address), "r"(parity)
+				     : "memory");
 		if (complete != 0)
 			return true;
 		if ((poll & 255u) == 0u) {

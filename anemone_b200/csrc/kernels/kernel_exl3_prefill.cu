@@ -370,17 +370,17 @@ __device__ __forceinline__ bool prefill_elected()
 }
 
 /* a whole warp's wait: its lanes go on, or give up, together */
-__device__ __forceinline__ bool warp_wait(uint64_t *barrier, uint32_t parity)
+template <bool ACROSS = false> __device__ __forceinline__ bool warp_wait(uint64_t *barrier, uint32_t parity)
 {
-	return __all_sync(0xFFFFFFFFu, barrier_wait(barrier, parity)) != 0;
+	return __all_sync(0xFFFFFFFFu, barrier_wait<ACROSS>(barrier, parity)) != 0;
 }
 
-/* whether the phase has completed by now, without a wait */
-__device__ __forceinline__ uint32_t barrier_test(uint32_t barrier, uint32_t parity)
+/* whether the phase, which arrivals of both CTAs complete, has completed by now, without a wait; pair_acquire follows */
+__device__ __forceinline__ uint32_t pair_barrier_test(uint32_t barrier, uint32_t parity)
 {
 	uint32_t complete;
 	asm volatile("{\n\t.reg .pred p;\n\t"
-		     "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+		     "mbarrier.test_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
 		     "selp.u32 %0, 1, 0, p;\n\t}"
 		     : "=r"(complete)
 		     : "r"(barrier), "r"(parity)
@@ -407,6 +407,23 @@ __device__ __forceinline__ uint32_t pair_address(const volatile void *here, uint
 		     : "=r"(there)
 		     : "r"((uint32_t)__cvta_generic_to_shared(const_cast<const void *>(here))), "r"(rank));
 	return there;
+}
+
+/* pair_arrive arrives at a barrier of the other CTA's; what this thread has seen in its own CTA's shared memory is in
+ * place for the thread that finds the phase complete there and then calls pair_acquire. Both fences order shared memory
+ * alone. The arrival's own .release.cluster, or fence.acq_rel.cluster before it, waits for all of memory and holds the one
+ * warp that arrives up for longer than a stage (4096 rows of 256 experts: 7.08 ms; that fence once for all the stages in
+ * place, 5.52), the waits' own .acquire.cluster costs 1 % (4.96); so 4.93, and 4.92 with no ordering at all. */
+__device__ __forceinline__ void pair_arrive(uint32_t there)
+{
+	asm volatile("fence.release.sync_restrict::shared::cta.cluster;\n\t"
+		     "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(there)
+		     : "memory");
+}
+
+__device__ __forceinline__ void pair_acquire()
+{
+	asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
 }
 
 /* Dynamic shared memory of a product CTA: MATRICES x GROUPS = 2 accumulators, gate and up of 128 outputs or down of
@@ -469,13 +486,16 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 		return false;
 	}
 	if (warp == 1 && rank != 0) {
-		/* rank 0 issues for both: a stage's arrival there says that this CTA's part of it is in place. The decode warps
-		 * do not tell rank 0 themselves: their arrival across the pair would wait for their stores. */
+		/* rank 0 issues for both: a stage's arrival there says that this CTA's part of it is in place. This warp has seen
+		 * the stage's phase complete, so the decode warps' stores (each behind its writer's proxy fence) and the rows'
+		 * copy happened before its arrival, whose release at cluster scope and the acquire behind rank 0's wait carry that
+		 * across. (The decode warps themselves have loads and stores in flight that a release would wait for.) */
 		bool good = true;
+		const uint32_t there = pair_address(shared->full, 0);
 		for (uint32_t block = 0; block < blocks && good; block++) {
 			good = warp_wait(&shared->full[block % S], (block / S) & 1u);
-			if (good && prefill_elected())
-				tensor_commit(&shared->full[block % S], 1u);
+			if (good && lane == 0)
+				pair_arrive(there + block % S * 8u);
 			__syncwarp();
 		}
 		if (!good)
@@ -495,7 +515,7 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 		const uint32_t full = warp_value(smem_address(shared->full)), r_second = MATRICES > 1u ? 2u * r_step : 0u;
 		for (uint32_t left = blocks; left != 0; left--) {
 			if (ready == 0) {
-				good = warp_wait(&shared->full[stage], parity);
+				good = warp_wait<true>(&shared->full[stage], parity);
 				if (!good)
 					break;
 			}
@@ -504,7 +524,8 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 			stage++;
 			if (stage == S)
 				stage = 0, parity ^= 1u;
-			ready = barrier_test(full + stage * 8u, parity);
+			pair_acquire();
+			ready = pair_barrier_test(full + stage * 8u, parity);
 			tensor_fence_after();
 			if (prefill_elected()) {
 				tensor_multiply(columns, w, r, instruction, accumulate);

@@ -326,6 +326,22 @@ def test_prefill_units_at_their_edges(api, oracle, rows):
         assert np.abs(got - expected).max() <= MAX_ABS and cosine(got, expected) >= COSINE, width
 
 
+@pytest.mark.parametrize("hidden,inner", [(32 * 8, 512), (32 * 96, 128)])
+def test_pairs_hand_their_stages_over(api, hidden, inner):
+    """A pair's second CTA tells the first when its half of a stage is in place: call after call the same bits, whatever
+    the CTAs' relative pace, for K of a ring and a stage (seven stages of 32 inputs) and of many turns of it."""
+    config = MoeConfig(hidden=hidden, inner=inner, experts=8, shared=1, picks=3, row_capacity=900)
+    widths, matrices, tokens, scores = make_inputs(41, config, 900)
+    card = api.Card(0, PrefillLayout(config, widths).arena_bytes)
+    try:
+        layer = PrefillLayer(card, config, widths, matrices)
+        first = layer.step(tokens, scores).view(np.uint32).copy()
+        for _ in range(40):
+            assert np.array_equal(layer.step(tokens, scores).view(np.uint32), first)
+    finally:
+        card.close()
+
+
 @pytest.mark.parametrize("rows,count", [(519, 2), (1100, 4)])
 def test_staged_call_in_pieces(api, monkeypatch, rows, count):
     """A staged call that takes its rows in pieces (beside the copies) against the whole: the same bits, call after call,
