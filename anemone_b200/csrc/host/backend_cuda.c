@@ -18,6 +18,7 @@
 #include "copy_pool.h"
 #include "driver_api.h"
 #include "kernel_images.h"
+#include "processor.h"
 
 #define CARD_MODULES_MOST 32u
 #define NANOSECONDS_PER_SECOND 1000000000ull
@@ -1633,7 +1634,7 @@ static result_status step_wait(const struct ab_driver *cu, struct device_card *c
 {
 	const uint64_t begun = now_nanoseconds();
 	for (uint32_t poll = 1; *done != run; poll++) {
-		__builtin_ia32_pause();
+		processor_pause();
 		if (poll % 4096u != 0 || now_nanoseconds() - begun < STEP_SPIN_NANOSECONDS)
 			continue;
 		const CUresult state = cu->cuStreamQuery(card->stream);
@@ -1746,7 +1747,7 @@ result_status backend_b200_step_call(struct device_card *card, uint32_t graph,
 		for (uint32_t sent = 0; sent < pieces;) {
 			if (!ab_copy_batch_is_done(&batch, sent)) { /* a piece more while the next to be sent is not there */
 				if (!ab_copy_batch_help(&batch))
-					__builtin_ia32_pause();
+					processor_pause();
 				continue;
 			}
 			DRIVER(card, cuMemcpyHtoDAsync(card->arena + inputs[range_of[sent]].arena_offset + within[sent],
@@ -1784,7 +1785,7 @@ result_status backend_b200_step_call(struct device_card *card, uint32_t graph,
 			CUresult state;
 			while ((state = cu->cuEventQuery(card->piece_events[piece])) == CUDA_ERROR_NOT_READY)
 				if (!ab_copy_batch_help(&batch))
-					__builtin_ia32_pause();
+					processor_pause();
 			if (state != CUDA_SUCCESS) {
 				status = driver_failure(card, "a step call", state);
 				batch.count = batch.allowed; /* what has not arrived is not copied on */

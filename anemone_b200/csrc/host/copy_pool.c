@@ -1,11 +1,14 @@
 /* copy_pool.c: host memory copies by a few threads at once (copy_pool.h). */
 #include "copy_pool.h"
 
-#include <emmintrin.h>
 #include <pthread.h>
 #include <sched.h>
 #include <string.h>
 #include <unistd.h>
+
+#ifdef __SSE2__
+#include <emmintrin.h>
+#endif
 
 #define POOL_THREADS_MOST 3u /* beside the caller: four copy 16.8 MB in 0.32 ms, eight in 0.28 */
 
@@ -18,6 +21,7 @@ static struct ab_copy_batch *current; /* one batch at a time: another caller cop
 
 /* Stores past the caches: what the device reads next lies in memory and not as dirty lines of some core's cache, which
  * PCIe reads at half its rate (a prompt of 2048 rows of 4096, 16.8 MB and 2 MB of scores: 1042 us, so 565). */
+#ifdef __SSE2__
 static void copy_past_caches(void *to, const void *from, size_t byte_count)
 {
 	unsigned char *out = to;
@@ -36,6 +40,12 @@ static void copy_past_caches(void *to, const void *from, size_t byte_count)
 	_mm_sfence();
 	memcpy(out, in, byte_count);
 }
+#else /* another processor: its own copy */
+static void copy_past_caches(void *to, const void *from, size_t byte_count)
+{
+	memcpy(to, from, byte_count);
+}
+#endif
 
 static void copy_make(struct ab_copy_batch *batch, uint32_t index)
 {
