@@ -578,3 +578,216 @@ def test_publish_reduce_bf16_prepare():
     graph = C.c_uint32(7)
     assert lib.backend_b200_step_capture(None, launch, 1, 0, None, 0, 0, None, 0, C.byref(graph)) == 1
     assert lib.backend_b200_graph_run_wait(None, 0) == 1 and graph.value == 7
+
+
+def mx_layer_records(wide, shared=1, block128=True, rows=None):
+    """An original-weights layer's records as the layer class fills them, on its own layout."""
+    from anemone_b200.moe import MoeConfig
+    from anemone_b200.mx import MxLayout
+    rows = rows or (300 if wide else 8)
+    c = MoeConfig(hidden=1024, inner=384, experts=12, shared=shared, picks=3, row_capacity=rows, activation_limit=7.0)
+    L = MxLayout(c, 1, 0, block128=block128, wide=wide)
+    quantize = R.MxQuantize(R.ActivationQuantize(L.tokens, L.at["codes"], L.at["exponents"], 0, c.hidden, 0),
+                            L.stream_codes, L.step, rows, 0)
+    d = R.MxLayerDescription()
+    d.workspace_offset, d.expert_table_offset, d.step_offset = L.workspace, L.expert_table, L.step
+    if wide:
+        d.row_codes = R.LinearRange(L.stream_codes, rows * c.hidden)
+        d.row_exponents = R.LinearRange(L.at["exponents"], L.sizes["exponents"])
+        for name in L.tile_sizes:
+            setattr(d, name, R.LinearRange(L.tile_at[name], L.tile_sizes[name]))
+    else:
+        d.jobs, d.codes = R.LinearRange(L.jobs, L.job_capacity * 96), R.LinearRange(L.stream_codes, rows * c.hidden)
+        for name in ("exponents", "hidden_codes", "hidden_exponents"):
+            setattr(d, name, R.LinearRange(L.at[name], L.sizes[name]))
+    d.pair_output = R.LinearRange(L.at["pair_output"], L.sizes["pair_output"])
+    if shared:
+        for name in ("hidden_codes", "hidden_exponents", "output"):
+            setattr(d, "shared_" + name, R.LinearRange(L.shared_at[name], L.shared_sizes[name]))
+        d.shared_weights_offset = (C.c_uint64 * 3)(*L.shared_matrices)
+        d.shared_format = 6 if block128 else 5
+    d.hidden_size, d.inner_size, d.expert_count, d.picks, d.row_capacity = c.hidden, 384, c.experts, c.picks, rows
+    d.activation_limit = 7.0
+    return c, L, quantize, d
+
+
+def changed(record, **values):
+    copy = type(record).from_buffer_copy(bytes(record))
+    for path, value in values.items():
+        *owners, name = path.split("__")
+        target = copy
+        for owner in owners:
+            target = getattr(target, owner)
+        assert hasattr(target, name), path
+        setattr(target, name, value)
+    return copy
+
+
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("shared,block128", [(0, False), (1, False), (1, True)])
+def test_mx_products_prepare(wide, shared, block128):
+    """The original-weights products on the tensor cores: launches and records of both forms, and what is refused: every
+    range too short, beyond the arena, off its alignment or over another; widths, counts and limits out of their range."""
+    lib, fake = api.library(), FakeBackend()
+    c, L, _, d = mx_layer_records(wide, shared, block128)
+    prepare = lib.mx_products_prepare
+    prepare.argtypes = [C.POINTER(R.MxLayerDescription), C.c_uint64, C.POINTER(api.BackendOperations), C.c_void_p,
+                        C.POINTER(R.KernelLaunch), U32P]
+    launches, count = (R.KernelLaunch * 3)(), C.c_uint32(9)
+
+    def status(record, arena=L.arena_bytes):
+        return prepare(C.byref(record), arena, C.byref(fake.table), fake.card, launches, C.byref(count))
+    assert status(d) == 0
+    names = (["mx_gather"] if wide else []) + ["mx_gate_up_" + ("many" if wide else "few"),
+                                               "mx_down_" + ("many" if wide else "few")]
+    assert [key[:2] for key in fake.asked] == [("kernel_mx_tensor", name) for name in names] and count.value == len(names)
+    made = list(launches)[:count.value]
+    assert all(bytes(l.argument[l.argument_byte_count:]).count(0) == 192 - l.argument_byte_count for l in made)
+    products = made[-2:]
+    assert [(tuple(l.grid), l.block[0], l.branch) for l in products] == \
+        [((148, 1, 1), 896, R.LAUNCH_CHAIN | R.LAUNCH_OVERLAPS_PREVIOUS)] * 2
+    if wide:
+        tiles = api.prefill_parts(c.row_capacity, c.picks, 0, c.experts, c.hidden, 384).tile_capacity
+        always_on = -(-c.row_capacity // (32 if block128 else 128)) if shared else 0
+        assert tuple(made[0].grid) == (tiles + always_on, 2, 1) and made[0].block[0] == 256
+    untouched = bytes(launches)
+    count.value = 9
+    ranges = ["codes", "exponents", "hidden_codes", "hidden_exponents", "pair_output"]
+    ranges += ["row_codes", "row_exponents"] if wide else ["jobs"]
+    ranges += ["shared_output"] if shared else []
+    ranges += ["shared_hidden_codes", "shared_hidden_exponents"] if shared and not wide else []
+    for name in ranges:
+        held = getattr(d, name)
+        exact = 64 * (held.byte_count // 64)  # the smallest that holds it may be a little less than what was laid out
+        assert status(changed(d, **{name + "__byte_offset": held.byte_offset + 8})) == 1, name
+        assert status(changed(d, **{name + "__byte_offset": L.arena_bytes})) == 1, name
+        assert status(changed(d, **{name + "__byte_offset": 2 ** 64 - 64})) == 1, name
+        assert status(changed(d, **{name + "__byte_count": L.arena_bytes + 64})) == 1, name
+        if name != "jobs":
+            assert status(changed(d, **{name + "__byte_count": exact // 2})) == 1, name
+            assert status(changed(d, **{name + "__byte_offset": d.expert_table_offset})) == 1, name
+    if not wide:
+        assert status(changed(d, jobs__byte_count=95)) == 1
+    for field, values in (("hidden_size", (0, 1088, 64, 2 ** 32 - 128)), ("inner_size", (0, 320, 2 ** 32 - 128)),
+                          ("expert_count", (0, 513)), ("picks", (0, 17)), ("row_capacity", (0, 65536)),
+                          ("activation_limit", (0.0, -1.0, float("nan"), float("inf"))), ("reserved_zero", (1,)),
+                          ("shared_format", (3, 4, 7)), ("step_offset", (d.step_offset + 8, L.arena_bytes)),
+                          ("expert_table_offset", (d.expert_table_offset + 4, L.arena_bytes, d.step_offset))):
+        for value in values:
+            assert status(changed(d, **{field: value})) == 1, (field, value)
+    if wide:
+        assert status(changed(d, workspace_offset=L.arena_bytes)) == 1
+    if shared:
+        for which in range(3):
+            for value in (L.shared_matrices[which] + 8, L.arena_bytes, d.codes.byte_offset):
+                broken = changed(d)
+                broken.shared_weights_offset[which] = value
+                assert status(broken) == 1, (which, value)
+        assert wide or status(changed(d, row_capacity=9)) == 1  # an always-on expert: eight rows in the short form
+    assert status(d, 4096) == 1
+    for index in range(6):
+        arguments = [C.byref(d), L.arena_bytes, C.byref(fake.table), fake.card, launches, C.byref(count)]
+        if index != 1:
+            arguments[index] = None
+            assert prepare(*arguments) == 1, index
+    assert bytes(launches) == untouched and count.value == 9
+
+
+def test_mx_quantize_prepare():
+    lib, fake = api.library(), FakeBackend()
+    for rows, blocks in ((8, 16), (4096, 8 * 148)):
+        c, L, quantize, _ = mx_layer_records(True, rows=rows)
+        prepare = lib.mx_quantize_prepare
+        prepare.argtypes = [C.POINTER(R.MxQuantize), C.c_uint64, C.POINTER(api.BackendOperations), C.c_void_p,
+                            C.POINTER(R.KernelLaunch)]
+        launch = R.KernelLaunch()
+
+        def status(record, arena=L.arena_bytes):
+            return prepare(C.byref(record), arena, C.byref(fake.table), fake.card, C.byref(launch))
+        assert status(quantize) == 0 and fake.asked[-1] == ("kernel_mx_tensor", "mx_quantize", C.sizeof(R.MxQuantize))
+        assert tuple(launch.grid) == (blocks, 1, 1) and launch.block[0] == 256 and launch.branch == R.LAUNCH_CHAIN
+        assert bytes(launch.argument[:launch.argument_byte_count]) == bytes(quantize)
+        untouched = bytes(launch)
+        for values in (dict(base__width=0), dict(base__width=96), dict(row_capacity=0), dict(row_capacity=2 ** 32 - 1),
+                       dict(reserved_zero=1), dict(base__reserved_zero=1), dict(stream_offset=quantize.base.codes_offset),
+                       dict(stream_offset=L.arena_bytes), dict(step_offset=L.step + 8), dict(step_offset=L.tokens),
+                       dict(base__values_offset=L.tokens + 2), dict(base__codes_offset=L.arena_bytes - 64),
+                       dict(base__exponents_offset=quantize.base.values_offset)):
+            assert status(changed(quantize, **values)) == 1, values
+        assert status(quantize, 4096) == 1
+        for index in (0, 2, 3, 4):
+            arguments = [C.byref(quantize), L.arena_bytes, C.byref(fake.table), fake.card, C.byref(launch)]
+            arguments[index] = None
+            assert prepare(*arguments) == 1, index
+        assert bytes(launch) == untouched
+
+
+def test_mx_route_quantize_prepare():
+    lib, fake = api.library(), FakeBackend()
+    c, L, quantize, _ = mx_layer_records(False)
+    router = R.RouterSelectB200(L.scores, L.expert_table, L.picks, L.weights, L.jobs, L.step, c.experts, 0, c.picks,
+                                c.row_capacity, L.job_capacity, c.scoring, c.route_scale, 0)
+    both, launch = R.MxRouteQuantize(router, quantize), R.KernelLaunch()
+    prepare = lib.mx_route_quantize_prepare
+    prepare.argtypes = [C.POINTER(R.MxRouteQuantize), C.c_uint64, C.POINTER(api.BackendOperations), C.c_void_p,
+                        C.POINTER(R.KernelLaunch)]
+
+    def status(record, arena=L.arena_bytes):
+        return prepare(C.byref(record), arena, C.byref(fake.table), fake.card, C.byref(launch))
+    assert status(both) == 0 and fake.asked[-1] == ("kernel_router_b200", "mx_route_quantize", C.sizeof(both))
+    assert tuple(launch.grid) == (1 + 8 * 16 // 32, 1, 1) and launch.block[0] == 1024
+    assert launch.branch == R.LAUNCH_CHAIN | R.LAUNCH_OVERLAPS_PREVIOUS
+    assert bytes(launch.argument[:launch.argument_byte_count]) == bytes(both)
+    untouched = bytes(launch)
+    for values in (dict(router__picks=0), dict(router__picks=17), dict(router__expert_count=513),
+                   dict(router__row_capacity=65), dict(router__scores_offset=L.scores + 4),
+                   dict(router__jobs_offset=L.arena_bytes), dict(router__scoring=9),
+                   dict(router__route_scale=float("nan")), dict(quantize__base__width=96),
+                   dict(quantize__row_capacity=0), dict(quantize__reserved_zero=1),
+                   dict(quantize__stream_offset=L.arena_bytes), dict(quantize__step_offset=L.step + 4),
+                   dict(quantize__base__codes_offset=L.tokens)):
+        assert status(changed(both, **values)) == 1, values
+    assert status(both, 4096) == 1
+    for index in (0, 2, 3, 4):
+        arguments = [C.byref(both), L.arena_bytes, C.byref(fake.table), fake.card, C.byref(launch)]
+        arguments[index] = None
+        assert prepare(*arguments) == 1, index
+    assert bytes(launch) == untouched
+
+
+def test_router_tiles_prepare():
+    lib, fake = api.library(), FakeBackend()
+    c, L, _, _ = mx_layer_records(True)
+    routing = R.Exl3Prefill()
+    routing.scores_offset, routing.expert_table_offset = L.scores, L.expert_table
+    routing.picks_offset, routing.weights_offset, routing.workspace_offset = L.picks, L.weights, L.workspace
+    routing.step_offset, routing.input_size, routing.inner_size = L.step, c.hidden, 384
+    routing.expert_count = routing.local_count = c.experts
+    routing.picks, routing.row_capacity, routing.scoring, routing.route_scale = c.picks, 300, 0, 1.0
+    prepare = lib.router_tiles_prepare
+    prepare.argtypes = [C.POINTER(R.Exl3Prefill), C.c_uint64, C.POINTER(api.BackendOperations), C.c_void_p,
+                        C.POINTER(R.KernelLaunch)]
+    launches = (R.KernelLaunch * 3)()
+
+    def status(record, arena=L.arena_bytes):
+        return prepare(C.byref(record), arena, C.byref(fake.table), fake.card, launches)
+    assert status(routing) == 0
+    assert [key[:2] for key in fake.asked] == [("kernel_exl3_prefill", "exl3_prefill_" + name)
+                                               for name in ("picks", "group", "tiles")]
+    assert [(l.grid[0], l.block[0]) for l in launches] == [(10, 1024), (12, 256), (1, 1024)]
+    for launch in launches:
+        assert bytes(launch.argument[:launch.argument_byte_count]) == bytes(routing)
+    untouched = bytes(launches)
+    for values in (dict(expert_count=0), dict(expert_count=513, local_count=513), dict(local_first=1),
+                   dict(local_count=11), dict(shared_count=1), dict(picks=0), dict(picks=13), dict(picks=17),
+                   dict(row_capacity=0), dict(row_capacity=65536), dict(scoring=9), dict(route_scale=0.0),
+                   dict(route_scale=float("inf")), dict(workspace_offset=L.workspace + 512),
+                   dict(workspace_offset=api.align(L.arena_bytes, 1024)), dict(scores_offset=L.scores + 4),
+                   dict(picks_offset=L.weights), dict(weights_offset=L.arena_bytes), dict(step_offset=L.scores)):
+        assert status(changed(routing, **values)) == 1, values
+    assert status(routing, 4096) == 1
+    for index in (0, 2, 3, 4):
+        arguments = [C.byref(routing), L.arena_bytes, C.byref(fake.table), fake.card, launches]
+        arguments[index] = None
+        assert prepare(*arguments) == 1, index
+    assert bytes(launches) == untouched
