@@ -1,6 +1,7 @@
 """The original-weights layer's tensor-core products (mx_gate_up_*, mx_down_*) against the CPU oracle, on the card's own
-picks and quantized rows: tiles that are full, ragged and of one row, widths whose last stage of 256 inputs is half
-empty, both storage forms of the always-on expert and none."""
+picks and quantized rows, and every product against 64 bits on the card's own quantized vectors: tiles that are full,
+ragged and of one row, widths whose last stage of 256 inputs is half empty, both storage forms of the always-on expert and
+none."""
 import ctypes as C
 
 import numpy as np
@@ -9,6 +10,7 @@ import pytest
 from anemone_b200 import records as R
 from anemone_b200 import synthetic
 from oracle.binding import ptr, u8p
+from tests import mx_exact
 
 pytestmark = pytest.mark.gpu
 
@@ -86,6 +88,10 @@ def test_layer_matches_oracle(oracle, rows, capacity, hidden, inner, experts, pi
         assert np.abs(got - want).max() <= max(2e-2, 2.0 ** -6 * np.abs(want).max())
         a, b = got.reshape(-1).astype(np.float64), want.reshape(-1).astype(np.float64)
         assert a @ b / (np.linalg.norm(a) * np.linalg.norm(b)) >= 0.9999
+        # Sums in another order round a gate or an up to its other bfloat16 neighbour for about one value in a thousand,
+        # and one in sixteen of those moves a hidden value by a step of E4M3 (2^-3.5 of it): 2^-3.5 sqrt(1e-3 / 16) is
+        # 7e-4 of the outputs' norm; four times that for the few hundred vectors of the smallest case
+        assert np.linalg.norm(a - b) <= 2.8e-3 * np.linalg.norm(b)
     got = outputs(received, at["pair_output"], rows * picks)
     close(got, outputs(expected, at["pair_output"], rows * picks))
     summed = np.zeros((rows, H), dtype=np.float32)
@@ -108,3 +114,58 @@ def test_layer_matches_oracle(oracle, rows, capacity, hidden, inner, experts, pi
         summed = (summed + joined).astype(np.float32)
     # row sums, the join and the reduction: bit for bit given what the card wrote
     assert np.array_equal(result, synthetic.to_bfloat16(np.float32(0.0) + summed))
+    check_products(received, L, rows, chosen, weights, matrices, always, block128)
+
+
+def check_products(received, L, rows, chosen, weights, matrices, always, block128):
+    """Every expert's hidden vectors from the card's quantized rows, and its outputs from the card's hidden vectors, in 64
+    bits, with the bound of FP32 sums."""
+    H, I, picks, experts = L.config.hidden, L.inner_local, L.config.picks, L.config.experts
+
+    def span(offset, count, dtype=np.uint8):
+        return received[offset:offset + count * np.dtype(dtype).itemsize].view(dtype)
+    row_values = mx_exact.vectors(mx_exact.from_stream_order(span(L.stream_codes, rows * H).reshape(rows, H)),
+                                  span(L.at["exponents"], rows * H // 32).reshape(rows, H // 32))
+    if L.wide:  # tiles of 128 vectors in operand order: 16 bytes of an input group a vector; 512 bytes of scales a block
+        tiles = L.tile_sizes["codes"] // (128 * H)
+        codes = span(L.tile_at["hidden_codes"], tiles * 128 * I).reshape(tiles, I // 16, 128, 16)
+        codes = codes.transpose(0, 2, 1, 3).reshape(tiles, 128, I)
+        scales = span(L.tile_at["hidden_exponents"], tiles * 4 * I).reshape(tiles, I // 128, 32, 4, 4)  # row % 32, row / 32
+        scales = scales.transpose(0, 3, 2, 1, 4).reshape(tiles, 128, I // 32)
+    else:
+        pair_codes = span(L.at["hidden_codes"], L.pairs * I).reshape(L.pairs, I)
+        pair_exponents = span(L.at["hidden_exponents"], L.pairs * I // 32).reshape(L.pairs, I // 32)
+
+    def check(at_rows, route, hidden, exponents, gate, up, down, outputs):
+        hidden = mx_exact.from_stream_order(hidden)
+        mx_exact.check_hidden(hidden, exponents, gate, up, row_values[at_rows], route, 7.0)
+        mx_exact.check_outputs(outputs, down, mx_exact.vectors(hidden, exponents))
+    pair_outputs = synthetic.from_bfloat16(span(L.at["pair_output"], L.pairs * H, np.uint16)).reshape(L.pairs, H)
+    tile = 0
+    for expert in range(experts):
+        at_rows, slots = np.nonzero(chosen == expert)
+        if at_rows.size == 0:
+            continue
+        pairs = at_rows * picks + slots
+        if L.wide:
+            count = -(-at_rows.size // 128)
+            hidden = codes[tile:tile + count].reshape(-1, I)[:at_rows.size]
+            exponents = scales[tile:tile + count].reshape(-1, I // 32)[:at_rows.size]
+            tile += count
+        else:
+            hidden, exponents = pair_codes[pairs], pair_exponents[pairs]
+        gate, up, down = (mx_exact.mx_weights(data, o, i) for data, (o, i) in zip(matrices[expert],
+                                                                                  ((I, H), (I, H), (H, I))))
+        check(at_rows, weights[at_rows, slots], hidden, exponents, gate, up, down, pair_outputs[pairs])
+    if always is None:
+        return
+    if L.wide:
+        first, held = tiles - (L.config.row_capacity + 31) // 32, 32 if block128 else 128
+        hidden = np.concatenate([codes[first + base // held, :min(held, rows - base)] for base in range(0, rows, held)])
+        exponents = np.concatenate([scales[first + base // held, :min(held, rows - base)] for base in range(0, rows, held)])
+    else:
+        hidden = span(L.shared_at["hidden_codes"], rows * I).reshape(rows, I)
+        exponents = span(L.shared_at["hidden_exponents"], rows * I // 32).reshape(rows, I // 32)
+    gate, up, down = (mx_exact.e4m3_weights(data, o, i, block128) for data, (o, i) in zip(always, ((I, H), (I, H), (H, I))))
+    outputs = synthetic.from_bfloat16(span(L.shared_at["output"], rows * H, np.uint16)).reshape(rows, H)
+    check(np.arange(rows), np.ones(rows), hidden, exponents, gate, up, down, outputs)
