@@ -33,16 +33,21 @@ WEIGHT_FORMAT_E4M3_SCALED = 5
 WEIGHT_FORMAT_E4M3_BLOCK128 = 6
 
 
-# Below this many weights a matrix a call of many rows keeps the mma.sync group products: a unit of the tensor-core
-# launches (128 rows of a matrix, all of its inputs) is then a handful of stages, and a tile of 128 batch rows hardly any.
-TENSOR_WIDE_WEIGHTS = 1 << 18
+# A prompt's products stay with mma.sync (group products) for matrices of fewer weights AND fewer (row, expert) pairs than
+# these: the launches are then mostly their own beginnings and ends, and five smaller ones do it as fast as the three
+# that set tensor memory up. The layer's graph, 12 to 256 experts of 2^14 to 2^17.6 weights: under 1024 pairs mma.sync
+# takes 0.89 to 1.30 of the tensor cores' time (59 to 117 us), level in the middle, from 1024 pairs on 0.96 to 3.1 of it
+# (256 experts, 512 x 256, top 8: 1024 rows 265 against 125 us). From 2^18 weights on 0.90 to 3.2 whatever the rows, 40 of
+# 45 points above 1.05.
+TENSOR_WIDE_WEIGHTS, TENSOR_WIDE_PAIRS = 1 << 18, 1024
 
 
 def tensor_products(config, inner_local, wide, many):
     """Whether the products run on the fifth-generation tensor cores: whole blocks of 128 inputs and units of 128
-    outputs, and for many rows matrices that are worth it."""
+    outputs, and for many rows matrices or rows that are worth it."""
     H = config.hidden
-    return H % 128 == 0 and inner_local % 128 == 0 and (not wide or (many and H * inner_local >= TENSOR_WIDE_WEIGHTS))
+    worth_it = H * inner_local >= TENSOR_WIDE_WEIGHTS or config.row_capacity * config.picks >= TENSOR_WIDE_PAIRS
+    return H % 128 == 0 and inner_local % 128 == 0 and (not wide or (many and worth_it))
 
 
 def matrix_bytes(outputs, inputs):
@@ -127,8 +132,11 @@ class MxLayer:
         """matrices: iterable over the routed experts of this rank's (gate, up, down) stored MXFP4 bytes;
         shared_matrices: the always-on expert's (gate, up, down) stored E4M3 bytes, where the configuration has one:
         WEIGHT_FORMAT_E4M3_SCALED, or with block128 WEIGHT_FORMAT_E4M3_BLOCK128 (one FP32 scale per 128 by 128).
-        side_run: the always-on expert's launches as a side run of the step's graph, beside the routed experts' (the
-        same values either way: the two touch disjoint ranges until the launch that joins them)."""
+        slices, shared_slices, side_run: of the mma.sync launches alone (where tensor_products says so, the tensor cores
+        sum all of K and the always-on expert stands in the same launches, and these say nothing): the chains a sum over K
+        is cut in, of the routed and of the always-on expert; the always-on expert's launches as a side run of the step's
+        graph, beside the routed experts' (the same values either way: the two touch disjoint ranges until the launch that
+        joins them)."""
         self.card, self.config = card, config
         self.layout = L = MxLayout(config, rank_count, rank, pool_entries, block128, wide)
         assert card.arena_bytes >= L.arena_bytes

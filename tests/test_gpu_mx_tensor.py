@@ -23,6 +23,9 @@ pytestmark = pytest.mark.gpu
     (130, 160, 1152, 256, 5, 2, "e8m0"),  # 1152 = four stages and a half; an always-on tile of two rows
     (203, 256, 1024, 384, 12, 3, "block128"),  # ragged tiles, one of two and more; 384 = a stage and a half
     (9, 16, 1024, 512, 40, 8, "block128"),  # a row or two an expert
+    (700, 700, 128, 128, 6, 2, "block128"),  # small matrices that many pairs bring here: a stage of one block, all through
+    (345, 512, 256, 128, 12, 4, "e8m0"),
+    (513, 513, 512, 384, 5, 2, None),
 ])
 def test_layer_matches_oracle(oracle, rows, capacity, hidden, inner, experts, picks, shared):
     from anemone_b200 import api
