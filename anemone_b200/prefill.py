@@ -115,6 +115,15 @@ class PrefillLayout:
         self.scores = layout.take(rows * c.experts * 4)
         self.input_bytes = layout.cursor - self.step
         assert self.tokens == self.step + 256 and self.scores == self.tokens + rows * H * 2
+        # What the ranks reach in one another's memory, in front of everything a rank's share sizes: the same offsets on
+        # every rank, however uneven the shares. The reduction's region (two parity slots of signal lines and this rank's
+        # FP32 rows) ...
+        self.slot_input = SIGNAL_BYTES
+        self.parity_stride = api.align(SIGNAL_BYTES + rows * H * 4, LINE)
+        self.region = layout.take(2 * self.parity_stride, LINE)
+        # ... and its result, the status block directly in front: one copy brings both back
+        self.status = layout.take(16 + rows * H * 2)
+        self.result = self.status + 16
         self.picks = layout.take(rows * c.picks * 4)
         self.weights = layout.take(rows * c.picks * 4)
         self.expert_table = layout.take(self.local_experts * 24)
@@ -124,13 +133,6 @@ class PrefillLayout:
         self.workspace = layout.take(self.parts.total, 1024)
         self.pair_outputs = layout.take(rows * self.pairs_per_row * H * 4)
         self.row_output = layout.take(rows * H * 4)
-        # the reduction's region (two parity slots of signal lines and this rank's FP32 rows) and its result
-        self.slot_input = SIGNAL_BYTES
-        self.parity_stride = api.align(SIGNAL_BYTES + rows * H * 4, LINE)
-        self.region = layout.take(2 * self.parity_stride, LINE)
-        # the status block stands directly in front of the result: one copy brings both back
-        self.status = layout.take(16 + rows * H * 2)
-        self.result = self.status + 16
         self.matrices = []
         for local in range(self.local_experts):
             width = int(widths[local])
