@@ -194,6 +194,54 @@ def test_prefill_expert_parallel(api, oracle, mode):
                 card.close()
 
 
+@pytest.mark.parametrize("count", [2, 4])
+def test_staged_prompt_in_pieces_across_cards(api, monkeypatch, count):
+    """A staged call in pieces on R cards, a thread a card: two or four reductions of different row counts a call through
+    the same two slots, call after call, against the whole call's bits."""
+    from concurrent.futures import ThreadPoolExecutor
+    from anemone_b200 import prefill
+    from anemone_b200.prefill import PrefillLayer, PrefillLayout, Share
+    rows = 1100
+    monkeypatch.setattr(prefill, "call_pieces", lambda *_: count)
+    for ranks in world_sizes(api):
+        config = MoeConfig(hidden=512, inner=128 * ranks, experts=8 * ranks + 1, shared=1, picks=4, row_capacity=rows)
+        rng = np.random.default_rng(600 + ranks)
+        widths = np.full(config.total_experts, 3, dtype=np.uint32)
+        matrices = [(synthetic.exl3_matrix(rng, config.hidden, config.inner, 3),
+                     synthetic.exl3_matrix(rng, config.hidden, config.inner, 3),
+                     synthetic.exl3_matrix(rng, config.inner, config.hidden, 3)) for _ in widths]
+        cards, layers = [], []
+        try:
+            for rank in range(ranks):
+                share = Share.expert_parallel(config, ranks, rank)  # uneven: an expert more on the last rank
+                held = share.experts(config)
+                card = api.Card(rank, PrefillLayout(config, widths[held], share).arena_bytes)
+                cards.append(card)
+                local = [share.matrices(config, e, 3, *matrices[e]) for e in held]
+                layers.append(PrefillLayer(card, config, widths[held], local, share, rank=rank, rank_count=ranks))
+            for layer in layers:
+                layer.connect_local(layers)
+            for card in cards:
+                card.wait()
+            with ThreadPoolExecutor(ranks) as pool:
+                for _ in range(3):
+                    tokens = synthetic.tokens(rng, rows, config.hidden)
+                    scores = rng.normal(0, 1, size=(rows, config.experts)).astype(np.float32)
+                    for layer in layers:
+                        layer.stage(0, tokens, scores)
+                    result_at = [api.align(layer.layout.input_bytes, 4096) for layer in layers]
+                    staged = list(pool.map(lambda pair: pair[0].call(0, pair[1]).copy(), zip(layers, result_at)))
+                    for layer in layers:  # queue every rank before waiting for any
+                        layer.load(tokens, scores)
+                    for layer in layers:
+                        layer.run()
+                    for layer, got in zip(layers, staged):
+                        assert np.array_equal(layer.result(rows), got)
+        finally:
+            for card in cards:
+                card.close()
+
+
 @pytest.mark.parametrize("payload", [0, 1])
 def test_push_and_owner_sums_across_cards(api, oracle, payload):
     """The one-shot push and the exchange's owner sums between real cards: every rank stores into every rank's inbox
