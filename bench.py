@@ -51,8 +51,8 @@ SEED = 20261125
 # one ncu capture of a 64-expert, 8-row launch over that launch's algorithmic bytes (the capture is too large for the
 # full workload; traffic grows in proportion to the experts streamed)
 GATE_UP_TRAFFIC_RATIO = 1.03
-# the same for the prefill's gate/up products (one capture at 32 experts and 1024 rows: 378.0 MB read and 27.0 MB
-# written against 418.8 MB of codes, scales, operands read and down operands written, some of which stay in L2) and for
+# the same for the prefill's gate/up products (one capture at 32 experts and 1024 rows: 379.4 MB read and 29.3 MB
+# written against 420.1 MB of codes, scales, operands read and down operands written, some of which stay in L2) and for
 # the original-weights gate/up products (one capture at 64 experts: 427.1 MB against 427.0 MB)
 PREFILL_TRAFFIC_RATIO = 0.97
 MX_GATE_UP_TRAFFIC_RATIO = 1.00
