@@ -99,7 +99,8 @@ def check_hidden(codes, exponents, gate, up, values, route_weights, limit):
         rounded.append(bfloat16(exact))
     g, u = rounded
     bounded_gate = np.minimum(g, np.float32(limit))
-    gated = (bounded_gate / (np.float32(1.0) + np.exp(-bounded_gate))).astype(np.float32)
+    with np.errstate(over="ignore"):  # a gate far below zero: its sigmoid is zero
+        gated = (bounded_gate / (np.float32(1.0) + np.exp(-bounded_gate))).astype(np.float32)
     hidden = (gated * np.clip(u, -np.float32(limit), np.float32(limit))).astype(np.float32)
     hidden = bfloat16((hidden * route_weights[:, None].astype(np.float32)).astype(np.float32))
     largest = np.maximum(np.abs(hidden.reshape(hidden.shape[0], -1, 32)).max(axis=2), np.float32(1e-4))
