@@ -136,26 +136,41 @@ __device__ __forceinline__ uint32_t exl3_pair(uint32_t low_state, uint32_t high_
 	return *reinterpret_cast<const uint32_t *>(&value);
 }
 
-/* state of the lane's symbol e from its two ring words, already shifted so that its first window starts at the top.
- * Widths whose windows start on a few distinct bit positions modulo 8 (K2: four, K4: two) take a state as two bytes of
- * the word shifted by that position (one shift serves every state that shares it, one byte permute a state: the
- * compiler keeps the shifted word); the other widths shift and mask. */
+/* A lane's windows lie in two words cut from its ring words: `first` begins with the first window, `last` ends with the
+ * last one, so that the first state is a shift and the last a mask. (With the second word at the first one's position the
+ * last state is a shift and a mask, and K4 needs two more shifts: 383 us a decode step instead of 373.) */
+struct exl3_windows {
+	uint32_t first, last;
+};
+
 template <uint32_t BX2>
-__device__ __forceinline__ uint32_t exl3_state_of(uint32_t high, uint32_t low, uint32_t e)
+__device__ __forceinline__ struct exl3_windows exl3_windows_of(uint32_t word0, uint32_t word1, uint32_t shift)
 {
+	constexpr uint32_t end = exl3_ring<BX2>::offset(7) + 16u;
+	struct exl3_windows windows;
+	windows.first = __funnelshift_l(word1, word0, shift);
+	/* shift + (end - 32) is 32 at most: K4's shift is 20 in every lane, the other widths' starts are even or 3 modulo 8 */
+	windows.last = end > 32u ? __funnelshift_lc(word1, word0, shift + (end - 32u)) : 0u;
+	return windows;
+}
+
+/* State of the lane's symbol e. Widths whose windows start on a few distinct bit positions modulo 8 (K2: four, K4: two)
+ * take a state as two bytes of a word shifted by that position (one shift serves every state that shares it, one byte
+ * permute a state: the compiler keeps the shifted word); the other widths shift and mask. */
+template <uint32_t BX2>
+__device__ __forceinline__ uint32_t exl3_state_of(const struct exl3_windows &windows, uint32_t e)
+{
+	constexpr uint32_t end = exl3_ring<BX2>::offset(7) + 16u;
 	const uint32_t offset = exl3_ring<BX2>::offset(e);
-	if (offset == 0u)
-		return high >> 16;
+	const uint32_t word = offset <= 16u ? windows.first : windows.last;
+	const uint32_t distance = offset <= 16u ? 16u - offset : end - 16u - offset; /* of the state's last bit from the word's */
+	if (distance == 16u)
+		return word >> 16;
 	if (BX2 == 4u || BX2 == 8u) {
-		/* the 32 bits the state lies in: the first word, or the window that begins 16 bits into it */
-		const uint32_t word = offset <= 16u ? high : __funnelshift_r(low, high, 16);
-		const uint32_t distance = (offset <= 16u ? 16u : 32u) - offset; /* of the state's last bit from the word's */
 		const uint32_t byte = distance / 8u; /* 0, 1 or 2: the state is bytes byte, byte + 1 of the shifted word */
 		return __byte_perm(word >> (distance % 8u), 0u, byte == 0u ? 0x4410u : byte == 1u ? 0x4421u : 0x4432u);
 	}
-	if (offset <= 16u)
-		return (high >> (16u - offset)) & 0xFFFFu;
-	return __funnelshift_r(low, high, 48u - offset) & 0xFFFFu;
+	return (word >> distance) & 0xFFFFu;
 }
 
 /* The four A registers of m16n8k16 for one tile: symbols {0,1}, {4,5}, {2,3}, {6,7} of the lane. */
@@ -163,12 +178,11 @@ template <uint32_t BX2>
 __device__ __forceinline__ void exl3_decode_fragment(uint32_t word0, uint32_t word1, uint32_t shift,
 						      uint32_t fragment[4])
 {
-	const uint32_t high = __funnelshift_l(word1, word0, shift);
-	const uint32_t low = word1 << shift;
-	fragment[0] = exl3_pair(exl3_state_of<BX2>(high, low, 0), exl3_state_of<BX2>(high, low, 1));
-	fragment[1] = exl3_pair(exl3_state_of<BX2>(high, low, 4), exl3_state_of<BX2>(high, low, 5));
-	fragment[2] = exl3_pair(exl3_state_of<BX2>(high, low, 2), exl3_state_of<BX2>(high, low, 3));
-	fragment[3] = exl3_pair(exl3_state_of<BX2>(high, low, 6), exl3_state_of<BX2>(high, low, 7));
+	const struct exl3_windows windows = exl3_windows_of<BX2>(word0, word1, shift);
+	fragment[0] = exl3_pair(exl3_state_of<BX2>(windows, 0), exl3_state_of<BX2>(windows, 1));
+	fragment[1] = exl3_pair(exl3_state_of<BX2>(windows, 4), exl3_state_of<BX2>(windows, 5));
+	fragment[2] = exl3_pair(exl3_state_of<BX2>(windows, 2), exl3_state_of<BX2>(windows, 3));
+	fragment[3] = exl3_pair(exl3_state_of<BX2>(windows, 6), exl3_state_of<BX2>(windows, 7));
 }
 
 __device__ __forceinline__ void mma_f16(float accumulator[4], const uint32_t a[4], uint32_t b0, uint32_t b1)
@@ -217,10 +231,15 @@ struct exl3_product_shared {
  * [step_begin, step_begin + step_count), a multiple of EXL3_STAGE_STEPS; operand_row: FP16 [inputs] of the pair that
  * stands in this lane's column (lane / 4; columns beyond the job's rows repeat column 0 and are ignored by the caller).
  * Warp w takes step 4 r + w of round r. A lane reads its two ring words of each of the eight tiles of a step straight
- * from global memory into registers (the warp's 16 loads of a step cover 8 x 16 bits_x2 contiguous bytes), one round
- * ahead of the round it decodes, together with that round's operands: no shared memory, no barrier and no producer
- * stand between the memory system and the decode, whose instruction issue is what bounds the kernel. The operands are
- * read past the L1 (they may have been written by a launch that still runs beside this one); the weights through it.
+ * from global memory into registers (the warp's 16 loads of a step cover 8 x 16 bits_x2 contiguous bytes), a tile's words
+ * of the next round as soon as this round's are decoded, and that round's operands: no shared memory, no barrier and no
+ * producer stand between the memory system and the decode, whose instruction issue is what bounds the kernel. One round
+ * of words in registers and one round a loop turn: with two of both the loop was 800 instructions a stored width, CTAs of
+ * several widths run beside one another on a SM, and a warp waited for instructions as often as for a pipe (0.71 of 7.4
+ * cycles an issue; 0.08 of 6.2 so). A decode step of eight rows, 256 experts of 8, H 4096, I 2048: 446 us with two
+ * rounds and a copy of the loop for gate/up and one for down, 383 with one round and one copy. The
+ * operands are read past the L1 (they may have been written by a launch that still runs beside this one); the weights
+ * through it.
  * Returns true (the signature keeps a verdict for callers written for a core with bounded waits). All 128 threads
  * call it. */
 template <uint32_t BX2>
@@ -237,56 +256,50 @@ __device__ __forceinline__ bool exl3_product_core(const unsigned char *matrix, u
 	const uint32_t begin = ring::begin(lane);
 	const uint32_t word_index = begin / 32u, shift = begin % 32u, next_index = (word_index + 1u) % ring::words;
 	/* this warp's first step, the CTA's first tile */
-	const uint32_t *const words = reinterpret_cast<const uint32_t *>(matrix) + (step_begin + warp) * step_words +
-				      (uint64_t)group * EXL3_GROUP_TILES * ring::words;
+	const uint32_t *words = reinterpret_cast<const uint32_t *>(matrix) + (step_begin + warp) * step_words +
+				(uint64_t)group * EXL3_GROUP_TILES * ring::words;
 	const uint64_t round_words = EXL3_STAGE_STEPS * step_words;
 	/* this lane's B operand of round r: inputs 2 t, 2 t + 1 and 2 t + 8, 2 t + 9 of step 4 r + warp */
-	const uint32_t *const fed = reinterpret_cast<const uint32_t *>(operand_row + (step_begin + warp) * EXL3_TILE +
-								      (lane % 4u) * 2u);
+	const uint32_t *fed =
+		reinterpret_cast<const uint32_t *>(operand_row + (step_begin + warp) * EXL3_TILE + (lane % 4u) * 2u);
 	constexpr uint32_t fed_round_words = EXL3_STAGE_STEPS * EXL3_TILE / 2u;
+	float4 *const partial = reinterpret_cast<float4 *>(dynamic_shared); /* [warp][tile][lane] */
+
+	uint32_t held[EXL3_GROUP_TILES][2], held_fed[2];
+#pragma unroll
+	for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++) {
+		held[tile][0] = __ldg(words + tile * ring::words + word_index);
+		held[tile][1] = __ldg(words + tile * ring::words + next_index);
+	}
+	held_fed[0] = __ldcg(fed);
+	held_fed[1] = __ldcg(fed + 4);
 	float accumulators[EXL3_GROUP_TILES][4];
 #pragma unroll
 	for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++)
 #pragma unroll
 		for (uint32_t c = 0; c < 4; c++)
 			accumulators[tile][c] = 0.0f;
-
-	uint32_t first[EXL3_GROUP_TILES][2], second[EXL3_GROUP_TILES][2], first_fed[2], second_fed[2];
-#define EXL3_ROUND_LOAD(set, set_fed, round)                                                                  \
-	do {                                                                                                   \
-		const uint32_t *const from = words + (uint64_t)(round) * round_words;                          \
-		_Pragma("unroll") for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++)                     \
-		{                                                                                              \
-			set[tile][0] = __ldg(from + tile * ring::words + word_index);                          \
-			set[tile][1] = __ldg(from + tile * ring::words + next_index);                          \
-		}                                                                                              \
-		set_fed[0] = __ldcg(fed + (uint64_t)(round) * fed_round_words);                                \
-		set_fed[1] = __ldcg(fed + (uint64_t)(round) * fed_round_words + 4);                            \
-	} while (0)
-#define EXL3_ROUND_MULTIPLY(set, set_fed)                                                                     \
-	do {                                                                                                   \
-		_Pragma("unroll") for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++)                     \
-		{                                                                                              \
-			uint32_t fragment[4];                                                                  \
-			exl3_decode_fragment<BX2>(set[tile][0], set[tile][1], shift, fragment);                \
-			mma_f16(accumulators[tile], fragment, set_fed[0], set_fed[1]);                         \
-		}                                                                                              \
-	} while (0)
-	EXL3_ROUND_LOAD(first, first_fed, 0u);
-	for (uint32_t round = 0; round < rounds; round += 2u) {
-		if (round + 1u < rounds)
-			EXL3_ROUND_LOAD(second, second_fed, round + 1u);
-		EXL3_ROUND_MULTIPLY(first, first_fed);
-		if (round + 1u >= rounds)
-			break;
-		if (round + 2u < rounds)
-			EXL3_ROUND_LOAD(first, first_fed, round + 2u);
-		EXL3_ROUND_MULTIPLY(second, second_fed);
+#pragma unroll 1
+	for (uint32_t round = 1; round <= rounds; round++) {
+		const uint32_t b0 = held_fed[0], b1 = held_fed[1];
+		const bool more = round < rounds;
+		words += round_words;
+		fed += fed_round_words;
+		if (more) {
+			held_fed[0] = __ldcg(fed);
+			held_fed[1] = __ldcg(fed + 4);
+		}
+#pragma unroll
+		for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++) {
+			uint32_t fragment[4];
+			exl3_decode_fragment<BX2>(held[tile][0], held[tile][1], shift, fragment);
+			if (more) {
+				held[tile][0] = __ldg(words + tile * ring::words + word_index);
+				held[tile][1] = __ldg(words + tile * ring::words + next_index);
+			}
+			mma_f16(accumulators[tile], fragment, b0, b1);
+		}
 	}
-#undef EXL3_ROUND_LOAD
-#undef EXL3_ROUND_MULTIPLY
-
-	float4 *const partial = reinterpret_cast<float4 *>(dynamic_shared); /* [warp][tile][lane] */
 #pragma unroll
 	for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++)
 		partial[(warp * EXL3_GROUP_TILES + tile) * EXL3_WARP + lane] = make_float4(
@@ -308,7 +321,7 @@ __device__ __forceinline__ bool exl3_product_core(const unsigned char *matrix, u
 		for (uint32_t c = 0; c < 4; c++)
 			sums[mine][c] = total[c];
 	}
-	__syncthreads(); /* the partial sums are consumed: the caller may reuse the dynamic shared memory */
+	__syncthreads(); /* the partial sums are consumed: the dynamic shared memory may be used again */
 	return true;
 }
 

@@ -17,20 +17,25 @@ __device__ __forceinline__ const uint32_t *moe_widths(const struct exl3_moe_reco
 		       nullptr;
 }
 
-/* this thread's sums (exl3_product_core's layout) to partial rows: row(column) + 128 group + output */
-__device__ __forceinline__ void store_partial(const float sums[2][4], float *const rows[LINEAR_MAXIMUM_ROWS],
-					      uint32_t row_count)
+/* this thread's sums (exl3_product_core's layout) to the partial rows of the job's pairs: first: the run's row of pair 0,
+ * at the group's first output; stride: floats from one pair's row to the next */
+__device__ __forceinline__ void store_partial(const float sums[2][4], float *first, uint64_t stride,
+					      const struct expert_job_record *job)
 {
 	const uint32_t lane = threadIdx.x % EXL3_WARP, warp = threadIdx.x / EXL3_WARP;
 	const uint32_t group_lane = lane / 4u, place = lane % 4u;
 #pragma unroll
-	for (uint32_t mine = 0; mine < 2; mine++)
+	for (uint32_t odd = 0; odd < 2; odd++) {
+		const uint32_t column = place * 2u + odd;
+		if (column >= job->row_count)
+			break;
+		float *const to = first + job->pair_index[column] * stride + warp * (2u * EXL3_TILE) + group_lane;
 #pragma unroll
-		for (uint32_t c = 0; c < 4; c++) {
-			const uint32_t column = place * 2u + (c & 1u);
-			if (column < row_count)
-				rows[column][(warp * 2u + mine) * EXL3_TILE + group_lane + (c >> 1) * 8u] = sums[mine][c];
+		for (uint32_t mine = 0; mine < 2; mine++) {
+			to[mine * EXL3_TILE] = sums[mine][odd];
+			to[mine * EXL3_TILE + 8u] = sums[mine][2u + odd];
 		}
+	}
 }
 
 /* true in exactly one CTA of the `expected` that work on this counter: the last to arrive. Every CTA's partial sums are
@@ -68,9 +73,8 @@ __device__ __forceinline__ void sum_runs(const float *first_run, uint64_t run_st
  * group's gate and up products: gate_first / up_first: run 0 of the FP32 partial rows [pair][inner] of each, the
  * further runs run_stride floats apart. Writes the bfloat16 hidden values and the FP16 down operands (behind the
  * gate/up operands, which other CTAs of the launch still read). All 128 threads call. */
-template <uint32_t BX2>
 __device__ __forceinline__ void exl3_gate_up_epilogue(const struct exl3_moe_record &moe, unsigned char *arena,
-						      const struct expert_job_record *job, uint32_t group,
+						      const struct expert_job_record *job, uint32_t bits_x2, uint32_t group,
 						      const float *gate_first, const float *up_first, uint64_t run_stride,
 						      uint32_t gate_runs, uint32_t up_runs)
 {
@@ -78,11 +82,11 @@ __device__ __forceinline__ void exl3_gate_up_epilogue(const struct exl3_moe_reco
 	const uint32_t lane = threadIdx.x % EXL3_WARP, warp = threadIdx.x / EXL3_WARP;
 	const uint32_t H = record.input_size, I = record.inner_size, pairs = record.pair_count;
 	const uint32_t channel = group * EXL3_TRANSFORM + lane * 4u;
-	const uint64_t codes = exl3_code_bytes(H, I, BX2);
+	const uint64_t codes = exl3_code_bytes(H, I, bits_x2);
 	float gate_scale[4], up_scale[4], down_scale[4];
 	load_half4(reinterpret_cast<const __half *>(arena + job->gate_offset + codes) + H + channel, gate_scale);
 	load_half4(reinterpret_cast<const __half *>(arena + job->up_offset + codes) + H + channel, up_scale);
-	load_half4(reinterpret_cast<const __half *>(arena + job->down_offset + exl3_code_bytes(I, H, BX2)) + channel,
+	load_half4(reinterpret_cast<const __half *>(arena + job->down_offset + exl3_code_bytes(I, H, bits_x2)) + channel,
 		   down_scale);
 	for (uint32_t column = warp; column < job->row_count; column += EXL3_PRODUCT_WARPS) {
 		const uint64_t at = (uint64_t)job->pair_index[column] * I + channel;
@@ -116,9 +120,9 @@ __device__ __forceinline__ void exl3_gate_up_epilogue(const struct exl3_moe_reco
 /* The finish of a job's rows for one group of 128 outputs by the CTA that completed the group's down products:
  * first: run 0 of the FP32 partial rows [pair][input_size]; writes the pair outputs (transform, scale, route
  * weight) at output_offset. All 128 threads call. */
-template <uint32_t BX2>
 __device__ __forceinline__ void exl3_down_epilogue(const struct exl3_moe_record &moe, unsigned char *arena,
-						   const struct expert_job_record *job, uint32_t group, const float *first,
+						   const struct expert_job_record *job, uint32_t bits_x2, uint32_t group,
+						   const float *first,
 						   uint64_t run_stride, uint32_t runs, uint64_t output_offset)
 {
 	const struct exl3_expert_record &record = moe.base;
@@ -126,7 +130,7 @@ __device__ __forceinline__ void exl3_down_epilogue(const struct exl3_moe_record 
 	const uint32_t H = record.input_size, I = record.inner_size;
 	const uint32_t channel = group * EXL3_TRANSFORM + lane * 4u;
 	float scale[4];
-	load_half4(reinterpret_cast<const __half *>(arena + job->down_offset + exl3_code_bytes(I, H, BX2)) + I + channel,
+	load_half4(reinterpret_cast<const __half *>(arena + job->down_offset + exl3_code_bytes(I, H, bits_x2)) + I + channel,
 		   scale);
 	for (uint32_t column = warp; column < job->row_count; column += EXL3_PRODUCT_WARPS) {
 		const uint64_t at = (uint64_t)job->pair_index[column] * H + channel;
@@ -148,41 +152,95 @@ struct moe_item {
 	uint32_t job, group, run, projection;
 };
 
-/* One item of gate or up: run item.run of K of 128 outputs of the job; the CTA that completes the (job, 128 outputs)
- * applies the activation. ready (may be null): a word a job that counts the groups whose down operands are in place. */
-template <uint32_t BX2>
-__device__ __forceinline__ void moe_gate_up(const struct exl3_moe_record &moe, unsigned char *arena,
-					    const struct expert_job_record *job, uint32_t runs,
-					    unsigned char *dynamic_shared, exl3_product_shared *shared, uint32_t *flag,
-					    uint32_t *ready, const struct moe_item &item, uint64_t)
+/* an item's product: a run of K of 128 outputs of one matrix, and this lane's column's operands */
+struct moe_product {
+	const unsigned char *matrix;
+	uint32_t outputs, group, step_begin, steps;
+	const __half *operand_row;
+};
+
+/* an item of gate or up: run item.run of K of 128 outputs of the job */
+__device__ __forceinline__ struct moe_product moe_gate_up_product(const struct exl3_moe_record &moe, unsigned char *arena,
+								  const struct expert_job_record *job,
+								  const struct moe_item &item, uint32_t runs)
 {
 	const struct exl3_expert_record &record = moe.base;
-	const uint32_t lane = threadIdx.x % EXL3_WARP;
-	const uint32_t H = record.input_size, I = record.inner_size, pairs = record.pair_count;
-	const uint32_t groups = I / EXL3_TRANSFORM;
-	const uint32_t group = item.group, run = item.run, projection = item.projection;
-	const uint32_t steps = H / EXL3_TILE / runs;
+	const uint32_t H = record.input_size, lane = threadIdx.x % EXL3_WARP;
 	const uint32_t fed_column = lane / 4u < job->row_count ? lane / 4u : 0u;
-	const __half *const operands = reinterpret_cast<const __half *>(arena + record.operands_offset);
-	float sums[2][4];
-	if (!exl3_product_core<BX2>(arena + (projection == 0 ? job->gate_offset : job->up_offset), I, group, run * steps,
-				    steps, operands + ((uint64_t)projection * pairs + job->pair_index[fed_column]) * H,
-				    dynamic_shared, shared, sums))
-		return;
+	struct moe_product product;
+	product.matrix = arena + (item.projection == 0 ? job->gate_offset : job->up_offset);
+	product.outputs = record.inner_size;
+	product.group = item.group;
+	product.steps = H / EXL3_TILE / runs;
+	product.step_begin = item.run * product.steps;
+	product.operand_row = reinterpret_cast<const __half *>(arena + record.operands_offset) +
+			      ((uint64_t)item.projection * record.pair_count + job->pair_index[fed_column]) * H;
+	return product;
+}
+
+/* the same of down, whose operands stand behind gate's and up's */
+__device__ __forceinline__ struct moe_product moe_down_product(const struct exl3_moe_record &moe, unsigned char *arena,
+							       const struct expert_job_record *job,
+							       const struct moe_item &item, uint32_t runs)
+{
+	const struct exl3_expert_record &record = moe.base;
+	const uint32_t H = record.input_size, I = record.inner_size, lane = threadIdx.x % EXL3_WARP;
+	const uint32_t fed_column = lane / 4u < job->row_count ? lane / 4u : 0u;
+	struct moe_product product;
+	product.matrix = arena + job->down_offset;
+	product.outputs = H;
+	product.group = item.group;
+	product.steps = I / EXL3_TILE / runs;
+	product.step_begin = item.run * product.steps;
+	product.operand_row = reinterpret_cast<const __half *>(arena + record.operands_offset) +
+			      (uint64_t)EXL3_PROJECTIONS * record.pair_count * H + (uint64_t)job->pair_index[fed_column] * I;
+	return product;
+}
+
+/* A product of any stored width. One call site a kernel: the K loop is unrolled over a step's tiles, once a width, and
+ * CTAs of several widths and of both kinds run beside one another on a SM and share its instruction cache
+ * (exl3_product_core). False: a width that is not stored. */
+__device__ __forceinline__ bool moe_multiply(uint32_t bits_x2, const struct moe_product &product,
+					     unsigned char *dynamic_shared, exl3_product_shared *shared, float sums[2][4])
+{
+	switch (bits_x2) {
+	case EXL3_BITS_X2_K2:
+		return exl3_product_core<EXL3_BITS_X2_K2>(product.matrix, product.outputs, product.group, product.step_begin,
+							  product.steps, product.operand_row, dynamic_shared, shared, sums);
+	case EXL3_BITS_X2_K2_5:
+		return exl3_product_core<EXL3_BITS_X2_K2_5>(product.matrix, product.outputs, product.group, product.step_begin,
+							    product.steps, product.operand_row, dynamic_shared, shared, sums);
+	case EXL3_BITS_X2_K3:
+		return exl3_product_core<EXL3_BITS_X2_K3>(product.matrix, product.outputs, product.group, product.step_begin,
+							  product.steps, product.operand_row, dynamic_shared, shared, sums);
+	case EXL3_BITS_X2_K4:
+		return exl3_product_core<EXL3_BITS_X2_K4>(product.matrix, product.outputs, product.group, product.step_begin,
+							  product.steps, product.operand_row, dynamic_shared, shared, sums);
+	default:
+		return false;
+	}
+}
+
+/* What follows a gate or up item's product; the CTA that completes the (job, 128 outputs) applies the activation. ready
+ * (may be null): a word a job that counts the groups whose down operands are in place. */
+__device__ __forceinline__ void moe_gate_up_finish(const struct exl3_moe_record &moe, unsigned char *arena,
+						   const struct expert_job_record *job, uint32_t bits_x2, uint32_t runs,
+						   uint32_t *flag, uint32_t *ready, const struct moe_item &item,
+						   const float sums[2][4])
+{
+	const struct exl3_expert_record &record = moe.base;
+	const uint32_t I = record.inner_size, pairs = record.pair_count, groups = I / EXL3_TRANSFORM;
+	const uint32_t group = item.group;
 	/* partial sums: FP32 [projection][run][pair][I] */
 	float *const partials = reinterpret_cast<float *>(arena + record.products_offset);
 	const uint64_t run_stride = (uint64_t)pairs * I;
-	float *rows[LINEAR_MAXIMUM_ROWS];
-#pragma unroll
-	for (uint32_t column = 0; column < LINEAR_MAXIMUM_ROWS; column++)
-		rows[column] = partials + ((uint64_t)projection * runs + run) * run_stride +
-			       (uint64_t)job->pair_index[column < job->row_count ? column : 0u] * I + group * EXL3_TRANSFORM;
-	store_partial(sums, rows, job->row_count);
+	store_partial(sums, partials + ((uint64_t)item.projection * runs + item.run) * run_stride + group * EXL3_TRANSFORM, I,
+		      job);
 	uint32_t *const counter = reinterpret_cast<uint32_t *>(arena + moe.counters_offset) + item.job * groups + group;
 	if (!last_of(counter, EXL3_PROJECTIONS * runs, flag))
 		return;
-	exl3_gate_up_epilogue<BX2>(moe, arena, job, group, partials, partials + (uint64_t)runs * run_stride, run_stride, runs,
-				   runs);
+	exl3_gate_up_epilogue(moe, arena, job, bits_x2, group, partials, partials + (uint64_t)runs * run_stride, run_stride,
+			      runs, runs);
 	if (ready != nullptr) { /* one more group of the job's down operands is in place, for a launch that runs beside */
 		__threadfence();
 		__syncthreads();
@@ -191,79 +249,24 @@ __device__ __forceinline__ void moe_gate_up(const struct exl3_moe_record &moe, u
 	}
 }
 
-/* The same for down: grid (input_size / 128 * runs, jobs). */
-template <uint32_t BX2>
-__device__ __forceinline__ void moe_down(const struct exl3_moe_record &moe, unsigned char *arena,
-					 const struct expert_job_record *job, uint32_t runs,
-					 unsigned char *dynamic_shared, exl3_product_shared *shared, uint32_t *flag,
-					 uint32_t *, const struct moe_item &item, uint64_t products_offset)
+/* The same for down. */
+__device__ __forceinline__ void moe_down_finish(const struct exl3_moe_record &moe, unsigned char *arena,
+						const struct expert_job_record *job, uint32_t bits_x2, uint32_t runs,
+						uint32_t *flag, const struct moe_item &item, uint64_t products_offset,
+						const float sums[2][4])
 {
 	const struct exl3_expert_record &record = moe.base;
-	const uint32_t lane = threadIdx.x % EXL3_WARP;
 	const uint32_t H = record.input_size, I = record.inner_size, pairs = record.pair_count;
-	const uint32_t groups = H / EXL3_TRANSFORM;
-	const uint32_t group = item.group, run = item.run;
-	const uint32_t steps = I / EXL3_TILE / runs;
-	const uint32_t fed_column = lane / 4u < job->row_count ? lane / 4u : 0u;
-	const __half *const operands =
-		reinterpret_cast<const __half *>(arena + record.operands_offset) + (uint64_t)EXL3_PROJECTIONS * pairs * H;
-	float sums[2][4];
-	if (!exl3_product_core<BX2>(arena + job->down_offset, H, group, run * steps, steps,
-				    operands + (uint64_t)job->pair_index[fed_column] * I, dynamic_shared, shared, sums))
-		return;
+	const uint32_t groups = H / EXL3_TRANSFORM, group = item.group;
 	/* partial sums: FP32 [run][pair][H] at products_offset; run 0's rows are also where the pair outputs go */
 	float *const partials = reinterpret_cast<float *>(arena + products_offset);
 	const uint64_t run_stride = (uint64_t)pairs * H;
-	float *rows[LINEAR_MAXIMUM_ROWS];
-#pragma unroll
-	for (uint32_t column = 0; column < LINEAR_MAXIMUM_ROWS; column++)
-		rows[column] = partials + run * run_stride +
-			       (uint64_t)job->pair_index[column < job->row_count ? column : 0u] * H + group * EXL3_TRANSFORM;
-	store_partial(sums, rows, job->row_count);
+	store_partial(sums, partials + item.run * run_stride + group * EXL3_TRANSFORM, H, job);
 	uint32_t *const counter = reinterpret_cast<uint32_t *>(arena + moe.counters_offset) +
 				  (uint64_t)record.job_count * (I / EXL3_TRANSFORM) + item.job * groups + group;
 	if (!last_of(counter, runs, flag))
 		return;
-	exl3_down_epilogue<BX2>(moe, arena, job, group, partials, run_stride, runs, products_offset);
-}
-
-#define EXL3_FUSED_WIDTH_SWITCH(function)                                                      \
-	switch (exl3_job_bits_x2(record.base, job, moe_widths(record, arena))) {               \
-	case EXL3_BITS_X2_K2:                                                                  \
-		function<EXL3_BITS_X2_K2>(record, arena, job, runs, dynamic_shared, shared, flag, ready, item, products_offset);   \
-		break;                                                                         \
-	case EXL3_BITS_X2_K2_5:                                                                \
-		function<EXL3_BITS_X2_K2_5>(record, arena, job, runs, dynamic_shared, shared, flag, ready, item, products_offset); \
-		break;                                                                         \
-	case EXL3_BITS_X2_K3:                                                                  \
-		function<EXL3_BITS_X2_K3>(record, arena, job, runs, dynamic_shared, shared, flag, ready, item, products_offset);   \
-		break;                                                                         \
-	case EXL3_BITS_X2_K4:                                                                  \
-		function<EXL3_BITS_X2_K4>(record, arena, job, runs, dynamic_shared, shared, flag, ready, item, products_offset);   \
-		break;                                                                         \
-	default:                                                                               \
-		break;                                                                         \
-	}
-
-/* one item of either kind, for an entry that walks a list of items (job: the item's) */
-__device__ __forceinline__ void exl3_moe_gate_up_item(const struct exl3_moe_record &record, unsigned char *arena,
-						      const struct moe_item &item, uint32_t runs,
-						      unsigned char *dynamic_shared, exl3_product_shared *shared,
-						      uint32_t *flag, uint32_t *ready)
-{
-	const uint64_t products_offset = 0;
-	const struct expert_job_record *const job = exl3_job(record.base, arena, item.job);
-	EXL3_FUSED_WIDTH_SWITCH(moe_gate_up)
-}
-
-__device__ __forceinline__ void exl3_moe_down_item(const struct exl3_moe_record &record, unsigned char *arena,
-						   const struct moe_item &item, uint32_t runs,
-						   unsigned char *dynamic_shared, exl3_product_shared *shared, uint32_t *flag,
-						   uint64_t products_offset)
-{
-	uint32_t *const ready = nullptr;
-	const struct expert_job_record *const job = exl3_job(record.base, arena, item.job);
-	EXL3_FUSED_WIDTH_SWITCH(moe_down)
+	exl3_down_epilogue(moe, arena, job, bits_x2, group, partials, run_stride, runs, products_offset);
 }
 
 /* the bodies of the two product kernels of the fixed cut, for any entry that holds a struct exl3_moe_record */
@@ -272,25 +275,28 @@ __device__ __forceinline__ void exl3_moe_gate_up_block(const struct exl3_moe_rec
 						       exl3_product_shared *shared, uint32_t *flag,
 						       uint32_t *ready = nullptr)
 {
-	const uint64_t products_offset = 0;
 	const struct moe_item item = { blockIdx.y, blockIdx.x / runs, blockIdx.x % runs, blockIdx.z };
 	const struct expert_job_record *const job = exl3_job(record.base, arena, blockIdx.y);
 	if (job->row_count == 0)
 		return;
-	EXL3_FUSED_WIDTH_SWITCH(moe_gate_up)
+	const uint32_t bits_x2 = exl3_job_bits_x2(record.base, job, moe_widths(record, arena));
+	float sums[2][4];
+	if (moe_multiply(bits_x2, moe_gate_up_product(record, arena, job, item, runs), dynamic_shared, shared, sums))
+		moe_gate_up_finish(record, arena, job, bits_x2, runs, flag, ready, item, sums);
 }
 
 __device__ __forceinline__ void exl3_moe_down_block(const struct exl3_moe_record &record, unsigned char *arena,
 						    uint32_t runs, unsigned char *dynamic_shared,
 						    exl3_product_shared *shared, uint32_t *flag)
 {
-	uint32_t *const ready = nullptr;
-	const uint64_t products_offset = record.base.products_offset;
 	const struct moe_item item = { blockIdx.y, blockIdx.x / runs, blockIdx.x % runs, 0u };
 	const struct expert_job_record *const job = exl3_job(record.base, arena, blockIdx.y);
 	if (job->row_count == 0)
 		return;
-	EXL3_FUSED_WIDTH_SWITCH(moe_down)
+	const uint32_t bits_x2 = exl3_job_bits_x2(record.base, job, moe_widths(record, arena));
+	float sums[2][4];
+	if (moe_multiply(bits_x2, moe_down_product(record, arena, job, item, runs), dynamic_shared, shared, sums))
+		moe_down_finish(record, arena, job, bits_x2, runs, flag, item, record.base.products_offset, sums);
 }
 
 #endif

@@ -64,6 +64,25 @@ def test_layer_single_rank(api, oracle, rows, form):
         card.close()
 
 
+@pytest.mark.parametrize("capacity, inner", [(8, 128), (32, 256), (64, 1024)])
+def test_steps_of_changing_row_counts(api, oracle, capacity, inner):
+    """One layer, steps of few and of many rows in turn: every step ends with the products' ticket at zero, whatever part
+    of the grid found work, at each cut of K the job count leads to."""
+    config = MoeConfig(hidden=1024, inner=inner, experts=16, shared=1, picks=4, row_capacity=capacity)
+    widths, matrices, tokens, scores = make_layer_inputs(70 + capacity, config, capacity)
+    layout = MoeLayout(config, widths, 1, 0)
+    card = api.Card(0, layout.arena_bytes)
+    try:
+        layer = MoeLayer(card, config, widths, matrices)
+        layer.connect_local([layer])
+        for rows in (1, capacity, 3, capacity - 1, 1):
+            expected = moe_reference.layer(oracle, config, widths, matrices, tokens[:rows], scores[:rows], 1)[0]
+            a, b = synthetic.from_bfloat16(layer.step(tokens[:rows], scores[:rows])), synthetic.from_bfloat16(expected)
+            assert np.abs(a - b).max() <= MAX_ABS and cosine(a, b) >= COSINE
+    finally:
+        card.close()
+
+
 @pytest.mark.parametrize("form", ["fused", "pull"])
 def test_router_job_table_matches_oracle(api, oracle, form):
     config = MoeConfig(hidden=512, inner=256, experts=256, shared=1, picks=8, row_capacity=32)
