@@ -165,6 +165,16 @@ def prefill_parts(row_capacity, picks, shared_count, expert_count, input_size, i
     return parts
 
 
+def rows_one(card, record):
+    """The launch behind the experts of a call of many rows on one rank (ordered_rows_one_prepare)."""
+    lib, launch = library(), R.KernelLaunch()
+    lib.ordered_rows_one_prepare.argtypes = [C.POINTER(R.OrderedRowsOne), C.c_uint64, C.POINTER(BackendOperations),
+                                             C.c_void_p, C.POINTER(R.KernelLaunch)]
+    check(lib.ordered_rows_one_prepare(C.byref(record), card.arena_bytes, card.ops_pointer, card.handle, C.byref(launch)),
+          "ordered_rows_one_prepare")
+    return launch
+
+
 def align(value, alignment):
     return (value + alignment - 1) // alignment * alignment
 

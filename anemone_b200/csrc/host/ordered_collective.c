@@ -358,3 +358,45 @@ result_status ordered_reduce_bf16_prepare(const struct ordered_reduce_bf16_descr
 	memcpy(launches_out, launches, sizeof(launches));
 	return STATUS_OK;
 }
+
+result_status ordered_rows_one_prepare(const struct ordered_rows_one_arguments *arguments, uint64_t arena_byte_count,
+				       const struct backend_operations *backend, struct device_card *card,
+				       struct kernel_launch *launch_out)
+{
+	if (arguments == NULL || backend == NULL || backend->kernel_prepare == NULL || card == NULL || launch_out == NULL)
+		return STATUS_INVALID_ARGUMENT;
+	const uint64_t rows = arguments->row_capacity;
+	const uint64_t elements = rows * arguments->width;
+	if (arguments->width == 0 || arguments->width % 8u != 0 || rows == 0 || rows > 65535u ||
+	    arguments->pairs_per_row == 0 || elements > ORDERED_B200_MAXIMUM_ELEMENTS || arguments->bf16_pairs > 1u ||
+	    arguments->reserved_zero != 0 ||
+	    (arguments->picks_offset != 0 && (arguments->picks == 0 || arguments->picks > arguments->pairs_per_row)) ||
+	    arguments->pair_output_offset % 16u != 0 || arguments->addend_offset % 16u != 0 ||
+	    arguments->row_output_offset % 16u != 0 || arguments->output_offset % 16u != 0 ||
+	    arguments->step_offset % ADDRESS_BYTES != 0 || arguments->picks_offset % 4u != 0)
+		return STATUS_INVALID_ARGUMENT;
+	const uint64_t pair_bytes = elements * (arguments->bf16_pairs != 0 ? 2u : 4u);
+	const struct checked_range ranges[6] = {
+		{ "result", arguments->output_offset, elements * 2u },
+		{ "row output", arguments->row_output_offset, elements * 4u },
+		{ "pair outputs", arguments->pair_output_offset, pair_bytes * arguments->pairs_per_row },
+		{ "picks", arguments->picks_offset, arguments->picks_offset != 0 ? rows * arguments->picks * 4u : 0u },
+		{ "addend", arguments->addend_offset, arguments->addend_offset != 0 ? elements * 2u : 0u },
+		{ "step block", arguments->step_offset, STEP_BLOCK_BYTES }
+	};
+	if (pair_bytes > UINT64_MAX / arguments->pairs_per_row ||
+	    !prepare_ranges_are_valid("ordered rows of one rank", ranges, 6, arena_byte_count))
+		return STATUS_INVALID_ARGUMENT;
+	uint32_t kernel = BACKEND_NO_KERNEL;
+	const result_status status = backend->kernel_prepare(card, KERNEL_FILE_ORDERED_B200, KERNEL_ORDERED_ROWS_ONE,
+							     sizeof(*arguments), &kernel);
+	if (status != STATUS_OK)
+		return status;
+	if (kernel == BACKEND_NO_KERNEL)
+		return STATUS_UNSUPPORTED;
+	const uint32_t vectors = arguments->width / 8u;
+	prepare_launch_fill(launch_out, kernel, (vectors + ORDERED_ROWS_ONE_THREADS - 1u) / ORDERED_ROWS_ONE_THREADS,
+			    arguments->row_capacity, 1, ORDERED_ROWS_ONE_THREADS, 0, arguments, sizeof(*arguments));
+	launch_out->branch = LAUNCH_CHAIN | LAUNCH_OVERLAPS_PREVIOUS;
+	return STATUS_OK;
+}

@@ -12,11 +12,15 @@
  *       (mode 1) a rank adds only its run of the vectors and stores the result into every rank's memory.
  *   ordered_rows_push        the two above as ONE launch for decode steps, by stores instead of loads: row sums into
  *       every rank's inbox, READY, the adds in rank order, one rounding, bfloat16 kept locally (ordered_push_device.cuh).
+ *   ordered_rows_one         grid (ceil(width / 1024), rows) x 128: one rank's whole tail of a call of many rows: row sums,
+ *       the always-on expert's rows, one rounding; no slot, no signal, no wait.
  * All read the live row count and the sequence from the step block. The read-complete barrier of the FP32
  * collectives is moved from the end of a step to the next refill of the same slot (two steps later), where it costs
  * nothing; the slot's input must therefore only ever be written by ordered_row_sum_publish.
  */
 #include "ordered_push_device.cuh"
+
+#include "anemone_b200_collective.h"
 
 /* true for exactly one block: the last of the grid to arrive. The counter is the owner's own, at `line` + 64. Every
  * block orders its stores at device scope before it counts itself; the block that sees the count complete then
@@ -190,6 +194,134 @@ extern "C" __global__ void __launch_bounds__(ORDERED_COLLECTIVE_THREADS)
 	}
 }
 
+/* ordered_rows_one: a thread eight channels of a row. Bound by the pair outputs' way from memory, each read once: 2048 rows
+ * of 4096, nine bfloat16 values each, 200 MB in all; the four launches it stands for with one rank (row sums, the
+ * always-on expert's rows, publish, reduce) wrote and read the FP32 rows three times more and met at two grid-wide counters:
+ * 134 us there, ROWS_ONE_2048 here; 333 rows 52 and ROWS_ONE_333. */
+template <bool BF16> __device__ __forceinline__ void rows_one_load(const unsigned char *at, float out[8])
+{
+	if (BF16) {
+		const uint4 raw = __ldcs(reinterpret_cast<const uint4 *>(at));
+		const uint32_t word[4] = { raw.x, raw.y, raw.z, raw.w };
+#pragma unroll
+		for (uint32_t i = 0; i < 4; i++) {
+			out[2u * i] = __uint_as_float(word[i] << 16);
+			out[2u * i + 1u] = __uint_as_float(word[i] & 0xFFFF0000u);
+		}
+	} else {
+#pragma unroll
+		for (uint32_t half = 0; half < 2; half++) {
+			const float4 value = __ldcs(reinterpret_cast<const float4 *>(at) + half);
+			out[4u * half] = value.x, out[4u * half + 1u] = value.y;
+			out[4u * half + 2u] = value.z, out[4u * half + 3u] = value.w;
+		}
+	}
+}
+
+template <bool BF16>
+__device__ __forceinline__ void rows_one(const struct ordered_rows_one_arguments &arguments, unsigned char *arena)
+{
+	const struct step_block step = *reinterpret_cast<const struct step_block *>(arena + arguments.step_offset);
+	const uint32_t channel = (blockIdx.x * blockDim.x + threadIdx.x) * 8u, width = arguments.width;
+	const uint64_t row = blockIdx.y;
+	if (channel >= width || row >= min(step.row_count, arguments.row_capacity))
+		return;
+	const uint32_t slots = arguments.pairs_per_row;
+	const uint32_t *const picked = reinterpret_cast<const uint32_t *>(arena + arguments.picks_offset) + row * arguments.picks;
+	constexpr uint32_t value_bytes = BF16 ? 2u : 4u, batch = 4u; /* batch: slots whose loads are in flight together */
+	const unsigned char *const pairs =
+		arena + arguments.pair_output_offset + (row * slots * width + channel) * value_bytes;
+	float sum[8] = { 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f };
+	for (uint32_t first = 0; first < slots; first += batch) {
+		float value[batch][8];
+		bool counts[batch];
+#pragma unroll
+		for (uint32_t place = 0; place < batch; place++) {
+			const uint32_t slot = first + place;
+			counts[place] = slot < slots && (arguments.picks_offset == 0 || slot >= arguments.picks ||
+							 picked[slot] - arguments.local_first < arguments.local_count);
+			if (counts[place])
+				rows_one_load<BF16>(pairs + (uint64_t)slot * width * value_bytes, value[place]);
+		}
+#pragma unroll
+		for (uint32_t place = 0; place < batch; place++)
+			if (counts[place])
+#pragma unroll
+				for (uint32_t i = 0; i < 8; i++)
+					sum[i] = __fadd_rn(sum[i], value[place][i]);
+	}
+	const uint64_t at = row * width + channel;
+	if (arguments.addend_offset != 0) {
+		float value[8];
+		rows_one_load<true>(arena + arguments.addend_offset + at * 2u, value);
+#pragma unroll
+		for (uint32_t i = 0; i < 8; i++)
+			sum[i] = __fadd_rn(sum[i], value[i]);
+	}
+	float4 *const kept = reinterpret_cast<float4 *>(arena + arguments.row_output_offset + at * 4u);
+	kept[0] = make_float4(sum[0], sum[1], sum[2], sum[3]);
+	kept[1] = make_float4(sum[4], sum[5], sum[6], sum[7]);
+	if (step.sequence != 0)
+		*reinterpret_cast<uint4 *>(arena + arguments.output_offset + at * 2u) =
+			make_uint4(bfloat16_bits(sum[0]) | bfloat16_bits(sum[1]) << 16, bfloat16_bits(sum[2]) | bfloat16_bits(sum[3]) << 16,
+				   bfloat16_bits(sum[4]) | bfloat16_bits(sum[5]) << 16, bfloat16_bits(sum[6]) | bfloat16_bits(sum[7]) << 16);
+}
+
+extern "C" __global__ void __launch_bounds__(ORDERED_ROWS_ONE_THREADS)
+	ordered_rows_one(struct ordered_rows_one_arguments arguments, unsigned char *arena)
+{
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+	if (arguments.bf16_pairs != 0)
+		rows_one<true>(arguments, arena);
+	else
+		rows_one<false>(arguments, arena);
+}
+
+/* four channels (vector) of a row's sum as they enter the slot: the row's pairs from +0 in ascending slot order and, of
+ * bfloat16 pairs, the addend's; its FP32 copy goes to row_output_offset */
+template <bool BF16_PAIRS>
+__device__ __forceinline__ float4 publish_row_sum(const struct ordered_publish_reduce_arguments &arguments,
+						  uint64_t addend_offset, uint64_t row_output_offset, unsigned char *arena,
+						  uint32_t vector, uint32_t row_vectors)
+{
+	const uint32_t row = vector / row_vectors, column = vector % row_vectors;
+	float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+	if (BF16_PAIRS) {
+		const uint2 *const pairs = reinterpret_cast<const uint2 *>(arena + arguments.pair_output_offset);
+		for (uint32_t slot = 0; slot < arguments.pairs_per_row; slot++) {
+			const uint2 value = __ldcg(pairs + ((uint64_t)row * arguments.pairs_per_row + slot) * row_vectors + column);
+			sum.x = __fadd_rn(sum.x, __uint_as_float(value.x << 16));
+			sum.y = __fadd_rn(sum.y, __uint_as_float(value.x & 0xFFFF0000u));
+			sum.z = __fadd_rn(sum.z, __uint_as_float(value.y << 16));
+			sum.w = __fadd_rn(sum.w, __uint_as_float(value.y & 0xFFFF0000u));
+		}
+		if (addend_offset != 0) {
+			const uint2 value = __ldcg(reinterpret_cast<const uint2 *>(arena + addend_offset) + vector);
+			sum.x = __fadd_rn(sum.x, __uint_as_float(value.x << 16));
+			sum.y = __fadd_rn(sum.y, __uint_as_float(value.x & 0xFFFF0000u));
+			sum.z = __fadd_rn(sum.z, __uint_as_float(value.y << 16));
+			sum.w = __fadd_rn(sum.w, __uint_as_float(value.y & 0xFFFF0000u));
+		}
+		if (row_output_offset != 0)
+			reinterpret_cast<float4 *>(arena + row_output_offset)[vector] = sum;
+		/* as the publish launch of one "pair" a row enters it: onto +0 */
+		sum = make_float4(__fadd_rn(0.0f, sum.x), __fadd_rn(0.0f, sum.y), __fadd_rn(0.0f, sum.z),
+				  __fadd_rn(0.0f, sum.w));
+	} else {
+		const float4 *const pairs = reinterpret_cast<const float4 *>(arena + arguments.pair_output_offset);
+		for (uint32_t slot = 0; slot < arguments.pairs_per_row; slot++) {
+			const float4 value =
+				__ldcg(pairs + ((uint64_t)row * arguments.pairs_per_row + slot) * row_vectors + column);
+			sum.x = __fadd_rn(sum.x, value.x);
+			sum.y = __fadd_rn(sum.y, value.y);
+			sum.z = __fadd_rn(sum.z, value.z);
+			sum.w = __fadd_rn(sum.w, value.w);
+		}
+	}
+	return sum;
+}
+
 /* The reduction of the decode step's four launches as ONE launch (struct exl3_layer_route_record explains the slot):
  *   - wait until every rank has said it is done with the slot's previous use (their DONE words arrive in this rank's
  *     own memory, so the wait is local and normally over at once);
@@ -223,6 +355,33 @@ __device__ __forceinline__ void publish_reduce_flags(const struct ordered_publis
 	const uint32_t row_vectors = arguments.width / 4u, vectors = live_rows * row_vectors;
 	/* the slot's previous use */
 	const uint64_t previous = *reinterpret_cast<const volatile uint64_t *>(local + ORDERED_LOCAL_PREVIOUS_OFFSET);
+	if (collective.rank_count == 1u) {
+		/* One rank: its own rows are all there is, and nothing of this launch waits for another block: the row sums are
+		 * rounded as they are formed. The slot's rows and words are left as the general form leaves them. (A decode
+		 * step's tail: 12 us by the general form, FLAGS_ONE so.) */
+		if (previous >= sequence) {
+			if (threadIdx.x == 0)
+				ordered_status_set(status, ORDERED_STATUS_BAD_SEQUENCE, ORDERED_READY_PHASE, collective.rank);
+		} else {
+			float4 *const rows = reinterpret_cast<float4 *>(mine + collective.input_offset);
+			uint2 *const own = reinterpret_cast<uint2 *>(arena + collective.output_offset);
+			for (uint32_t vector = blockIdx.x * blockDim.x + threadIdx.x; vector < vectors; vector += gridDim.x * blockDim.x) {
+				const float4 sum = publish_row_sum<BF16_PAIRS>(arguments, addend_offset, row_output_offset, arena, vector,
+									       row_vectors);
+				rows[vector] = sum;
+				own[vector] = make_uint2(bfloat16_bits(sum.x) | bfloat16_bits(sum.y) << 16,
+							 bfloat16_bits(sum.z) | bfloat16_bits(sum.w) << 16);
+			}
+		}
+		if (last_block_of_grid(local, &last) && threadIdx.x == 0) {
+			if (previous < sequence) {
+				*reinterpret_cast<volatile uint64_t *>(local + ORDERED_LOCAL_PREVIOUS_OFFSET) = sequence;
+				signal_store(mine + EXL3_LAYER_READY_LINE * ORDERED_COLLECTIVE_LINE_BYTES, sequence);
+			}
+			signal_store(mine + EXL3_LAYER_DONE_LINE * ORDERED_COLLECTIVE_LINE_BYTES, sequence);
+		}
+		return;
+	}
 	if (threadIdx.x == 0)
 		verdict = 1u;
 	__syncthreads();
@@ -247,41 +406,8 @@ __device__ __forceinline__ void publish_reduce_flags(const struct ordered_publis
 	if (verdict != 0u) {
 		float4 *const rows = reinterpret_cast<float4 *>(mine + collective.input_offset);
 		for (uint32_t vector = blockIdx.x * blockDim.x + threadIdx.x; vector < vectors; vector += gridDim.x * blockDim.x) {
-			const uint32_t row = vector / row_vectors, column = vector % row_vectors;
-			float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-			if (BF16_PAIRS) {
-				const uint2 *const pairs = reinterpret_cast<const uint2 *>(arena + arguments.pair_output_offset);
-				for (uint32_t slot = 0; slot < arguments.pairs_per_row; slot++) {
-					const uint2 value = __ldcg(pairs + ((uint64_t)row * arguments.pairs_per_row + slot) * row_vectors + column);
-					sum.x = __fadd_rn(sum.x, __uint_as_float(value.x << 16));
-					sum.y = __fadd_rn(sum.y, __uint_as_float(value.x & 0xFFFF0000u));
-					sum.z = __fadd_rn(sum.z, __uint_as_float(value.y << 16));
-					sum.w = __fadd_rn(sum.w, __uint_as_float(value.y & 0xFFFF0000u));
-				}
-				if (addend_offset != 0) {
-					const uint2 value = __ldcg(reinterpret_cast<const uint2 *>(arena + addend_offset) + vector);
-					sum.x = __fadd_rn(sum.x, __uint_as_float(value.x << 16));
-					sum.y = __fadd_rn(sum.y, __uint_as_float(value.x & 0xFFFF0000u));
-					sum.z = __fadd_rn(sum.z, __uint_as_float(value.y << 16));
-					sum.w = __fadd_rn(sum.w, __uint_as_float(value.y & 0xFFFF0000u));
-				}
-				if (row_output_offset != 0)
-					reinterpret_cast<float4 *>(arena + row_output_offset)[vector] = sum;
-				/* as the publish launch of one "pair" a row enters it: onto +0 */
-				sum = make_float4(__fadd_rn(0.0f, sum.x), __fadd_rn(0.0f, sum.y), __fadd_rn(0.0f, sum.z),
-						  __fadd_rn(0.0f, sum.w));
-			} else {
-				const float4 *const pairs = reinterpret_cast<const float4 *>(arena + arguments.pair_output_offset);
-				for (uint32_t slot = 0; slot < arguments.pairs_per_row; slot++) {
-					const float4 value =
-						__ldcg(pairs + ((uint64_t)row * arguments.pairs_per_row + slot) * row_vectors + column);
-					sum.x = __fadd_rn(sum.x, value.x);
-					sum.y = __fadd_rn(sum.y, value.y);
-					sum.z = __fadd_rn(sum.z, value.z);
-					sum.w = __fadd_rn(sum.w, value.w);
-				}
-			}
-			rows[vector] = sum;
+			rows[vector] = publish_row_sum<BF16_PAIRS>(arguments, addend_offset, row_output_offset, arena, vector,
+								   row_vectors);
 		}
 	} else if (threadIdx.x == 0) {
 		atomicExch(gave_up, 1u);

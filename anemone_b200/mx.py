@@ -5,6 +5,7 @@ multiples of 128 (tensor_products):
 and for many rows
     exl3_prefill_picks -> exl3_prefill_group -> exl3_prefill_tiles -> mx_quantize -> mx_gather -> mx_gate_up_many
     -> mx_down_many -> expert_row_sum_entry -> trunk_rows_add_entry -> ordered_row_sum_publish -> ordered_reduce_bf16
+(the last four as one launch, ordered_rows_one, where there is one rank)
 (the products of the routed and the always-on experts on the fifth-generation tensor cores); otherwise
     router_select_b200 -> activation_quantize_entry -> expert_gate_up_<S> -> activation_quantize_entry (hidden)
     -> expert_down_<S> -> expert_row_sum_entry
@@ -235,6 +236,12 @@ class MxLayer:
                                           C.byref(count)), "mx_products_prepare")
         self.expert_launches = list(launches)[count.value - 2:count.value]  # gate/up, down
         head += list(launches)[:count.value - 2]
+        if L.wide and self.rank_count == 1:
+            # no peers: row sums, the always-on expert's rows and the rounding are one launch
+            one = R.OrderedRowsOne(L.at["pair_output"], 0, L.shared_at["output"] if c.shared else 0, L.at["row_output"],
+                                   L.result, L.step, H, c.picks, rows, 0, 0, 0, 1, 0)
+            self.launches = head + self.expert_launches + [api.rows_one(card, one)]
+            return
         behind = [] if L.flags else self._row_sums()
         reduce_launches = self._reduce()
         if L.flags:

@@ -4,6 +4,7 @@ Launches of one call, all from libanemone_b200.so (kernel file kernel_exl3_prefi
     exl3_prefill_picks -> exl3_prefill_group -> exl3_prefill_tiles -> exl3_prefill_operands
     -> exl3_prefill_gate_up -> exl3_prefill_down -> exl3_prefill_row_sum
     -> ordered_row_sum_publish -> ordered_reduce_bf16 (owner runs)
+or, on one rank, ordered_rows_one in the place of the last three.
 Rows are grouped per expert into tiles of 128; each (row tile, 128 outputs) is a tensor-core contraction with the
 expert's trellis tiles decoded on the way. The result is this rank's FP32 [rows][hidden] row sums over the pairs whose
 experts it holds. A rank holds a run of the routed experts with their full intermediate width (expert parallelism) or
@@ -202,6 +203,12 @@ class PrefillLayer:
         launches = (R.KernelLaunch * 7)()
         api.check(lib.exl3_prefill_prepare(C.byref(record), card.arena_bytes, card.ops_pointer, card.handle, launches),
                   "exl3_prefill_prepare")
+        if self.rank_count == 1:
+            # no peers: the row sums and their rounding are one launch, in the place of the last and of the reduction's two
+            one = R.OrderedRowsOne(L.pair_outputs + first * L.pairs_per_row * H * 4, L.picks + first * c.picks * 4, 0,
+                                   L.row_output + first * H * 4, L.result + first * H * 2, step, H, L.pairs_per_row, rows,
+                                   c.picks, share.local_first, share.local_count, 0, 0)
+            return record, launches[:6], [api.rows_one(card, one)]
         reduce = R.OrderedReduceBf16Description()
         reduce.reduce.collective = R.OrderedCollective(L.peer_table, L.region, L.slot_input, L.result + first * H * 2, 0,
                                                        step, L.parity_stride, c.deadline_cycles, rows * H,

@@ -168,6 +168,13 @@ class OrderedPublishReduceBf16(C.Structure):
     _fields_ = [("base", OrderedPublishReduce), ("addend_offset", C.c_uint64), ("row_output_offset", C.c_uint64)]
 
 
+class OrderedRowsOne(C.Structure):
+    _fields_ = [(name, C.c_uint64) for name in ("pair_output_offset", "picks_offset", "addend_offset",
+                                                "row_output_offset", "output_offset", "step_offset")] + \
+               [(name, C.c_uint32) for name in ("width", "pairs_per_row", "row_capacity", "picks", "local_first",
+                                                "local_count", "bf16_pairs", "reserved_zero")]
+
+
 class OrderedRowSumPublish(C.Structure):
     _fields_ = [("collective", OrderedCollective), ("pair_output_offset", C.c_uint64), ("width", C.c_uint32),
                 ("pairs_per_row", C.c_uint32), ("status_offset", C.c_uint64)]

@@ -119,6 +119,35 @@ MUST_CHECK result_status ordered_publish_reduce_bf16_prepare(const struct ordere
 							     const struct backend_operations *backend,
 							     struct device_card *card, struct kernel_launch *launch_out);
 
+/* B200 extension: what stands behind the experts of a layer call on ONE rank, in one launch ("ordered_rows_one"): a row's
+ * pairs added from +0 in ascending slot order, the optional bfloat16 addend row, the FP32 sum kept at row_output_offset,
+ * the same sum rounded once to bfloat16 at output_offset (not where the step's sequence is 0). The values are those of
+ * exl3_prefill_row_sum, or expert_row_sum_entry and trunk_rows_add_entry, and of ordered_reduce_bf16_prepare's two
+ * launches with one rank; with no peer there is no slot, no signal and no wait. */
+struct ordered_rows_one_arguments {
+	uint64_t pair_output_offset; /* FP32, or with bf16_pairs bfloat16, [row_capacity * pairs_per_row][width] */
+	uint64_t picks_offset; /* uint32 [row_capacity][picks]: the pair of slot s < picks counts where its pick is one of
+				* local_count experts from local_first; 0: every pair counts */
+	uint64_t addend_offset; /* bfloat16 [row_capacity][width], 0: none */
+	uint64_t row_output_offset; /* FP32 [row_capacity][width] */
+	uint64_t output_offset; /* bfloat16 [row_capacity][width] */
+	uint64_t step_offset;
+	uint32_t width; /* a multiple of 8 */
+	uint32_t pairs_per_row;
+	uint32_t row_capacity;
+	uint32_t picks;
+	uint32_t local_first;
+	uint32_t local_count;
+	uint32_t bf16_pairs; /* 0 or 1 */
+	uint32_t reserved_zero;
+};
+AB_RECORD_HAS(ordered_rows_one_arguments, 80);
+#define KERNEL_ORDERED_ROWS_ONE "ordered_rows_one"
+#define ORDERED_ROWS_ONE_THREADS 128u
+MUST_CHECK result_status ordered_rows_one_prepare(const struct ordered_rows_one_arguments *arguments,
+						  uint64_t arena_byte_count, const struct backend_operations *backend,
+						  struct device_card *card, struct kernel_launch *launch_out);
+
 /* ---- one-shot push all-reduce (include/anemone/ordered_push.h:37-59) ---- */
 
 struct ordered_push_description {

@@ -12,6 +12,7 @@ import numpy as np
 import pytest
 
 from anemone_b200 import records as R
+from anemone_b200 import synthetic
 from tests import golden_util
 from oracle.binding import f32p, pointer_array, ptr, u16p
 
@@ -234,3 +235,46 @@ def test_wait_runs_out_without_fault(api):
         assert (card.download(world.result, 2 * rows * width, np.uint16) == 0x4040).all()  # 1 + 2 = 3.0
     finally:
         world.close()
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("width, rows, live, slots, picks, held, addend", [
+    (8, 1, 1, 1, 0, (0, 0), False), (1032, 5, 3, 4, 0, (0, 0), True), (1024, 7, 7, 9, 8, (4, 5), False),
+    (2048, 33, 33, 5, 5, (0, 3), True), (128, 3, 0, 6, 6, (0, 16), False)])
+def test_rows_of_one_rank(api, width, rows, live, slots, picks, held, addend, bf16):
+    """ordered_rows_one: every FP32 sum and its one rounding, bit for bit; rows that are not live stay as they were."""
+    rng = np.random.default_rng([width, rows, slots, bf16])
+    pairs = rng.standard_normal((rows, slots, width), dtype=np.float32)
+    extra = rng.standard_normal((rows, width), dtype=np.float32)
+    choice = rng.integers(0, 16, size=(rows, max(picks, 1)), dtype=np.uint32)
+    pairs[0, 0, :4] = np.inf, -0.0, np.nan, 3e38
+    pair_bits, extra_bits = (pairs if not bf16 else synthetic.to_bfloat16(pairs)), synthetic.to_bfloat16(extra)
+    layout = api.Layout(256)
+    at = [layout.take(size) for size in (16, pair_bits.nbytes, choice.nbytes, extra_bits.nbytes, rows * width * 4,
+                                         rows * width * 2)]
+    card = api.Card(0, api.align(layout.cursor, 4096) + 4096)
+    try:
+        for offset, data in zip(at, (np.array([7, live], dtype=np.uint64), pair_bits, choice, extra_bits)):
+            card.upload(offset, data)
+        card.fill(at[4], 0xA5, rows * width * 4)
+        card.fill(at[5], 0xA5, rows * width * 2)
+        card.run([api.rows_one(card, R.OrderedRowsOne(at[1], at[2] if picks else 0, at[3] if addend else 0, at[4], at[5], at[0],
+                                                      width, slots, rows, picks, held[0], held[1], int(bf16), 0))])
+        kept = card.download(at[4], rows * width * 4, np.float32).reshape(rows, width)
+        got = card.download(at[5], rows * width * 2, np.uint16).reshape(rows, width)
+    finally:
+        card.close()
+    values = synthetic.from_bfloat16(pair_bits) if bf16 else pairs
+    expected = np.zeros((rows, width), dtype=np.float32)
+    for slot in range(slots):
+        counts = np.ones((rows, 1), dtype=bool) if slot >= picks else \
+            ((choice[:, slot] >= held[0]) & (choice[:, slot] < held[0] + held[1]))[:, None]
+        expected = np.where(counts, expected + values[:, slot], expected)
+    if addend:
+        expected = expected + synthetic.from_bfloat16(extra_bits)
+    number = ~np.isnan(expected[:live])
+    assert np.array_equal(np.isnan(kept[:live]), ~number)
+    assert np.array_equal(kept[:live].view(np.uint32)[number], expected[:live].view(np.uint32)[number])
+    rounded = np.where(number, synthetic.to_bfloat16(expected[:live]), 0x7FC0)
+    assert np.array_equal(got[:live], rounded)
+    assert (kept[live:].view(np.uint8) == 0xA5).all() and (got[live:].view(np.uint8) == 0xA5).all()

@@ -408,6 +408,29 @@ def test_layer_cut_of_k_follows_the_prepared_jobs(rows, hidden, inner, runs):
     assert R.Exl3LayerProducts.from_buffer_copy(bytes(products.argument[:128])).gate_up_runs == runs
 
 
+def test_rows_of_one_rank_prepare():
+    lib, fake, launch = api.library(), FakeBackend(), R.KernelLaunch()
+    prepare = lib.ordered_rows_one_prepare
+    prepare.argtypes = [C.POINTER(R.OrderedRowsOne), C.c_uint64, C.POINTER(api.BackendOperations), C.c_void_p,
+                        C.POINTER(R.KernelLaunch)]
+
+    def record(**change):
+        made = R.OrderedRowsOne(1 << 20, 4096, 0, 1 << 16, 1 << 14, 256, 1032, 9, 3, 8, 0, 4, 0, 0)
+        for name, value in change.items():
+            setattr(made, name, value)
+        return C.byref(made)
+    assert prepare(record(), 1 << 24, C.byref(fake.table), fake.card, C.byref(launch)) == 0
+    assert fake.asked[-1][1:3] == ("ordered_rows_one", 80) and tuple(launch.grid) == (2, 3, 1) and launch.block[0] == 128
+    assert launch.branch == 0x100  # it waits for the launch before it, whose place it may overlap
+    untouched = bytes(launch)
+    for change in (dict(width=0), dict(width=1028), dict(row_capacity=0), dict(row_capacity=65536), dict(pairs_per_row=0),
+                   dict(picks=0), dict(picks=10), dict(bf16_pairs=2), dict(reserved_zero=1), dict(output_offset=(1 << 14) + 8),
+                   dict(pair_output_offset=(1 << 24) - 16), dict(output_offset=1 << 16), dict(addend_offset=1 << 20),
+                   dict(step_offset=260)):
+        assert prepare(record(**change), 1 << 24, C.byref(fake.table), fake.card, C.byref(launch)) == 1, change
+        assert bytes(launch) == untouched
+
+
 def test_router_wide_prepare():
     """The job table of many rows: three launches (the prefill's picks and grouping, then router_wide_jobs)."""
     lib, fake = api.library(), FakeBackend()
