@@ -197,7 +197,7 @@ extern "C" __global__ void __launch_bounds__(ORDERED_COLLECTIVE_THREADS)
 /* ordered_rows_one: a thread eight channels of a row. Bound by the pair outputs' way from memory, each read once: 2048 rows
  * of 4096, nine bfloat16 values each, 200 MB in all; the four launches it stands for with one rank (row sums, the
  * always-on expert's rows, publish, reduce) wrote and read the FP32 rows three times more and met at two grid-wide counters:
- * 134 us there, ROWS_ONE_2048 here; 333 rows 52 and ROWS_ONE_333. */
+ * 134 us there, 41 here; 333 rows 52 and 6. */
 template <bool BF16> __device__ __forceinline__ void rows_one_load(const unsigned char *at, float out[8])
 {
 	if (BF16) {
@@ -358,7 +358,7 @@ __device__ __forceinline__ void publish_reduce_flags(const struct ordered_publis
 	if (collective.rank_count == 1u) {
 		/* One rank: its own rows are all there is, and nothing of this launch waits for another block: the row sums are
 		 * rounded as they are formed. The slot's rows and words are left as the general form leaves them. (A decode
-		 * step's tail: 12 us by the general form, FLAGS_ONE so.) */
+		 * step's tail: 12 us by the general form, 8 so.) */
 		if (previous >= sequence) {
 			if (threadIdx.x == 0)
 				ordered_status_set(status, ORDERED_STATUS_BAD_SEQUENCE, ORDERED_READY_PHASE, collective.rank);
