@@ -204,15 +204,48 @@ __device__ __forceinline__ void hadamard128_warp(float v[4], uint32_t lane)
 	v[1] = __fadd_rn(b, d);
 	v[2] = __fsub_rn(a, c);
 	v[3] = __fsub_rn(b, d);
-	/* strides 4 .. 64 across lanes: the lower partner takes a + b, the upper one (lower - upper) */
+	/* strides 4 .. 64 across lanes: the lower partner takes a + b, the upper one (lower - upper): its own value times -1
+	 * and the other's, rounded once */
 #pragma unroll
 	for (uint32_t distance = 1; distance < EXL3_WARP; distance <<= 1) {
-		const bool upper = (lane & distance) != 0;
+		const float sign = (lane & distance) != 0 ? -1.0f : 1.0f;
 #pragma unroll
-		for (uint32_t i = 0; i < 4; i++) {
-			const float other = __shfl_xor_sync(0xFFFFFFFFu, v[i], distance);
-			v[i] = upper ? __fsub_rn(other, v[i]) : __fadd_rn(v[i], other);
-		}
+		for (uint32_t i = 0; i < 4; i++)
+			v[i] = __fmaf_rn(v[i], sign, __shfl_xor_sync(0xFFFFFFFFu, v[i], distance));
+	}
+}
+
+/* The same transform with a row in eight lanes, four rows a warp: v[k][j] is value 32 k + 4 (lane % 8) + j. The same FP32
+ * operations in the same stage order, so the same bits; three of the seven stages cross lanes instead of five: 12 shuffles
+ * a row instead of 20. For many rows: a warp's chain is twice as long. All 32 lanes call. */
+__device__ __forceinline__ void hadamard128_rows(float v[4][4], uint32_t lane)
+{
+#pragma unroll
+	for (uint32_t k = 0; k < 4; k++) {
+		const float a = __fadd_rn(v[k][0], v[k][1]), b = __fsub_rn(v[k][0], v[k][1]);
+		const float c = __fadd_rn(v[k][2], v[k][3]), d = __fsub_rn(v[k][2], v[k][3]);
+		v[k][0] = __fadd_rn(a, c);
+		v[k][1] = __fadd_rn(b, d);
+		v[k][2] = __fsub_rn(a, c);
+		v[k][3] = __fsub_rn(b, d);
+	}
+#pragma unroll
+	for (uint32_t distance = 1; distance < 8u; distance <<= 1) {
+		const float sign = (lane & distance) != 0 ? -1.0f : 1.0f;
+#pragma unroll
+		for (uint32_t k = 0; k < 4; k++)
+#pragma unroll
+			for (uint32_t j = 0; j < 4; j++)
+				v[k][j] = __fmaf_rn(v[k][j], sign, __shfl_xor_sync(0xFFFFFFFFu, v[k][j], distance));
+	}
+#pragma unroll
+	for (uint32_t j = 0; j < 4; j++) {
+		const float a = __fadd_rn(v[0][j], v[1][j]), b = __fsub_rn(v[0][j], v[1][j]);
+		const float c = __fadd_rn(v[2][j], v[3][j]), d = __fsub_rn(v[2][j], v[3][j]);
+		v[0][j] = __fadd_rn(a, c);
+		v[1][j] = __fadd_rn(b, d);
+		v[2][j] = __fsub_rn(a, c);
+		v[3][j] = __fsub_rn(b, d);
 	}
 }
 

@@ -91,12 +91,14 @@ AB_INLINE uint64_t exl3_layer_gate_up_product_bytes(uint32_t pair_count, uint32_
 /* ---- prefill (kernel_exl3_prefill) ---- */
 #define EXL3_PREFILL_GEMM_THREADS 576u /* a copy warp, an issuing warp, sixteen decode warps */
 #define EXL3_PREFILL_OPERAND_PARTS 4u /* an operand CTA takes a quarter of a tile's rows */
-#define EXL3_PREFILL_STAGE_STEPS 2u /* steps of 16 inputs of one stage */
-/* a stage's turn in the ring (decoded, told to the issuing warp, multiplied, freed) is 3500 cycles and more, its products
- * 512: as many as fit */
-#define EXL3_PREFILL_STAGES 7u
-#define EXL3_PREFILL_STAGE_BYTES 32768u /* gate/up: two blocks of rows, two of weights; down: one and two */
-#define EXL3_PREFILL_DYNAMIC_BYTES (EXL3_PREFILL_STAGES * EXL3_PREFILL_STAGE_BYTES)
+#define EXL3_PREFILL_STAGE_STEPS 4u /* steps of 16 inputs of one stage */
+/* A ring of stages of 64 inputs: three of gate/up (two blocks of rows, two of weights, 64 KB), four of down (one and two).
+ * What a stage costs whatever its inputs (the issuing warp's wait, products and commit, 515 cycles; the hand-over across the
+ * pair) is paid half as often as with stages of 32, of which seven fit: 413 rows of 256 experts 621 us of gate/up and
+ * 357 of down, 596 and 356 so; 4096 rows 1880 and 1140, 1855 and 1079. More stages where the rows are few leave room for
+ * them (six for 16 rows a CTA): no gain. */
+#define EXL3_PREFILL_DYNAMIC_BYTES 196608u
+#define EXL3_PREFILL_MOST_STAGES 4u
 #define EXL3_PREFILL_STAGING_ROW 132u /* floats of a staged accumulator row */
 
 #endif

@@ -24,14 +24,18 @@ __device__ __forceinline__ uint32_t exl3_job_bits_x2(const struct exl3_expert_re
 	return exl3_bits_x2(widths != nullptr ? widths[job->expert] : record.bits_per_weight);
 }
 
-__device__ __forceinline__ void load_half4(const __half *source, float out[4])
+__device__ __forceinline__ void half4_values(const uint2 raw, float out[4])
 {
-	const uint2 raw = *reinterpret_cast<const uint2 *>(source);
 	const __half2 low = *reinterpret_cast<const __half2 *>(&raw.x), high = *reinterpret_cast<const __half2 *>(&raw.y);
 	out[0] = __low2float(low);
 	out[1] = __high2float(low);
 	out[2] = __low2float(high);
 	out[3] = __high2float(high);
+}
+
+__device__ __forceinline__ void load_half4(const __half *source, float out[4])
+{
+	half4_values(*reinterpret_cast<const uint2 *>(source), out);
 }
 
 __device__ __forceinline__ void store_half4(__half *destination, const float v[4])

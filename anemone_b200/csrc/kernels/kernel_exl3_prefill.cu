@@ -6,7 +6,7 @@
  *   - streams its rows' FP16 operands (pre-tiled in the tensor cores' no-swizzle K-major layout) into a ring of
  *     shared-memory stages, one bulk asynchronous copy a stage (one warp),
  *   - loads the trellis words of its outputs into registers a turn of the decode teams ahead, decodes them and stores
- *     them as the A operand blocks of the stage (sixteen warps in four teams, a team a stage; the decode's fragment order
+ *     them as the A operand blocks of the stage (sixteen warps in two teams, a team a stage; the decode's fragment order
  *     makes every store a contiguous 128 bytes of the block),
  *   - multiplies with tcgen05.mma of cta_group::2 (one thread of the pair), FP32 accumulators in tensor memory, the stage
  *     released by tcgen05.commit,
@@ -22,18 +22,34 @@
 #define PREFILL_FIRST_DECODE_WARP 2u /* behind the copy warp and the issuing warp */
 #define PREFILL_DECODE_WARPS 16u
 #define PREFILL_DECODE_THREADS (PREFILL_DECODE_WARPS * EXL3_WARP)
-#define PREFILL_TEAMS 4u /* of four decode warps */
+#define PREFILL_PARTS (2u * EXL3_PREFILL_STAGE_STEPS) /* of a stage's weights, a decode warp each */
+#define PREFILL_TEAMS (PREFILL_DECODE_WARPS / PREFILL_PARTS) /* of decode warps */
 #define PREFILL_GROUP_THREADS 256u
 
 struct prefill_shared {
-	uint64_t full[EXL3_PREFILL_STAGES]; /* the stage's weights are decoded and its rows have landed; rank 0: the other CTA's too */
-	uint64_t free[EXL3_PREFILL_STAGES]; /* the products that read it are done */
+	uint64_t full[EXL3_PREFILL_MOST_STAGES]; /* the stage's weights are decoded and its rows have landed; rank 0: the other CTA's too */
+	uint64_t free[EXL3_PREFILL_MOST_STAGES]; /* the products that read it are done */
 	uint64_t done; /* every product of the pair is done */
 	uint32_t tensor_memory;
 	volatile uint32_t failed;
 	uint32_t expired; /* an earlier wait had run out when the CTA began */
 	uint32_t armed; /* stages whose row copies were started */
+	uint32_t stages; /* of the ring */
+	/* of the CTA's 128 outputs: gate's, up's and down's input-side scales; down: of its two groups */
+	__half __align__(16) scales[3][EXL3_TRANSFORM];
 };
+
+/* The epilogue's scales, brought beside the K loop: read by the epilogue from memory they were its longest wait (1500 cycles
+ * each time, four times in a row for a warp's rows). A decode warp a run of 256 bytes, half its lanes; complete at the
+ * decode warps' barrier behind the K loop. */
+__device__ __forceinline__ void prefill_fetch_scales(prefill_shared *shared, uint32_t place, const __half *scales)
+{
+	const uint32_t lane = threadIdx.x % EXL3_WARP;
+	if (threadIdx.x / EXL3_WARP == PREFILL_FIRST_DECODE_WARP + place && lane < 16u)
+		asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_address(shared->scales[place] + lane * 8u)),
+			     "l"(scales + lane * 8u)
+			     : "memory");
+}
 
 struct prefill_view {
 	const struct exl3_prefill_parts parts;
@@ -187,7 +203,7 @@ __device__ __forceinline__ uint32_t prefill_tiles_of_unit(const prefill_view &vi
 	return tile_index + 1u < tile_count && tiles[tile_index + 1u].expert == tile.expert ? 2u : 1u;
 }
 
-/* Where a tile's operands lie: what a CTA of the pair takes for one stage of 32 inputs is ONE run of bytes, [matrix][four
+/* Where a tile's operands lie: what a CTA of the pair takes for one stage of 64 inputs is ONE run of bytes, [matrix][eight
  * pieces of eight inputs][half rows][16 bytes], the stages one behind the other. The second CTA's runs are in the second
  * tile's region, or behind the first CTA's for a single tile. (With a fixed place for each of 128 rows a stage of fewer
  * rows was up to eight copies, and their issue, 1070 cycles a stage, was what bounded the products.) */
@@ -210,23 +226,37 @@ __device__ __forceinline__ uint64_t prefill_operand_byte(const prefill_rows &row
 							 uint32_t input)
 {
 	const uint32_t rank = row / rows.half, piece = input / 8u;
-	return rank * rows.second + (uint64_t)((piece / 4u * matrices + m) * 4u + piece % 4u) * (rows.half * 16u) +
+	constexpr uint32_t pieces = 2u * EXL3_PREFILL_STAGE_STEPS; /* of a stage */
+	return rank * rows.second + (uint64_t)((piece / pieces * matrices + m) * pieces + piece % pieces) * (rows.half * 16u) +
 	       (row - rank * rows.half) * 16u + input % 8u * 2u;
 }
 
-/* grid (tile capacity, ceil(H / 128 / 4) x EXL3_PREFILL_OPERAND_PARTS, 2) x 128: x . suh, Hadamard, FP16 operands of
- * gate (z = 0) and up (z = 1). A warp takes one 128-channel block of a quarter of the tile's rows, eight rows at a time:
- * the eight transforms are independent, and their FP16 rows go through shared memory so that every store to the
- * operand blocks is a whole 128-byte piece (eight rows x eight inputs). Rows beyond the tile's count are written as
- * zeros. */
-#define OPERAND_ROW_BYTES 272u /* 128 FP16 and a pad that spreads eight rows over the banks */
+/* Four rows a warp, eight lanes a row: what a lane holds of a block of 128 channels is four runs of four channels, at
+ * 32 k + 4 (lane % 8) (hadamard128_rows' layout). */
+#define PREFILL_WARP_ROWS 4u
+/* A tile of at most this many rows is finished a row a warp (hadamard128_warp), whose chain is a third as long: an
+ * epilogue of gate/up of up to 16 rows is 4 k cycles so, 9 k four rows a warp; of 128 rows 18 k and 15 k. */
+#define PREFILL_FEW_ROWS 32u
+__device__ __forceinline__ void prefill_scales(const __half *scales, uint32_t first_channel, uint2 out[4])
+{
+#pragma unroll
+	for (uint32_t k = 0; k < 4; k++)
+		out[k] = *reinterpret_cast<const uint2 *>(scales + first_channel + 32u * k);
+}
+
+/* grid (tile capacity, ceil(H / 128 / 4) x EXL3_PREFILL_OPERAND_PARTS) x 128: x . suh, Hadamard, FP16 operands of gate and
+ * of up. A warp takes one 128-channel block of a quarter of the tile's rows, four rows at a time; four rows' stores to a
+ * piece of the operand blocks are 64 adjacent bytes. Bound by instruction issue beside the operands' way to memory: 4096
+ * rows of H 4096, 36864 pairs, 1.14 GB written, 238 us (321 with a row a warp, a launch half each of gate and up
+ * and the rows through shared memory). Rows beyond the tile's count are not written: what the products make of them
+ * stays in their own columns of the accumulators, which nobody reads. */
 extern "C" __global__ void __launch_bounds__(EXL3_TRANSFORM_THREADS)
 	exl3_prefill_operands(struct exl3_prefill_record record, unsigned char *arena)
 {
-	__shared__ __align__(16) unsigned char staged[EXL3_TRANSFORM_WARPS][8u * OPERAND_ROW_BYTES];
 	const prefill_view view = prefill_view_of(record, arena);
 	const uint32_t tile_index = blockIdx.x;
-	if (tile_index >= reinterpret_cast<const uint32_t *>(view.workspace + view.parts.counts)[view.experts])
+	const uint32_t tile_count = reinterpret_cast<const uint32_t *>(view.workspace + view.parts.counts)[view.experts];
+	if (tile_index >= tile_count)
 		return;
 	const struct exl3_prefill_tile tile =
 		reinterpret_cast<const struct exl3_prefill_tile *>(view.workspace + view.parts.tiles)[tile_index];
@@ -237,57 +267,53 @@ extern "C" __global__ void __launch_bounds__(EXL3_TRANSFORM_THREADS)
 	constexpr uint32_t part_rows = EXL3_PREFILL_TILE_ROWS / EXL3_PREFILL_OPERAND_PARTS;
 	if (block >= H / EXL3_TRANSFORM || part * part_rows >= tile.row_count)
 		return;
-	const uint32_t channel = block * EXL3_TRANSFORM + lane * 4u;
+	const uint32_t channel = block * EXL3_TRANSFORM + lane % 8u * 4u;
 	const uint32_t bits_x2 = exl3_bits_x2(reinterpret_cast<const uint32_t *>(arena + record.widths_offset)[tile.expert]);
-	const uint64_t matrix =
-		reinterpret_cast<const uint64_t *>(arena + record.expert_table_offset)[3u * tile.expert + blockIdx.z];
-	float scale[4];
-	load_half4(reinterpret_cast<const __half *>(arena + matrix +
-						    exl3_code_bytes(H, prefill_inner_of(record, tile.expert), bits_x2)) +
-			   channel,
-		   scale);
+	const uint64_t codes = exl3_code_bytes(H, prefill_inner_of(record, tile.expert), bits_x2);
+	const uint64_t *const table = reinterpret_cast<const uint64_t *>(arena + record.expert_table_offset) + 3u * tile.expert;
+	uint2 scales[EXL3_PROJECTIONS][4];
+#pragma unroll
+	for (uint32_t m = 0; m < EXL3_PROJECTIONS; m++)
+		prefill_scales(reinterpret_cast<const __half *>(arena + table[m] + codes), channel, scales[m]);
 	const struct exl3_prefill_entry *const entries =
 		reinterpret_cast<const struct exl3_prefill_entry *>(view.workspace + view.parts.entries) +
 		(uint64_t)tile.expert * record.row_capacity + tile.first_entry;
-	const __nv_bfloat16 *const input = reinterpret_cast<const __nv_bfloat16 *>(arena + record.input_offset);
-	const uint32_t count = prefill_tiles_of_unit(
-		view, tile, tile_index, reinterpret_cast<const uint32_t *>(view.workspace + view.parts.counts)[view.experts]);
-	const prefill_rows rows = prefill_rows_of(count, tile.row_count, EXL3_PROJECTIONS, H);
+	const __nv_bfloat16 *const input = reinterpret_cast<const __nv_bfloat16 *>(arena + record.input_offset) + channel;
+	const prefill_rows rows = prefill_rows_of(prefill_tiles_of_unit(view, tile, tile_index, tile_count), tile.row_count,
+						  EXL3_PROJECTIONS, H);
 	unsigned char *const region = view.workspace + view.parts.gate_up_operands + (uint64_t)tile_index * H * 512u;
-	unsigned char *const mine = staged[warp];
-	for (uint32_t first = part * part_rows; first < (part + 1u) * part_rows && first < tile.row_count; first += 8u) {
-		uint2 raw[8];
+	const uint32_t end = min((part + 1u) * part_rows, tile.row_count);
+	for (uint32_t first = part * part_rows; first < end; first += PREFILL_WARP_ROWS) {
+		const uint32_t row = first + lane / 8u;
+		const uint64_t source = (uint64_t)(entries[min(row, end - 1u)].pair / view.pairs_per_row) * H;
+		uint2 raw[4];
 #pragma unroll
-		for (uint32_t r = 0; r < 8; r++) {
-			raw[r] = make_uint2(0u, 0u);
-			if (first + r < tile.row_count) {
-				const uint32_t source_row = entries[first + r].pair / view.pairs_per_row;
-				raw[r] = *reinterpret_cast<const uint2 *>(input + (uint64_t)source_row * H + channel);
+		for (uint32_t k = 0; k < 4; k++)
+			raw[k] = *reinterpret_cast<const uint2 *>(input + source + 32u * k);
+#pragma unroll
+		for (uint32_t m = 0; m < EXL3_PROJECTIONS; m++) {
+			float v[4][4];
+#pragma unroll
+			for (uint32_t k = 0; k < 4; k++) {
+				float scale[4];
+				half4_values(scales[m][k], scale);
+				v[k][0] = __fmul_rn(__uint_as_float(raw[k].x << 16), scale[0]);
+				v[k][1] = __fmul_rn(__uint_as_float(raw[k].x & 0xFFFF0000u), scale[1]);
+				v[k][2] = __fmul_rn(__uint_as_float(raw[k].y << 16), scale[2]);
+				v[k][3] = __fmul_rn(__uint_as_float(raw[k].y & 0xFFFF0000u), scale[3]);
+			}
+			hadamard128_rows(v, lane);
+#pragma unroll
+			for (uint32_t k = 0; k < 4; k++) {
+#pragma unroll
+				for (uint32_t j = 0; j < 4; j++)
+					v[k][j] = __fmul_rn(v[k][j], EXL3_NORMALIZATION);
+				if (row < end)
+					store_half4(reinterpret_cast<__half *>(
+							    region + prefill_operand_byte(rows, EXL3_PROJECTIONS, m, row, channel + 32u * k)),
+						    v[k]);
 			}
 		}
-#pragma unroll
-		for (uint32_t r = 0; r < 8; r++) {
-			float v[4] = { __uint_as_float(raw[r].x << 16), __uint_as_float(raw[r].x & 0xFFFF0000u),
-				       __uint_as_float(raw[r].y << 16), __uint_as_float(raw[r].y & 0xFFFF0000u) };
-#pragma unroll
-			for (uint32_t i = 0; i < 4; i++)
-				v[i] = __fmul_rn(v[i], scale[i]);
-			hadamard128_warp(v, lane);
-#pragma unroll
-			for (uint32_t i = 0; i < 4; i++)
-				v[i] = __fmul_rn(v[i], EXL3_NORMALIZATION);
-			store_half4(reinterpret_cast<__half *>(mine + r * OPERAND_ROW_BYTES + lane * 8u), v);
-		}
-		__syncwarp();
-		/* piece p (eight inputs) of the eight rows: 128 contiguous bytes of the block; lane = 8 (p % 4) + row */
-#pragma unroll
-		for (uint32_t turn = 0; turn < 4; turn++) {
-			const uint32_t piece = turn * 4u + lane / 8u, row = lane % 8u;
-			const uint4 value = *reinterpret_cast<const uint4 *>(mine + row * OPERAND_ROW_BYTES + piece * 16u);
-			*reinterpret_cast<uint4 *>(region + prefill_operand_byte(rows, EXL3_PROJECTIONS, blockIdx.z, first + row,
-										 block * EXL3_TRANSFORM + piece * 8u)) = value;
-		}
-		__syncwarp();
 	}
 }
 
@@ -300,8 +326,8 @@ extern "C" __global__ void __launch_bounds__(EXL3_TRANSFORM_THREADS)
  * (its 128 outputs and its 128 rows per 128 cycles). One CTA on its own with two row tiles of 128 x 128 products needs
  * 128 bytes a cycle for the instructions alone, all there is, and takes every row's operands from L2 twice as often.
  * The rows' number is the instruction's N, so a last tile of few rows costs the tensor cores little; the decode is the
- * same for any. 4096 rows of H 4096, I 2048, 256 experts of 8: gate/up 2202 us with single CTAs, 1880 so; down 1211,
- * 1137. Neither end is full (1024 rows of 32 experts: 67 % of the issue slots, the tensor cores 43 % of the cycles): a
+ * same for any. 4096 rows of H 4096, I 2048, 256 experts of 8: gate/up 2202 us with single CTAs, 1811 so; down 1211,
+ * 1015. Neither end is full (1024 rows of 32 experts: 67 % of the issue slots, the tensor cores 43 % of the cycles): a
  * stage's turn in the ring, about 600 cycles of which the products take 512 at most, and a unit's beginning and epilogue,
  * a sixth of gate/up and a quarter of down, lie between them. */
 #define PREFILL_PAIR 2u /* CTAs of a unit */
@@ -427,9 +453,9 @@ __device__ __forceinline__ void pair_acquire()
 }
 
 /* Dynamic shared memory of a product CTA: MATRICES x GROUPS = 2 accumulators, gate and up of 128 outputs or down of
- * 2 x 128; a ring of EXL3_PREFILL_STAGES stages of 32 inputs, each
- *   [matrix] the CTA's rows (up to 128 x 32 FP16, 8 KB): one bulk copy, mostly from L2
- *   [matrix x group] decoded weights, 128 outputs x 32 FP16, 8 KB in the same layout: written by the decode warps
+ * 2 x 128; a ring of stages of 64 inputs, each
+ *   [matrix] the CTA's rows (up to 128 x 64 FP16, 16 KB): one bulk copy, mostly from L2
+ *   [matrix x group] decoded weights, 128 outputs x 64 FP16, 16 KB in the same layout: written by the decode warps
  * Rows and weights share the stage so that the issuing warp waits for ONE barrier a stage: a wait on a barrier that is
  * long complete takes it 150 cycles, three of them and the issue of four products 730, where the products of 256 rows
  * last 512. The trellis words do not pass here: the start of a bulk copy takes a warp 300 to 500 cycles, whatever the
@@ -438,11 +464,10 @@ __device__ __forceinline__ void pair_acquire()
 #define PREFILL_BLOCK (PREFILL_STEPS * 4096u) /* 512 units of 16 bytes, 256 a step */
 template <uint32_t MATRICES, uint32_t GROUPS> struct prefill_rings {
 	static constexpr uint32_t weights_at = MATRICES * PREFILL_BLOCK; /* in a stage, behind the rows */
-	static constexpr uint32_t stage = EXL3_PREFILL_STAGE_BYTES;
-	static constexpr uint32_t bytes = EXL3_PREFILL_STAGES * stage;
-	static_assert(weights_at + MATRICES * GROUPS * PREFILL_BLOCK <= stage, "a stage holds its blocks");
+	static constexpr uint32_t stage = weights_at + MATRICES * GROUPS * PREFILL_BLOCK;
+	static constexpr uint32_t stages = EXL3_PREFILL_DYNAMIC_BYTES / stage;
 	static_assert(MATRICES * GROUPS * PREFILL_SUM_COLUMNS == 512u, "tensor memory has 512 columns");
-	static_assert(bytes == EXL3_PREFILL_DYNAMIC_BYTES, "the host sizes the rings");
+	static_assert(stages <= EXL3_PREFILL_MOST_STAGES && MATRICES * GROUPS == 2u, "the rings' barriers; a stage's parts");
 };
 
 /* The K loop of one CTA of the pair. matrices[m]: the codes of matrix m (`outputs` outputs), of which this CTA decodes
@@ -461,7 +486,7 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 {
 	typedef exl3_ring<BX2> ring;
 	typedef prefill_rings<MATRICES, GROUPS> rings;
-	constexpr uint32_t S = EXL3_PREFILL_STAGES;
+	constexpr uint32_t S = rings::stages;
 	const uint32_t lane = threadIdx.x % EXL3_WARP, warp = threadIdx.x / EXL3_WARP;
 	const uint64_t step_words = (uint64_t)(outputs / EXL3_TILE) * ring::words; /* of one step of 16 inputs */
 	const uint32_t accumulators = shared->tensor_memory;
@@ -512,7 +537,7 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 		const uint32_t r_low = warp_value(prefill_descriptor_low(dynamic_shared, half * 16u));
 		const uint32_t w_low = warp_value(prefill_descriptor_low(dynamic_shared + rings::weights_at, 2048u));
 		const uint32_t r_step = warp_value(2u * half), columns = warp_value(accumulators), live = warp_value(sums);
-		const uint32_t full = warp_value(smem_address(shared->full)), r_second = MATRICES > 1u ? 2u * r_step : 0u;
+		const uint32_t full = warp_value(smem_address(shared->full)), r_second = MATRICES > 1u ? PREFILL_STEPS * r_step : 0u;
 		for (uint32_t left = blocks; left != 0; left--) {
 			if (ready == 0) {
 				good = warp_wait<true>(&shared->full[stage], parity);
@@ -528,12 +553,14 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 			ready = pair_barrier_test(full + stage * 8u, parity);
 			tensor_fence_after();
 			if (prefill_elected()) {
-				tensor_multiply(columns, w, r, instruction, accumulate);
-				tensor_multiply(columns, w + 256u, r + r_step, instruction, 1u);
-				if (GROUPS == 1u || live > 1u) {
-					tensor_multiply(columns + PREFILL_SUM_COLUMNS, w + 512u, r + r_second, instruction, accumulate);
-					tensor_multiply(columns + PREFILL_SUM_COLUMNS, w + 768u, r + r_second + r_step, instruction, 1u);
-				}
+#pragma unroll
+				for (uint32_t step = 0; step < PREFILL_STEPS; step++)
+					tensor_multiply(columns, w + step * 256u, r + step * r_step, instruction, step == 0u ? accumulate : 1u);
+				if (GROUPS == 1u || live > 1u)
+#pragma unroll
+					for (uint32_t step = 0; step < PREFILL_STEPS; step++)
+						tensor_multiply(columns + PREFILL_SUM_COLUMNS, w + (PREFILL_STEPS + step) * 256u,
+								r + r_second + step * r_step, instruction, step == 0u ? accumulate : 1u);
 				tensor_commit(freed, 3u);
 				if (left == 1u)
 					tensor_commit(&shared->done, 3u);
@@ -557,14 +584,15 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 		return false;
 	}
 
-	/* decode: the sixteen warps are four teams of four; team q decodes the WHOLE stages q, q + 4, ..., so that the
-	 * teams work on four different stages at once and a warp crosses a barrier and a proxy fence once per stage of
+	/* decode: the sixteen warps are two teams of eight; team q decodes the WHOLE stages q, q + 2, ..., so that the
+	 * teams work on two different stages at once and a warp crosses a barrier and a proxy fence once per stage of
 	 * eight tiles. A warp's part of a stage is the eight adjacent tiles of one (matrix, group, step). A lane loads
-	 * its ring words straight into registers, a tile's words for the team's next stage as soon as this one's are decoded: four
-	 * stages, two microseconds, ahead. */
+	 * its ring words straight into registers, a tile's words for the team's next stage as soon as this one's are decoded: two
+	 * stages, more than a microsecond, ahead. */
 	{
-		static_assert(MATRICES * GROUPS * PREFILL_STEPS == 4u && PREFILL_DECODE_WARPS == 4u * PREFILL_TEAMS, "a part a warp");
-		const uint32_t decoder = warp - PREFILL_FIRST_DECODE_WARP, team = decoder / 4u, member = decoder % 4u;
+		static_assert(MATRICES * GROUPS * PREFILL_STEPS == PREFILL_PARTS && PREFILL_DECODE_WARPS == PREFILL_PARTS * PREFILL_TEAMS,
+			      "a part a warp");
+		const uint32_t decoder = warp - PREFILL_FIRST_DECODE_WARP, team = decoder / PREFILL_PARTS, member = decoder % PREFILL_PARTS;
 		const uint32_t step = member % PREFILL_STEPS, g = GROUPS > 1u ? member / PREFILL_STEPS : 0u;
 		const uint32_t m = MATRICES > 1u ? member / PREFILL_STEPS : 0u;
 		const uint32_t begin = ring::begin(lane);
@@ -620,7 +648,8 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 		if (!good)
 			shared->failed = 1;
 		tensor_fence_after();
-		decode_sync(); /* every decode warp has its verdict in */
+		asm volatile("cp.async.wait_all;" ::: "memory");
+		decode_sync(); /* every decode warp has its verdict in, and the scales are in place */
 		return shared->failed == 0;
 	}
 }
@@ -628,18 +657,19 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 /* Begins a product CTA: barriers, tensor memory, and the pair's agreement on whether to run. All threads of both CTAs
  * call; false: an earlier wait ran out, the pair is to go (the flag is never cleared while the kernel file stays loaded:
  * later CTAs do not queue up behind the same fault, the host reads the flag and rejects the result). */
-__device__ __forceinline__ bool prefill_begin(prefill_shared *shared, uint32_t rank)
+__device__ __forceinline__ bool prefill_begin(prefill_shared *shared, uint32_t rank, uint32_t stages)
 {
 	const uint32_t warp = threadIdx.x / EXL3_WARP;
 	if (threadIdx.x == 0) {
-		for (uint32_t stage = 0; stage < EXL3_PREFILL_STAGES; stage++) {
-			/* the four warps of the team that decodes the stage, the rows' copies, at rank 0 the other CTA */
-			barrier_init(&shared->full[stage], rank == 0 ? 6u : 5u);
+		for (uint32_t stage = 0; stage < stages; stage++) {
+			/* the warps of the team that decodes the stage, the rows' copies, at rank 0 the other CTA */
+			barrier_init(&shared->full[stage], PREFILL_PARTS + (rank == 0 ? 2u : 1u));
 			barrier_init(&shared->free[stage], 1);
 		}
 		barrier_init(&shared->done, 1);
 		shared->failed = 0;
 		shared->armed = 0;
+		shared->stages = stages;
 		shared->expired = *reinterpret_cast<volatile unsigned int *>(&exl3_wait_expired);
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
@@ -700,9 +730,9 @@ __device__ __forceinline__ void prefill_release(prefill_shared *shared)
 	__syncthreads();
 	if (shared->failed != 0 && threadIdx.x == 0) {
 		/* a stage whose other arrivals are missing holds this thread up to the bound, long past its copies' end */
-		for (uint32_t back = 0; back < EXL3_PREFILL_STAGES && back < shared->armed; back++) {
+		for (uint32_t back = 0; back < shared->stages && back < shared->armed; back++) {
 			const uint32_t block = shared->armed - 1u - back;
-			(void)barrier_wait(&shared->full[block % EXL3_PREFILL_STAGES], (block / EXL3_PREFILL_STAGES) & 1u);
+			(void)barrier_wait(&shared->full[block % shared->stages], (block / shared->stages) & 1u);
 		}
 	}
 	__syncthreads();
@@ -737,40 +767,90 @@ __device__ __forceinline__ prefill_tile_view prefill_tile_of(const struct exl3_p
 
 /* The gate/up epilogue of one row tile and one group of 128 outputs, from the staged accumulators (gate rows, then up
  * rows): Hadamard, scales, SwiGLU, down-side transform, FP16 down operand blocks. Decode warps; a warp a row. */
-template <uint32_t BX2>
-__device__ __forceinline__ void prefill_gate_up_rows(const struct exl3_prefill_record &record, unsigned char *arena,
-						     const prefill_view &view, const prefill_tile_view &tile,
-						     uint32_t tile_index, uint32_t count, uint32_t group,
-						     const float *staging)
+__device__ __forceinline__ void prefill_gate_up_rows(const struct exl3_prefill_record &record, const prefill_view &view,
+						     const prefill_shared *shared, const prefill_tile_view &tile,
+						     uint32_t tile_index, uint32_t count, uint32_t group, float *staging)
 {
-	const uint32_t H = record.input_size, I = prefill_inner_of(record, tile.tile.expert);
+	const uint32_t I = prefill_inner_of(record, tile.tile.expert);
 	const uint32_t lane = threadIdx.x % EXL3_WARP, warp = threadIdx.x / EXL3_WARP;
-	const uint32_t channel = group * EXL3_TRANSFORM + lane * 4u;
-	const uint64_t codes = exl3_code_bytes(H, I, BX2);
-	float gate_scale[4], up_scale[4], down_scale[4];
-	load_half4(reinterpret_cast<const __half *>(arena + tile.gate + codes) + H + channel, gate_scale);
-	load_half4(reinterpret_cast<const __half *>(arena + tile.up + codes) + H + channel, up_scale);
-	load_half4(reinterpret_cast<const __half *>(arena + tile.down + exl3_code_bytes(I, H, BX2)) + channel, down_scale);
+	const uint32_t channel = group * EXL3_TRANSFORM + lane % 8u * 4u;
+	const __half *const scales = shared->scales[0] + lane % 8u * 4u;
 	const prefill_rows rows = prefill_rows_of(count, tile.tile.row_count, 1u, I);
 	unsigned char *const region = view.workspace + view.parts.down_operands + (uint64_t)tile_index * view.widest * 256u;
-	for (uint32_t row = warp - PREFILL_FIRST_DECODE_WARP; row < tile.tile.row_count; row += PREFILL_DECODE_WARPS) {
-		const float4 gate_raw = *reinterpret_cast<const float4 *>(staging + row * EXL3_PREFILL_STAGING_ROW + lane * 4u);
-		const float4 up_raw = *reinterpret_cast<const float4 *>(
-			staging + (EXL3_PREFILL_TILE_ROWS + row) * EXL3_PREFILL_STAGING_ROW + lane * 4u);
-		float gate[4] = { gate_raw.x, gate_raw.y, gate_raw.z, gate_raw.w };
-		float up[4] = { up_raw.x, up_raw.y, up_raw.z, up_raw.w };
-		hadamard128_warp(gate, lane);
-		hadamard128_warp(up, lane);
-		float hidden[4], fed[4];
-		exl3_swiglu4(gate, up, gate_scale, up_scale, record.activation_limit, hidden);
+	if (tile.tile.row_count <= PREFILL_FEW_ROWS) {
+		const uint32_t at = lane * 4u;
+		for (uint32_t row = warp - PREFILL_FIRST_DECODE_WARP; row < tile.tile.row_count; row += PREFILL_DECODE_WARPS) {
+			const float4 g = *reinterpret_cast<const float4 *>(staging + row * EXL3_PREFILL_STAGING_ROW + at);
+			const float4 u = *reinterpret_cast<const float4 *>(staging +
+									   (EXL3_PREFILL_TILE_ROWS + row) * EXL3_PREFILL_STAGING_ROW + at);
+			float gate[4] = { g.x, g.y, g.z, g.w }, up[4] = { u.x, u.y, u.z, u.w };
+			float gate_scale[4], up_scale[4], down_scale[4], fed[4];
+			load_half4(shared->scales[0] + at, gate_scale);
+			load_half4(shared->scales[1] + at, up_scale);
+			load_half4(shared->scales[2] + at, down_scale);
+			hadamard128_warp(gate, lane);
+			hadamard128_warp(up, lane);
+			exl3_swiglu4(gate, up, gate_scale, up_scale, record.activation_limit, fed);
 #pragma unroll
-		for (uint32_t i = 0; i < 4; i++)
-			fed[i] = __fmul_rn(hidden[i], down_scale[i]);
-		hadamard128_warp(fed, lane);
+			for (uint32_t i = 0; i < 4; i++)
+				fed[i] = __fmul_rn(fed[i], down_scale[i]);
+			hadamard128_warp(fed, lane);
 #pragma unroll
-		for (uint32_t i = 0; i < 4; i++)
-			fed[i] = __fmul_rn(fed[i], EXL3_NORMALIZATION);
-		store_half4(reinterpret_cast<__half *>(region + prefill_operand_byte(rows, 1u, 0u, row, channel)), fed);
+			for (uint32_t i = 0; i < 4; i++)
+				fed[i] = __fmul_rn(fed[i], EXL3_NORMALIZATION);
+			store_half4(reinterpret_cast<__half *>(
+					    region + prefill_operand_byte(rows, 1u, 0u, row, group * EXL3_TRANSFORM + at)),
+				    fed);
+		}
+		return;
+	}
+#pragma unroll 1
+	for (uint32_t first = (warp - PREFILL_FIRST_DECODE_WARP) * PREFILL_WARP_ROWS; first < tile.tile.row_count;
+	     first += PREFILL_DECODE_WARPS * PREFILL_WARP_ROWS) {
+		const uint32_t row = first + lane / 8u; /* beyond the tile's count: a row of whatever stands there, not stored */
+		/* the staged rows: up's, then gate's, which become the hidden values' */
+		float *const gate_at = staging + row * EXL3_PREFILL_STAGING_ROW + lane % 8u * 4u;
+		float *const up_at = gate_at + EXL3_PREFILL_TILE_ROWS * EXL3_PREFILL_STAGING_ROW;
+		/* One copy of the transform for up, gate and the down-side one, and of the hidden step for four values: what these
+		 * cost a unit of few rows is the fetch of their instructions (16 values of each unrolled: 10 to 13 k cycles an
+		 * epilogue of up to 16 rows, 4 k so). What a lane stores here it alone reads again. */
+#pragma unroll 1
+		for (uint32_t pass = 0; pass < 3u; pass++) {
+			float *const at = pass == 0u ? up_at : gate_at;
+			if (pass == 2u)
+#pragma unroll 1
+				for (uint32_t k = 0; k < 4; k++) {
+					float gate_scale[4], up_scale[4], down_scale[4], hidden[4];
+					load_half4(scales + 32u * k, gate_scale);
+					load_half4(scales + EXL3_TRANSFORM + 32u * k, up_scale);
+					load_half4(scales + 2u * EXL3_TRANSFORM + 32u * k, down_scale);
+					float4 *const to = reinterpret_cast<float4 *>(gate_at + 32u * k);
+					const float4 g = *to, u = *reinterpret_cast<const float4 *>(up_at + 32u * k);
+					float gate[4] = { g.x, g.y, g.z, g.w }, up[4] = { u.x, u.y, u.z, u.w };
+					exl3_swiglu4(gate, up, gate_scale, up_scale, record.activation_limit, hidden);
+					*to = make_float4(__fmul_rn(hidden[0], down_scale[0]), __fmul_rn(hidden[1], down_scale[1]),
+							  __fmul_rn(hidden[2], down_scale[2]), __fmul_rn(hidden[3], down_scale[3]));
+				}
+			float v[4][4];
+#pragma unroll
+			for (uint32_t k = 0; k < 4; k++) {
+				const float4 raw = *reinterpret_cast<const float4 *>(at + 32u * k);
+				v[k][0] = raw.x, v[k][1] = raw.y, v[k][2] = raw.z, v[k][3] = raw.w;
+			}
+			hadamard128_rows(v, lane);
+#pragma unroll
+			for (uint32_t k = 0; k < 4; k++) {
+				if (pass != 2u) {
+					*reinterpret_cast<float4 *>(at + 32u * k) = make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
+				} else if (row < tile.tile.row_count) {
+#pragma unroll
+					for (uint32_t j = 0; j < 4; j++)
+						v[k][j] = __fmul_rn(v[k][j], EXL3_NORMALIZATION);
+					store_half4(reinterpret_cast<__half *>(region + prefill_operand_byte(rows, 1u, 0u, row, channel + 32u * k)),
+						    v[k]);
+				}
+			}
+		}
 	}
 }
 
@@ -788,6 +868,13 @@ __device__ __forceinline__ void prefill_gate_up(const struct exl3_prefill_record
 	const unsigned char *const row_runs = view.workspace + view.parts.gate_up_operands +
 					      (uint64_t)(tile_index + (count == 2u ? rank : 0u)) * H * 512u +
 					      (count == 2u ? 0u : rank * rows.second);
+	if (mine != 0) {
+		const uint64_t codes = exl3_code_bytes(H, I, BX2), first_scale = group * EXL3_TRANSFORM;
+		prefill_fetch_scales(shared, 0u, reinterpret_cast<const __half *>(arena + first.gate + codes) + H + first_scale);
+		prefill_fetch_scales(shared, 1u, reinterpret_cast<const __half *>(arena + first.up + codes) + H + first_scale);
+		prefill_fetch_scales(shared, 2u, reinterpret_cast<const __half *>(arena + first.down + exl3_code_bytes(I, H, BX2)) +
+							 first_scale);
+	}
 	const bool complete = prefill_products<BX2, 2, 1>(matrices, I, group, mine, 1, row_runs, rows.half,
 							  H / (PREFILL_STEPS * EXL3_TILE), rank, dynamic_shared, shared);
 	if (threadIdx.x / EXL3_WARP >= PREFILL_FIRST_DECODE_WARP && complete && mine != 0) {
@@ -795,7 +882,7 @@ __device__ __forceinline__ void prefill_gate_up(const struct exl3_prefill_record
 		for (uint32_t tile = 0; tile < count; tile++) {
 			const prefill_tile_view rows_of = prefill_tile_of(record, arena, view, tile_index + tile);
 			prefill_stage_out(shared->tensor_memory, 2, tile * EXL3_PREFILL_TILE_ROWS, rows_of.tile.row_count, staging);
-			prefill_gate_up_rows<BX2>(record, arena, view, rows_of, tile_index + tile, count, group, staging);
+			prefill_gate_up_rows(record, view, shared, rows_of, tile_index + tile, count, group, staging);
 			decode_sync(); /* the staging rows are read: the next tile may overwrite them */
 		}
 	}
@@ -819,6 +906,9 @@ __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &r
 	const unsigned char *const row_runs = view.workspace + view.parts.down_operands +
 					      (uint64_t)(tile_index + (count == 2u ? rank : 0u)) * view.widest * 256u +
 					      (count == 2u ? 0u : rank * rows.second);
+	for (uint32_t g = 0; g < groups; g++)
+		prefill_fetch_scales(shared, g, reinterpret_cast<const __half *>(arena + first.down + exl3_code_bytes(I, H, BX2)) + I +
+							 (first_group + g) * EXL3_TRANSFORM);
 	const bool complete = prefill_products<BX2, 1, 2>(matrices, H, first_group, groups, sums, row_runs, rows.half,
 							  I / (PREFILL_STEPS * EXL3_TILE), rank, dynamic_shared, shared);
 	if (warp >= PREFILL_FIRST_DECODE_WARP && complete) {
@@ -829,23 +919,53 @@ __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &r
 			prefill_stage_out(shared->tensor_memory, groups, tile * EXL3_PREFILL_TILE_ROWS, rows_of.tile.row_count,
 					  staging);
 			for (uint32_t g = 0; g < groups; g++) {
-				const uint32_t channel = (first_group + g) * EXL3_TRANSFORM + lane * 4u;
-				float scale[4];
-				load_half4(reinterpret_cast<const __half *>(arena + first.down + exl3_code_bytes(I, H, BX2)) + I + channel,
-					   scale);
-				for (uint32_t row = warp - PREFILL_FIRST_DECODE_WARP; row < rows_of.tile.row_count;
-				     row += PREFILL_DECODE_WARPS) {
-					const struct exl3_prefill_entry entry = rows_of.entries[row];
-					const float4 raw = *reinterpret_cast<const float4 *>(
-						staging + (g * EXL3_PREFILL_TILE_ROWS + row) * EXL3_PREFILL_STAGING_ROW + lane * 4u);
-					float v[4] = { raw.x, raw.y, raw.z, raw.w };
-					hadamard128_warp(v, lane);
+				const uint32_t channel = (first_group + g) * EXL3_TRANSFORM + lane % 8u * 4u;
+				const __half *const scales = shared->scales[g] + lane % 8u * 4u;
+				if (rows_of.tile.row_count <= PREFILL_FEW_ROWS) {
+					float scale[4];
+					load_half4(shared->scales[g] + lane * 4u, scale);
+					for (uint32_t row = warp - PREFILL_FIRST_DECODE_WARP; row < rows_of.tile.row_count;
+					     row += PREFILL_DECODE_WARPS) {
+						const struct exl3_prefill_entry entry = rows_of.entries[row];
+						const float4 raw = *reinterpret_cast<const float4 *>(
+							staging + (g * EXL3_PREFILL_TILE_ROWS + row) * EXL3_PREFILL_STAGING_ROW + lane * 4u);
+						float v[4] = { raw.x, raw.y, raw.z, raw.w };
+						hadamard128_warp(v, lane);
 #pragma unroll
-					for (uint32_t i = 0; i < 4; i++)
-						v[i] = __fmul_rn(__fmul_rn(__fmul_rn(v[i], EXL3_NORMALIZATION), scale[i]),
-								 entry.route_weight);
-					*reinterpret_cast<float4 *>(outputs + (uint64_t)entry.pair * H + channel) =
-						make_float4(v[0], v[1], v[2], v[3]);
+						for (uint32_t i = 0; i < 4; i++)
+							v[i] = __fmul_rn(__fmul_rn(__fmul_rn(v[i], EXL3_NORMALIZATION), scale[i]),
+									 entry.route_weight);
+						*reinterpret_cast<float4 *>(outputs + (uint64_t)entry.pair * H +
+									    (first_group + g) * EXL3_TRANSFORM + lane * 4u) =
+							make_float4(v[0], v[1], v[2], v[3]);
+					}
+					continue;
+				}
+				for (uint32_t from = (warp - PREFILL_FIRST_DECODE_WARP) * PREFILL_WARP_ROWS; from < rows_of.tile.row_count;
+				     from += PREFILL_DECODE_WARPS * PREFILL_WARP_ROWS) {
+					const uint32_t row = from + lane / 8u;
+					const struct exl3_prefill_entry entry = rows_of.entries[min(row, rows_of.tile.row_count - 1u)];
+					const float *const at =
+						staging + (g * EXL3_PREFILL_TILE_ROWS + row) * EXL3_PREFILL_STAGING_ROW + lane % 8u * 4u;
+					float v[4][4];
+#pragma unroll
+					for (uint32_t k = 0; k < 4; k++) {
+						const float4 raw = *reinterpret_cast<const float4 *>(at + 32u * k);
+						v[k][0] = raw.x, v[k][1] = raw.y, v[k][2] = raw.z, v[k][3] = raw.w;
+					}
+					hadamard128_rows(v, lane);
+#pragma unroll
+					for (uint32_t k = 0; k < 4; k++) {
+						float scale[4];
+						load_half4(scales + 32u * k, scale);
+#pragma unroll
+						for (uint32_t j = 0; j < 4; j++)
+							v[k][j] = __fmul_rn(__fmul_rn(__fmul_rn(v[k][j], EXL3_NORMALIZATION), scale[j]),
+									    entry.route_weight);
+						if (row < rows_of.tile.row_count)
+							*reinterpret_cast<float4 *>(outputs + (uint64_t)entry.pair * H + channel + 32u * k) =
+								make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
+					}
 				}
 			}
 			decode_sync();
@@ -893,7 +1013,7 @@ extern "C" __global__ void __cluster_dims__(PREFILL_PAIR, 1, 1) __launch_bounds_
 	const uint32_t count = prefill_tiles_of_unit(view, tile, tile_index, tile_count);
 	if (count == 0 || first_group >= prefill_inner_of(record, tile.expert) / EXL3_TRANSFORM)
 		return;
-	if (!prefill_begin(&shared, rank)) {
+	if (!prefill_begin(&shared, rank, prefill_rings<2, 1>::stages)) {
 		prefill_release(&shared);
 		return;
 	}
@@ -917,7 +1037,7 @@ extern "C" __global__ void __cluster_dims__(PREFILL_PAIR, 1, 1) __launch_bounds_
 	const uint32_t count = prefill_tiles_of_unit(view, tile, tile_index, tile_count);
 	if (count == 0)
 		return;
-	if (!prefill_begin(&shared, rank)) {
+	if (!prefill_begin(&shared, rank, prefill_rings<1, 2>::stages)) {
 		prefill_release(&shared);
 		return;
 	}

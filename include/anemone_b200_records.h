@@ -673,7 +673,7 @@ struct router_select_b200_arguments {
  *   exl3_prefill_group     grid (local + shared) x 256: entries[local expert][...]: the pairs routed to the expert in
  *                          ascending row order, and their count
  *   exl3_prefill_tiles     grid 1 x 1024: the tile table: (expert, first entry, rows) per 128-row tile, tile count
- *   exl3_prefill_operands  grid (tile capacity, 4 ceil(H / 512), 2) x 128: FP16 gate and up operands of every tile row
+ *   exl3_prefill_operands  grid (tile capacity, 4 ceil(H / 512)) x 128: FP16 gate and up operands of every tile row
  *   exl3_prefill_gate_up   grid (ceil(max(I, shared I) / 256), tile capacity) pairs of CTAs x 576: both products, SwiGLU,
  *                          FP16 down operands
  *   exl3_prefill_down      grid (ceil(H / 512), tile capacity) pairs of CTAs x 576: down product, output transform: FP32
@@ -684,7 +684,7 @@ struct router_select_b200_arguments {
  *   counts uint32 [local + shared + 1] (the last: tile count) | tiles struct exl3_prefill_tile [tile capacity] |
  *   entries struct exl3_prefill_entry [local + shared][row_capacity] |
  *   gate/up operands FP16, H * 512 bytes a tile | down operands FP16, max(I, shared I) * 256 bytes a tile
- * stored as the tensor cores read them without swizzling, and so that what a CTA of a pair reads for 32 inputs is one
+ * stored as the tensor cores read them without swizzling, and so that what a CTA of a pair reads for 64 inputs is one
  * run of bytes: [H / 32][gate, up][4 pieces of eight inputs][rows][16 bytes] (down: without the second part), the rows
  * being the tile's 128, or, for an expert's last tile if its number is even (counted from 0), half its rows rounded up
  * to whole sixteens, the other half's runs behind them.
