@@ -38,8 +38,8 @@
 
 #define MX_THREADS MX_PRODUCTS_THREADS
 #define MX_WARP_WEIGHTS 12u /* behind the epilogue's, the multiplying, the scheduling and the rows' warps */
-#define MX_TEAMS 2u
-#define MX_TEAM_WARPS 8u /* a warp a tile of 16 weight rows */
+#define MX_WEIGHT_WARPS 16u
+#define MX_TILES 8u /* of 16 weight rows, of a unit */
 
 #define MX_BLOCK_INPUTS 128u /* a block: the inputs whose scales one tcgen05.cp brings */
 #define MX_STAGE_BLOCKS 2u
@@ -56,7 +56,7 @@
 /* units the scheduler may be ahead: more than the units a warp's loads in flight can reach into (two stages of its team's,
  * four units where K is 256 or less), so that no role waits for a unit that waits for it */
 #define MX_UNITS 8u
-#define MX_WEIGHTS_AHEAD 8u /* loads of a lane in flight */
+#define MX_CHUNK 4u /* loads of a lane stored, and asked for again, together; two chunks are in flight */
 #define MX_SCALE_COLUMN 256u /* tensor memory: two accumulators of 128 columns, then the stages' scales */
 #define MX_MOST_STAGES 5u
 
@@ -69,6 +69,11 @@ template <bool FEW> struct mx_form {
 	static constexpr uint32_t stages = FEW ? 5u : 3u;
 	static constexpr uint32_t epilogue_warps = FEW ? 4u : 8u;
 	static constexpr uint32_t row_warps = FEW ? 4u : 1u;
+	/* The weights' warps in teams that take the stages in turns, each warp MX_TILES / team_warps tiles of its team's. What a
+	 * stage costs a warp beside its stores (the wait for the place, the fence, the arrival, the next unit's pointers: about
+	 * as much as one tile) is paid once for two tiles by teams of four, and four stages of the ring of five are filled at
+	 * once; the many rows' ring holds three. */
+	static constexpr uint32_t team_warps = FEW ? 4u : 8u, teams = MX_WEIGHT_WARPS / team_warps;
 	static constexpr uint32_t multiply = epilogue_warps, schedule = multiply + 1u, rows = schedule + 1u;
 	static constexpr uint32_t b_at = stages * MX_OPERAND;
 	static constexpr uint32_t scales_at = b_at + stages * b_operand;
@@ -78,7 +83,7 @@ template <bool FEW> struct mx_form {
 	static_assert(bytes <= MX_PRODUCTS_DYNAMIC_BYTES && stages <= MX_MOST_STAGES, "the host sizes the shared memory");
 	static_assert(rows + row_warps <= MX_WARP_WEIGHTS, "the warps' order");
 };
-static_assert((MX_WARP_WEIGHTS + MX_TEAMS * MX_TEAM_WARPS) * EXL3_WARP == MX_THREADS, "the warps of a CTA");
+static_assert((MX_WARP_WEIGHTS + MX_WEIGHT_WARPS) * EXL3_WARP == MX_THREADS, "the warps of a CTA");
 
 struct mx_unit {
 	const unsigned char *matrix[2];
@@ -382,101 +387,137 @@ template <bool BYTES> __device__ __forceinline__ void mx_store_scales(unsigned c
 template <uint32_t STAGES> struct mx_weights_place {
 	struct mx_place units;
 	struct mx_stage_place<STAGES> stage;
-	uint32_t begun; /* stages of the units entered so far: their parity says whose the next unit's first stage is */
+	uint32_t begun; /* stages of the units entered so far: they say whose the next unit's first stage is */
 };
 
-/* The units of one kind that follow one another, by one warp of a team: its tile of 16 weight rows of every second
- * stage. False once a wait ran out. */
+/* The units of one kind that follow one another, by one warp of a team: its tiles of 16 weight rows of every stage of its
+ * team's. A stage is a run of chunks of MX_CHUNK loads (MXFP4: a tile; E4M3: half a tile, a block); a chunk's registers are
+ * asked for the chunk after next as soon as they are stored, across the stages' and the units' ends. False once a wait ran
+ * out. */
 template <bool DOWN, bool FEW, bool BYTES>
-__device__ __forceinline__ bool mx_weights(const struct mx_products_arguments &arguments, struct mx_shared &shared,
-					   unsigned char *dynamic_shared, uint32_t lane, uint32_t team, uint32_t warp,
-					   struct mx_weights_place<mx_form<FEW>::stages> &place)
+__device__ __forceinline__ bool mx_weights(const struct mx_products_arguments &arguments, const unsigned char *arena,
+					   struct mx_shared &shared, unsigned char *dynamic_shared, uint32_t lane, uint32_t team,
+					   uint32_t warp, struct mx_weights_place<mx_form<FEW>::stages> &place)
 {
+	typedef mx_form<FEW> form;
 	constexpr uint32_t kind = BYTES ? MX_UNIT_SHARED : MX_UNIT_ROUTED;
-	constexpr uint32_t block_items = BYTES ? 4u : 2u, items = MX_STAGE_BLOCKS * block_items; /* loads of a stage */
-	constexpr uint32_t ahead = MX_WEIGHTS_AHEAD / items; /* the team's stages in flight */
+	constexpr uint32_t tiles = MX_TILES / form::team_warps, halves = BYTES ? 2u : 1u, chunks = tiles * halves;
+	constexpr uint32_t block_items = BYTES ? 4u : 2u, stage_items = MX_STAGE_BLOCKS * block_items; /* of a tile */
+	constexpr uint32_t turn = chunks < 2u ? 2u : chunks; /* chunks of one turn of the loop */
+	static_assert(halves * MX_CHUNK == stage_items && turn % 2u == 0u && turn % chunks == 0u, "chunks make stages");
 	const uint32_t K = arguments.input_size, blocks = K / MX_BLOCK_INPUTS, stages = mx_stages_of(K);
 	const uint64_t weights = (uint64_t)arguments.output_size * K;
 	const bool constant_scales = BYTES && arguments.shared_format == WEIGHT_FORMAT_E4M3_BLOCK128;
-	uint4 ring[MX_WEIGHTS_AHEAD];
-	uint32_t scales[ahead];
-	const uint4 *from = nullptr;
-	const uint32_t *scales_from = nullptr;
-	uint32_t at = stages, pending = 0; /* at: the next stage of the unit entered last; from `stages` on: it has no more */
+	uint4 held[2][MX_CHUNK];
+	uint32_t scales[2];
+	const uint4 *from[tiles]; /* of the stage whose chunks are asked for */
+	const uint32_t *scales_from[tiles];
+	uint32_t at = stages, pending = 0; /* at: that stage of its unit; from `stages` on: the unit has no more */
 	bool more = true, good = true;
-	/* the team's next stage into place `t` of those in flight */
-#define MX_WEIGHTS_LOAD(t)                                                                                             \
-	do {                                                                                                           \
-		while (more && at >= stages) {                                                                         \
-			const struct mx_unit *const unit = place.units.peek(shared);                                   \
-			good = unit != nullptr;                                                                        \
-			more = good && unit->kind == kind;                                                             \
-			if (more) {                                                                                    \
-				const uint32_t tile = DOWN ? unit->group * 8u + warp : unit->group * 4u + warp % 4u;   \
-				const unsigned char *const matrix = unit->matrix[DOWN ? 0u : warp / 4u];               \
-				at = (place.begun ^ team) & 1u;                                                        \
-				place.begun += stages;                                                                 \
-				from = reinterpret_cast<const uint4 *>(matrix) +                                       \
-				       ((uint64_t)tile * blocks + at * MX_STAGE_BLOCKS) * (block_items * EXL3_WARP) + lane; \
-				if (BYTES)                                                                             \
-					scales_from = reinterpret_cast<const uint32_t *>(                              \
-							      matrix + weights + (uint64_t)(tile / 2u) * (K / 32u)) +  \
-						      at * MX_STAGE_BLOCKS + lane / 16u;                               \
-				else                                                                                   \
-					scales_from = reinterpret_cast<const uint32_t *>(matrix + weights / 2u) +      \
-						      ((uint64_t)tile * blocks + at * MX_STAGE_BLOCKS) * 16u + lane;   \
-				place.units.release(shared, lane);                                                     \
-			}                                                                                              \
-		}                                                                                                      \
-		if (more) {                                                                                            \
-			/* a last stage of one block: nothing reads what its second block's place holds */             \
-			const bool whole = at * MX_STAGE_BLOCKS + 1u < blocks;                                         \
-			_Pragma("unroll") for (uint32_t item = 0; item < items; item++)                                \
-				if (item < block_items || whole)                                                       \
-					ring[(t) * items + item] = __ldcs(from + item * EXL3_WARP);                    \
-			scales[t] = 0x7F7F7F7Fu;                                                                       \
-			if (!constant_scales && (whole || lane < 16u))                                                 \
-				scales[t] = __ldg(scales_from);                                                        \
-			from += MX_TEAMS * items * EXL3_WARP;                                                          \
-			scales_from += MX_TEAMS * MX_STAGE_BLOCKS * (BYTES ? 1u : 16u);                                \
-			at += MX_TEAMS;                                                                                \
-			pending++;                                                                                     \
-		}                                                                                                      \
-	} while (0)
 #pragma unroll
-	for (uint32_t t = 0; t < ahead; t++)
-		MX_WEIGHTS_LOAD(t);
+	for (uint32_t tile = 0; tile < tiles; tile++) {
+		from[tile] = reinterpret_cast<const uint4 *>(arena);
+		scales_from[tile] = reinterpret_cast<const uint32_t *>(arena);
+	}
+	/* the next stage of the team's, in this unit or one behind it */
+	auto enter = [&]() {
+		if (more) {
+			at += form::teams;
+#pragma unroll
+			for (uint32_t tile = 0; tile < tiles; tile++) {
+				from[tile] += form::teams * stage_items * EXL3_WARP;
+				scales_from[tile] += form::teams * MX_STAGE_BLOCKS * (BYTES ? 1u : 16u);
+			}
+		}
+		while (more && at >= stages) {
+			const struct mx_unit *const unit = place.units.peek(shared);
+			good = unit != nullptr;
+			more = good && unit->kind == kind;
+			if (more) {
+				at = (team - place.begun) % form::teams;
+				place.begun += stages;
+#pragma unroll
+				for (uint32_t tile = 0; tile < tiles; tile++) {
+					const uint32_t local = tile * form::team_warps + warp;
+					const uint32_t row_tile = DOWN ? unit->group * 8u + local : unit->group * 4u + local % 4u;
+					const unsigned char *const matrix = unit->matrix[DOWN ? 0u : local / 4u];
+					from[tile] = reinterpret_cast<const uint4 *>(matrix) +
+						     ((uint64_t)row_tile * blocks + at * MX_STAGE_BLOCKS) * (block_items * EXL3_WARP) + lane;
+					if (BYTES)
+						scales_from[tile] = reinterpret_cast<const uint32_t *>(
+									    matrix + weights + (uint64_t)(row_tile / 2u) * (K / 32u)) +
+								    at * MX_STAGE_BLOCKS + lane / 16u;
+					else
+						scales_from[tile] = reinterpret_cast<const uint32_t *>(matrix + weights / 2u) +
+								    ((uint64_t)row_tile * blocks + at * MX_STAGE_BLOCKS) * 16u + lane;
+				}
+				place.units.release(shared, lane);
+			}
+		}
+		pending += more ? 1u : 0u;
+	};
+	/* Chunk `sub` of that stage into place `to`. Every register is loaded on every path (the arena's first bytes where there
+	 * is no stage left; a last stage of one block brings its first block twice, and nothing reads the second's place): a
+	 * load under a condition would make a copy of the register where the paths meet, and the copy waits for the load. */
+	auto ask = [&](uint32_t to, uint32_t sub) {
+		const uint32_t tile = sub / halves, half = sub % halves;
+		const bool whole = at * MX_STAGE_BLOCKS + 1u < blocks;
+		const uint4 *const first = more ? from[tile] : reinterpret_cast<const uint4 *>(arena);
+		const uint32_t step = more ? EXL3_WARP : 0u, second = more && whole ? block_items * EXL3_WARP : 0u;
+#pragma unroll
+		for (uint32_t item = 0; item < MX_CHUNK; item++) {
+			const uint32_t stage_item = half * MX_CHUNK + item;
+			held[to][item] = __ldcs(first + stage_item % block_items * step + (stage_item < block_items ? 0u : second));
+		}
+		if (half == 0u)
+			scales[to] = __ldg(more && !constant_scales ?
+						   scales_from[tile] - (whole || lane < 16u ? 0u : BYTES ? 1u : 16u) :
+						   reinterpret_cast<const uint32_t *>(arena));
+	};
+	enter();
+	ask(0u, 0u);
+	if (chunks == 1u)
+		enter();
+	ask(1u, 1u % chunks);
 	/* lane 4 g + t: row g of the tile, its quarter t of the block's inputs */
 	unsigned char *const lane_at = dynamic_shared + (lane % 4u / 2u) * MX_PIECE + (warp * 16u + lane / 4u) * 16u +
 				       (lane % 2u) * (BYTES ? 8u : 4u);
 	const uint32_t row = warp * 16u + (BYTES ? lane % 16u : lane % 8u);
-	unsigned char *const lane_scales = dynamic_shared + mx_form<FEW>::scales_at + row % 32u * 16u + row / 32u * 4u +
+	unsigned char *const lane_scales = dynamic_shared + form::scales_at + row % 32u * 16u + row / 32u * 4u +
 					   lane / 16u * (2u * MX_SCALE_BYTES) + (BYTES ? 0u : lane / 8u % 2u * 2u);
 	while (good && pending != 0) {
 #pragma unroll
-		for (uint32_t t = 0; t < ahead; t++) {
-			if (!good || pending == 0)
-				break;
-			good = mx_wait(&shared.empty[place.stage.slot], place.stage.parity ^ 1u);
-			unsigned char *const to = lane_at + place.stage.slot * MX_OPERAND;
+		for (uint32_t chunk = 0; chunk < turn; chunk++) {
+			const uint32_t sub = chunk % chunks, tile = sub / halves, half = sub % halves, here = chunk % 2u;
+			if (sub == 0u) {
+				if (!good || pending == 0)
+					break;
+				good = mx_wait(&shared.empty[place.stage.slot], place.stage.parity ^ 1u);
+			}
+			unsigned char *const to = lane_at + place.stage.slot * MX_OPERAND + tile * (form::team_warps * 256u);
 #pragma unroll
-			for (uint32_t item = 0; item < items; item++)
+			for (uint32_t item = 0; item < MX_CHUNK; item++)
 				if (BYTES)
-					mx_store_bytes(to + item * 2u * MX_PIECE, ring[t * items + item]);
+					mx_store_bytes(to + (half * MX_CHUNK + item) * 2u * MX_PIECE, held[here][item]);
 				else
-					mx_store_nibbles(to + item * 4u * MX_PIECE, ring[t * items + item]);
-			mx_store_scales<BYTES>(lane_scales + place.stage.slot * MX_STAGE_SCALES, scales[t]);
-			mx_proxy_fence();
-			__syncwarp();
-			if (lane == 0)
-				barrier_arrive(&shared.full[place.stage.slot]);
-			place.stage.advance(MX_TEAMS);
-			pending--;
-			if (good)
-				MX_WEIGHTS_LOAD(t);
+					mx_store_nibbles(to + item * 4u * MX_PIECE, held[here][item]);
+			if (half == 0u)
+				mx_store_scales<BYTES>(lane_scales + place.stage.slot * MX_STAGE_SCALES + tile * (form::team_warps / 2u * 4u),
+						       constant_scales ? 0x7F7F7F7Fu : scales[here]);
+			if (sub == chunks - 1u) {
+				mx_proxy_fence();
+				__syncwarp();
+				if (lane == 0)
+					barrier_arrive(&shared.full[place.stage.slot]);
+				place.stage.advance(form::teams);
+				pending--;
+			}
+			more = more && good;
+			if ((chunk + 2u) % chunks == 0u)
+				enter();
+			ask(here, (chunk + 2u) % chunks);
 		}
 	}
-#undef MX_WEIGHTS_LOAD
 	return good;
 }
 
@@ -893,10 +934,10 @@ __device__ __forceinline__ void mx_run(const struct mx_products_arguments &argum
 			barrier_init(&shared.unit_full[slot], 1);
 			/* the weights', the rows', the multiplying and the epilogue's warps */
 			barrier_init(&shared.unit_free[slot],
-				     MX_TEAMS * MX_TEAM_WARPS + form::row_warps + 1u + form::epilogue_warps);
+				     MX_WEIGHT_WARPS + form::row_warps + 1u + form::epilogue_warps);
 		}
 		for (uint32_t stage = 0; stage < form::stages; stage++) {
-			barrier_init(&shared.full[stage], MX_TEAM_WARPS + 1u); /* the stage's team, and the warp that brings its rows */
+			barrier_init(&shared.full[stage], form::team_warps + 1u); /* the stage's team, and the warp that brings its rows */
 			barrier_init(&shared.empty[stage], 1);
 		}
 		for (uint32_t sum = 0; sum < 2u; sum++) {
@@ -928,10 +969,10 @@ __device__ __forceinline__ void mx_run(const struct mx_products_arguments &argum
 	} else if (warp == form::schedule) {
 		mx_schedule<DOWN, FEW>(arguments, arena, shared, lane);
 	} else if (warp >= MX_WARP_WEIGHTS) {
-		const uint32_t team = (warp - MX_WARP_WEIGHTS) / MX_TEAM_WARPS, tile = (warp - MX_WARP_WEIGHTS) % MX_TEAM_WARPS;
+		const uint32_t team = (warp - MX_WARP_WEIGHTS) / form::team_warps, tile = (warp - MX_WARP_WEIGHTS) % form::team_warps;
 		struct mx_weights_place<form::stages> place = { { 0u }, { team, 0u }, 0u };
-		if (mx_weights<DOWN, FEW, true>(arguments, shared, dynamic_shared, lane, team, tile, place))
-			(void)mx_weights<DOWN, FEW, false>(arguments, shared, dynamic_shared, lane, team, tile, place);
+		if (mx_weights<DOWN, FEW, true>(arguments, arena, shared, dynamic_shared, lane, team, tile, place))
+			(void)mx_weights<DOWN, FEW, false>(arguments, arena, shared, dynamic_shared, lane, team, tile, place);
 	} else if (warp < form::rows + form::row_warps) {
 		if (DOWN)
 			asm volatile("griddepcontrol.wait;" ::: "memory");
