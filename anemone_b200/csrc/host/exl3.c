@@ -484,11 +484,12 @@ result_status exl3_prefill_prepare(const struct exl3_prefill_record *record, uin
 								  "exl3_prefill_tiles",	   "exl3_prefill_operands",
 								  "exl3_prefill_gate_up",  "exl3_prefill_down",
 								  "exl3_prefill_row_sum" };
-	const uint32_t row_warps = ROUTER_B200_THREADS / EXL3_WARP;
+	/* a warp a row, four to a block: a few hundred rows in blocks of 32 stand on a dozen SMs and share their issue slots */
+	const uint32_t row_warps = 4u;
 	const struct {
 		uint32_t x, y, z, threads, shared;
 	} shapes[EXL3_PREFILL_LAUNCHES] = {
-		{ (record->row_capacity + row_warps - 1u) / row_warps, 1, 1, ROUTER_B200_THREADS, 0 },
+		{ (record->row_capacity + row_warps - 1u) / row_warps, 1, 1, row_warps * EXL3_WARP, 0 },
 		{ experts, 1, 1, 256u, 0 },
 		{ 1, 1, 1, ROUTER_B200_THREADS, 0 },
 		{ parts.tile_capacity, transform_grid(H) * EXL3_PREFILL_OPERAND_PARTS, 1, EXL3_TRANSFORM_THREADS, 0 },

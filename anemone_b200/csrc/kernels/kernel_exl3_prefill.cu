@@ -81,7 +81,7 @@ extern "C" __global__ void __launch_bounds__(ROUTER_B200_THREADS)
 	const struct step_block step = *reinterpret_cast<const struct step_block *>(arena + record.step_offset);
 	const uint32_t live = min(step.row_count, record.row_capacity);
 	const uint32_t warp = threadIdx.x / WARP, lane = threadIdx.x % WARP;
-	const uint32_t row = blockIdx.x * (ROUTER_B200_THREADS / WARP) + warp;
+	const uint32_t row = blockIdx.x * (blockDim.x / WARP) + warp;
 	if (row >= live)
 		return;
 	router_row(reinterpret_cast<const float *>(arena + record.scores_offset) + (uint64_t)row * record.expert_count,

@@ -87,41 +87,72 @@ __device__ __forceinline__ float router_affinity(float score, uint32_t scoring)
 	return __fdiv_rn(1.0f, __fadd_rn(1.0f, router_exponential(-score)));
 }
 
-/* One row by one warp: `picks` rounds of a warp-wide maximum over 64-bit keys of affinity + bias (bias may be null:
- * none), as the reference's router_row (source/kernel_router.cuh:47-119); the weights come from the affinities alone.
+/* The order of router_key's upper half: the score as the top-k orders it, never 0, which stands for no expert. */
+__device__ __forceinline__ uint32_t router_order(float score)
+{
+	return (uint32_t)(router_key(score, 0) >> 32);
+}
+
+/* One warp's `picks` largest of PLACES keys a lane: orders[place] of expert first + place * stride + lane, 0 where there is
+ * none; lane p gets the expert of pick p, and keys_out (may be null) the keys. Within a lane a later place is a higher expert, so that a strict comparison
+ * keeps the lower one of equals and 32 bits are enough; across lanes the largest order, then the lowest expert that holds
+ * it, by two 32-bit reductions. (With 64-bit keys, five shuffles of two words a pick and room for 512 experts whatever
+ * their number, 512 rows of 256 experts took 17 us, a warp a row; 10 so.) */
+template <uint32_t PLACES>
+__device__ __forceinline__ uint32_t router_pick(uint32_t (&orders)[PLACES], uint32_t stride, uint32_t first, uint32_t picks,
+						uint32_t lane, uint64_t *keys_out)
+{
+	uint32_t mine = 0;
+	for (uint32_t pick = 0; pick < picks; pick++) {
+		uint32_t best = 0, at = 0;
+#pragma unroll
+		for (uint32_t place = 0; place < PLACES; place++)
+			if (orders[place] > best)
+				best = orders[place], at = place;
+		const uint32_t expert = first + at * stride + lane;
+		const uint32_t largest = __reduce_max_sync(0xFFFFFFFFu, best);
+		const uint32_t chosen = ~__reduce_max_sync(0xFFFFFFFFu, best == largest ? ~expert : 0u);
+		const uint32_t gone = chosen == expert ? at : PLACES;
+#pragma unroll
+		for (uint32_t place = 0; place < PLACES; place++)
+			orders[place] = place == gone ? 0u : orders[place];
+		if (lane == pick)
+			mine = chosen;
+		/* the key of a pick, 0 where there were fewer experts */
+		if (keys_out != nullptr && lane == pick)
+			keys_out[pick] = largest != 0u ? (uint64_t)largest << 32 | ~chosen : 0ull;
+	}
+	return mine;
+}
+
+template <uint32_t PLACES>
+__device__ __forceinline__ uint32_t router_row_picks(const float *scores, const float *bias, uint32_t experts, uint32_t picks,
+						     uint32_t scoring, uint32_t lane)
+{
+	uint32_t orders[PLACES];
+#pragma unroll
+	for (uint32_t place = 0; place < PLACES; place++) {
+		const uint32_t expert = place * WARP + lane;
+		orders[place] = 0u;
+		if (expert < experts) {
+			const float affinity = router_affinity(scores[expert], scoring);
+			orders[place] = router_order(bias != nullptr ? __fadd_rn(affinity, bias[expert]) : affinity);
+		}
+	}
+	return router_pick<PLACES>(orders, WARP, 0u, picks, lane, nullptr);
+}
+
+/* One row by one warp: `picks` rounds of a warp-wide maximum over the keys of affinity + bias (bias may be null: none), as
+ * the reference's router_row (source/kernel_router.cuh:47-119); the weights come from the affinities alone.
  * chosen and weight: the row's ROUTER_B200_MAXIMUM_PICKS entries in shared memory, filled by slot; the same values go
  * to picks_out and weights_out (the row's entries in the arena) unless those are null. All 32 lanes call. */
 __device__ __forceinline__ void router_row(const float *scores, const float *bias, uint32_t experts, uint32_t picks,
 					   uint32_t scoring, float route_scale, uint32_t lane, uint32_t *chosen,
 					   float *weight, uint32_t *picks_out, float *weights_out)
 {
-	uint64_t keys[EXPERTS_PER_LANE];
-#pragma unroll
-	for (uint32_t place = 0; place < EXPERTS_PER_LANE; place++) {
-		const uint32_t expert = place * WARP + lane;
-		if (expert < experts) {
-			const float affinity = router_affinity(scores[expert], scoring);
-			keys[place] = router_key(bias != nullptr ? __fadd_rn(affinity, bias[expert]) : affinity, expert);
-		} else {
-			keys[place] = 0ull;
-		}
-	}
-	uint32_t mine = 0; /* lane p keeps pick p */
-	for (uint32_t pick = 0; pick < picks; pick++) {
-		uint64_t best = 0;
-#pragma unroll
-		for (uint32_t place = 0; place < EXPERTS_PER_LANE; place++)
-			best = keys[place] > best ? keys[place] : best;
-		for (uint32_t distance = WARP / 2u; distance != 0; distance >>= 1) {
-			const uint64_t other = __shfl_xor_sync(0xFFFFFFFFu, best, distance);
-			best = other > best ? other : best;
-		}
-#pragma unroll
-		for (uint32_t place = 0; place < EXPERTS_PER_LANE; place++)
-			keys[place] = keys[place] == best ? 0ull : keys[place];
-		if (lane == pick)
-			mine = ~(uint32_t)best;
-	}
+	/* lane p keeps pick p */
+	const uint32_t mine = experts <= 8u * WARP ? router_row_picks<8u>(scores, bias, experts, picks, scoring, lane) :
+						     router_row_picks<EXPERTS_PER_LANE>(scores, bias, experts, picks, scoring, lane);
 	/* slot = the number of picked experts below mine */
 	uint32_t slot = 0;
 	for (uint32_t pick = 0; pick < picks; pick++) {
@@ -170,29 +201,18 @@ __device__ __forceinline__ void router_row_team(const float *scores, const float
 						uint32_t barrier, uint64_t *candidates, uint32_t *chosen, float *weight,
 						uint32_t *picks_out, float *weights_out)
 {
-	uint64_t keys[ROUTER_TEAM_SLOTS];
+	uint32_t orders[ROUTER_TEAM_SLOTS];
 #pragma unroll
 	for (uint32_t place = 0; place < ROUTER_TEAM_SLOTS; place++) {
 		const uint32_t expert = (place * ROUTER_TEAM_WARPS + member) * WARP + lane;
+		orders[place] = 0u;
 		if (expert < experts) {
 			const float affinity = router_affinity(scores[expert], scoring);
-			keys[place] = router_key(bias != nullptr ? __fadd_rn(affinity, bias[expert]) : affinity, expert);
-		} else {
-			keys[place] = 0ull;
+			orders[place] = router_order(bias != nullptr ? __fadd_rn(affinity, bias[expert]) : affinity);
 		}
 	}
-	for (uint32_t pick = 0; pick < picks; pick++) {
-		uint64_t best = 0;
-#pragma unroll
-		for (uint32_t place = 0; place < ROUTER_TEAM_SLOTS; place++)
-			best = keys[place] > best ? keys[place] : best;
-		best = router_warp_largest(best);
-#pragma unroll
-		for (uint32_t place = 0; place < ROUTER_TEAM_SLOTS; place++)
-			keys[place] = keys[place] == best ? 0ull : keys[place];
-		if (lane == pick)
-			candidates[member * ROUTER_B200_MAXIMUM_PICKS + pick] = best;
-	}
+	(void)router_pick<ROUTER_TEAM_SLOTS>(orders, ROUTER_TEAM_WARPS * WARP, member * WARP, picks, lane,
+					     candidates + member * ROUTER_B200_MAXIMUM_PICKS);
 	asm volatile("bar.sync %0, %1;" ::"r"(barrier), "n"(ROUTER_TEAM_WARPS * WARP) : "memory");
 	if (member != 0)
 		return;
