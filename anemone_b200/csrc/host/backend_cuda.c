@@ -28,6 +28,9 @@
 #define STEP_WORDS 16u /* 64-bit words a graph: a line of 128 bytes of its own, the first two used */
 #define STEP_COPY_BLOCKS 64u
 #define CALL_PIECE_BYTES (1u << 19) /* 10 us of PCIe, 30 of a core's copy */
+/* Up to here half of that, since the first piece's copy hides behind nothing, and the pool's threads look out for a result's
+ * pieces: 333 rows of 4096 490 us a call, 455 so. (A prompt of 2048 rows: 2650, 2700 with both.) */
+#define CALL_SHORT_BYTES (8u << 20)
 #define STEP_SPIN_NANOSECONDS 2000000ull /* a step's wait looks at its word alone for so long */
 
 struct prepared_kernel {
@@ -1687,7 +1690,7 @@ static uint32_t call_pieces(struct ab_copy_batch *batch, const struct backend_b2
 	uint64_t total = 0;
 	for (uint32_t range = 0; range < count; range++)
 		total += ranges[range].byte_count;
-	uint64_t piece = CALL_PIECE_BYTES;
+	uint64_t piece = total <= CALL_SHORT_BYTES ? CALL_PIECE_BYTES / 2u : CALL_PIECE_BYTES;
 	while (total / piece + count > AB_COPY_BATCH_MOST)
 		piece *= 2u;
 	uint32_t pieces = 0;
@@ -1788,10 +1791,12 @@ result_status backend_b200_step_call(struct device_card *card, uint32_t graph,
 					processor_pause();
 			if (state != CUDA_SUCCESS) {
 				status = driver_failure(card, "a step call", state);
-				batch.count = batch.allowed; /* what has not arrived is not copied on */
+				ab_copy_batch_cut(&batch); /* what has not arrived is not copied on */
 				goto done;
 			}
 			ab_copy_batch_allow(&batch, piece + 1u);
+			if (piece == 0 && batch.copies[0].byte_count < CALL_PIECE_BYTES) /* a short call: the others follow closely */
+				ab_copy_batch_soon(&batch);
 		}
 		ab_copy_batch_end(&batch);
 		begun = false;

@@ -1,5 +1,6 @@
 /* copy_pool.c: host memory copies by a few threads at once (copy_pool.h). */
 #include "copy_pool.h"
+#include "processor.h"
 
 #include <pthread.h>
 #include <sched.h>
@@ -62,6 +63,13 @@ static void *pool_thread(void *unused)
 	(void)unused;
 	(void)pthread_mutex_lock(&mutex);
 	while (!ending) {
+		if (current != NULL && current->soon && current->next >= current->allowed && current->next < current->count) {
+			(void)pthread_mutex_unlock(&mutex);
+			for (uint32_t turn = 0; turn < 32u; turn++)
+				processor_pause();
+			(void)pthread_mutex_lock(&mutex);
+			continue;
+		}
 		if (current == NULL || current->next >= current->allowed) {
 			(void)pthread_cond_wait(&wake, &mutex);
 			continue;
@@ -108,7 +116,7 @@ void ab_copy_pool_leave(void)
 void ab_copy_batch_begin(struct ab_copy_batch *batch)
 {
 	batch->next = 0;
-	batch->shared = false;
+	batch->shared = batch->soon = false;
 	memset(batch->done, 0, sizeof(batch->done));
 	if (batch->count < 2)
 		return; /* not worth waking anyone */
@@ -132,6 +140,23 @@ void ab_copy_batch_allow(struct ab_copy_batch *batch, uint32_t allowed)
 	batch->allowed = allowed;
 	if (batch->shared)
 		(void)pthread_cond_signal(&wake);
+	(void)pthread_mutex_unlock(&mutex);
+}
+
+void ab_copy_batch_soon(struct ab_copy_batch *batch)
+{
+	(void)pthread_mutex_lock(&mutex);
+	if (batch->shared && !batch->soon) {
+		batch->soon = true;
+		(void)pthread_cond_broadcast(&wake);
+	}
+	(void)pthread_mutex_unlock(&mutex);
+}
+
+void ab_copy_batch_cut(struct ab_copy_batch *batch)
+{
+	(void)pthread_mutex_lock(&mutex);
+	batch->count = batch->allowed;
 	(void)pthread_mutex_unlock(&mutex);
 }
 

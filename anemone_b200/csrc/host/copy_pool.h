@@ -26,6 +26,7 @@ struct ab_copy_batch {
 	uint32_t done[AB_COPY_BATCH_MOST];
 	bool to_device; /* the copies' targets are read by the device next: written past the caches */
 	bool shared; /* the pool's threads help (else they are busy with another thread's batch) */
+	bool soon; /* under the pool's mutex: the rest will be allowed within microseconds */
 };
 
 void ab_copy_pool_enter(void); /* one more user (a card opens) */
@@ -34,6 +35,10 @@ void ab_copy_pool_leave(void); /* the last one ends the threads */
 /* offers the batch (copies, count and allowed filled in) to the pool; must be ended by the same thread */
 void ab_copy_batch_begin(struct ab_copy_batch *batch);
 void ab_copy_batch_allow(struct ab_copy_batch *batch, uint32_t allowed);
+/* The rest of the batch will be allowed piece by piece from now on: the pool's threads are woken and look out for it
+ * instead of being woken, 30 to 50 us each time, for every piece. */
+void ab_copy_batch_soon(struct ab_copy_batch *batch);
+void ab_copy_batch_cut(struct ab_copy_batch *batch); /* what is not allowed yet is not made */
 bool ab_copy_batch_help(struct ab_copy_batch *batch); /* makes one copy; false: none may be taken */
 bool ab_copy_batch_is_done(const struct ab_copy_batch *batch, uint32_t copy);
 void ab_copy_batch_end(struct ab_copy_batch *batch); /* makes or awaits the rest */
