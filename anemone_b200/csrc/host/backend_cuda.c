@@ -1770,6 +1770,9 @@ result_status backend_b200_step_call(struct device_card *card, uint32_t graph,
 	if (output_count != 0) {
 		const uint32_t pieces =
 			call_pieces(&batch, outputs, output_count, staged + input_count, true, range_of, within);
+		uint64_t out_bytes = 0;
+		for (uint32_t index = 0; index < output_count; index++)
+			out_bytes += outputs[index].byte_count;
 		for (uint32_t piece = 0; piece < pieces; piece++) {
 			if (card->piece_events[piece] == NULL)
 				DRIVER(card, cuEventCreate(&card->piece_events[piece], CU_EVENT_DISABLE_TIMING));
@@ -1795,7 +1798,7 @@ result_status backend_b200_step_call(struct device_card *card, uint32_t graph,
 				goto done;
 			}
 			ab_copy_batch_allow(&batch, piece + 1u);
-			if (piece == 0 && batch.copies[0].byte_count < CALL_PIECE_BYTES) /* a short call: the others follow closely */
+			if (piece == 0 && out_bytes <= CALL_SHORT_BYTES) /* the others follow closely */
 				ab_copy_batch_soon(&batch);
 		}
 		ab_copy_batch_end(&batch);
