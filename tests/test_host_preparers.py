@@ -394,8 +394,8 @@ def test_layer_prepare_three_launches():
 
 
 @pytest.mark.parametrize("rows, hidden, inner, runs", [(8, 4096, 2048, 4), (15, 4096, 2048, 4), (16, 4096, 2048, 2),
-                                                       (32, 4096, 2048, 1), (64, 4096, 2048, 1), (16, 4096, 256, 4),
-                                                       (32, 4096, 256, 2), (64, 4096, 256, 1), (8, 1536, 256, 4)])
+                                                       (32, 4096, 2048, 2), (64, 4096, 2048, 2), (16, 4096, 256, 4),
+                                                       (32, 4096, 256, 2), (64, 4096, 256, 2), (8, 1536, 256, 4)])
 def test_layer_cut_of_k_follows_the_prepared_jobs(rows, hidden, inner, runs):
     fake = FakeBackend()
     config = MoeConfig(hidden=hidden, inner=inner, row_capacity=rows)
