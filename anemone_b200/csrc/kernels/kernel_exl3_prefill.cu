@@ -71,6 +71,14 @@ __device__ __forceinline__ prefill_view prefill_view_of(const struct exl3_prefil
 	return view;
 }
 
+/* The first act of the launches that may each be given their places while the one before them still runs: all of that one
+ * first; then the next may take its places. */
+__device__ __forceinline__ void prefill_follow()
+{
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 /* ------------------------------------------------------------------ routing */
 
 extern "C" __global__ void __launch_bounds__(ROUTER_B200_THREADS)
@@ -78,6 +86,7 @@ extern "C" __global__ void __launch_bounds__(ROUTER_B200_THREADS)
 {
 	__shared__ uint32_t chosen[ROUTER_B200_THREADS / WARP][ROUTER_B200_MAXIMUM_PICKS];
 	__shared__ float weight[ROUTER_B200_THREADS / WARP][ROUTER_B200_MAXIMUM_PICKS];
+	prefill_follow();
 	const struct step_block step = *reinterpret_cast<const struct step_block *>(arena + record.step_offset);
 	const uint32_t live = min(step.row_count, record.row_capacity);
 	const uint32_t warp = threadIdx.x / WARP, lane = threadIdx.x % WARP;
@@ -96,6 +105,7 @@ extern "C" __global__ void __launch_bounds__(PREFILL_GROUP_THREADS)
 	exl3_prefill_group(struct exl3_prefill_record record, unsigned char *arena)
 {
 	__shared__ uint32_t warp_total[PREFILL_GROUP_THREADS / WARP];
+	prefill_follow();
 	const prefill_view view = prefill_view_of(record, arena);
 	const uint32_t expert = blockIdx.x, lane = threadIdx.x % WARP, warp = threadIdx.x / WARP;
 	const uint32_t *const picked = reinterpret_cast<const uint32_t *>(arena + record.picks_offset);
@@ -149,6 +159,7 @@ extern "C" __global__ void __launch_bounds__(ROUTER_B200_THREADS)
 	exl3_prefill_tiles(struct exl3_prefill_record record, unsigned char *arena)
 {
 	__shared__ uint32_t warp_total[ROUTER_B200_THREADS / WARP];
+	prefill_follow();
 	const prefill_view view = prefill_view_of(record, arena);
 	uint32_t *const counts = reinterpret_cast<uint32_t *>(view.workspace + view.parts.counts);
 	struct exl3_prefill_tile *const tiles =
@@ -253,6 +264,7 @@ __device__ __forceinline__ void prefill_scales(const __half *scales, uint32_t fi
 extern "C" __global__ void __launch_bounds__(EXL3_TRANSFORM_THREADS)
 	exl3_prefill_operands(struct exl3_prefill_record record, unsigned char *arena)
 {
+	prefill_follow();
 	const prefill_view view = prefill_view_of(record, arena);
 	const uint32_t tile_index = blockIdx.x;
 	const uint32_t tile_count = reinterpret_cast<const uint32_t *>(view.workspace + view.parts.counts)[view.experts];
@@ -1003,11 +1015,14 @@ extern "C" __global__ void __cluster_dims__(PREFILL_PAIR, 1, 1) __launch_bounds_
 {
 	extern __shared__ __align__(1024) unsigned char dynamic_shared[];
 	__shared__ prefill_shared shared;
+	prefill_follow();
 	const prefill_view view = prefill_view_of(record, arena);
 	const uint32_t tile_count = reinterpret_cast<const uint32_t *>(view.workspace + view.parts.counts)[view.experts];
-	const uint32_t tile_index = blockIdx.y, rank = blockIdx.x % PREFILL_PAIR, first_group = blockIdx.x / PREFILL_PAIR * 2u;
-	if (tile_index >= tile_count)
+	if (blockIdx.y >= tile_count)
 		return;
+	/* the last tiles first: the always-on expert's, two to a unit, take half as long again as the median expert's */
+	const uint32_t tile_index = tile_count - 1u - blockIdx.y;
+	const uint32_t rank = blockIdx.x % PREFILL_PAIR, first_group = blockIdx.x / PREFILL_PAIR * 2u;
 	const struct exl3_prefill_tile tile =
 		reinterpret_cast<const struct exl3_prefill_tile *>(view.workspace + view.parts.tiles)[tile_index];
 	const uint32_t count = prefill_tiles_of_unit(view, tile, tile_index, tile_count);
@@ -1027,11 +1042,14 @@ extern "C" __global__ void __cluster_dims__(PREFILL_PAIR, 1, 1) __launch_bounds_
 {
 	extern __shared__ __align__(1024) unsigned char dynamic_shared[];
 	__shared__ prefill_shared shared;
+	prefill_follow();
 	const prefill_view view = prefill_view_of(record, arena);
 	const uint32_t tile_count = reinterpret_cast<const uint32_t *>(view.workspace + view.parts.counts)[view.experts];
-	const uint32_t tile_index = blockIdx.y, rank = blockIdx.x % PREFILL_PAIR, first_group = blockIdx.x / PREFILL_PAIR * 4u;
-	if (tile_index >= tile_count)
+	if (blockIdx.y >= tile_count)
 		return;
+	/* the last tiles first: the always-on expert's, two to a unit, take half as long again as the median expert's */
+	const uint32_t tile_index = tile_count - 1u - blockIdx.y;
+	const uint32_t rank = blockIdx.x % PREFILL_PAIR, first_group = blockIdx.x / PREFILL_PAIR * 4u;
 	const struct exl3_prefill_tile tile =
 		reinterpret_cast<const struct exl3_prefill_tile *>(view.workspace + view.parts.tiles)[tile_index];
 	const uint32_t count = prefill_tiles_of_unit(view, tile, tile_index, tile_count);
