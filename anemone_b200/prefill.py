@@ -25,15 +25,19 @@ from .moe import LINE, SIGNAL_BYTES, rank_columns
 
 PIECE_ROWS = 128  # a staged call's pieces begin on whole row tiles
 STEP_SPACE = 48  # a piece's step block and its status, behind the call's own in the 256 bytes of the step's space
-PCIE_BYTES, WEIGHT_RATE = 53e9, 2.4e12  # a second: measured copies; weights decoded and multiplied with up to 256 rows
-PIECE_SECONDS = 1e-4  # routing, grouping, the reduction and the gaps between their launches, whatever the rows
+# A second: measured copies; weights decoded and multiplied with up to 256 rows, as if every held expert had rows (a
+# prompt's popularity leaves a third to a half of them without). PIECE_SECONDS: routing, grouping, the reduction and the gaps
+# between their launches, whatever the rows. Both fitted to calls in 1, 2 and 4 pieces of 512 to 4096 rows on a whole
+# layer of 64 and of 256 experts and on halves to eighths of it: the estimate takes the fastest of each.
+PCIE_BYTES, WEIGHT_RATE = 53e9, 7e12
+PIECE_SECONDS = 8e-5
 
 
 def call_pieces(config, share, rank_count):
     """In how many pieces a staged call takes its rows: 1, 2 or 4, by an estimate of the call's time. More pieces hide more
     of the copies, but each decodes every expert's weights again, so few rows of many experts stay whole. 4096 rows of
-    H 4096, I 2048 on 32 of 256 experts: 1.35 ms of copies, 0.5 of products; two pieces. All 256: 3.5 ms of products
-    against 5 in two pieces; one. The ranks of a reduction must agree: theirs is the largest share of equal ones."""
+    H 4096, I 2048, Zipf(1.1), ms a call in 1, 2, 4 pieces: 32 of 256 experts 1.78, 1.39, 1.41; 64 of them 2.17, 1.81, 2.00;
+    128 2.71, 2.54, 3.05; all 4.56, 4.86, 6.08; 1024 rows on 64 of them 0.75, 0.84, 1.12. The ranks of a reduction must agree: theirs is the largest share of equal ones."""
     rows, H = config.row_capacity, config.hidden
     if rank_count > 1:
         matrices, pairs = -(-config.experts // rank_count), config.picks / rank_count
