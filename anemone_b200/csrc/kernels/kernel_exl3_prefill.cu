@@ -12,6 +12,7 @@
  *     released by tcgen05.commit,
  *   - reads the accumulators back with tcgen05.ld and applies the chain's FP32 epilogue (exl3_passes.cuh: Hadamard,
  *     scales, SwiGLU, down-side transform / route weight) a warp a row.
+ * A tile of at most eight rows takes none of it: mma.sync on what the decode leaves in registers (prefill_thin_products).
  * Arithmetic per value is the retained chain's; only the association of the FP32 sums over K is the tensor cores'.
  * Every wait is bounded: one that runs out raises exl3_wait_expired, the CTA stores nothing, waits (bounded) for what
  * it has in flight, frees its tensor memory and returns.
@@ -866,11 +867,111 @@ __device__ __forceinline__ void prefill_gate_up_rows(const struct exl3_prefill_r
 	}
 }
 
+/* The products of a single tile of at most PREFILL_THIN_ROWS rows, by mma.sync on what the decode leaves in registers, as a
+ * decode step's (exl3_product_core): no stage, no hand-over to another warp, no tensor memory. Sixteen warps: eight take
+ * the K steps of the first of the two (matrix, group)s in turns, eight the second's; a lane loads its ring words a round
+ * ahead, and the eight rows' operands of a step as two runs of 128 bytes. The eight partial sums are added in warp order from
+ * +0 into the staged rows the epilogues read. Decode warps only; ends with their barrier.
+ * Such a tile's time is its decode and what a unit costs beside it (a pair's beginning, 5 k cycles, the stages' hand-overs, a
+ * fifth of its 70 k). 413 rows of 256 experts, 59 of 97 with at most eight rows: gate/up and down 596 and 342 us through the
+ * stages, 552 and 319 so; 4096 rows, 95 of 173: 1852 and 1017, 1806 and 1002. More than eight rows would be a second
+ * product a fragment and 32 registers more than the launch has. */
+#define PREFILL_THIN_ROWS 8u
+#define PREFILL_THIN_PARTIALS 73728u /* bytes, behind both accumulators' first eight staged rows */
+static_assert((EXL3_PREFILL_TILE_ROWS + PREFILL_THIN_ROWS) * EXL3_PREFILL_STAGING_ROW * 4u <= PREFILL_THIN_PARTIALS &&
+		      PREFILL_THIN_PARTIALS + PREFILL_DECODE_WARPS * EXL3_GROUP_TILES * EXL3_WARP * 16u <= EXL3_PREFILL_DYNAMIC_BYTES,
+	      "the partial sums lie behind the staged rows");
+template <uint32_t BX2, uint32_t MATRICES, uint32_t GROUPS>
+__device__ __forceinline__ void prefill_thin_products(const unsigned char *const (&matrices)[MATRICES], uint32_t outputs,
+						      uint32_t first_group, uint32_t groups, const unsigned char *row_runs,
+						      uint32_t half, uint32_t row_count, uint32_t steps, unsigned char *dynamic_shared)
+{
+	typedef exl3_ring<BX2> ring;
+	constexpr uint32_t turns = PREFILL_DECODE_WARPS / 2u; /* warps that share the steps */
+	const uint32_t lane = threadIdx.x % EXL3_WARP, decoder = threadIdx.x / EXL3_WARP - PREFILL_FIRST_DECODE_WARP;
+	const uint32_t which = decoder / turns, member = decoder % turns;
+	const uint32_t g = GROUPS > 1u ? which : 0u, m = MATRICES > 1u ? which : 0u;
+	float4 *const partials = reinterpret_cast<float4 *>(dynamic_shared + PREFILL_THIN_PARTIALS);
+	if (g < groups) {
+		const uint64_t step_words = (uint64_t)(outputs / EXL3_TILE) * ring::words;
+		const uint32_t begin = ring::begin(lane);
+		const uint32_t word_index = begin / 32u, shift = begin % 32u, next_index = (word_index + 1u) % ring::words;
+		const uint32_t *words = reinterpret_cast<const uint32_t *>(MATRICES > 1u && m != 0u ? matrices[MATRICES - 1u] : matrices[0]) +
+					member * step_words + (uint64_t)(first_group + g) * EXL3_GROUP_TILES * ring::words;
+		/* step s stands in stage s / PREFILL_STEPS: [matrix][pieces][half rows][16 bytes]; the lane's two words of it */
+		const uint32_t piece = half * 16u, stage_bytes = MATRICES * PREFILL_STEPS * 2u * piece;
+		const unsigned char *fed = row_runs + (uint64_t)(member / PREFILL_STEPS) * stage_bytes +
+					   (m * PREFILL_STEPS + member % PREFILL_STEPS) * 2u * piece + lane / 4u * 16u + lane % 4u * 4u;
+		const uint64_t turn_words = turns * step_words, turn_bytes = (uint64_t)(turns / PREFILL_STEPS) * stage_bytes;
+		static_assert(turns % PREFILL_STEPS == 0u, "a turn of the warps is whole stages");
+		const uint32_t rounds = steps / turns;
+		float sums[EXL3_GROUP_TILES][4];
+		uint32_t held[EXL3_GROUP_TILES][2], held_fed[2];
+#pragma unroll
+		for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++) {
+#pragma unroll
+			for (uint32_t c = 0; c < 4; c++)
+				sums[tile][c] = 0.0f;
+			held[tile][0] = __ldg(words + tile * ring::words + word_index);
+			held[tile][1] = __ldg(words + tile * ring::words + next_index);
+		}
+		held_fed[0] = __ldcg(reinterpret_cast<const uint32_t *>(fed));
+		held_fed[1] = __ldcg(reinterpret_cast<const uint32_t *>(fed + piece));
+#pragma unroll 1
+		for (uint32_t round = 1; round <= rounds; round++) {
+			const uint32_t b0 = held_fed[0], b1 = held_fed[1];
+			const bool more = round < rounds;
+			words += turn_words;
+			fed += turn_bytes;
+			if (more) {
+				held_fed[0] = __ldcg(reinterpret_cast<const uint32_t *>(fed));
+				held_fed[1] = __ldcg(reinterpret_cast<const uint32_t *>(fed + piece));
+			}
+#pragma unroll
+			for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++) {
+				uint32_t fragment[4];
+				exl3_decode_fragment<BX2>(held[tile][0], held[tile][1], shift, fragment);
+				if (more) {
+					held[tile][0] = __ldg(words + tile * ring::words + word_index);
+					held[tile][1] = __ldg(words + tile * ring::words + next_index);
+				}
+				mma_f16(sums[tile], fragment, b0, b1);
+			}
+		}
+#pragma unroll
+		for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++)
+			partials[(decoder * EXL3_GROUP_TILES + tile) * EXL3_WARP + lane] =
+				make_float4(sums[tile][0], sums[tile][1], sums[tile][2], sums[tile][3]);
+	}
+	asm volatile("cp.async.wait_all;" ::: "memory"); /* the scales */
+	decode_sync();
+	if (g < groups) {
+		static_assert(EXL3_GROUP_TILES == turns, "a tile a warp");
+		float total[4] = { 0.0f, 0.0f, 0.0f, 0.0f };
+#pragma unroll
+		for (uint32_t slice = 0; slice < turns; slice++) {
+			const float4 part = partials[((which * turns + slice) * EXL3_GROUP_TILES + member) * EXL3_WARP + lane];
+			total[0] = __fadd_rn(total[0], part.x);
+			total[1] = __fadd_rn(total[1], part.y);
+			total[2] = __fadd_rn(total[2], part.z);
+			total[3] = __fadd_rn(total[3], part.w);
+		}
+#pragma unroll
+		for (uint32_t c = 0; c < 4; c++) {
+			const uint32_t row = lane % 4u * 2u + (c & 1u);
+			if (row < row_count)
+				reinterpret_cast<float *>(dynamic_shared)[(which * EXL3_PREFILL_TILE_ROWS + row) * EXL3_PREFILL_STAGING_ROW +
+									  member * EXL3_TILE + lane / 4u + (c >> 1) * 8u] = total[c];
+		}
+	}
+	decode_sync();
+}
+
 /* gate and up of a unit's `count` row tiles (tile_index, + 1) by 256 outputs: this CTA's group is `group` */
 template <uint32_t BX2>
 __device__ __forceinline__ void prefill_gate_up(const struct exl3_prefill_record &record, unsigned char *arena,
 						const prefill_view &view, uint32_t tile_index, uint32_t count, uint32_t group,
-						uint32_t rank, unsigned char *dynamic_shared, prefill_shared *shared)
+						uint32_t rank, bool thin, unsigned char *dynamic_shared, prefill_shared *shared)
 {
 	const prefill_tile_view first = prefill_tile_of(record, arena, view, tile_index);
 	const uint32_t H = record.input_size, I = prefill_inner_of(record, first.tile.expert);
@@ -887,6 +988,15 @@ __device__ __forceinline__ void prefill_gate_up(const struct exl3_prefill_record
 		prefill_fetch_scales(shared, 2u, reinterpret_cast<const __half *>(arena + first.down + exl3_code_bytes(I, H, BX2)) +
 							 first_scale);
 	}
+	if (thin) {
+		if (threadIdx.x / EXL3_WARP < PREFILL_FIRST_DECODE_WARP || mine == 0)
+			return;
+		prefill_thin_products<BX2, 2, 1>(matrices, I, group, mine, view.workspace + view.parts.gate_up_operands +
+						 (uint64_t)tile_index * H * 512u, rows.half, first.tile.row_count, H / EXL3_TILE,
+						 dynamic_shared);
+		prefill_gate_up_rows(record, view, shared, first, tile_index, 1u, group, reinterpret_cast<float *>(dynamic_shared));
+		return;
+	}
 	const bool complete = prefill_products<BX2, 2, 1>(matrices, I, group, mine, 1, row_runs, rows.half,
 							  H / (PREFILL_STEPS * EXL3_TILE), rank, dynamic_shared, shared);
 	if (threadIdx.x / EXL3_WARP >= PREFILL_FIRST_DECODE_WARP && complete && mine != 0) {
@@ -901,13 +1011,72 @@ __device__ __forceinline__ void prefill_gate_up(const struct exl3_prefill_record
 	prefill_release(shared);
 }
 
+/* The down epilogue of one row tile from the staged accumulators, a group each: output transform, scale, route weight, FP32
+ * pair outputs. Decode warps. */
+__device__ __forceinline__ void prefill_down_rows(const prefill_shared *shared, const prefill_tile_view &rows_of,
+						  uint32_t first_group, uint32_t groups, uint32_t H, float *outputs,
+						  const float *staging)
+{
+	const uint32_t lane = threadIdx.x % EXL3_WARP, warp = threadIdx.x / EXL3_WARP;
+	for (uint32_t g = 0; g < groups; g++) {
+		const uint32_t channel = (first_group + g) * EXL3_TRANSFORM + lane % 8u * 4u;
+		const __half *const scales = shared->scales[g] + lane % 8u * 4u;
+		if (rows_of.tile.row_count <= PREFILL_FEW_ROWS) {
+			float scale[4];
+			load_half4(shared->scales[g] + lane * 4u, scale);
+			for (uint32_t row = warp - PREFILL_FIRST_DECODE_WARP; row < rows_of.tile.row_count;
+			     row += PREFILL_DECODE_WARPS) {
+				const struct exl3_prefill_entry entry = rows_of.entries[row];
+				const float4 raw = *reinterpret_cast<const float4 *>(
+					staging + (g * EXL3_PREFILL_TILE_ROWS + row) * EXL3_PREFILL_STAGING_ROW + lane * 4u);
+				float v[4] = { raw.x, raw.y, raw.z, raw.w };
+				hadamard128_warp(v, lane);
+#pragma unroll
+				for (uint32_t i = 0; i < 4; i++)
+					v[i] = __fmul_rn(__fmul_rn(__fmul_rn(v[i], EXL3_NORMALIZATION), scale[i]),
+							 entry.route_weight);
+				*reinterpret_cast<float4 *>(outputs + (uint64_t)entry.pair * H +
+							    (first_group + g) * EXL3_TRANSFORM + lane * 4u) =
+					make_float4(v[0], v[1], v[2], v[3]);
+			}
+			continue;
+		}
+		for (uint32_t from = (warp - PREFILL_FIRST_DECODE_WARP) * PREFILL_WARP_ROWS; from < rows_of.tile.row_count;
+		     from += PREFILL_DECODE_WARPS * PREFILL_WARP_ROWS) {
+			const uint32_t row = from + lane / 8u;
+			const struct exl3_prefill_entry entry = rows_of.entries[min(row, rows_of.tile.row_count - 1u)];
+			const float *const at =
+				staging + (g * EXL3_PREFILL_TILE_ROWS + row) * EXL3_PREFILL_STAGING_ROW + lane % 8u * 4u;
+			float v[4][4];
+#pragma unroll
+			for (uint32_t k = 0; k < 4; k++) {
+				const float4 raw = *reinterpret_cast<const float4 *>(at + 32u * k);
+				v[k][0] = raw.x, v[k][1] = raw.y, v[k][2] = raw.z, v[k][3] = raw.w;
+			}
+			hadamard128_rows(v, lane);
+#pragma unroll
+			for (uint32_t k = 0; k < 4; k++) {
+				float scale[4];
+				load_half4(scales + 32u * k, scale);
+#pragma unroll
+				for (uint32_t j = 0; j < 4; j++)
+					v[k][j] = __fmul_rn(__fmul_rn(__fmul_rn(v[k][j], EXL3_NORMALIZATION), scale[j]),
+							    entry.route_weight);
+				if (row < rows_of.tile.row_count)
+					*reinterpret_cast<float4 *>(outputs + (uint64_t)entry.pair * H + channel + 32u * k) =
+						make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
+			}
+		}
+	}
+}
+
 /* down of a unit's `count` row tiles by 512 outputs: this CTA's groups are first_group, + 1; `sums`: 2, or 1 where the
  * last unit has no second group for either CTA */
 template <uint32_t BX2>
 __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &record, unsigned char *arena,
 					     const prefill_view &view, uint32_t tile_index, uint32_t count,
-					     uint32_t first_group, uint32_t sums, uint32_t rank, unsigned char *dynamic_shared,
-					     prefill_shared *shared)
+					     uint32_t first_group, uint32_t sums, uint32_t rank, bool thin,
+					     unsigned char *dynamic_shared, prefill_shared *shared)
 {
 	const prefill_tile_view first = prefill_tile_of(record, arena, view, tile_index);
 	const uint32_t H = record.input_size, I = prefill_inner_of(record, first.tile.expert);
@@ -921,6 +1090,16 @@ __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &r
 	for (uint32_t g = 0; g < groups; g++)
 		prefill_fetch_scales(shared, g, reinterpret_cast<const __half *>(arena + first.down + exl3_code_bytes(I, H, BX2)) + I +
 							 (first_group + g) * EXL3_TRANSFORM);
+	if (thin) {
+		if (warp < PREFILL_FIRST_DECODE_WARP || groups == 0)
+			return;
+		prefill_thin_products<BX2, 1, 2>(matrices, H, first_group, groups, view.workspace + view.parts.down_operands +
+						 (uint64_t)tile_index * view.widest * 256u, rows.half, first.tile.row_count, I / EXL3_TILE,
+						 dynamic_shared);
+		prefill_down_rows(shared, first, first_group, groups, H, reinterpret_cast<float *>(arena + record.pair_output_offset),
+				  reinterpret_cast<const float *>(dynamic_shared));
+		return;
+	}
 	const bool complete = prefill_products<BX2, 1, 2>(matrices, H, first_group, groups, sums, row_runs, rows.half,
 							  I / (PREFILL_STEPS * EXL3_TILE), rank, dynamic_shared, shared);
 	if (warp >= PREFILL_FIRST_DECODE_WARP && complete) {
@@ -930,56 +1109,7 @@ __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &r
 			const prefill_tile_view rows_of = prefill_tile_of(record, arena, view, tile_index + tile);
 			prefill_stage_out(shared->tensor_memory, groups, tile * EXL3_PREFILL_TILE_ROWS, rows_of.tile.row_count,
 					  staging);
-			for (uint32_t g = 0; g < groups; g++) {
-				const uint32_t channel = (first_group + g) * EXL3_TRANSFORM + lane % 8u * 4u;
-				const __half *const scales = shared->scales[g] + lane % 8u * 4u;
-				if (rows_of.tile.row_count <= PREFILL_FEW_ROWS) {
-					float scale[4];
-					load_half4(shared->scales[g] + lane * 4u, scale);
-					for (uint32_t row = warp - PREFILL_FIRST_DECODE_WARP; row < rows_of.tile.row_count;
-					     row += PREFILL_DECODE_WARPS) {
-						const struct exl3_prefill_entry entry = rows_of.entries[row];
-						const float4 raw = *reinterpret_cast<const float4 *>(
-							staging + (g * EXL3_PREFILL_TILE_ROWS + row) * EXL3_PREFILL_STAGING_ROW + lane * 4u);
-						float v[4] = { raw.x, raw.y, raw.z, raw.w };
-						hadamard128_warp(v, lane);
-#pragma unroll
-						for (uint32_t i = 0; i < 4; i++)
-							v[i] = __fmul_rn(__fmul_rn(__fmul_rn(v[i], EXL3_NORMALIZATION), scale[i]),
-									 entry.route_weight);
-						*reinterpret_cast<float4 *>(outputs + (uint64_t)entry.pair * H +
-									    (first_group + g) * EXL3_TRANSFORM + lane * 4u) =
-							make_float4(v[0], v[1], v[2], v[3]);
-					}
-					continue;
-				}
-				for (uint32_t from = (warp - PREFILL_FIRST_DECODE_WARP) * PREFILL_WARP_ROWS; from < rows_of.tile.row_count;
-				     from += PREFILL_DECODE_WARPS * PREFILL_WARP_ROWS) {
-					const uint32_t row = from + lane / 8u;
-					const struct exl3_prefill_entry entry = rows_of.entries[min(row, rows_of.tile.row_count - 1u)];
-					const float *const at =
-						staging + (g * EXL3_PREFILL_TILE_ROWS + row) * EXL3_PREFILL_STAGING_ROW + lane % 8u * 4u;
-					float v[4][4];
-#pragma unroll
-					for (uint32_t k = 0; k < 4; k++) {
-						const float4 raw = *reinterpret_cast<const float4 *>(at + 32u * k);
-						v[k][0] = raw.x, v[k][1] = raw.y, v[k][2] = raw.z, v[k][3] = raw.w;
-					}
-					hadamard128_rows(v, lane);
-#pragma unroll
-					for (uint32_t k = 0; k < 4; k++) {
-						float scale[4];
-						load_half4(scales + 32u * k, scale);
-#pragma unroll
-						for (uint32_t j = 0; j < 4; j++)
-							v[k][j] = __fmul_rn(__fmul_rn(__fmul_rn(v[k][j], EXL3_NORMALIZATION), scale[j]),
-									    entry.route_weight);
-						if (row < rows_of.tile.row_count)
-							*reinterpret_cast<float4 *>(outputs + (uint64_t)entry.pair * H + channel + 32u * k) =
-								make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
-					}
-				}
-			}
+			prefill_down_rows(shared, rows_of, first_group, groups, H, outputs, staging);
 			decode_sync();
 		}
 	}
@@ -1005,7 +1135,8 @@ __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &r
 		call;                                                                                  \
 	} break;                                                                                       \
 	default:                                                                                       \
-		prefill_release(&shared);                                                           \
+		if (!thin)                                                                             \
+			prefill_release(&shared);                                                      \
 		break;                                                                                 \
 	}
 
@@ -1028,11 +1159,12 @@ extern "C" __global__ void __cluster_dims__(PREFILL_PAIR, 1, 1) __launch_bounds_
 	const uint32_t count = prefill_tiles_of_unit(view, tile, tile_index, tile_count);
 	if (count == 0 || first_group >= prefill_inner_of(record, tile.expert) / EXL3_TRANSFORM)
 		return;
-	if (!prefill_begin(&shared, rank, prefill_rings<2, 1>::stages)) {
+	const bool thin = count == 1u && tile.row_count <= PREFILL_THIN_ROWS;
+	if (!thin && !prefill_begin(&shared, rank, prefill_rings<2, 1>::stages)) {
 		prefill_release(&shared);
 		return;
 	}
-	PREFILL_WIDTH_SWITCH((prefill_gate_up<BX2>(record, arena, view, tile_index, count, first_group + rank, rank,
+	PREFILL_WIDTH_SWITCH((prefill_gate_up<BX2>(record, arena, view, tile_index, count, first_group + rank, rank, thin,
 						   dynamic_shared, &shared)))
 }
 
@@ -1055,12 +1187,13 @@ extern "C" __global__ void __cluster_dims__(PREFILL_PAIR, 1, 1) __launch_bounds_
 	const uint32_t count = prefill_tiles_of_unit(view, tile, tile_index, tile_count);
 	if (count == 0)
 		return;
-	if (!prefill_begin(&shared, rank, prefill_rings<1, 2>::stages)) {
+	const bool thin = count == 1u && tile.row_count <= PREFILL_THIN_ROWS;
+	if (!thin && !prefill_begin(&shared, rank, prefill_rings<1, 2>::stages)) {
 		prefill_release(&shared);
 		return;
 	}
 	PREFILL_WIDTH_SWITCH((prefill_down<BX2>(record, arena, view, tile_index, count, first_group + 2u * rank,
-						min(2u, record.input_size / EXL3_TRANSFORM - first_group), rank, dynamic_shared,
+						min(2u, record.input_size / EXL3_TRANSFORM - first_group), rank, thin, dynamic_shared,
 						&shared)))
 }
 

@@ -37,7 +37,8 @@ def call_pieces(config, share, rank_count):
     """In how many pieces a staged call takes its rows: 1, 2 or 4, by an estimate of the call's time. More pieces hide more
     of the copies, but each decodes every expert's weights again, so few rows of many experts stay whole. 4096 rows of
     H 4096, I 2048, Zipf(1.1), ms a call in 1, 2, 4 pieces: 32 of 256 experts 1.78, 1.39, 1.41; 64 of them 2.17, 1.81, 2.00;
-    128 2.71, 2.54, 3.05; all 4.56, 4.86, 6.08; 1024 rows on 64 of them 0.75, 0.84, 1.12. The ranks of a reduction must agree: theirs is the largest share of equal ones."""
+    128 2.71, 2.54, 3.05; all 4.56, 4.86, 6.08; 1024 rows on 64 of them 0.75, 0.84, 1.12. The ranks of a reduction must
+    agree: theirs is the largest share of equal ones."""
     rows, H = config.row_capacity, config.hidden
     if rank_count > 1:
         matrices, pairs = -(-config.experts // rank_count), config.picks / rank_count

@@ -326,6 +326,13 @@ def test_prefill_units_at_their_edges(api, oracle, rows):
         assert np.abs(got - expected).max() <= MAX_ABS and cosine(got, expected) >= COSINE, width
 
 
+@pytest.mark.parametrize("rows", [1, 7, 8, 9, 264])
+def test_prefill_tiles_of_few_rows(api, oracle, rows):
+    """Tiles of at most eight rows are multiplied without stages and tensor memory: the fewest and the most of them, the
+    first tile beyond, a last tile of eight behind a unit of two; odd numbers of groups, every stored width."""
+    test_prefill_units_at_their_edges(api, oracle, rows)
+
+
 @pytest.mark.parametrize("hidden,inner", [(32 * 8, 512), (32 * 96, 128)])
 def test_pairs_hand_their_stages_over(api, hidden, inner):
     """A pair's second CTA tells the first when its half of a stage is in place: call after call the same bits, whatever
