@@ -332,7 +332,7 @@ result_status exl3_layer_prepare(const struct exl3_layer_description *descriptio
 		return STATUS_INVALID_ARGUMENT;
 	/* the cut of the products: the caller's, or the measured default of exl3_geometry.h */
 	const uint32_t gate_up_runs =
-		description->gate_up_runs != 0 ? description->gate_up_runs : exl3_layer_gate_up_runs(H, I, base->job_count);
+		description->gate_up_runs != 0 ? description->gate_up_runs : exl3_layer_gate_up_runs(H, I);
 	const uint32_t down_runs = description->down_runs != 0 ? description->down_runs : 1u;
 	if (!layer_runs_are_valid(gate_up_runs, H / EXL3_TRANSFORM) || !layer_runs_are_valid(down_runs, I / EXL3_TRANSFORM))
 		return STATUS_INVALID_ARGUMENT;

@@ -51,17 +51,13 @@ AB_INLINE uint32_t exl3_moe_splits(uint32_t inputs, uint32_t outputs)
 /* The default cut of the layer's products, measured on one to eight ranks' shapes of a hidden width of 4096 and an
  * intermediate width of 2048 (a CTA an item; an item's fixed cost, the chain of dependent loads from its ticket to its
  * first weights, is about 2.5 us of its place on the card): gate and up in 4 runs of K where the rank holds at least
- * 1024 inner channels, in 8 below (more items of the fewer outputs); down in one run. A layer prepared for more jobs has
- * items enough with fewer, longer runs: half as many for every doubling of the jobs beyond eight rows of eight picks, two
- * at least (32 rows of 256 experts: 1055 us a step in four runs, 1026 in two, 1010 in one; one row in such a layer 126, 145,
- * 185; a rank of eight's 256 columns and 64 rows: 456 in eight, 434 in two; eight rows keep the four that one row wants,
- * 106 us against 135 in two, where the eight would gain 2 %). Halved too while it does not divide the K blocks of 128. */
-#define EXL3_LAYER_RUNS_JOBS 64u
-AB_INLINE uint32_t exl3_layer_gate_up_runs(uint32_t input_size, uint32_t inner_size, uint32_t job_count)
+ * 1024 inner channels, in 8 below (more items of the fewer outputs); down in one run. Halved while it does not divide
+ * the K blocks of 128. The same whatever the rows, although a layer of many jobs has items enough with fewer runs (32 rows of
+ * 256 experts: 1055 us a step in four, 1026 in two): the tensor cores' FP32 sums of a longer run are less exact (the row
+ * sums' error against 64 bits, 32 rows of 2048 x 2048: 1.00e-5 of their norm in four runs, 1.78e-5 in two). */
+AB_INLINE uint32_t exl3_layer_gate_up_runs(uint32_t input_size, uint32_t inner_size)
 {
 	uint32_t runs = inner_size >= 1024u ? 4u : 8u;
-	for (uint32_t jobs = job_count; runs > 2u && jobs >= 2u * EXL3_LAYER_RUNS_JOBS; jobs /= 2u)
-		runs /= 2u;
 	while (runs > 1u && (input_size / EXL3_TRANSFORM) % runs != 0)
 		runs /= 2u;
 	return runs;

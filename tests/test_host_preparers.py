@@ -2,14 +2,12 @@
 reference's own host tests drive them: tests/exl3_tp_test.c:23-48, tests/exl3_fast_prepare_test.c) and, where the
 reference's host code was compiled (oracle/_ref), byte for byte against its preparers."""
 import ctypes as C
-import types
 
 import numpy as np
 import pytest
 
 from anemone_b200 import api, synthetic
 from anemone_b200 import records as R
-from anemone_b200.moe import MoeConfig, MoeLayer, MoeLayout
 
 U32P = C.POINTER(C.c_uint32)
 
@@ -391,21 +389,6 @@ def test_layer_prepare_three_launches():
     bad.route.moe.counters_offset = bad.route.moe.base.products_offset  # overlaps the partial sums
     assert lib.exl3_layer_prepare(C.byref(bad), C.byref(fake.table), fake.card, launches) == 1
     assert bytes(launches) == untouched
-
-
-@pytest.mark.parametrize("rows, hidden, inner, runs", [(8, 4096, 2048, 4), (15, 4096, 2048, 4), (16, 4096, 2048, 2),
-                                                       (32, 4096, 2048, 2), (64, 4096, 2048, 2), (16, 4096, 256, 4),
-                                                       (32, 4096, 256, 2), (64, 4096, 256, 2), (8, 1536, 256, 4)])
-def test_layer_cut_of_k_follows_the_prepared_jobs(rows, hidden, inner, runs):
-    fake = FakeBackend()
-    config = MoeConfig(hidden=hidden, inner=inner, row_capacity=rows)
-    layer = MoeLayer.__new__(MoeLayer)
-    layer.config, layer.layout = config, MoeLayout(config, np.full(config.total_experts, 3), 1, 0)
-    layer.card = types.SimpleNamespace(ops_pointer=C.pointer(fake.table), handle=fake.card,
-                                       arena_bytes=layer.layout.arena_bytes)
-    layer.cut, layer.rank, layer.rank_count = (0, 0), 0, 1
-    products = layer._prepare_fused()[1]
-    assert R.Exl3LayerProducts.from_buffer_copy(bytes(products.argument[:128])).gate_up_runs == runs
 
 
 def test_rows_of_one_rank_prepare():
