@@ -11,10 +11,10 @@
  * One persistent CTA a SM walks units: a tile of rows of one expert by 64 columns of gate and the same 64 of up (or
  * 128 outputs of down), all of K in stages of 256 inputs. Its warps:
  *   schedule  finds the CTA's units ahead of the others (matrices, rows, route weights) into a ring of eight
- *   weights   two teams of eight warps that take the stages in turns; a lane keeps eight 128-bit loads of its warp's tile
- *             in flight in registers, across the units' ends, and stores a stage's codes as the A operand and its
- *             scales in the order tcgen05.cp takes them (no shared-memory copy of the raw words: the SM's
- *             shared-memory bandwidth is the next limit behind HBM). Two teams because one warp's chain of wait,
+ *   weights   few: four teams of four warps, many: two teams of eight, that take the stages in turns; a lane keeps eight
+ *             128-bit loads of its warp's tiles in flight in registers, across the units' ends, and stores a stage's
+ *             codes as the A operand and its scales in the order tcgen05.cp takes them (no shared-memory copy of the raw words: the SM's
+ *             shared-memory bandwidth is the next limit behind HBM). Teams because one warp's chain of wait,
  *             stores, fence and arrival is longer than a stage at the HBM rate (about 390 ns)
  *   rows      few: four warps, a stage each in turns, gather the rows' codes and exponents by cp.async as the B operand;
  *             many: one warp copies them in bulk from where mx_gather and the gate/up launch laid them in operand order
@@ -26,8 +26,8 @@
  * Every wait is bounded; one that runs out raises exl3_wait_expired, and the CTA ends without its remaining units.
  *
  * Measured (hidden 4096, intermediate 2048, 256 experts, top 8, CUDA events, one launch alone): eight rows, 508 MB of
- * gate and up in 127 us (4.0 TB/s; the mma.sync launch 208), down 69 us (115), the always-on expert inside them (63 us
- * of launches of its own before); 2048 rows, 867 + 444 us (6209 + 3337, and the always-on expert's 1415). Stages of 128
+ * gate and up in 116 us (4.4 TB/s; by two teams 127, the mma.sync launch 208), down 60 us (69, 115), the always-on expert
+ * inside them (63 us of launches of its own before); 2048 rows, 867 + 444 us (6209 + 3337, and the always-on expert's 1415). Stages of 128
  * inputs, one team of weight warps or the products issued behind a lane test each made the multiplying or the weight
  * warps' chain the limit (246, 212 and 169 us at eight rows).
  */
@@ -53,8 +53,8 @@
 #define MX_UNIT_ROUTED 0u
 #define MX_UNIT_SHARED 1u
 #define MX_UNIT_END 2u
-/* units the scheduler may be ahead: more than the units a warp's loads in flight can reach into (two stages of its team's,
- * four units where K is 256 or less), so that no role waits for a unit that waits for it */
+/* units the scheduler may be ahead: more than the units a warp's loads in flight can reach into (its team's next stage, or,
+ * of eight warps, next two: four units where K is 256 or less), so that no role waits for a unit that waits for it */
 #define MX_UNITS 8u
 #define MX_CHUNK 4u /* loads of a lane stored, and asked for again, together; two chunks are in flight */
 #define MX_SCALE_COLUMN 256u /* tensor memory: two accumulators of 128 columns, then the stages' scales */
@@ -72,7 +72,7 @@ template <bool FEW> struct mx_form {
 	/* The weights' warps in teams that take the stages in turns, each warp MX_TILES / team_warps tiles of its team's. What a
 	 * stage costs a warp beside its stores (the wait for the place, the fence, the arrival, the next unit's pointers: about
 	 * as much as one tile) is paid once for two tiles by teams of four, and four stages of the ring of five are filled at
-	 * once; the many rows' ring holds three. */
+	 * once (a call of eight rows 221 us by two teams of eight, 214 by four of four); the many rows' ring holds three. */
 	static constexpr uint32_t team_warps = FEW ? 4u : 8u, teams = MX_WEIGHT_WARPS / team_warps;
 	static constexpr uint32_t multiply = epilogue_warps, schedule = multiply + 1u, rows = schedule + 1u;
 	static constexpr uint32_t b_at = stages * MX_OPERAND;

@@ -668,8 +668,8 @@ struct router_select_b200_arguments {
  * chain's (FP16 operands from the FP32 Hadamard transform, exactly decoded FP16 weights, FP32 accumulation, FP32
  * transforms, SwiGLU, route weight last); only the association of the FP32 sums over K is the tensor cores'.
  * Seven launches, one record:
- *   exl3_prefill_picks     grid (ceil(rows / 32)) x 1024: each live row's picks and weights (router_select_b200's
- *                          conventions), from scores
+ *   exl3_prefill_picks     grid (ceil(rows / 4)) x 128, or any number of whole warps a block (router_wide_prepare: 1024
+ *                          threads): each live row's picks and weights (router_select_b200's conventions), from scores
  *   exl3_prefill_group     grid (local + shared) x 256: entries[local expert][...]: the pairs routed to the expert in
  *                          ascending row order, and their count
  *   exl3_prefill_tiles     grid 1 x 1024: the tile table: (expert, first entry, rows) per 128-row tile, tile count
