@@ -867,103 +867,88 @@ __device__ __forceinline__ void prefill_gate_up_rows(const struct exl3_prefill_r
 	}
 }
 
-/* The products of a single tile of at most PREFILL_THIN_ROWS rows, by mma.sync on what the decode leaves in registers, as a
- * decode step's (exl3_product_core): no stage, no hand-over to another warp, no tensor memory. Sixteen warps: eight take
- * the K steps of the first of the two (matrix, group)s in turns, eight the second's; a lane loads its ring words a round
- * ahead, and the eight rows' operands of a step as two runs of 128 bytes. The eight partial sums are added in warp order from
- * +0 into the staged rows the epilogues read. Decode warps only; ends with their barrier.
+/* The products of a single tile of at most PREFILL_THIN_ROWS rows, by mma.sync on what the decode leaves in registers: no
+ * stage, no hand-over to another warp, no tensor memory. Sixteen warps, 16 outputs each of the two (matrix, group)s; a lane
+ * holds its ring words and the rows' operands (two runs of 128 bytes a step, shared by eight warps in the L1) a turn of eight
+ * steps ahead, and asks the L2 for the turn after the next, a lane a step. The sums go into the staged rows the epilogues read.
+ * Decode warps only; ends with their barrier.
+ * A warp walks ALL of K in one accumulator: the sums are then the same bits as the tensor cores' accumulators in tensor memory
+ * (both instructions add sixteen products to an FP32 sum, with the same roundings; nothing documents it, the tests hold it at
+ * every width), so a row's result does not depend on how many rows its expert has in the call. K shared out over eight warps,
+ * a step's eight tiles a warp, is faster (below) but gives a row other bits in a short tile than in a long one.
  * Such a tile's time is its decode and what a unit costs beside it (a pair's beginning, 5 k cycles, the stages' hand-overs, a
- * fifth of its 70 k). 413 rows of 256 experts, 59 of 97 with at most eight rows: gate/up and down 596 and 342 us through the
- * stages, 552 and 319 so; 4096 rows, 95 of 173: 1852 and 1017, 1806 and 1002. More than eight rows would be a second
- * product a fragment and 32 registers more than the launch has. */
+ * fifth of its 70 k). More than eight rows would be a second product a fragment. */
 #define PREFILL_THIN_ROWS 8u
-#define PREFILL_THIN_PARTIALS 73728u /* bytes, behind both accumulators' first eight staged rows */
-static_assert((EXL3_PREFILL_TILE_ROWS + PREFILL_THIN_ROWS) * EXL3_PREFILL_STAGING_ROW * 4u <= PREFILL_THIN_PARTIALS &&
-		      PREFILL_THIN_PARTIALS + PREFILL_DECODE_WARPS * EXL3_GROUP_TILES * EXL3_WARP * 16u <= EXL3_PREFILL_DYNAMIC_BYTES,
-	      "the partial sums lie behind the staged rows");
+#define PREFILL_THIN_HALF 16u /* rows of the first CTA's half of such a tile's operands (prefill_rows_of) */
+#define PREFILL_THIN_TURN 8u /* steps a lane holds: four take 603 and 339 us; K is a multiple of 128 inputs */
 template <uint32_t BX2, uint32_t MATRICES, uint32_t GROUPS>
 __device__ __forceinline__ void prefill_thin_products(const unsigned char *const (&matrices)[MATRICES], uint32_t outputs,
 						      uint32_t first_group, uint32_t groups, const unsigned char *row_runs,
-						      uint32_t half, uint32_t row_count, uint32_t steps, unsigned char *dynamic_shared)
+						      uint32_t row_count, uint32_t steps, unsigned char *dynamic_shared)
 {
 	typedef exl3_ring<BX2> ring;
-	constexpr uint32_t turns = PREFILL_DECODE_WARPS / 2u; /* warps that share the steps */
+	static_assert(PREFILL_DECODE_WARPS == MATRICES * GROUPS * EXL3_GROUP_TILES, "16 outputs a warp");
+	static_assert(PREFILL_THIN_TURN % PREFILL_STEPS == 0u && EXL3_TRANSFORM / EXL3_TILE % PREFILL_THIN_TURN == 0u,
+		      "a turn is whole stages, K whole turns");
 	const uint32_t lane = threadIdx.x % EXL3_WARP, decoder = threadIdx.x / EXL3_WARP - PREFILL_FIRST_DECODE_WARP;
-	const uint32_t which = decoder / turns, member = decoder % turns;
+	const uint32_t which = decoder / EXL3_GROUP_TILES, tile = decoder % EXL3_GROUP_TILES;
 	const uint32_t g = GROUPS > 1u ? which : 0u, m = MATRICES > 1u ? which : 0u;
-	float4 *const partials = reinterpret_cast<float4 *>(dynamic_shared + PREFILL_THIN_PARTIALS);
 	if (g < groups) {
 		const uint64_t step_words = (uint64_t)(outputs / EXL3_TILE) * ring::words;
 		const uint32_t begin = ring::begin(lane);
 		const uint32_t word_index = begin / 32u, shift = begin % 32u, next_index = (word_index + 1u) % ring::words;
-		const uint32_t *words = reinterpret_cast<const uint32_t *>(MATRICES > 1u && m != 0u ? matrices[MATRICES - 1u] : matrices[0]) +
-					member * step_words + (uint64_t)(first_group + g) * EXL3_GROUP_TILES * ring::words;
+		const uint64_t first = (uint64_t)(MATRICES > 1u && m != 0u ? matrices[MATRICES - 1u] : matrices[0]) +
+				       ((uint64_t)(first_group + g) * EXL3_GROUP_TILES + tile) * ring::words * 4u;
+		/* the warp's address, known to be one: a step's is one addition */
+		const uint32_t *words = reinterpret_cast<const uint32_t *>((uint64_t)warp_value((uint32_t)(first >> 32)) << 32 |
+									   warp_value((uint32_t)first));
+		const uint32_t *ahead = words + (2u * PREFILL_THIN_TURN + lane % PREFILL_THIN_TURN) * step_words;
 		/* step s stands in stage s / PREFILL_STEPS: [matrix][pieces][half rows][16 bytes]; the lane's two words of it */
-		const uint32_t piece = half * 16u, stage_bytes = MATRICES * PREFILL_STEPS * 2u * piece;
-		const unsigned char *fed = row_runs + (uint64_t)(member / PREFILL_STEPS) * stage_bytes +
-					   (m * PREFILL_STEPS + member % PREFILL_STEPS) * 2u * piece + lane / 4u * 16u + lane % 4u * 4u;
-		const uint64_t turn_words = turns * step_words, turn_bytes = (uint64_t)(turns / PREFILL_STEPS) * stage_bytes;
-		static_assert(turns % PREFILL_STEPS == 0u, "a turn of the warps is whole stages");
-		const uint32_t rounds = steps / turns;
-		float sums[EXL3_GROUP_TILES][4];
-		uint32_t held[EXL3_GROUP_TILES][2], held_fed[2];
+		constexpr uint32_t piece = PREFILL_THIN_HALF * 16u, stage_bytes = MATRICES * PREFILL_STEPS * 2u * piece;
+		const unsigned char *fed = row_runs + m * PREFILL_STEPS * 2u * piece + lane / 4u * 16u + lane % 4u * 4u;
+		float sums[4] = { 0.0f, 0.0f, 0.0f, 0.0f };
+		uint32_t held[PREFILL_THIN_TURN][2], held_fed[PREFILL_THIN_TURN][2];
 #pragma unroll
-		for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++) {
-#pragma unroll
-			for (uint32_t c = 0; c < 4; c++)
-				sums[tile][c] = 0.0f;
-			held[tile][0] = __ldg(words + tile * ring::words + word_index);
-			held[tile][1] = __ldg(words + tile * ring::words + next_index);
+		for (uint32_t step = 0; step < PREFILL_THIN_TURN; step++) {
+			const unsigned char *const at = fed + step / PREFILL_STEPS * stage_bytes + step % PREFILL_STEPS * 2u * piece;
+			held[step][0] = __ldg(words + word_index);
+			held[step][1] = __ldg(words + next_index);
+			held_fed[step][0] = *reinterpret_cast<const uint32_t *>(at);
+			held_fed[step][1] = *reinterpret_cast<const uint32_t *>(at + piece);
+			words += step_words;
 		}
-		held_fed[0] = __ldcg(reinterpret_cast<const uint32_t *>(fed));
-		held_fed[1] = __ldcg(reinterpret_cast<const uint32_t *>(fed + piece));
 #pragma unroll 1
-		for (uint32_t round = 1; round <= rounds; round++) {
-			const uint32_t b0 = held_fed[0], b1 = held_fed[1];
-			const bool more = round < rounds;
-			words += turn_words;
-			fed += turn_bytes;
-			if (more) {
-				held_fed[0] = __ldcg(reinterpret_cast<const uint32_t *>(fed));
-				held_fed[1] = __ldcg(reinterpret_cast<const uint32_t *>(fed + piece));
+		for (uint32_t left = steps / PREFILL_THIN_TURN; left != 0; left--) {
+			if (left == 1u) /* the last turn loads its own once more */
+				words -= PREFILL_THIN_TURN * step_words;
+			else
+				fed += PREFILL_THIN_TURN / PREFILL_STEPS * stage_bytes;
+			if (left > 2u && lane < PREFILL_THIN_TURN) {
+				asm volatile("prefetch.global.L2 [%0];" ::"l"(ahead));
+				ahead += PREFILL_THIN_TURN * step_words;
 			}
 #pragma unroll
-			for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++) {
+			for (uint32_t step = 0; step < PREFILL_THIN_TURN; step++) {
+				const unsigned char *const at = fed + step / PREFILL_STEPS * stage_bytes + step % PREFILL_STEPS * 2u * piece;
 				uint32_t fragment[4];
-				exl3_decode_fragment<BX2>(held[tile][0], held[tile][1], shift, fragment);
-				if (more) {
-					held[tile][0] = __ldg(words + tile * ring::words + word_index);
-					held[tile][1] = __ldg(words + tile * ring::words + next_index);
-				}
-				mma_f16(sums[tile], fragment, b0, b1);
+				exl3_decode_fragment<BX2>(held[step][0], held[step][1], shift, fragment);
+				held[step][0] = __ldg(words + word_index);
+				held[step][1] = __ldg(words + next_index);
+				words += step_words;
+				mma_f16(sums, fragment, held_fed[step][0], held_fed[step][1]);
+				held_fed[step][0] = *reinterpret_cast<const uint32_t *>(at);
+				held_fed[step][1] = *reinterpret_cast<const uint32_t *>(at + piece);
 			}
-		}
-#pragma unroll
-		for (uint32_t tile = 0; tile < EXL3_GROUP_TILES; tile++)
-			partials[(decoder * EXL3_GROUP_TILES + tile) * EXL3_WARP + lane] =
-				make_float4(sums[tile][0], sums[tile][1], sums[tile][2], sums[tile][3]);
-	}
-	asm volatile("cp.async.wait_all;" ::: "memory"); /* the scales */
-	decode_sync();
-	if (g < groups) {
-		static_assert(EXL3_GROUP_TILES == turns, "a tile a warp");
-		float total[4] = { 0.0f, 0.0f, 0.0f, 0.0f };
-#pragma unroll
-		for (uint32_t slice = 0; slice < turns; slice++) {
-			const float4 part = partials[((which * turns + slice) * EXL3_GROUP_TILES + member) * EXL3_WARP + lane];
-			total[0] = __fadd_rn(total[0], part.x);
-			total[1] = __fadd_rn(total[1], part.y);
-			total[2] = __fadd_rn(total[2], part.z);
-			total[3] = __fadd_rn(total[3], part.w);
 		}
 #pragma unroll
 		for (uint32_t c = 0; c < 4; c++) {
 			const uint32_t row = lane % 4u * 2u + (c & 1u);
 			if (row < row_count)
 				reinterpret_cast<float *>(dynamic_shared)[(which * EXL3_PREFILL_TILE_ROWS + row) * EXL3_PREFILL_STAGING_ROW +
-									  member * EXL3_TILE + lane / 4u + (c >> 1) * 8u] = total[c];
+									  tile * EXL3_TILE + lane / 4u + (c >> 1) * 8u] = sums[c];
 		}
 	}
+	asm volatile("cp.async.wait_all;" ::: "memory"); /* the scales */
 	decode_sync();
 }
 
@@ -992,7 +977,7 @@ __device__ __forceinline__ void prefill_gate_up(const struct exl3_prefill_record
 		if (threadIdx.x / EXL3_WARP < PREFILL_FIRST_DECODE_WARP || mine == 0)
 			return;
 		prefill_thin_products<BX2, 2, 1>(matrices, I, group, mine, view.workspace + view.parts.gate_up_operands +
-						 (uint64_t)tile_index * H * 512u, rows.half, first.tile.row_count, H / EXL3_TILE,
+						 (uint64_t)tile_index * H * 512u, first.tile.row_count, H / EXL3_TILE,
 						 dynamic_shared);
 		prefill_gate_up_rows(record, view, shared, first, tile_index, 1u, group, reinterpret_cast<float *>(dynamic_shared));
 		return;
@@ -1094,7 +1079,7 @@ __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &r
 		if (warp < PREFILL_FIRST_DECODE_WARP || groups == 0)
 			return;
 		prefill_thin_products<BX2, 1, 2>(matrices, H, first_group, groups, view.workspace + view.parts.down_operands +
-						 (uint64_t)tile_index * view.widest * 256u, rows.half, first.tile.row_count, I / EXL3_TILE,
+						 (uint64_t)tile_index * view.widest * 256u, first.tile.row_count, I / EXL3_TILE,
 						 dynamic_shared);
 		prefill_down_rows(shared, first, first_group, groups, H, reinterpret_cast<float *>(arena + record.pair_output_offset),
 				  reinterpret_cast<const float *>(dynamic_shared));

@@ -254,6 +254,12 @@ def test_prefill_full_size_properties(api):
         second = layer.step(tokens[order], scores[order])
         assert np.isfinite(first).all() and np.abs(first).max() > 0
         assert np.array_equal(second.view(np.uint32), first[order].view(np.uint32))
+        # (1) again for the rows in front of the first place where an expert has one to eight rows behind whole pairs of tiles
+        seen = np.cumsum([np.bincount(row, minlength=config.experts) for row in picks[:4000]], axis=0)
+        fewer = int(np.flatnonzero(((seen > 256) & (seen % 256 >= 1) & (seen % 256 <= 8)).any(axis=1))[0]) + 1
+        order = rng.permutation(fewer)
+        third = layer.step(tokens[order], scores[order])
+        assert np.array_equal(third.view(np.uint32), first[order].view(np.uint32))
     finally:
         card.close()
     small = MoeConfig(hidden=4096, inner=2048, experts=256, shared=1, picks=8, row_capacity=8)
@@ -333,6 +339,37 @@ def test_prefill_tiles_of_few_rows(api, oracle, rows):
     test_prefill_units_at_their_edges(api, oracle, rows)
 
 
+@pytest.mark.parametrize("hidden,inner", [(128, 128), (640, 384), (4096, 2048)])
+def test_prefill_row_bits_whatever_the_tiling(api, hidden, inner):
+    """A row has the same FP32 bits whatever stands beside it: alone, in a tile of at most eight rows, in a longer one, as the
+    last of a unit of two tiles and as the few rows behind one. Every expert (one a stored width, and an always-on one) sees
+    every row of a call, so a call of n rows makes tiles of n everywhere. Rows of zeros, of one large value and of widely
+    different sizes among them."""
+    capacity = 300
+    config = MoeConfig(hidden=hidden, inner=inner, experts=4, shared=1, picks=4, row_capacity=capacity)
+    widths, matrices, tokens, scores = make_inputs(83, config, capacity)
+    widths = np.array([2, 40, 3, 4, 3], dtype=np.uint32)
+    rng = np.random.default_rng(84)
+    matrices = [(synthetic.exl3_matrix(rng, hidden, inner, int(w)), synthetic.exl3_matrix(rng, hidden, inner, int(w)),
+                 synthetic.exl3_matrix(rng, inner, hidden, int(w))) for w in widths]
+    values = synthetic.from_bfloat16(tokens).copy()
+    values[3], values[4] = 0.0, 0.0
+    values[4, 77], values[5, ::3] = 60.0, 0.0
+    values[6] *= np.exp2(rng.integers(-20, 4, size=hidden)).astype(np.float32)
+    tokens = synthetic.to_bfloat16(values)
+    card = api.Card(0, PrefillLayout(config, widths).arena_bytes)
+    try:
+        layer = PrefillLayer(card, config, widths, matrices)
+        whole = layer.step(tokens, scores).view(np.uint32).copy()
+        for count in (1, 2, 7, 8, 9, 16, 17, 33, 64, 130, 257, 262, 264):
+            for order in (rng.permutation(capacity)[:count], (np.arange(count) + 3) % capacity, np.arange(count)[::-1]):
+                got = layer.step(tokens[order], scores[order]).view(np.uint32)
+                differ = got != whole[order]
+                assert not differ.any(), (count, int(differ.sum()), np.flatnonzero(differ.any(axis=1))[:20])
+    finally:
+        card.close()
+
+
 @pytest.mark.parametrize("hidden,inner", [(32 * 8, 512), (32 * 96, 128)])
 def test_pairs_hand_their_stages_over(api, hidden, inner):
     """A pair's second CTA tells the first when its half of a stage is in place: call after call the same bits, whatever
@@ -378,5 +415,32 @@ def test_staged_call_in_pieces(api, monkeypatch, rows, count):
             card.step_pieces([(1 << 20, [], [])])
         with pytest.raises(api.StatusError):
             card.step_pieces([(layer.graph, [(card.arena_bytes, 0, 16)], [])])
+    finally:
+        card.close()
+
+
+@pytest.mark.parametrize("rows,count,experts", [(600, 2, 48), (1100, 4, 64)])
+def test_staged_call_in_pieces_of_few_rows_an_expert(api, monkeypatch, rows, count, experts):
+    """Pieces in which experts have at most eight rows that have more in the whole call: still the whole's bits."""
+    config = MoeConfig(hidden=512, inner=256, experts=experts, shared=1, picks=2, row_capacity=rows)
+    widths, matrices, tokens, scores = make_inputs(rows, config, rows)
+    monkeypatch.setattr(prefill, "call_pieces", lambda *_: count)
+    layout = PrefillLayout(config, widths)
+    card = api.Card(0, layout.arena_bytes)
+    try:
+        layer = PrefillLayer(card, config, widths, matrices)
+        layer.connect_local([layer])
+        card.wait()
+        layer.stage(0, tokens, scores)
+        staged = layer.call(0, api.align(layout.input_bytes, 4096)).copy()
+        sums = layer.rows(rows)
+        picks = card.download(layout.picks, rows * 2 * 4, np.uint32).reshape(rows, 2)
+        whole = np.bincount(picks.reshape(-1), minlength=experts)
+        parts = [np.bincount(picks[first:first + held].reshape(-1), minlength=experts) for first, held, _ in layer.pieces]
+        assert sum(int(((part >= 1) & (part <= 8) & (whole > 8)).sum()) for part in parts) >= 8
+        layer.load(tokens, scores)
+        layer.run()
+        assert np.array_equal(layer.result(rows), staged)
+        assert np.array_equal(layer.rows(rows).view(np.uint32), sums.view(np.uint32))
     finally:
         card.close()
