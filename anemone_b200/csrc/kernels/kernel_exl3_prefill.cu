@@ -877,7 +877,9 @@ __device__ __forceinline__ void prefill_gate_up_rows(const struct exl3_prefill_r
  * every width), so a row's result does not depend on how many rows its expert has in the call. K shared out over eight warps,
  * a step's eight tiles a warp, is faster (below) but gives a row other bits in a short tile than in a long one.
  * Such a tile's time is its decode and what a unit costs beside it (a pair's beginning, 5 k cycles, the stages' hand-overs, a
- * fifth of its 70 k). More than eight rows would be a second product a fragment. */
+ * fifth of its 70 k). 413 rows of 256 experts, 59 of 97 with at most eight rows: gate/up and down 538 and 311 us through the
+ * stages, 519 and 298 so, 506 and 294 with K shared out; 4096 rows, 95 of 173: 1872 and 1002, 1843 and 991, 1824 and 977.
+ * Without the L2's request 523 and 305. More than eight rows would be a second product a fragment. */
 #define PREFILL_THIN_ROWS 8u
 #define PREFILL_THIN_HALF 16u /* rows of the first CTA's half of such a tile's operands (prefill_rows_of) */
 #define PREFILL_THIN_TURN 8u /* steps a lane holds: four take 603 and 339 us; K is a multiple of 128 inputs */
@@ -956,7 +958,7 @@ __device__ __forceinline__ void prefill_thin_products(const unsigned char *const
 template <uint32_t BX2>
 __device__ __forceinline__ void prefill_gate_up(const struct exl3_prefill_record &record, unsigned char *arena,
 						const prefill_view &view, uint32_t tile_index, uint32_t count, uint32_t group,
-						uint32_t rank, bool thin, unsigned char *dynamic_shared, prefill_shared *shared)
+						uint32_t rank, unsigned char *dynamic_shared, prefill_shared *shared)
 {
 	const prefill_tile_view first = prefill_tile_of(record, arena, view, tile_index);
 	const uint32_t H = record.input_size, I = prefill_inner_of(record, first.tile.expert);
@@ -972,15 +974,6 @@ __device__ __forceinline__ void prefill_gate_up(const struct exl3_prefill_record
 		prefill_fetch_scales(shared, 1u, reinterpret_cast<const __half *>(arena + first.up + codes) + H + first_scale);
 		prefill_fetch_scales(shared, 2u, reinterpret_cast<const __half *>(arena + first.down + exl3_code_bytes(I, H, BX2)) +
 							 first_scale);
-	}
-	if (thin) {
-		if (threadIdx.x / EXL3_WARP < PREFILL_FIRST_DECODE_WARP || mine == 0)
-			return;
-		prefill_thin_products<BX2, 2, 1>(matrices, I, group, mine, view.workspace + view.parts.gate_up_operands +
-						 (uint64_t)tile_index * H * 512u, first.tile.row_count, H / EXL3_TILE,
-						 dynamic_shared);
-		prefill_gate_up_rows(record, view, shared, first, tile_index, 1u, group, reinterpret_cast<float *>(dynamic_shared));
-		return;
 	}
 	const bool complete = prefill_products<BX2, 2, 1>(matrices, I, group, mine, 1, row_runs, rows.half,
 							  H / (PREFILL_STEPS * EXL3_TILE), rank, dynamic_shared, shared);
@@ -1060,7 +1053,7 @@ __device__ __forceinline__ void prefill_down_rows(const prefill_shared *shared, 
 template <uint32_t BX2>
 __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &record, unsigned char *arena,
 					     const prefill_view &view, uint32_t tile_index, uint32_t count,
-					     uint32_t first_group, uint32_t sums, uint32_t rank, bool thin,
+					     uint32_t first_group, uint32_t sums, uint32_t rank,
 					     unsigned char *dynamic_shared, prefill_shared *shared)
 {
 	const prefill_tile_view first = prefill_tile_of(record, arena, view, tile_index);
@@ -1075,16 +1068,6 @@ __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &r
 	for (uint32_t g = 0; g < groups; g++)
 		prefill_fetch_scales(shared, g, reinterpret_cast<const __half *>(arena + first.down + exl3_code_bytes(I, H, BX2)) + I +
 							 (first_group + g) * EXL3_TRANSFORM);
-	if (thin) {
-		if (warp < PREFILL_FIRST_DECODE_WARP || groups == 0)
-			return;
-		prefill_thin_products<BX2, 1, 2>(matrices, H, first_group, groups, view.workspace + view.parts.down_operands +
-						 (uint64_t)tile_index * view.widest * 256u, first.tile.row_count, I / EXL3_TILE,
-						 dynamic_shared);
-		prefill_down_rows(shared, first, first_group, groups, H, reinterpret_cast<float *>(arena + record.pair_output_offset),
-				  reinterpret_cast<const float *>(dynamic_shared));
-		return;
-	}
 	const bool complete = prefill_products<BX2, 1, 2>(matrices, H, first_group, groups, sums, row_runs, rows.half,
 							  I / (PREFILL_STEPS * EXL3_TILE), rank, dynamic_shared, shared);
 	if (warp >= PREFILL_FIRST_DECODE_WARP && complete) {
@@ -1101,7 +1084,47 @@ __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &r
 	prefill_release(shared);
 }
 
-#define PREFILL_WIDTH_SWITCH(call)                                                                     \
+/* gate and up of a tile of few rows (its own only one) by the 128 outputs of group `group`. Decode warps. The tiles of few rows
+ * and the others part at their launch's beginning: with both forms behind one switch over the widths gate/up's launch spilled
+ * 48 bytes of registers (32 experts of 1024 rows: gate/up 427 us, 422 so). */
+template <uint32_t BX2>
+__device__ __forceinline__ void prefill_thin_gate_up(const struct exl3_prefill_record &record, unsigned char *arena,
+						     const prefill_view &view, uint32_t tile_index, uint32_t group,
+						     unsigned char *dynamic_shared, prefill_shared *shared)
+{
+	const prefill_tile_view tile = prefill_tile_of(record, arena, view, tile_index);
+	const uint32_t H = record.input_size, I = prefill_inner_of(record, tile.tile.expert);
+	const unsigned char *const matrices[2] = { arena + tile.gate, arena + tile.up };
+	const uint64_t codes = exl3_code_bytes(H, I, BX2), first_scale = group * EXL3_TRANSFORM;
+	prefill_fetch_scales(shared, 0u, reinterpret_cast<const __half *>(arena + tile.gate + codes) + H + first_scale);
+	prefill_fetch_scales(shared, 1u, reinterpret_cast<const __half *>(arena + tile.up + codes) + H + first_scale);
+	prefill_fetch_scales(shared, 2u, reinterpret_cast<const __half *>(arena + tile.down + exl3_code_bytes(I, H, BX2)) +
+						 first_scale);
+	prefill_thin_products<BX2, 2, 1>(matrices, I, group, 1u, view.workspace + view.parts.gate_up_operands +
+					 (uint64_t)tile_index * H * 512u, tile.tile.row_count, H / EXL3_TILE, dynamic_shared);
+	prefill_gate_up_rows(record, view, shared, tile, tile_index, 1u, group, reinterpret_cast<float *>(dynamic_shared));
+}
+
+/* down of such a tile by the groups first_group, + 1. Decode warps. */
+template <uint32_t BX2>
+__device__ __forceinline__ void prefill_thin_down(const struct exl3_prefill_record &record, unsigned char *arena,
+						  const prefill_view &view, uint32_t tile_index, uint32_t first_group,
+						  unsigned char *dynamic_shared, prefill_shared *shared)
+{
+	const prefill_tile_view tile = prefill_tile_of(record, arena, view, tile_index);
+	const uint32_t H = record.input_size, I = prefill_inner_of(record, tile.tile.expert);
+	const uint32_t groups = min(2u, H / EXL3_TRANSFORM - first_group);
+	const unsigned char *const matrices[1] = { arena + tile.down };
+	for (uint32_t g = 0; g < groups; g++)
+		prefill_fetch_scales(shared, g, reinterpret_cast<const __half *>(arena + tile.down + exl3_code_bytes(I, H, BX2)) + I +
+							 (first_group + g) * EXL3_TRANSFORM);
+	prefill_thin_products<BX2, 1, 2>(matrices, H, first_group, groups, view.workspace + view.parts.down_operands +
+					 (uint64_t)tile_index * view.widest * 256u, tile.tile.row_count, I / EXL3_TILE, dynamic_shared);
+	prefill_down_rows(shared, tile, first_group, groups, H, reinterpret_cast<float *>(arena + record.pair_output_offset),
+			  reinterpret_cast<const float *>(dynamic_shared));
+}
+
+#define PREFILL_WIDTH_SWITCH(call, otherwise)                                                          \
 	switch (exl3_bits_x2(reinterpret_cast<const uint32_t *>(arena + record.widths_offset)[tile.expert])) { \
 	case EXL3_BITS_X2_K2: {                                                                        \
 		constexpr uint32_t BX2 = EXL3_BITS_X2_K2;                                              \
@@ -1120,8 +1143,7 @@ __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &r
 		call;                                                                                  \
 	} break;                                                                                       \
 	default:                                                                                       \
-		if (!thin)                                                                             \
-			prefill_release(&shared);                                                      \
+		otherwise;                                                                             \
 		break;                                                                                 \
 	}
 
@@ -1144,13 +1166,19 @@ extern "C" __global__ void __cluster_dims__(PREFILL_PAIR, 1, 1) __launch_bounds_
 	const uint32_t count = prefill_tiles_of_unit(view, tile, tile_index, tile_count);
 	if (count == 0 || first_group >= prefill_inner_of(record, tile.expert) / EXL3_TRANSFORM)
 		return;
-	const bool thin = count == 1u && tile.row_count <= PREFILL_THIN_ROWS;
-	if (!thin && !prefill_begin(&shared, rank, prefill_rings<2, 1>::stages)) {
+	if (count == 1u && tile.row_count <= PREFILL_THIN_ROWS) {
+		if (threadIdx.x / EXL3_WARP >= PREFILL_FIRST_DECODE_WARP &&
+		    first_group + rank < prefill_inner_of(record, tile.expert) / EXL3_TRANSFORM)
+			PREFILL_WIDTH_SWITCH((prefill_thin_gate_up<BX2>(record, arena, view, tile_index, first_group + rank,
+									dynamic_shared, &shared)), (void)0)
+		return;
+	}
+	if (!prefill_begin(&shared, rank, prefill_rings<2, 1>::stages)) {
 		prefill_release(&shared);
 		return;
 	}
-	PREFILL_WIDTH_SWITCH((prefill_gate_up<BX2>(record, arena, view, tile_index, count, first_group + rank, rank, thin,
-						   dynamic_shared, &shared)))
+	PREFILL_WIDTH_SWITCH((prefill_gate_up<BX2>(record, arena, view, tile_index, count, first_group + rank, rank, dynamic_shared,
+						   &shared)), prefill_release(&shared))
 }
 
 /* grid (ceil(H / 512), tile capacity) CTA pairs x 576 */
@@ -1172,14 +1200,19 @@ extern "C" __global__ void __cluster_dims__(PREFILL_PAIR, 1, 1) __launch_bounds_
 	const uint32_t count = prefill_tiles_of_unit(view, tile, tile_index, tile_count);
 	if (count == 0)
 		return;
-	const bool thin = count == 1u && tile.row_count <= PREFILL_THIN_ROWS;
-	if (!thin && !prefill_begin(&shared, rank, prefill_rings<1, 2>::stages)) {
+	if (count == 1u && tile.row_count <= PREFILL_THIN_ROWS) {
+		if (threadIdx.x / EXL3_WARP >= PREFILL_FIRST_DECODE_WARP && first_group + 2u * rank < record.input_size / EXL3_TRANSFORM)
+			PREFILL_WIDTH_SWITCH((prefill_thin_down<BX2>(record, arena, view, tile_index, first_group + 2u * rank, dynamic_shared,
+								     &shared)), (void)0)
+		return;
+	}
+	if (!prefill_begin(&shared, rank, prefill_rings<1, 2>::stages)) {
 		prefill_release(&shared);
 		return;
 	}
 	PREFILL_WIDTH_SWITCH((prefill_down<BX2>(record, arena, view, tile_index, count, first_group + 2u * rank,
-						min(2u, record.input_size / EXL3_TRANSFORM - first_group), rank, thin, dynamic_shared,
-						&shared)))
+						min(2u, record.input_size / EXL3_TRANSFORM - first_group), rank, dynamic_shared,
+						&shared)), prefill_release(&shared))
 }
 
 /* grid (ceil(H / 512), row capacity) x 128: FP32 row sums over the row's local pairs from +0 in ascending slot order,
