@@ -87,14 +87,15 @@ AB_INLINE uint64_t exl3_layer_gate_up_product_bytes(uint32_t pair_count, uint32_
 /* ---- prefill (kernel_exl3_prefill) ---- */
 #define EXL3_PREFILL_GEMM_THREADS 576u /* a copy warp, an issuing warp, sixteen decode warps */
 #define EXL3_PREFILL_OPERAND_PARTS 4u /* an operand CTA takes a quarter of a tile's rows */
-#define EXL3_PREFILL_STAGE_STEPS 4u /* steps of 16 inputs of one stage */
-/* A ring of stages of 64 inputs: three of gate/up (two blocks of rows, two of weights, 64 KB), four of down (one and two).
- * What a stage costs whatever its inputs (the issuing warp's wait, products and commit, 515 cycles; the hand-over across the
- * pair) is paid half as often as with stages of 32, of which seven fit: 413 rows of 256 experts 621 us of gate/up and
- * 357 of down, 596 and 356 so; 4096 rows 1880 and 1140, 1855 and 1079. More stages where the rows are few leave room for
- * them (six for 16 rows a CTA): no gain. */
+/* Steps of 16 inputs of one stage, by the launch's matrices. Gate and up (two blocks of rows and two of weights): stages of 32
+ * inputs, six of 32 KB; down (one and two): of 64, four of 48 KB. What a stage costs whatever its inputs (the issuing
+ * warp's wait, products and commit, 515 cycles; the hand-over across the pair) is paid half as often with 64 inputs, which
+ * counts where the rows are few; but only three such stages of gate and up fit, and with 256 rows the copies' latency
+ * shows. us of gate/up in stages of 32 and of 64: 1024 rows of 32 experts 421, 423; 4096 rows of 32 1246, 1289; 4096 rows of 256 1812,
+ * 1846; of rank 0 of eight 195, 198; 413 rows of 256 528, 518. Of down: 238, 236; 687, 670 (4096 rows of 32); 413 rows 299, 297. */
+#define EXL3_PREFILL_STAGE_STEPS(matrices) ((matrices) == 1u ? 4u : 2u)
 #define EXL3_PREFILL_DYNAMIC_BYTES 196608u
-#define EXL3_PREFILL_MOST_STAGES 4u
+#define EXL3_PREFILL_MOST_STAGES 6u
 #define EXL3_PREFILL_STAGING_ROW 132u /* floats of a staged accumulator row */
 
 #endif

@@ -6,7 +6,7 @@
  *   - streams its rows' FP16 operands (pre-tiled in the tensor cores' no-swizzle K-major layout) into a ring of
  *     shared-memory stages, one bulk asynchronous copy a stage (one warp),
  *   - loads the trellis words of its outputs into registers a turn of the decode teams ahead, decodes them and stores
- *     them as the A operand blocks of the stage (sixteen warps in two teams, a team a stage; the decode's fragment order
+ *     them as the A operand blocks of the stage (sixteen warps in teams, a team a stage; the decode's fragment order
  *     makes every store a contiguous 128 bytes of the block),
  *   - multiplies with tcgen05.mma of cta_group::2 (one thread of the pair), FP32 accumulators in tensor memory, the stage
  *     released by tcgen05.commit,
@@ -23,8 +23,6 @@
 #define PREFILL_FIRST_DECODE_WARP 2u /* behind the copy warp and the issuing warp */
 #define PREFILL_DECODE_WARPS 16u
 #define PREFILL_DECODE_THREADS (PREFILL_DECODE_WARPS * EXL3_WARP)
-#define PREFILL_PARTS (2u * EXL3_PREFILL_STAGE_STEPS) /* of a stage's weights, a decode warp each */
-#define PREFILL_TEAMS (PREFILL_DECODE_WARPS / PREFILL_PARTS) /* of decode warps */
 #define PREFILL_GROUP_THREADS 256u
 
 struct prefill_shared {
@@ -215,8 +213,8 @@ __device__ __forceinline__ uint32_t prefill_tiles_of_unit(const prefill_view &vi
 	return tile_index + 1u < tile_count && tiles[tile_index + 1u].expert == tile.expert ? 2u : 1u;
 }
 
-/* Where a tile's operands lie: what a CTA of the pair takes for one stage of 64 inputs is ONE run of bytes, [matrix][eight
- * pieces of eight inputs][half rows][16 bytes], the stages one behind the other. The second CTA's runs are in the second
+/* Where a tile's operands lie: what a CTA of the pair takes for one stage (gate and up 32 inputs, down 64) is ONE run of bytes,
+ * [matrix][pieces of eight inputs][half rows][16 bytes], the stages one behind the other. The second CTA's runs are in the second
  * tile's region, or behind the first CTA's for a single tile. (With a fixed place for each of 128 rows a stage of fewer
  * rows was up to eight copies, and their issue, 1070 cycles a stage, was what bounded the products.) */
 struct prefill_rows {
@@ -238,7 +236,7 @@ __device__ __forceinline__ uint64_t prefill_operand_byte(const prefill_rows &row
 							 uint32_t input)
 {
 	const uint32_t rank = row / rows.half, piece = input / 8u;
-	constexpr uint32_t pieces = 2u * EXL3_PREFILL_STAGE_STEPS; /* of a stage */
+	const uint32_t pieces = 2u * EXL3_PREFILL_STAGE_STEPS(matrices); /* of a stage */
 	return rank * rows.second + (uint64_t)((piece / pieces * matrices + m) * pieces + piece % pieces) * (rows.half * 16u) +
 	       (row - rank * rows.half) * 16u + input % 8u * 2u;
 }
@@ -339,8 +337,8 @@ extern "C" __global__ void __launch_bounds__(EXL3_TRANSFORM_THREADS)
  * (its 128 outputs and its 128 rows per 128 cycles). One CTA on its own with two row tiles of 128 x 128 products needs
  * 128 bytes a cycle for the instructions alone, all there is, and takes every row's operands from L2 twice as often.
  * The rows' number is the instruction's N, so a last tile of few rows costs the tensor cores little; the decode is the
- * same for any. 4096 rows of H 4096, I 2048, 256 experts of 8: gate/up 2202 us with single CTAs, 1811 so; down 1211,
- * 1015. Neither end is full (1024 rows of 32 experts: 67 % of the issue slots, the tensor cores 43 % of the cycles): a
+ * same for any. 4096 rows of H 4096, I 2048, 256 experts of 8: gate/up 2202 us with single CTAs, 1812 so; down 1211,
+ * 993. Neither end is full (1024 rows of 32 experts: 67 % of the issue slots, the tensor cores 43 % of the cycles): a
  * stage's turn in the ring, about 600 cycles of which the products take 512 at most, and a unit's beginning and epilogue,
  * a sixth of gate/up and a quarter of down, lie between them. */
 #define PREFILL_PAIR 2u /* CTAs of a unit */
@@ -466,18 +464,20 @@ __device__ __forceinline__ void pair_acquire()
 }
 
 /* Dynamic shared memory of a product CTA: MATRICES x GROUPS = 2 accumulators, gate and up of 128 outputs or down of
- * 2 x 128; a ring of stages of 64 inputs, each
- *   [matrix] the CTA's rows (up to 128 x 64 FP16, 16 KB): one bulk copy, mostly from L2
- *   [matrix x group] decoded weights, 128 outputs x 64 FP16, 16 KB in the same layout: written by the decode warps
+ * 2 x 128; a ring of stages of 32 (gate and up) or 64 inputs (EXL3_PREFILL_STAGE_STEPS), each
+ *   [matrix] the CTA's rows (up to 128 x 32 or 64 FP16, 8 or 16 KB): one bulk copy, mostly from L2
+ *   [matrix x group] decoded weights, 128 outputs by as many inputs in the same layout: written by the decode warps
  * Rows and weights share the stage so that the issuing warp waits for ONE barrier a stage: a wait on a barrier that is
  * long complete takes it 150 cycles, three of them and the issue of four products 730, where the products of 256 rows
  * last 512. The trellis words do not pass here: the start of a bulk copy takes a warp 300 to 500 cycles, whatever the
  * bytes, and a stage's words were four runs (5 copies a stage: 650 cycles a stage; 12: 900). */
-#define PREFILL_STEPS EXL3_PREFILL_STAGE_STEPS
-#define PREFILL_BLOCK (PREFILL_STEPS * 4096u) /* 512 units of 16 bytes, 256 a step */
 template <uint32_t MATRICES, uint32_t GROUPS> struct prefill_rings {
-	static constexpr uint32_t weights_at = MATRICES * PREFILL_BLOCK; /* in a stage, behind the rows */
-	static constexpr uint32_t stage = weights_at + MATRICES * GROUPS * PREFILL_BLOCK;
+	static constexpr uint32_t steps = EXL3_PREFILL_STAGE_STEPS(MATRICES); /* of 16 inputs */
+	static constexpr uint32_t block = steps * 4096u; /* of 128 rows or outputs */
+	static constexpr uint32_t weights_at = MATRICES * block; /* in a stage, behind the rows */
+	static constexpr uint32_t stage = weights_at + MATRICES * GROUPS * block;
+	static constexpr uint32_t parts = MATRICES * GROUPS * steps; /* of a stage's weights, a decode warp each */
+	static constexpr uint32_t teams = PREFILL_DECODE_WARPS / parts; /* of decode warps */
 	static constexpr uint32_t stages = EXL3_PREFILL_DYNAMIC_BYTES / stage;
 	static_assert(MATRICES * GROUPS * PREFILL_SUM_COLUMNS == 512u, "tensor memory has 512 columns");
 	static_assert(stages <= EXL3_PREFILL_MOST_STAGES && MATRICES * GROUPS == 2u, "the rings' barriers; a stage's parts");
@@ -507,7 +507,7 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 	if (warp == 0) {
 		/* the rows' operands: a copy a stage */
 		if (lane == 0) {
-			const uint32_t bytes = MATRICES * PREFILL_STEPS * 32u * half;
+			const uint32_t bytes = MATRICES * rings::steps * 32u * half;
 			uint32_t block = 0;
 			for (; block < blocks; block++) {
 				const uint32_t stage = block % S;
@@ -550,7 +550,7 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 		const uint32_t r_low = warp_value(prefill_descriptor_low(dynamic_shared, half * 16u));
 		const uint32_t w_low = warp_value(prefill_descriptor_low(dynamic_shared + rings::weights_at, 2048u));
 		const uint32_t r_step = warp_value(2u * half), columns = warp_value(accumulators), live = warp_value(sums);
-		const uint32_t full = warp_value(smem_address(shared->full)), r_second = MATRICES > 1u ? PREFILL_STEPS * r_step : 0u;
+		const uint32_t full = warp_value(smem_address(shared->full)), r_second = MATRICES > 1u ? rings::steps * r_step : 0u;
 		for (uint32_t left = blocks; left != 0; left--) {
 			if (ready == 0) {
 				good = warp_wait<true>(&shared->full[stage], parity);
@@ -567,12 +567,12 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 			tensor_fence_after();
 			if (prefill_elected()) {
 #pragma unroll
-				for (uint32_t step = 0; step < PREFILL_STEPS; step++)
+				for (uint32_t step = 0; step < rings::steps; step++)
 					tensor_multiply(columns, w + step * 256u, r + step * r_step, instruction, step == 0u ? accumulate : 1u);
 				if (GROUPS == 1u || live > 1u)
 #pragma unroll
-					for (uint32_t step = 0; step < PREFILL_STEPS; step++)
-						tensor_multiply(columns + PREFILL_SUM_COLUMNS, w + (PREFILL_STEPS + step) * 256u,
+					for (uint32_t step = 0; step < rings::steps; step++)
+						tensor_multiply(columns + PREFILL_SUM_COLUMNS, w + (rings::steps + step) * 256u,
 								r + r_second + step * r_step, instruction, step == 0u ? accumulate : 1u);
 				tensor_commit(freed, 3u);
 				if (left == 1u)
@@ -597,26 +597,25 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 		return false;
 	}
 
-	/* decode: the sixteen warps are two teams of eight; team q decodes the WHOLE stages q, q + 2, ..., so that the
-	 * teams work on two different stages at once and a warp crosses a barrier and a proxy fence once per stage of
-	 * eight tiles. A warp's part of a stage is the eight adjacent tiles of one (matrix, group, step). A lane loads
-	 * its ring words straight into registers, a tile's words for the team's next stage as soon as this one's are decoded: two
-	 * stages, more than a microsecond, ahead. */
+	/* decode: the sixteen warps are teams of a warp a part, four for gate and up and two for down; team q of T decodes the
+	 * WHOLE stages q, q + T, ..., so that the teams work on different stages at once and a warp crosses a barrier and a
+	 * proxy fence once per stage of eight tiles. A warp's part of a stage is the eight adjacent tiles of one (matrix, group, step).
+	 * A lane loads its ring words straight into registers, a tile's words for the team's next stage as soon as this one's are
+	 * decoded: 128 inputs, more than a microsecond, ahead. */
 	{
-		static_assert(MATRICES * GROUPS * PREFILL_STEPS == PREFILL_PARTS && PREFILL_DECODE_WARPS == PREFILL_PARTS * PREFILL_TEAMS,
-			      "a part a warp");
-		const uint32_t decoder = warp - PREFILL_FIRST_DECODE_WARP, team = decoder / PREFILL_PARTS, member = decoder % PREFILL_PARTS;
-		const uint32_t step = member % PREFILL_STEPS, g = GROUPS > 1u ? member / PREFILL_STEPS : 0u;
-		const uint32_t m = MATRICES > 1u ? member / PREFILL_STEPS : 0u;
+		static_assert(PREFILL_DECODE_WARPS == rings::parts * rings::teams, "a part a warp");
+		const uint32_t decoder = warp - PREFILL_FIRST_DECODE_WARP, team = decoder / rings::parts, member = decoder % rings::parts;
+		const uint32_t step = member % rings::steps, g = GROUPS > 1u ? member / rings::steps : 0u;
+		const uint32_t m = MATRICES > 1u ? member / rings::steps : 0u;
 		const uint32_t begin = ring::begin(lane);
 		const uint32_t word_index = begin / 32u, shift = begin % 32u, next_index = (word_index + 1u) % ring::words;
 		const bool taken = g < groups; /* the CTA has this group */
-		unsigned char *const to_part = dynamic_shared + rings::weights_at + (m + g) * PREFILL_BLOCK + step * 4096u + lane * 4u;
+		unsigned char *const to_part = dynamic_shared + rings::weights_at + (m + g) * rings::block + step * 4096u + lane * 4u;
 		const uint32_t *words_at =
 			reinterpret_cast<const uint32_t *>(MATRICES > 1u && m != 0u ? matrices[MATRICES - 1u] : matrices[0]) +
-			(uint64_t)(team * PREFILL_STEPS + step) * step_words +
+			(uint64_t)(team * rings::steps + step) * step_words +
 			(uint64_t)(first_group + g) * EXL3_GROUP_TILES * ring::words;
-		const uint64_t turn_words = (uint64_t)(PREFILL_TEAMS * PREFILL_STEPS) * step_words;
+		const uint64_t turn_words = (uint64_t)(rings::teams * rings::steps) * step_words;
 		bool good = true;
 		uint32_t words[EXL3_GROUP_TILES][2];
 		if (taken && team < blocks)
@@ -625,9 +624,9 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 				words[tile][0] = __ldg(words_at + tile * ring::words + word_index);
 				words[tile][1] = __ldg(words_at + tile * ring::words + next_index);
 			}
-		for (uint32_t block = team; block < blocks; block += PREFILL_TEAMS) {
+		for (uint32_t block = team; block < blocks; block += rings::teams) {
 			const uint32_t stage = block % S;
-			if (block + PREFILL_TEAMS < blocks)
+			if (block + rings::teams < blocks)
 				words_at += turn_words; /* of the next turn; the last loads its own once more */
 			if (block >= S) {
 				good = warp_wait(&shared->free[stage], (block / S - 1u) & 1u);
@@ -670,13 +669,13 @@ __device__ __forceinline__ bool prefill_products(const unsigned char *const (&ma
 /* Begins a product CTA: barriers, tensor memory, and the pair's agreement on whether to run. All threads of both CTAs
  * call; false: an earlier wait ran out, the pair is to go (the flag is never cleared while the kernel file stays loaded:
  * later CTAs do not queue up behind the same fault, the host reads the flag and rejects the result). */
-__device__ __forceinline__ bool prefill_begin(prefill_shared *shared, uint32_t rank, uint32_t stages)
+__device__ __forceinline__ bool prefill_begin(prefill_shared *shared, uint32_t rank, uint32_t stages, uint32_t parts)
 {
 	const uint32_t warp = threadIdx.x / EXL3_WARP;
 	if (threadIdx.x == 0) {
 		for (uint32_t stage = 0; stage < stages; stage++) {
 			/* the warps of the team that decodes the stage, the rows' copies, at rank 0 the other CTA */
-			barrier_init(&shared->full[stage], PREFILL_PARTS + (rank == 0 ? 2u : 1u));
+			barrier_init(&shared->full[stage], parts + (rank == 0 ? 2u : 1u));
 			barrier_init(&shared->free[stage], 1);
 		}
 		barrier_init(&shared->done, 1);
@@ -878,7 +877,8 @@ __device__ __forceinline__ void prefill_gate_up_rows(const struct exl3_prefill_r
  * a step's eight tiles a warp, is faster (below) but gives a row other bits in a short tile than in a long one.
  * Such a tile's time is its decode and what a unit costs beside it (a pair's beginning, 5 k cycles, the stages' hand-overs, a
  * fifth of its 70 k). 413 rows of 256 experts, 59 of 97 with at most eight rows: gate/up and down 538 and 311 us through the
- * stages, 519 and 298 so, 506 and 294 with K shared out; 4096 rows, 95 of 173: 1872 and 1002, 1843 and 991, 1824 and 977.
+ * stages, 519 and 298 so, 506 and 294 with K shared out; 4096 rows, 95 of 173: 1872 and 1002, 1843 and 991, 1824 and 977 (all
+ * with stages of 64 inputs).
  * Without the L2's request 523 and 305. More than eight rows would be a second product a fragment. */
 #define PREFILL_THIN_ROWS 8u
 #define PREFILL_THIN_HALF 16u /* rows of the first CTA's half of such a tile's operands (prefill_rows_of) */
@@ -889,8 +889,9 @@ __device__ __forceinline__ void prefill_thin_products(const unsigned char *const
 						      uint32_t row_count, uint32_t steps, unsigned char *dynamic_shared)
 {
 	typedef exl3_ring<BX2> ring;
+	constexpr uint32_t stage_steps = EXL3_PREFILL_STAGE_STEPS(MATRICES);
 	static_assert(PREFILL_DECODE_WARPS == MATRICES * GROUPS * EXL3_GROUP_TILES, "16 outputs a warp");
-	static_assert(PREFILL_THIN_TURN % PREFILL_STEPS == 0u && EXL3_TRANSFORM / EXL3_TILE % PREFILL_THIN_TURN == 0u,
+	static_assert(PREFILL_THIN_TURN % stage_steps == 0u && EXL3_TRANSFORM / EXL3_TILE % PREFILL_THIN_TURN == 0u,
 		      "a turn is whole stages, K whole turns");
 	const uint32_t lane = threadIdx.x % EXL3_WARP, decoder = threadIdx.x / EXL3_WARP - PREFILL_FIRST_DECODE_WARP;
 	const uint32_t which = decoder / EXL3_GROUP_TILES, tile = decoder % EXL3_GROUP_TILES;
@@ -905,14 +906,14 @@ __device__ __forceinline__ void prefill_thin_products(const unsigned char *const
 		const uint32_t *words = reinterpret_cast<const uint32_t *>((uint64_t)warp_value((uint32_t)(first >> 32)) << 32 |
 									   warp_value((uint32_t)first));
 		const uint32_t *ahead = words + (2u * PREFILL_THIN_TURN + lane % PREFILL_THIN_TURN) * step_words;
-		/* step s stands in stage s / PREFILL_STEPS: [matrix][pieces][half rows][16 bytes]; the lane's two words of it */
-		constexpr uint32_t piece = PREFILL_THIN_HALF * 16u, stage_bytes = MATRICES * PREFILL_STEPS * 2u * piece;
-		const unsigned char *fed = row_runs + m * PREFILL_STEPS * 2u * piece + lane / 4u * 16u + lane % 4u * 4u;
+		/* step s stands in stage s / stage_steps: [matrix][pieces][half rows][16 bytes]; the lane's two words of it */
+		constexpr uint32_t piece = PREFILL_THIN_HALF * 16u, stage_bytes = MATRICES * stage_steps * 2u * piece;
+		const unsigned char *fed = row_runs + m * stage_steps * 2u * piece + lane / 4u * 16u + lane % 4u * 4u;
 		float sums[4] = { 0.0f, 0.0f, 0.0f, 0.0f };
 		uint32_t held[PREFILL_THIN_TURN][2], held_fed[PREFILL_THIN_TURN][2];
 #pragma unroll
 		for (uint32_t step = 0; step < PREFILL_THIN_TURN; step++) {
-			const unsigned char *const at = fed + step / PREFILL_STEPS * stage_bytes + step % PREFILL_STEPS * 2u * piece;
+			const unsigned char *const at = fed + step / stage_steps * stage_bytes + step % stage_steps * 2u * piece;
 			held[step][0] = __ldg(words + word_index);
 			held[step][1] = __ldg(words + next_index);
 			held_fed[step][0] = *reinterpret_cast<const uint32_t *>(at);
@@ -924,14 +925,14 @@ __device__ __forceinline__ void prefill_thin_products(const unsigned char *const
 			if (left == 1u) /* the last turn loads its own once more */
 				words -= PREFILL_THIN_TURN * step_words;
 			else
-				fed += PREFILL_THIN_TURN / PREFILL_STEPS * stage_bytes;
+				fed += PREFILL_THIN_TURN / stage_steps * stage_bytes;
 			if (left > 2u && lane < PREFILL_THIN_TURN) {
 				asm volatile("prefetch.global.L2 [%0];" ::"l"(ahead));
 				ahead += PREFILL_THIN_TURN * step_words;
 			}
 #pragma unroll
 			for (uint32_t step = 0; step < PREFILL_THIN_TURN; step++) {
-				const unsigned char *const at = fed + step / PREFILL_STEPS * stage_bytes + step % PREFILL_STEPS * 2u * piece;
+				const unsigned char *const at = fed + step / stage_steps * stage_bytes + step % stage_steps * 2u * piece;
 				uint32_t fragment[4];
 				exl3_decode_fragment<BX2>(held[step][0], held[step][1], shift, fragment);
 				held[step][0] = __ldg(words + word_index);
@@ -976,7 +977,7 @@ __device__ __forceinline__ void prefill_gate_up(const struct exl3_prefill_record
 							 first_scale);
 	}
 	const bool complete = prefill_products<BX2, 2, 1>(matrices, I, group, mine, 1, row_runs, rows.half,
-							  H / (PREFILL_STEPS * EXL3_TILE), rank, dynamic_shared, shared);
+							  H / (prefill_rings<2, 1>::steps * EXL3_TILE), rank, dynamic_shared, shared);
 	if (threadIdx.x / EXL3_WARP >= PREFILL_FIRST_DECODE_WARP && complete && mine != 0) {
 		float *const staging = reinterpret_cast<float *>(dynamic_shared);
 		for (uint32_t tile = 0; tile < count; tile++) {
@@ -1069,7 +1070,7 @@ __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &r
 		prefill_fetch_scales(shared, g, reinterpret_cast<const __half *>(arena + first.down + exl3_code_bytes(I, H, BX2)) + I +
 							 (first_group + g) * EXL3_TRANSFORM);
 	const bool complete = prefill_products<BX2, 1, 2>(matrices, H, first_group, groups, sums, row_runs, rows.half,
-							  I / (PREFILL_STEPS * EXL3_TILE), rank, dynamic_shared, shared);
+							  I / (prefill_rings<1, 2>::steps * EXL3_TILE), rank, dynamic_shared, shared);
 	if (warp >= PREFILL_FIRST_DECODE_WARP && complete) {
 		float *const staging = reinterpret_cast<float *>(dynamic_shared);
 		float *const outputs = reinterpret_cast<float *>(arena + record.pair_output_offset);
@@ -1173,7 +1174,7 @@ extern "C" __global__ void __cluster_dims__(PREFILL_PAIR, 1, 1) __launch_bounds_
 									dynamic_shared, &shared)), (void)0)
 		return;
 	}
-	if (!prefill_begin(&shared, rank, prefill_rings<2, 1>::stages)) {
+	if (!prefill_begin(&shared, rank, prefill_rings<2, 1>::stages, prefill_rings<2, 1>::parts)) {
 		prefill_release(&shared);
 		return;
 	}
@@ -1206,7 +1207,7 @@ extern "C" __global__ void __cluster_dims__(PREFILL_PAIR, 1, 1) __launch_bounds_
 								     &shared)), (void)0)
 		return;
 	}
-	if (!prefill_begin(&shared, rank, prefill_rings<1, 2>::stages)) {
+	if (!prefill_begin(&shared, rank, prefill_rings<1, 2>::stages, prefill_rings<1, 2>::parts)) {
 		prefill_release(&shared);
 		return;
 	}

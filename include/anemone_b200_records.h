@@ -684,8 +684,8 @@ struct router_select_b200_arguments {
  *   counts uint32 [local + shared + 1] (the last: tile count) | tiles struct exl3_prefill_tile [tile capacity] |
  *   entries struct exl3_prefill_entry [local + shared][row_capacity] |
  *   gate/up operands FP16, H * 512 bytes a tile | down operands FP16, max(I, shared I) * 256 bytes a tile
- * stored as the tensor cores read them without swizzling, and so that what a CTA of a pair reads for 64 inputs is one
- * run of bytes: [H / 32][gate, up][4 pieces of eight inputs][rows][16 bytes] (down: without the second part), the rows
+ * stored as the tensor cores read them without swizzling, and so that what a CTA of a pair reads for a stage is one
+ * run of bytes: [H / 32][gate, up][4 pieces of eight inputs][rows][16 bytes], down [I / 64][8 pieces][rows][16 bytes], the rows
  * being the tile's 128, or, for an expert's last tile if its number is even (counted from 0), half its rows rounded up
  * to whole sixteens, the other half's runs behind them.
  * tile capacity = ceil(row_capacity * (picks + shared) / 128) + local + shared; exl3_prefill_parts_of takes the local
