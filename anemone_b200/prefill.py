@@ -25,12 +25,15 @@ from .moe import LINE, SIGNAL_BYTES, rank_columns
 
 PIECE_ROWS = 128  # a staged call's pieces begin on whole row tiles
 STEP_SPACE = 48  # a piece's step block and its status, behind the call's own in the 256 bytes of the step's space
-# A second: measured copies; weights decoded and multiplied with up to 256 rows, as if every held expert had rows (a
-# prompt's popularity leaves a third to a half of them without). PIECE_SECONDS: routing, grouping, the reduction and the gaps
-# between their launches, whatever the rows. Both fitted to calls in 1, 2 and 4 pieces of 512 to 4096 rows on a whole
-# layer of 64 and of 256 experts and on halves to eighths of it: the estimate takes the fastest of each.
-PCIE_BYTES, WEIGHT_RATE = 53e9, 7e12
-PIECE_SECONDS = 8e-5
+PCIE_BYTES = 53e9  # a second: measured copies
+# (weights a second, seconds a piece). The first: weights decoded and multiplied with up to 256 rows, as if every held expert
+# had rows (a prompt's popularity leaves a third to a half of them without). The second: routing, grouping, the reduction and
+# the gaps between their launches, whatever the rows. ONE_RANK is fitted to calls in 1, 2 and 4 pieces of 512 to 4096 rows of a
+# hidden width of 4096 and Zipf(1.1) popularity, on a whole layer of 64 and of 256 experts and on halves to eighths of it, on
+# one card: the estimate takes the fastest of each. A fit and no rate of this card: 7e12 is above what its memory delivers.
+# Where every piece has a reduction between ranks, no call in pieces has been timed: SEVERAL_RANKS are the products' own rate and
+# a generous piece, which cut a call only where its copies outweigh its products by far.
+ONE_RANK, SEVERAL_RANKS = (7e12, 8e-5), (2.4e12, 1e-4)
 
 
 def call_pieces(config, share, rank_count):
@@ -39,6 +42,7 @@ def call_pieces(config, share, rank_count):
     H 4096, I 2048, Zipf(1.1), ms a call in 1, 2, 4 pieces: 32 of 256 experts 1.78, 1.39, 1.41; 64 of them 2.17, 1.81, 2.00;
     128 2.71, 2.54, 3.05; all 4.56, 4.86, 6.08; 1024 rows on 64 of them 0.75, 0.84, 1.12. The ranks of a reduction must
     agree: theirs is the largest share of equal ones."""
+    weight_rate, piece_seconds = SEVERAL_RANKS if rank_count > 1 else ONE_RANK
     rows, H = config.row_capacity, config.hidden
     if rank_count > 1:
         matrices, pairs = -(-config.experts // rank_count), config.picks / rank_count
@@ -51,7 +55,7 @@ def call_pieces(config, share, rank_count):
     def estimate(count):
         weights = 3 * H * (inner * (count * matrices + rows * pairs / 256) + always_on * (count + rows / 256))
         hidden = (count - 1) / count
-        return taken / count + max(count * PIECE_SECONDS + weights / WEIGHT_RATE, taken * hidden, returned * hidden) + returned / count
+        return taken / count + max(count * piece_seconds + weights / weight_rate, taken * hidden, returned * hidden) + returned / count
     return min((count for count in (1, 2, 4) if rows >= 2 * PIECE_ROWS * count), key=estimate, default=1)
 
 

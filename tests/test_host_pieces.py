@@ -92,6 +92,24 @@ def test_ranks_agree_on_the_pieces(ranks, rows, held):
         assert len(counts) == 1 and counts <= {1, 2, 4}
 
 
+@pytest.mark.parametrize("rows,experts,counts", [
+    (512, 64, (1, 1, 1)), (1024, 64, (1, 1, 1)), (2048, 64, (1, 2, 2)), (4096, 64, (2, 2, 2)),
+    (512, 256, (1, 1, 1)), (1024, 256, (1, 1, 1)), (2048, 256, (1, 1, 1)), (4096, 256, (1, 1, 2))])
+def test_pieces_of_several_ranks(rows, experts, counts):
+    """What is measured on one card decides nothing for 2, 4 and 8 ranks, whose pieces hold a reduction each."""
+    config = MoeConfig(hidden=4096, inner=2048, experts=experts, shared=1, picks=8, row_capacity=rows)
+    for split in (Share.expert_parallel, Share.tensor_parallel):
+        assert tuple(prefill.call_pieces(config, split(config, ranks, 0), ranks) for ranks in (2, 4, 8)) == counts
+
+
+@pytest.mark.parametrize("rows,experts,held,count", [(4096, 256, 32, 2), (4096, 256, 64, 2), (4096, 256, 128, 2),
+                                                     (4096, 256, 256, 1), (1024, 256, 64, 1)])
+def test_pieces_of_one_rank(rows, experts, held, count):
+    """The fastest of 1, 2 and 4 pieces where they were timed."""
+    config = MoeConfig(hidden=4096, inner=2048, experts=experts, shared=1, picks=8, row_capacity=rows)
+    assert prefill.call_pieces(config, Share.expert_parallel(config, experts // held, 0), 1) == count
+
+
 def walk(layers, calls, values, rng):
     """Runs the ranks' calls as coroutines, one random step at a time; returns [rank][call] the results. A coroutine yields
     False while it waits."""
