@@ -3,7 +3,9 @@ the target, and the copy pool's plain form copies like the one it stands for."""
 import ctypes as C
 import glob
 import os
+import re
 import subprocess
+import time
 
 import numpy as np
 import pytest
@@ -19,7 +21,111 @@ class Copy(C.Structure):
 
 class Batch(C.Structure):
     _fields_ = [("copies", Copy * BATCH_MOST), ("count", C.c_uint32), ("next", C.c_uint32), ("allowed", C.c_uint32),
-                ("done", C.c_uint32 * BATCH_MOST), ("to_device", C.c_bool), ("shared", C.c_bool)]
+                ("done", C.c_uint32 * BATCH_MOST), ("to_device", C.c_bool), ("shared", C.c_bool), ("soon", C.c_bool)]
+
+
+def test_the_batch_here_is_the_librarys(tmp_path):
+    """Every field, in order, and every one's place: the library writes them all."""
+    header = open(os.path.join(build.CSRC, "host", "copy_pool.h")).read()
+    body = re.sub(r"/\*.*?\*/", "", re.search(r"struct ab_copy_batch \{(.*?)\};", header, flags=re.S).group(1), flags=re.S)
+    names = re.findall(r"(\w+)(?:\[\w+\])?\s*[,;]", body)
+    assert names == [field[0] for field in Batch._fields_]
+    source = "#include <stdio.h>\n#include \"copy_pool.h\"\nint main(void){" + "".join(
+        'printf("%%zu ", offsetof(struct ab_copy_batch, %s));' % name for name in names) + \
+        'printf("%zu", sizeof(struct ab_copy_batch)); return 0; }'
+    program = str(tmp_path / "places")
+    made = subprocess.run([build.GCC, "-I" + os.path.join(build.CSRC, "host"), "-x", "c", "-", "-o", program], input=source,
+                          capture_output=True, text=True)
+    assert made.returncode == 0, made.stderr
+    places = subprocess.run([program], capture_output=True, text=True, check=True).stdout.split()
+    assert [int(place) for place in places] == [getattr(Batch, name).offset for name in names] + [C.sizeof(Batch)]
+
+
+@pytest.fixture
+def pool(tmp_path):
+    """The pool as the library has it, with one user."""
+    path = str(tmp_path / "libpool.so")
+    made = subprocess.run([build.GCC] + build.GCC_FLAGS + ["-shared", "-o", path,
+                          os.path.join(build.CSRC, "host", "copy_pool.c"), "-lpthread"], capture_output=True, text=True)
+    assert made.returncode == 0, made.stderr
+    library = C.CDLL(path)
+    library.ab_copy_batch_help.restype = library.ab_copy_batch_is_done.restype = C.c_bool
+    library.ab_copy_pool_enter()
+    yield library
+    library.ab_copy_pool_leave()
+
+
+def batch_of(count, size=5000):
+    sources = np.random.default_rng(count).integers(0, 256, size=(count, size), dtype=np.uint8)
+    targets = np.full((count, size), 0xA5, dtype=np.uint8)
+    batch = Batch()
+    for index in range(count):
+        batch.copies[index] = Copy(targets[index].ctypes.data, sources[index].ctypes.data, size)
+    batch.count = count
+    return batch, sources, targets
+
+
+@pytest.mark.parametrize("soon_at", [None, 0, 3])
+def test_pieces_allowed_one_by_one(pool, soon_at):
+    """A result's pieces as they arrive: none is made before it is allowed, each is then made by a thread of the pool (the
+    caller only where there is none), the batch ends, and the pool takes the next."""
+    for count in (9, 2, BATCH_MOST):
+        batch, sources, targets = batch_of(count)
+        pool.ab_copy_batch_begin(C.byref(batch))
+        for piece in range(count):
+            time.sleep(0.0005)
+            assert (targets[piece:] == 0xA5).all()
+            pool.ab_copy_batch_allow(C.byref(batch), piece + 1)
+            if piece == soon_at:
+                pool.ab_copy_batch_soon(C.byref(batch))
+                assert batch.soon == batch.shared
+            until = time.monotonic() + 20
+            while not pool.ab_copy_batch_is_done(C.byref(batch), piece):
+                if not batch.shared:
+                    pool.ab_copy_batch_help(C.byref(batch))
+                assert time.monotonic() < until
+        pool.ab_copy_batch_end(C.byref(batch))
+        assert np.array_equal(targets, sources) and not pool.ab_copy_batch_help(C.byref(batch))
+
+
+@pytest.mark.parametrize("soon", [False, True])
+@pytest.mark.parametrize("allowed", [0, 1, 7])
+def test_a_cut_batch_makes_what_was_allowed(pool, soon, allowed):
+    """After a failure in the middle of a result: what was allowed is made, the rest never, with the pool's threads looking
+    out for it or not; they are free for the next batch and for the pool's end."""
+    batch, sources, targets = batch_of(12)
+    pool.ab_copy_batch_begin(C.byref(batch))
+    pool.ab_copy_batch_allow(C.byref(batch), allowed)
+    if soon:
+        pool.ab_copy_batch_soon(C.byref(batch))
+        time.sleep(0.002)
+    pool.ab_copy_batch_cut(C.byref(batch))
+    pool.ab_copy_batch_end(C.byref(batch))
+    time.sleep(0.002)
+    assert np.array_equal(targets[:allowed], sources[:allowed]) and (targets[allowed:] == 0xA5).all()
+    following, others, copied = batch_of(BATCH_MOST)
+    following.allowed = BATCH_MOST
+    pool.ab_copy_batch_begin(C.byref(following))
+    assert following.shared == batch.shared and not following.soon
+    pool.ab_copy_batch_end(C.byref(following))
+    assert np.array_equal(copied, others)
+
+
+def test_two_batches_at_once(pool):
+    """One batch at a time has the pool's threads; a second is made by its caller alone, with the same calls."""
+    first, sources, targets = batch_of(10)
+    pool.ab_copy_batch_begin(C.byref(first))
+    pool.ab_copy_batch_allow(C.byref(first), 1)
+    pool.ab_copy_batch_soon(C.byref(first))
+    second, others, copied = batch_of(11)
+    pool.ab_copy_batch_begin(C.byref(second))
+    assert not (first.shared and second.shared)
+    pool.ab_copy_batch_allow(C.byref(second), 4)
+    pool.ab_copy_batch_soon(C.byref(second))
+    assert not second.soon or second.shared
+    pool.ab_copy_batch_end(C.byref(second))
+    pool.ab_copy_batch_end(C.byref(first))
+    assert np.array_equal(copied, others) and np.array_equal(targets, sources)
 
 
 def on_x86():
