@@ -28,8 +28,13 @@
 #define STEP_WORDS 16u /* 64-bit words a graph: a line of 128 bytes of its own, the first two used */
 #define STEP_COPY_BLOCKS 64u
 #define CALL_PIECE_BYTES (1u << 19) /* 10 us of PCIe, 30 of a core's copy */
-/* Up to here half of that, since the first piece's copy hides behind nothing, and the pool's threads look out for a result's
- * pieces: 333 rows of 4096 490 us a call, 455 so. (A prompt of 2048 rows: 2650, 2700 with both.) */
+/* Up to CALL_HALF_BYTES in one direction half of that, since the first piece's copy hides behind nothing; beyond, the pieces'
+ * own cost counts for more. Up to CALL_SHORT_BYTES of result the pool's threads look out for its pieces instead of being woken
+ * for each. us a call with neither, with the look-out, with both; rows of 4096 of a rank of eight, original weights: 128 rows
+ * (1.1 MB) 288, 273, 262; 333 (2.9) 497, 452, 446; 400 (3.5) 519, 498, 494; 440 (3.8) 534, 504, 519; 512 (4.5) 568, 536, 555;
+ * 700 (6.1) 673, 652, 692; 1000 (8.7) 837, 830, 908; 1500 (13.1) 1162, 1136, 1270; EXL3, 64 experts: 128 rows 481, 458, 410;
+ * 400 (3.4) 701, 712, 659; 500 (4.2) 772, 748, 744; 700 (5.9) 905, 880, 903. Above 8 MB of result the look-out is level. */
+#define CALL_HALF_BYTES (4u << 20)
 #define CALL_SHORT_BYTES (8u << 20)
 #define STEP_SPIN_NANOSECONDS 2000000ull /* a step's wait looks at its word alone for so long */
 
@@ -1690,7 +1695,7 @@ static uint32_t call_pieces(struct ab_copy_batch *batch, const struct backend_b2
 	uint64_t total = 0;
 	for (uint32_t range = 0; range < count; range++)
 		total += ranges[range].byte_count;
-	uint64_t piece = total <= CALL_SHORT_BYTES ? CALL_PIECE_BYTES / 2u : CALL_PIECE_BYTES;
+	uint64_t piece = total <= CALL_HALF_BYTES ? CALL_PIECE_BYTES / 2u : CALL_PIECE_BYTES;
 	while (total / piece + count > AB_COPY_BATCH_MOST)
 		piece *= 2u;
 	uint32_t pieces = 0;

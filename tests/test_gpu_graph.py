@@ -95,7 +95,8 @@ def test_side_runs_and_copies(api):
         card.close()
 
 
-@pytest.mark.parametrize("sizes", [(1,), (63, 65, 17), ((1 << 19) - 1, (1 << 19) + 1), (1 << 20, 3, 5 << 20), (40 << 20,)])
+@pytest.mark.parametrize("sizes", [(1,), (63, 65, 17), ((1 << 19) - 1, (1 << 19) + 1), (1 << 20, 3, 5 << 20), (40 << 20,),
+                                   (4 << 20,), ((4 << 20) - 5, 6), (8 << 20,), ((8 << 20) - 1, 2)])
 def test_a_call_copies_ordinary_memory(api, sizes):
     """backend_b200_step_call without a graph: ranges of ordinary memory in and out again, at the edges of the pieces
     they are cut in (one piece, ragged ones, longer pieces where there would be too many), odd addresses and sizes."""
