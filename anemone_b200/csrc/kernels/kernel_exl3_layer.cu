@@ -46,12 +46,13 @@ extern "C" __global__ void __launch_bounds__(EXL3_LAYER_ROUTE_THREADS)
 	const float *const bias =
 		record.bias_offset != 0 ? reinterpret_cast<const float *>(arena + record.bias_offset) : nullptr;
 	/* every CTA chooses every live row's experts itself (the same arithmetic, the same picks): the launch lasts as long
-	 * as one row's chain of dependent instructions. Up to eight rows a team of four warps takes one, whose chain is a
-	 * third of a warp's; more rows a warp each (32 rows of 256 experts by teams, four behind one another: 52 us; 23 so) */
+	 * as one row's chain of dependent instructions. Few rows of many experts a team of four warps each, others a warp each
+	 * (router_by_teams; 9 rows of 256 experts by teams, two behind one another: 24.6 us, 18.2 so; 16 rows 29.7, 19.1; 32 rows
+	 * 52.9, 26.0) */
 	uint32_t *const picks_out = reinterpret_cast<uint32_t *>(arena + record.picks_offset);
 	float *const weights_out = reinterpret_cast<float *>(arena + record.weights_offset);
 	const uint32_t team = warp / ROUTER_TEAM_WARPS, teams = warps / ROUTER_TEAM_WARPS;
-	if (live <= teams) {
+	if (router_by_teams(live, teams, routed, picks)) {
 		if (team < live)
 			router_row_team(scores + (uint64_t)team * routed, bias, routed, picks, record.scoring, record.route_scale, lane,
 					warp % ROUTER_TEAM_WARPS, 1u + team, candidates[team], chosen[team], weight[team],

@@ -39,9 +39,9 @@ __device__ __forceinline__ void router_select_block(const struct router_select_b
 	uint32_t *const picks_out = reinterpret_cast<uint32_t *>(arena + arguments.picks_offset);
 	float *const weights_out = reinterpret_cast<float *>(arena + arguments.weights_offset);
 	const uint32_t team = warp / ROUTER_TEAM_WARPS, teams = blockDim.x / WARP / ROUTER_TEAM_WARPS;
-	if (live <= teams) {
+	if (router_by_teams(live, teams, experts, picks)) {
 		/* a team of four warps a row (the same picks and weights): the launch lasts as long as one row's chain of
-		 * dependent instructions, which a team shortens */
+		 * dependent instructions, which a team shortens where the experts are many */
 		if (team < live)
 			router_row_team(scores + (uint64_t)team * experts, bias, experts, picks, arguments.scoring,
 					arguments.route_scale, lane, warp % ROUTER_TEAM_WARPS, 1u + team, candidates[team],

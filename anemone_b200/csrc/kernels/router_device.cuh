@@ -196,6 +196,17 @@ __device__ __forceinline__ uint64_t router_warp_largest(uint64_t key)
  * are found; slots, weights and their sum are formed as there. All lanes of all members call. */
 #define ROUTER_TEAM_WARPS 4u
 #define ROUTER_TEAM_SLOTS (ROUTER_B200_MAXIMUM_EXPERTS / (ROUTER_TEAM_WARPS * WARP))
+/* Whether a block's rows, at most a team each, are taken by teams; else a warp takes a row. A team reads and orders the experts
+ * four times as fast, but merges its candidates pick by pick, with the other teams beside it on the same schedulers. us of the
+ * routing launch of a decode step, teams / a warp a row. 8 picks of 256 experts: 1 row 9.7 / 11.3, 4 rows 11.3 / 12.8,
+ * 6 12.9 / 13.2, 8 13.5 / 13.5; of 128: 1 row 9.7 / 10.4, 4 11.3 / 10.9, 8 13.3 / 11.3; of 64: 1 row 9.5 / 9.4, 8 13.2 / 9.9; of 384:
+ * 8 rows 14.2 / 16.4. 16 picks of 256: 3 rows 13.0 / 13.2, 5 15.1 / 14.0, 8 17.8 / 14.4; of 384: 6 rows 16.3 / 17.6, 8 19.1 / 18.1.
+ * 4 picks of 128: 5 rows 10.2 / 10.6, 8 11.2 / 11.1; of 64: 4 rows 9.6 / 9.3, 8 11.3 / 9.3. */
+__device__ __forceinline__ bool router_by_teams(uint32_t rows, uint32_t teams, uint32_t experts, uint32_t picks)
+{
+	return rows <= teams && rows * picks * 4u <= experts;
+}
+
 __device__ __forceinline__ void router_row_team(const float *scores, const float *bias, uint32_t experts, uint32_t picks,
 						uint32_t scoring, float route_scale, uint32_t lane, uint32_t member,
 						uint32_t barrier, uint64_t *candidates, uint32_t *chosen, float *weight,

@@ -132,6 +132,38 @@ def test_router_job_table_matches_oracle(api, oracle, form):
 
 
 @pytest.mark.parametrize("form", ["fused", "pull"])
+@pytest.mark.parametrize("experts,picks,rows", [(256, 8, (1, 8)), (255, 8, (7, 8)), (128, 8, (4, 5)), (32, 8, (1, 2)), (31, 8, (1,)),
+                                                (64, 16, (1, 2)), (500, 16, (7, 8, 9)), (128, 4, (8, 9)), (17, 16, (1, 8))])
+def test_router_by_teams_and_by_warps(api, oracle, form, experts, picks, rows):
+    """Both ways a block takes its rows, at the line between them: picks, their order and their weights are the oracle's bits,
+    ties, not-a-numbers, infinities and equal scores among them."""
+    config = MoeConfig(hidden=256, inner=128, experts=experts, shared=0, picks=picks, row_capacity=max(rows))
+    widths = np.full(experts, 2, dtype=np.uint32)
+    tiny = [tuple(np.zeros(synthetic.matrix_bytes(i, o, 2), dtype=np.uint8) for i, o in
+                  ((256, 128), (256, 128), (128, 256)))] * experts
+    card = api.Card(0, MoeLayout(config, widths, 1, 0, reduce_form=form).arena_bytes)
+    try:
+        layer = MoeLayer(card, config, widths, tiny, reduce_form=form)
+        layer.connect_local([layer])
+        for count in rows:
+            rng = np.random.default_rng([experts, picks, count])
+            scores = rng.normal(0, 1, size=(count, experts)).astype(np.float32)
+            scores[0, experts // 2] = scores[0, 1] = 9.0
+            scores[-1, [0, experts - 1]] = np.nan, np.inf
+            scores[count // 2, ::3] = -np.inf if picks < 2 * experts // 3 else 0.25
+            layer.step(np.zeros((count, config.hidden), dtype=np.uint16), scores)
+            got = card.download(layer.layout.picks, count * picks * 4, np.uint32).reshape(count, picks)
+            weights = card.download(layer.layout.weights, count * picks * 4, np.uint32).reshape(count, picks)
+            wanted, want = moe_reference.route(oracle, config, scores)
+            assert np.array_equal(got, wanted), count
+            number = ~np.isnan(want)
+            assert np.array_equal(np.isnan(weights.view(np.float32)), ~number)
+            assert np.array_equal(weights[number], want[number].view(np.uint32))
+    finally:
+        card.close()
+
+
+@pytest.mark.parametrize("form", ["fused", "pull"])
 def test_router_at_the_reference_geometry(api, form):
     """384 experts, 6 picks, route scale 1.5, sqrt(softplus) affinities and a selection bias: picks, slot order,
     weights and job table equal the answers of the reference's own router reference (committed fixtures), bit for
