@@ -11,8 +11,8 @@
  *   - multiplies with tcgen05.mma of cta_group::2 (one thread of the pair), FP32 accumulators in tensor memory, the stage
  *     released by tcgen05.commit,
  *   - reads the accumulators back with tcgen05.ld and applies the chain's FP32 epilogue (exl3_passes.cuh: Hadamard,
- *     scales, SwiGLU, down-side transform / route weight) a warp a row.
- * A tile of at most eight rows takes none of it: mma.sync on what the decode leaves in registers (prefill_thin_products).
+ *     scales, SwiGLU, down-side transform / route weight), four rows a warp, a row a warp to PREFILL_FEW_ROWS.
+ * A single tile of at most eight rows takes none of it: mma.sync on what the decode leaves in registers (prefill_thin_products).
  * Arithmetic per value is the retained chain's; only the association of the FP32 sums over K is the tensor cores'.
  * Every wait is bounded: one that runs out raises exl3_wait_expired, the CTA stores nothing, waits (bounded) for what
  * it has in flight, frees its tensor memory and returns.
@@ -244,8 +244,11 @@ __device__ __forceinline__ uint64_t prefill_operand_byte(const prefill_rows &row
 /* Four rows a warp, eight lanes a row: what a lane holds of a block of 128 channels is four runs of four channels, at
  * 32 k + 4 (lane % 8) (hadamard128_rows' layout). */
 #define PREFILL_WARP_ROWS 4u
-/* A tile of at most this many rows is finished a row a warp (hadamard128_warp), whose chain is a third as long: an
- * epilogue of gate/up of up to 16 rows is 4 k cycles so, 9 k four rows a warp; of 128 rows 18 k and 15 k. */
+/* A tile of at most this many rows is finished a row a warp (hadamard128_warp), whose chain is a third as long; the bits are
+ * the same. gate/up and down together, us, 17 experts of as many rows each, H 4096, I 2048, a row a warp / four rows a
+ * warp: 12 rows 165.7 / 169.7, 16 167.4 / 170.5, 32 171.7 / 174.6, 33 176.7 / 179.4, 40 178.3 / 177.7, 48 179.7 / 178.9,
+ * 64 184.2 / 182.4, 128 204.7 / 202.3 (65 and 80 rows, where four rows a warp begin a second turn, 187.9 / 190.0 and 189.6 /
+ * 190.5). */
 #define PREFILL_FEW_ROWS 32u
 __device__ __forceinline__ void prefill_scales(const __half *scales, uint32_t first_channel, uint2 out[4])
 {
@@ -339,8 +342,9 @@ extern "C" __global__ void __launch_bounds__(EXL3_TRANSFORM_THREADS)
  * The rows' number is the instruction's N, so a last tile of few rows costs the tensor cores little; the decode is the
  * same for any. 4096 rows of H 4096, I 2048, 256 experts of 8: gate/up 2202 us with single CTAs, 1812 so; down 1211,
  * 993. Neither end is full (1024 rows of 32 experts: 67 % of the issue slots, the tensor cores 43 % of the cycles): a
- * stage's turn in the ring, about 600 cycles of which the products take 512 at most, and a unit's beginning and epilogue,
- * a sixth of gate/up and a quarter of down, lie between them. */
+ * stage's turn in the ring, about 600 cycles for 64 inputs of which the products take 512 at most, and a unit's beginning,
+ * epilogue and release lie between them: a third of a unit of 256 rows (gate/up 77 k cycles in its K loop and 41 k beside it,
+ * down 41 and 27), a tenth of one of 9 to 32 (78 and 9, 42 and 9). */
 #define PREFILL_PAIR 2u /* CTAs of a unit */
 #define PREFILL_SUM_COLUMNS 256u /* tensor-memory columns of one accumulator: a row a column */
 
@@ -778,7 +782,7 @@ __device__ __forceinline__ prefill_tile_view prefill_tile_of(const struct exl3_p
 }
 
 /* The gate/up epilogue of one row tile and one group of 128 outputs, from the staged accumulators (gate rows, then up
- * rows): Hadamard, scales, SwiGLU, down-side transform, FP16 down operand blocks. Decode warps; a warp a row. */
+ * rows): Hadamard, scales, SwiGLU, down-side transform, FP16 down operand blocks. Decode warps; four rows a warp, a row a warp to PREFILL_FEW_ROWS. */
 __device__ __forceinline__ void prefill_gate_up_rows(const struct exl3_prefill_record &record, const prefill_view &view,
 						     const prefill_shared *shared, const prefill_tile_view &tile,
 						     uint32_t tile_index, uint32_t count, uint32_t group, float *staging)
@@ -1060,7 +1064,7 @@ __device__ __forceinline__ void prefill_down(const struct exl3_prefill_record &r
 	const prefill_tile_view first = prefill_tile_of(record, arena, view, tile_index);
 	const uint32_t H = record.input_size, I = prefill_inner_of(record, first.tile.expert);
 	const uint32_t groups = first_group < H / EXL3_TRANSFORM ? min(2u, H / EXL3_TRANSFORM - first_group) : 0u;
-	const uint32_t lane = threadIdx.x % EXL3_WARP, warp = threadIdx.x / EXL3_WARP;
+	const uint32_t warp = threadIdx.x / EXL3_WARP;
 	const unsigned char *const matrices[1] = { arena + first.down };
 	const prefill_rows rows = prefill_rows_of(count, first.tile.row_count, 1u, I);
 	const unsigned char *const row_runs = view.workspace + view.parts.down_operands +

@@ -4,7 +4,7 @@ Host-side mirror of how the reference's model program uses the path (source/mode
 at load, matrices are placed in the arena, every launch is prepared by the library's preparers and captured into one
 graph; per step the caller writes the step block, the tokens and the router scores, runs the graph and reads the
 bfloat16 result. Launches of one step, all from libanemone_b200.so, in the default form ("fused", exl3_layer_prepare):
-    exl3_layer_route_input -> exl3_layer_gate_up -> exl3_layer_down_publish -> ordered_reduce_flags
+    exl3_layer_route_input -> exl3_layer_products -> ordered_publish_reduce_flags
 and in the forms kept for callers of the separate preparers ("pull": six launches, "push": five):
     router_select_b200 -> exl3_moe_input -> exl3_moe_gate_up -> exl3_moe_down -> ordered_row_sum_publish
     -> ordered_reduce_bf16

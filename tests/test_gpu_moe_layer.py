@@ -67,7 +67,7 @@ def test_layer_single_rank(api, oracle, rows, form):
 @pytest.mark.parametrize("capacity, inner", [(8, 128), (32, 256), (64, 1024)])
 def test_steps_of_changing_row_counts(api, oracle, capacity, inner):
     """One layer, steps of few and of many rows in turn: every step ends with the products' ticket at zero, whatever part
-    of the grid found work, at each cut of K the job count leads to."""
+    of the grid found work, at several cuts of K (by the intermediate width)."""
     config = MoeConfig(hidden=1024, inner=inner, experts=16, shared=1, picks=4, row_capacity=capacity)
     widths, matrices, tokens, scores = make_layer_inputs(70 + capacity, config, capacity)
     layout = MoeLayout(config, widths, 1, 0)

@@ -373,7 +373,8 @@ def test_prefill_row_bits_whatever_the_tiling(api, hidden, inner):
 @pytest.mark.parametrize("hidden,inner", [(32 * 8, 512), (32 * 96, 128)])
 def test_pairs_hand_their_stages_over(api, hidden, inner):
     """A pair's second CTA tells the first when its half of a stage is in place: call after call the same bits, whatever
-    the CTAs' relative pace, for K of a ring and a stage (seven stages of 32 inputs) and of many turns of it."""
+    the CTAs' relative pace: gate and up over eight stages of 32 inputs (a ring and two) and over 96, down over eight stages of
+    64 (two rings) and over two (half of one)."""
     config = MoeConfig(hidden=hidden, inner=inner, experts=8, shared=1, picks=3, row_capacity=900)
     widths, matrices, tokens, scores = make_inputs(41, config, 900)
     card = api.Card(0, PrefillLayout(config, widths).arena_bytes)
